@@ -19,6 +19,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "../common/ptx.cuh"
 #include "gla.cuh"
 
 namespace tb {
@@ -144,7 +145,329 @@ __global__ void __launch_bounds__(D* NPART) gdn_recurrent_kernel(
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// The same recurrence, eight tokens at a time, for prompts.
+//
+// One token at a time the recurrence is a chain: a contraction over all key rows, its sum across threads, then the update
+// that the next token's contraction waits for (2100 clocks a token in the kernel above). Eight tokens share ONE such round:
+// with P_j = product of the decays up to and including token j of the block and S the state before it,
+//   x_j  = v_j - (k_j P_{j-1})^T S                                     eight contractions with the same S
+//   u_j  = x_j - sum_{i<j} L_ji u_i      L_ji = sum_d k_j (beta k)_i dec_{i+1..j-1}
+//   o_j  = (q_j P_j)^T S + sum_{i<=j} A_ji u_i    A_ji = sum_d q_j (beta k)_i dec_{i+1..j}
+//   S   <- P_7 S + sum_j (beta k_j dec_{j+1..7}) u_j^T
+// Everything is fp32 with exponents <= 0, as in the token form. What does not depend on the state (the scaled vectors and
+// the small triangles) is formed once per head by gdn_block_prep_kernel, one warp per block of tokens, instead of by every
+// group of value columns; it leaves records of 25 D + 128 floats. Value columns never mix, so the walk runs on
+// B * H * D / 16 CTAs of 16 columns: a half warp holds two columns, 16 lanes x D / 16 rows each, and sums the 32
+// partial results of a block (2 columns x 8 tokens x {k, q}) with one 30-exchange reduce-scatter that leaves two of them
+// in each lane. Products run in packed f32x2 over row pairs. Bound by the latency of that chain (issue slots 37 % used at
+// one warp per scheduler), not by memory (DRAM 3 %). Measured, 16 heads of 128, 8192 tokens: one sequence 9010 -> 1155 us
+// (four tokens a round: 1853 us), four sequences 9056 -> 3460 us; 6 heads of 64: 5007 -> 896 us. The token kernel keeps
+// prompts of fewer than GDN_BLOCK_MIN_T tokens, where one launch beats two.
+// ------------------------------------------------------------------------------------------------
+constexpr int GB = 8;  // tokens per block
+constexpr int GDN_TRI = 2 * GB * GB;
+template <int D>
+constexpr int gdn_rec_floats() { return (1 + 3 * GB) * D + GDN_TRI; }  // P_7 | k P | q P | (beta k) dec | L | A
+
+// Reduce-scatter of N values over the sixteen lanes of a half warp: lane l gets the sums of values l * N / 16 + [0, N / 16).
+template <int N>
+__device__ __forceinline__ void reduce_scatter16(float (&v)[N], int lane) {
+  int n = N / 2;
+#pragma unroll
+  for (int s = 8; s >= 1; s >>= 1, n >>= 1) {
+    const bool up = (lane & s) != 0;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+    }
+  }
+}
+
+template <int N>
+__device__ __forceinline__ void load_bf16_row(const __nv_bfloat16* p, bool ok, float (&f)[N]) {
+  uint32_t w[N / 2];
+  if constexpr (N == 4) {
+    const uint2 x = ok ? *reinterpret_cast<const uint2*>(p) : make_uint2(0u, 0u);
+    w[0] = x.x;
+    w[1] = x.y;
+  } else {
+    w[0] = ok ? *reinterpret_cast<const uint32_t*>(p) : 0u;
+  }
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+
+template <int N>
+__device__ __forceinline__ void store_rec(float* p, const float (&f)[N]) {
+  if constexpr (N == 4)
+    *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
+  else
+    *reinterpret_cast<float2*>(p) = make_float2(f[0], f[1]);
+}
+
+// Tokens [t0, t0 + nt) of every sequence -> records [B * H, ceil(nt / GB)]. One warp per record; D / 32 dims per lane.
+template <int D>
+__global__ void __launch_bounds__(128) gdn_block_prep_kernel(
+    const __nv_bfloat16* __restrict__ q, long long q_ld, int qcol, const __nv_bfloat16* __restrict__ k, long long k_ld,
+    int kcol, const __nv_bfloat16* __restrict__ g, long long g_ld, int gcol, const float* __restrict__ beta, int beta_mode,
+    float* __restrict__ rec, int T, int t0, int nt, int H, int logits, int nrec) {
+  constexpr int N = D / 32, REC = gdn_rec_floats<D>();
+  const int lane = threadIdx.x & 31, id = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (id >= nrec) return;
+  const int nb = (nt + GB - 1) / GB, bh = id / nb, blk = id % nb, h = bh % H;
+  const long long row0 = (long long)(bh / H) * T + t0 + blk * GB;
+  const int left = nt - blk * GB, d0 = h * D + lane * N;
+  float qv[GB][N], kv[GB][N], dec[GB][N], bt[GB][N];
+#pragma unroll
+  for (int j = 0; j < GB; ++j) {
+    const bool ok = j < left;
+    const long long r = row0 + j;
+    load_bf16_row<N>(q + r * q_ld + qcol + d0, ok, qv[j]);
+    load_bf16_row<N>(k + r * k_ld + kcol + d0, ok, kv[j]);
+    load_bf16_row<N>(g + r * g_ld + gcol + d0, ok, dec[j]);
+    const float b1 = (ok && beta_mode == 1) ? beta[r * H + h] : 1.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) bt[j][i] = (ok && beta_mode == 2) ? beta[r * H * D + d0 + i] : b1;
+  }
+  float* out = rec + (long long)id * REC + lane * N;
+  float p[N], f[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = 1.f;
+#pragma unroll
+  for (int j = 0; j < GB; ++j) {  // k_j P_{j-1}, q_j P_j; tokens past the end write nothing and leave the state as it is
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      dec[j][i] = j < left ? __expf(gdn_log_decay(dec[j][i], logits != 0)) : 1.f;
+      f[i] = kv[j][i] * p[i];
+    }
+    store_rec<N>(out + (1 + j) * D, f);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      p[i] *= dec[j][i];
+      f[i] = qv[j][i] * p[i];
+    }
+    store_rec<N>(out + (1 + GB + j) * D, f);
+  }
+  store_rec<N>(out, p);
+  float* tri = rec + (long long)id * REC + (1 + 3 * GB) * D;
+#pragma unroll
+  for (int i = 0; i < GB; ++i) {  // w = (beta k)_i carried forward through the decays of the later tokens
+    float w[N], sums[2 * GB];
+#pragma unroll
+    for (int j = 0; j < 2 * GB; ++j) sums[j] = 0.f;
+#pragma unroll
+    for (int n = 0; n < N; ++n) w[n] = bt[i][n] * kv[i][n];
+#pragma unroll
+    for (int j = i; j < GB; ++j) {
+      if (j > i) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          sums[j] += kv[j][n] * w[n];
+          w[n] *= dec[j][n];
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < N; ++n) sums[GB + j] += qv[j][n] * w[n];
+    }
+    store_rec<N>(out + (1 + 2 * GB + i) * D, w);
+    reduce_scatter16(sums, lane);
+    const float s = sums[0] + __shfl_xor_sync(0xffffffffu, sums[0], 16);
+    if (lane < 16) tri[lane * GB + i] = s;  // lanes 0..7: L[j = lane][i] (zero for i >= j); lanes 8..15: A[j = lane - 8][i]
+  }
+}
+
+constexpr int GDN_COLS = 16;  // value columns per CTA
+constexpr int GDN_STAGES = 3;
+
+template <int D>
+__global__ void __launch_bounds__(128) gdn_block_walk_kernel(const float* __restrict__ rec, const __nv_bfloat16* __restrict__ v,
+                                                             long long v_ld, int vcol, float* __restrict__ state,
+                                                             __nv_bfloat16* __restrict__ out, long long o_ld, int ocol, int T,
+                                                             int t0, int nt, int H, float scale) {
+  constexpr int REC = gdn_rec_floats<D>(), NP = D / 32, NV = REC / 4;  // NP row pairs per lane
+  __shared__ __align__(16) float stage[GDN_STAGES][REC];
+  const int tid = threadIdx.x, lane = tid & 31, l16 = lane & 15;
+  const int bh = blockIdx.x / (D / GDN_COLS), h = bh % H;
+  const int c0 = (blockIdx.x % (D / GDN_COLS)) * GDN_COLS + (tid >> 4) * 2;  // two columns per half warp
+  const int nb = (nt + GB - 1) / GB;
+  const long long row0 = (long long)(bh / H) * T + t0;
+  const float* src = rec + (long long)bh * nb * REC;
+  auto row = [&](int pr) { return (pr >> 1) * 64 + l16 * 4 + (pr & 1) * 2; };  // 16 lanes read 256 consecutive bytes
+
+  uint64_t S[2][NP];
+  float* sp = state + (long long)bh * D * D + c0;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const float2 x = *reinterpret_cast<const float2*>(sp + (long long)row(i) * D);
+    const float2 y = *reinterpret_cast<const float2*>(sp + (long long)(row(i) + 1) * D);
+    S[0][i] = pack_f2(x.x, y.x);
+    S[1][i] = pack_f2(x.y, y.y);
+  }
+  auto fetch = [&](int blk) {
+    if (blk < nb) {
+      const float4* from = reinterpret_cast<const float4*>(src + (long long)blk * REC);
+      float4* to = reinterpret_cast<float4*>(&stage[blk % GDN_STAGES][0]);
+      for (int i = tid; i < NV; i += 128)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + i)), "l"(from + i)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // lane l of a half warp ends up with the results of tokens j, j + 1 for {k, q}[l >> 3] and column (l >> 2) & 1
+  const int j = (l16 & 3) * 2, col = (l16 >> 2) & 1;
+  const bool reads = l16 >= 8;
+  const unsigned short* vp = reinterpret_cast<const unsigned short*>(v) + vcol + h * D + c0 + col;
+  uint32_t vraw[2], vnext[2];
+  auto values = [&](int blk) {  // raw bits: converting here would wait for the load
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = blk * GB + j + e;
+      vnext[e] = (!reads && t < nt) ? (uint32_t)vp[(row0 + t) * v_ld] : 0u;
+    }
+  };
+  values(0);
+  fetch(0);
+  fetch(1);
+  for (int blk = 0; blk < nb; ++blk) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // this block's record has landed for every thread, and the one before it has been read by every thread
+    fetch(blk + 2);
+    vraw[0] = vnext[0];
+    vraw[1] = vnext[1];
+    values(blk + 1);
+    const float* r = &stage[blk % GDN_STAGES][0];
+    float val[4 * GB];
+#pragma unroll
+    for (int w = 0; w < 2 * GB; ++w) {
+      uint64_t a0, a1;
+#pragma unroll
+      for (int i = 0; i < NP; i += 2) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(r + (1 + w) * D + row(i));
+        a0 = i == 0 ? mul2(x.x, S[0][0]) : fma2(x.x, S[0][i], a0);
+        a1 = i == 0 ? mul2(x.x, S[1][0]) : fma2(x.x, S[1][i], a1);
+        a0 = fma2(x.y, S[0][i + 1], a0);
+        a1 = fma2(x.y, S[1][i + 1], a1);
+      }
+      float lo, hi;
+      unpack_f2(a0, lo, hi);
+      val[(w / GB) * 2 * GB + w % GB] = lo + hi;
+      unpack_f2(a1, lo, hi);
+      val[(w / GB) * 2 * GB + GB + w % GB] = lo + hi;
+    }
+    reduce_scatter16(val, lane);
+    const float x0 = __uint_as_float(vraw[0] << 16) - val[0], x1 = __uint_as_float(vraw[1] << 16) - val[1];
+    const float* tri = r + (1 + 3 * GB) * D;
+    float u[2][GB];
+#pragma unroll
+    for (int i = 0; i < GB; ++i) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) u[c][i] = __shfl_sync(0xffffffffu, (i & 1) ? x1 : x0, (lane & 16) + c * 4 + i / 2);
+    }
+#pragma unroll
+    for (int i = 1; i < GB; ++i) {
+      float l[GB];
+      *reinterpret_cast<float4*>(l) = *reinterpret_cast<const float4*>(tri + i * GB);
+      if (i > 4) *reinterpret_cast<float4*>(l + 4) = *reinterpret_cast<const float4*>(tri + i * GB + 4);
+#pragma unroll
+      for (int m = 0; m < i; ++m) {
+        u[0][i] -= l[m] * u[0][m];
+        u[1][i] -= l[m] * u[1][m];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NP; i += 2) {
+      const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(r + row(i));
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        S[c][i] = mul2(S[c][i], p.x);
+        S[c][i + 1] = mul2(S[c][i + 1], p.y);
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < GB; ++w) {
+      const uint64_t u0 = pack_f2(u[0][w], u[0][w]), u1 = pack_f2(u[1][w], u[1][w]);
+#pragma unroll
+      for (int i = 0; i < NP; i += 2) {
+        const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(r + (1 + 2 * GB + w) * D + row(i));
+        S[0][i] = fma2(e.x, u0, S[0][i]);
+        S[0][i + 1] = fma2(e.y, u0, S[0][i + 1]);
+        S[1][i] = fma2(e.x, u1, S[1][i]);
+        S[1][i + 1] = fma2(e.y, u1, S[1][i + 1]);
+      }
+    }
+    if (reads) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = blk * GB + j + e;
+        if (t < nt) {
+          const float* a = tri + GB * GB + (j + e) * GB;
+          float o = val[e];
+#pragma unroll
+          for (int m = 0; m < GB; ++m) o += a[m] * (col ? u[1][m] : u[0][m]);
+          out[(row0 + t) * o_ld + ocol + h * D + c0 + col] = __float2bfloat16(o * scale);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    float a, b, c, d;
+    unpack_f2(S[0][i], a, b);
+    unpack_f2(S[1][i], c, d);
+    *reinterpret_cast<float2*>(sp + (long long)row(i) * D) = make_float2(a, c);
+    *reinterpret_cast<float2*>(sp + (long long)(row(i) + 1) * D) = make_float2(b, d);
+  }
+}
+
+template <int D>
+void run_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode, float* state,
+                const GlaMat& O, int B, int T, int H, bool logits, float scale, float* rec, int seg, cudaStream_t s) {
+  auto p = [](const GlaMat& m) { return reinterpret_cast<const __nv_bfloat16*>(m.ptr); };
+  for (int t0 = 0; t0 < T; t0 += seg) {
+    const int nt = T - t0 < seg ? T - t0 : seg, nrec = B * H * ((nt + GB - 1) / GB);
+    gdn_block_prep_kernel<D><<<(nrec + 3) / 4, 128, 0, s>>>(p(Q), Q.ld, Q.col0, p(K), K.ld, K.col0, p(G), G.ld, G.col0, beta,
+                                                           beta_mode, rec, T, t0, nt, H, logits ? 1 : 0, nrec);
+    gdn_block_walk_kernel<D><<<B * H * (D / GDN_COLS), 128, 0, s>>>(rec, p(V), V.ld, V.col0, state,
+                                                                   reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(O.ptr)), O.ld,
+                                                                   O.col0, T, t0, nt, H, scale);
+  }
+}
+
+// Tokens per segment: whole blocks whose records fill at most 48 MB (they are read back from the 126 MB L2), at least 128
+// tokens so that the two launches of a segment stay small beside its walk.
+int segment_tokens(int BH, int D) {
+  const long long per_block = (long long)BH * ((1 + 3 * GB) * D + GDN_TRI) * 4;
+  const long long blocks = (48ll << 20) / per_block;
+  return (int)(blocks < 16 ? 16 : blocks) * GB;
+}
+
 }  // namespace
+
+long long gdn_block_workspace_floats(int B, int T, int H, int D) {
+  if (T < GDN_BLOCK_MIN_T || (D != 64 && D != 128)) return 0;
+  const int seg = segment_tokens(B * H, D), nt = T < seg ? T : seg;
+  return (long long)B * H * ((nt + GB - 1) / GB) * ((1 + 3 * GB) * D + GDN_TRI);
+}
+
+void launch_gdn_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode,
+                       float* state, const GlaMat& O, int B, int T, int H, int D, bool logits, float scale, float* workspace,
+                       cudaStream_t s) {
+  if (B <= 0 || T <= 0) return;
+  const int seg = segment_tokens(B * H, D);
+  if (D == 64)
+    run_blocks<64>(Q, K, V, G, beta, beta_mode, state, O, B, T, H, logits, scale, workspace, seg, s);
+  else if (D == 128)
+    run_blocks<128>(Q, K, V, G, beta, beta_mode, state, O, B, T, H, logits, scale, workspace, seg, s);
+  else
+    throw std::runtime_error("gdn_blocks: head dimension must be 64 or 128");
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) throw std::runtime_error(std::string("gdn_blocks launch failed: ") + cudaGetErrorString(e));
+}
 
 void launch_gdn_recurrent(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta,
                           int beta_mode, float* state, const GlaMat& O, int B, int T, int H, int D, bool logits,

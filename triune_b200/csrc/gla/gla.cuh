@@ -54,6 +54,14 @@ void launch_gdn_recurrent(const GlaMat& Q, const GlaMat& K, const GlaMat& V, con
                           int beta_mode, float* state, const GlaMat& O, int B, int T, int H, int D, bool gate_logits,
                           float scale, cudaStream_t s);
 
+// The same for T >= GDN_BLOCK_MIN_T, eight tokens per round; `workspace`: fp32 [gdn_block_workspace_floats(...)], 16-byte
+// aligned. q, k, g rows must start on 8-byte boundaries.
+constexpr int GDN_BLOCK_MIN_T = 8;
+long long gdn_block_workspace_floats(int B, int T, int H, int D);
+void launch_gdn_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode,
+                       float* state, const GlaMat& O, int B, int T, int H, int D, bool gate_logits, float scale, float* workspace,
+                       cudaStream_t s);
+
 // ---- Gated DeltaNet, chunk-parallel training path (gdn_chunk_kernels.cu) ----
 struct GdnDims {
   int B, T, H, D;    // T a multiple of 64, D = 64 or 128 (keys and values)

@@ -111,6 +111,13 @@ void gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol,
     else TORCH_CHECK(false, "beta must be [B,T,H] or [B,T,H,D]");
     bp = beta->data_ptr<float>();
   }
+  const int64_t ws = tb::gdn_block_workspace_floats((int)B, (int)T, (int)H, (int)D);
+  if (ws > 0) {
+    Tensor work = torch::empty({ws}, state.options());
+    tb::launch_gdn_blocks(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), bp, mode, state.data_ptr<float>(), mat(out, ocol),
+                          (int)B, (int)T, (int)H, (int)D, gate_logits, (float)scale, work.data_ptr<float>(), cur_stream());
+    return;
+  }
   tb::launch_gdn_recurrent(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), bp, mode, state.data_ptr<float>(),
                            mat(out, ocol), (int)B, (int)T, (int)H, (int)D, gate_logits, (float)scale, cur_stream());
 }
