@@ -33,3 +33,19 @@ def test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims):
     oo, ss = ref.gated_deltanet_recurrent(q.double(), k.double(), v.double(), gl, None if beta is None else beta.double(), s0.double(), 0.7)
     assert _rel(o, oo) < 2.0 ** -8   # outputs are rounded to bf16: at most 2^-9 each
     assert _rel(s, ss) < 1e-6        # the state is fp32 throughout
+
+
+def test_a_thread_without_a_context_of_its_own_runs_tensor_map_kernels():
+    import threading
+
+    from triune_b200 import ops
+
+    x, w = torch.randn(256, 128, device="cuda").bfloat16(), torch.randn(64, 128, device="cuda").bfloat16()
+    want = ops.linear(x, w)
+    spare = torch.empty_like(want)
+    del spare  # the thread's output comes from the allocator's cache: no CUDA call before the tensor map
+    got = []
+    t = threading.Thread(target=lambda: got.append(ops.linear(x, w)))
+    t.start()
+    t.join()
+    assert got and torch.equal(got[0], want)

@@ -30,6 +30,16 @@ inline EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
+// A thread that has made no CUDA call of its own yet (a backward pass on autograd's thread whose first buffers come from the
+// caching allocator) has no current context, and the encoder needs one: make the device's primary context current and retry.
+template <typename... A>
+CUresult encode_tiled(A... args) {
+  CUresult r = get_encode_fn()(args...);
+  int dev = 0;
+  if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = get_encode_fn()(args...);
+  return r;
+}
+
 // 3-D tiled map over a [d2][d1][d0] array (d0 contiguous). Strides in BYTES for d1 and d2 (multiples of
 // 16). Boxes are {b0, b1, 1}. 128-byte swizzle when b0 * elem_bytes == 128, 64-byte swizzle when it is 64, none otherwise.
 inline CUtensorMap make_tmap_3d(const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t d0, uint64_t d1,
@@ -46,7 +56,7 @@ inline CUtensorMap make_tmap_3d(const void* base, CUtensorMapDataType dt, int el
   cuuint32_t estr[3] = {1, 1, 1};
   CUtensorMapSwizzle sw = (b0 * elem_bytes == 128) ? CU_TENSOR_MAP_SWIZZLE_128B
                           : (b0 * elem_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
-  CUresult r = get_encode_fn()(&m, dt, 3, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = encode_tiled(&m, dt, 3, const_cast<void*>(base), dims, strides, box, estr,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
@@ -64,7 +74,7 @@ inline CUtensorMap make_tmap_4d_bf16(const void* base, const uint64_t (&d)[4], c
   }
   cuuint32_t box[4] = {64, b1, 1, 1}, estr[4] = {1, 1, 1, 1};
   CUtensorMap m;
-  CUresult r = get_encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = encode_tiled(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
