@@ -49,3 +49,44 @@ def test_a_thread_without_a_context_of_its_own_runs_tensor_map_kernels():
     t.start()
     t.join()
     assert got and torch.equal(got[0], want)
+
+
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [
+    (1536, 384, 32768, True, True), (384, 1536, 4100, True, True), (384, 384, 1536, True, True), (8, 384, 32761, True, True),
+    (37, 1536, 6144, False, False), (129, 72, 1544, False, False), (512, 512, 1472, False, True), (640, 1024, 8192, False, True),
+    (600, 1536, 384, False, False),
+])
+@pytest.mark.parametrize("what", ["plain", "bias", "gelu", "dgelu", "f32"])
+def test_products_of_few_tiles_against_fp32(M, N, K, a_mn, b_mn, what):
+    from triune_b200 import ops
+
+    if what in ("gelu", "dgelu") and a_mn:
+        pytest.skip("activation epilogues follow row-major activations")
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    Mp = (M + 7) // 8 * 8
+    a = rnd(K, Mp)[:, :M] if a_mn else rnd(M, K)
+    b = rnd(K, N) if b_mn else rnd(N, K)
+    bias = rnd(N) if what in ("bias", "gelu") else None
+    alpha = K ** -0.5
+    want = alpha * (a.float().t() if a_mn else a.float()) @ (b.float() if b_mn else b.float().t())
+    if bias is not None:
+        want = want + bias.float()
+    # fp32 sums of K products in another order: relative error about sqrt(K) 2^-24 (4e-6 for the longest), before the rounding
+    bf16 = 2.0 ** -8
+    if what == "gelu":
+        aux = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        got = ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, alpha=alpha, gelu=True, aux_out=aux)
+        x = want.clone().requires_grad_(True)
+        y = F.gelu(x, approximate="tanh")
+        (d,) = torch.autograd.grad(y.sum(), x)
+        assert _rel(got, y.detach()) < bf16 and _rel(aux, d) < bf16
+    elif what == "dgelu":
+        aux = rnd(M, N)
+        got = ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, alpha=alpha, dgelu_aux=aux)
+        assert _rel(got, want * aux.float()) < bf16
+    else:
+        kw = {"out_dtype": torch.float32} if what == "f32" else {}
+        got = ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, alpha=alpha, **kw)
+        assert _rel(got, want) < (2e-5 if what == "f32" else bf16)
+    assert torch.isfinite(got.float()).all()

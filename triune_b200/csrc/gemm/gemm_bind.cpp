@@ -114,6 +114,11 @@ void tc_gemm(const Tensor& a, const Tensor& b, Tensor& c, bool a_mn_major, bool 
                 "k_runs must be a contiguous CUDA int32 tensor [runs, 2]");
     g.k_runs = k_runs->data_ptr<int>();
   }
+  Tensor parts;
+  if (const long long floats = tb::tc_gemm_split_floats(g)) {
+    parts = torch::empty({(int64_t)floats}, a.options().dtype(at::kFloat));
+    g.split_ws = parts.data_ptr<float>();
+  }
   tb::launch_tc_gemm(g, cur_stream());
 }
 

@@ -296,7 +296,137 @@ int sm_count() {
   return n;
 }
 
+bool pairs_enabled() {
+  static const bool on = [] {
+    const char* e = std::getenv("TRIUNE_GEMM_PAIR");  // "0" keeps every product on the one-CTA kernel
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
+// widest tile that divides N: the tensor core is most efficient at N = 256, then 192 (e.g. N = 384), then 128
+int tile_width(int N) {
+  static const int forced = [] {
+    const char* e = std::getenv("TRIUNE_GEMM_BN");  // experiments only: force the tile width
+    return e ? std::atoi(e) : 0;
+  }();
+  if (forced == 64 || forced == 128 || forced == 192 || forced == 256) return forced;
+  return (N >= 256 && N % 256 == 0) ? 256 : ((N >= 192 && N % 192 == 0) ? 192 : (N > 64 ? 128 : 64));
+}
+
+int dense_tiles(const GemmArgs& a, int BN) {
+  return ((a.M + BM - 1) / BM) * ((a.N + BN - 1) / BN) * (a.batch < 1 ? 1 : a.batch);
+}
+
+// A reduction is split over idle SMs where the tiles fill at most half of them and the time saved (0.4 us an iteration of
+// 64, measured with operands in L2) outweighs the second kernel (about 5 us with the write and read of the parts). Weight
+// gradients of narrow layers are the case: 1536 x 384 over 32768 rows 224 -> 44 us, 384 x 384 146 -> 22 us.
+constexpr int SPLIT_MIN_ITERS = 24;  // shorter: narrower tiles instead
+struct SplitPlan {
+  int splits, pair;
+};
+SplitPlan split_plan(const GemmArgs& a) {
+  SplitPlan p{1, 0};
+  if (a.mode != GEMM_DENSE || a.batch > 1 || a.strideA != 0 || a.strideB != 0 || a.row_scale != nullptr ||
+      (a.flags & (GF_ACCUMULATE | GF_SWIGLU | GF_DSWIGLU | GF_ADDAUX | GF_SPLIT_SLICES)))
+    return p;
+  const int iters = (a.K + BK - 1) / BK;
+  if (iters < SPLIT_MIN_ITERS) return p;
+  GemmArgs part = a;
+  part.flags &= ~(GF_GELU | GF_DGELU);
+  p.pair = pairs_enabled() ? tc_gemm_pair_config(part) : 0;
+  const int slots = p.pair ? sm_count() / 2 : sm_count();
+  const int tiles = p.pair ? ((a.M + 2 * BM - 1) / (2 * BM)) * (a.N / p.pair) : dense_tiles(a, tile_width(a.N));
+  if (tiles * 2 > slots) return p;
+  int splits = slots / tiles;
+  if (splits > iters / 8) splits = iters / 8;
+  if (splits > 1) p.splits = splits;
+  return p;
+}
+
+// Few tiles and a short reduction (or one split as far as it goes): narrower tiles put more SMs to work.
+int narrowed_width(const GemmArgs& a, int BN, int splits) {
+  if (splits == 1 && (a.flags & GF_ACCUMULATE) && (a.K + BK - 1) / BK >= 16) return BN;  // splits by itself, into the accumulator
+  while (BN > 64 && dense_tiles(a, BN) * splits * 2 <= sm_count()) BN = BN == 256 ? 128 : 64;
+  return BN;
+}
+
+// Sum of the parts of a split reduction, eight columns a thread, through the epilogue that the product asked for. Bound by
+// reading the parts, which the product has just left in L2.
+__global__ void __launch_bounds__(256) split_finish_kernel(const float* __restrict__ ws, int splits, int M, int N, float alpha,
+                                                           const __nv_bfloat16* __restrict__ bias, int flags,
+                                                           const __nv_bfloat16* __restrict__ aux_in, __nv_bfloat16* __restrict__ aux_out,
+                                                           void* __restrict__ C, long long ldc) {
+  const int per_row = N / 8;
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x, part = (long long)M * N;
+  if (i >= (long long)M * per_row) return;
+  const int m = (int)(i / per_row), n = (int)(i % per_row) * 8;
+  const float* p = ws + (long long)m * N + n;
+  float v[8] = {};
+  for (int s = 0; s < splits; ++s) {
+    const float4 x = __ldcs(reinterpret_cast<const float4*>(p + s * part)), y = __ldcs(reinterpret_cast<const float4*>(p + s * part + 4));
+    v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+    v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+  }
+  const long long at = m * ldc + n;
+  float b[8] = {};
+  if (bias != nullptr) {
+    const uint4 w = *reinterpret_cast<const uint4*>(bias + n);
+    const uint32_t q[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) unpack_f2(bf16x2_to_f2(q[j]), b[2 * j], b[2 * j + 1]);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = fmaf(v[j], alpha, b[j]);
+  if (flags & GF_OUT_F32) {
+    float* c = reinterpret_cast<float*>(C) + at;
+    *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(c + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    return;
+  }
+  if (flags & GF_GELU) {  // the formulas of EPI_GELU
+    float d[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float x = v[j], x2 = x * x, h = 0.5f * x;
+      float t;
+      asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(x * fmaf(x2, 0.0356774081363001f, 0.7978845608028654f)));
+      v[j] = fmaf(h, t, h);
+      d[j] = fmaf(h * fmaf(-t, t, 1.f), fmaf(x2, 0.1070322244089003f, 0.7978845608028654f), fmaf(t, 0.5f, 0.5f));
+    }
+    if (aux_out != nullptr)
+      *reinterpret_cast<uint4*>(aux_out + at) =
+          make_uint4(pack_bf16x2(d[0], d[1]), pack_bf16x2(d[2], d[3]), pack_bf16x2(d[4], d[5]), pack_bf16x2(d[6], d[7]));
+  } else if (flags & GF_DGELU) {
+    const uint4 w = *reinterpret_cast<const uint4*>(aux_in + at);
+    const uint32_t q[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float x, y;
+      unpack_f2(bf16x2_to_f2(q[j]), x, y);
+      v[2 * j] *= x;
+      v[2 * j + 1] *= y;
+    }
+  }
+  *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(C) + at) =
+      make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+
+void launch_split_finish(const GemmArgs& a, int splits, cudaStream_t s) {
+  const int iters = (a.K + BK - 1) / BK, per = (iters + splits - 1) / splits;
+  const long long vecs = (long long)a.M * (a.N / 8);
+  split_finish_kernel<<<(unsigned)((vecs + 255) / 256), 256, 0, s>>>(a.split_ws, (iters + per - 1) / per, a.M, a.N, a.alpha, a.bias,
+                                                                    a.flags, a.aux_in, a.aux_out, a.C, a.ldc);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) throw std::runtime_error(std::string("tc_gemm split launch failed: ") + cudaGetErrorString(e));
+}
+
 }  // namespace
+
+long long tc_gemm_split_floats(const GemmArgs& a) {
+  const SplitPlan p = split_plan(a);
+  return p.splits > 1 ? (long long)p.splits * a.M * a.N : 0;
+}
 
 static long long* g_gemm_dbg = nullptr;
 void tc_gemm_set_debug_buffer(long long* p) { g_gemm_dbg = p; }
@@ -331,25 +461,31 @@ void launch_tc_gemm(const GemmArgs& a, cudaStream_t stream) {
     if (dswiglu && a.aux_in == nullptr) throw std::runtime_error("tc_gemm: gate/up rows missing");
   }
 
-  {
-    static const bool pairs = [] {
-      const char* e = std::getenv("TRIUNE_GEMM_PAIR");  // "0" keeps every product on the one-CTA kernel
-      return !(e && e[0] == '0');
-    }();
-    if (pairs && launch_tc_gemm_pair(a, stream)) return;
+  const SplitPlan plan = (a.flags & GF_SPLIT_SLICES) ? SplitPlan{a.splits, 0} : split_plan(a);
+  if (!(a.flags & GF_SPLIT_SLICES) && a.split_ws != nullptr && plan.splits > 1) {
+    GemmArgs part = a;  // bare fp32 products of the parts, then their sum through the epilogue that was asked for
+    part.flags = (a.flags & ~(GF_GELU | GF_DGELU)) | GF_OUT_F32 | GF_SPLIT_SLICES;
+    part.C = a.split_ws;
+    part.ldc = a.N;
+    part.strideC = (long long)a.M * a.N;
+    part.alpha = 1.f;
+    part.bias = nullptr;
+    part.aux_in = nullptr;
+    part.aux_out = nullptr;
+    part.splits = plan.splits;
+    launch_tc_gemm(part, stream);
+    launch_split_finish(a, plan.splits, stream);
+    return;
   }
+  if (pairs_enabled() && launch_tc_gemm_pair(a, stream)) return;
 
-  // widest tile that divides N: the tensor core is most efficient at N = 256, then 192 (e.g. N = 384), then 128
-  int BN = (a.N >= 256 && a.N % 256 == 0) ? 256 : ((a.N >= 192 && a.N % 192 == 0) ? 192 : (a.N > 64 ? 128 : 64));
-  {
-    static const int forced = [] {
-      const char* e = std::getenv("TRIUNE_GEMM_BN");  // experiments only: force the tile width
-      return e ? std::atoi(e) : 0;
-    }();
-    if (forced == 64 || forced == 128 || forced == 192 || forced == 256) BN = forced;
-  }
+  int BN = tile_width(a.N);
   // SwiGLU forward: a tile of BN accumulator columns yields BN / 2 output columns
-  if (swiglu) BN = (a.N % 128 == 0) ? 256 : ((a.N % 64 == 0) ? 128 : 64);
+  if (swiglu) {
+    BN = (a.N % 128 == 0) ? 256 : ((a.N % 64 == 0) ? 128 : 64);
+  } else if (a.mode == GEMM_DENSE) {
+    BN = narrowed_width(a, BN, (a.flags & GF_SPLIT_SLICES) ? a.splits : 1);
+  }
   const int n_out = swiglu ? BN / 2 : BN;
   KParams kp;
   kp.M = a.M; kp.N = a.N; kp.K = a.K;
@@ -376,7 +512,10 @@ void launch_tc_gemm(const GemmArgs& a, cudaStream_t stream) {
   kp.group_m = raster_group_m(kp.num_m, kp.num_n, sm_count());
   // Split-K: weight gradients reduce over tens of thousands of tokens into a handful of output tiles; spread the
   // reduction over idle SMs. Only when the output is an fp32 accumulator (partials are added with red.add).
-  if (a.mode == GEMM_DENSE && (kp.flags & GF_OUT_F32) && (kp.flags & GF_ACCUMULATE) && a.bias == nullptr &&
+  if (kp.flags & GF_SPLIT_SLICES) {
+    set_split_slices(kp, a.splits);
+    kp.total_tiles *= kp.splits;
+  } else if (a.mode == GEMM_DENSE && (kp.flags & GF_OUT_F32) && (kp.flags & GF_ACCUMULATE) && a.bias == nullptr &&
       a.row_scale == nullptr && !(kp.flags & (GF_GELU | GF_DGELU))) {
     const int total_iters = (a.K + BK - 1) / BK;
     const int sms = sm_count();
@@ -420,7 +559,7 @@ void launch_tc_gemm(const GemmArgs& a, cudaStream_t stream) {
   // output maps: rows of 64 bytes (32 bf16 / 16 fp32) x 32 rows, one box per epilogue warp and column chunk
   const bool c_f32 = (kp.flags & GF_OUT_F32) != 0;
   const int c_elem = c_f32 ? 4 : 2;
-  const uint64_t c_batches = (a.mode == GEMM_GROUPED_M) ? 1 : (uint64_t)kp.batch;
+  const uint64_t c_batches = (kp.flags & GF_SPLIT_SLICES) ? (uint64_t)kp.splits : (a.mode == GEMM_GROUPED_M) ? 1 : (uint64_t)kp.batch;
   const uint64_t c_bstride = (c_batches > 1 ? (uint64_t)a.strideC : (uint64_t)a.ldc * (uint64_t)a.M) * c_elem;
   const uint64_t c_cols = dswiglu ? 2ull * (uint64_t)a.N : (uint64_t)a.N;  // d(gate) | d(up)
   CUtensorMap tmC = make_tmap_3d(a.C, c_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, c_elem,

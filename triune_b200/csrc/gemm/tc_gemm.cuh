@@ -21,6 +21,7 @@ enum GemmFlags : int {
   // SwiGLU over a fused gate/up weight B = [gate rows (n_split) ; up rows (n_split)], dense mode, K-major operands:
   GF_SWIGLU = 32,   // C [M, N = n_split] = silu(A gate^T) * (A up^T); aux_out [M, 2 N] optionally receives both pre-activations
   GF_ADDAUX = 128,  // C = alpha * A B^T + beta * aux_in (aux_in: bf16, C's layout; bf16 output, no bias)
+  GF_SPLIT_SLICES = 256,  // internal: the parts of a split reduction go to separate fp32 matrices C + part * strideC
   GF_DSWIGLU = 64,  // acc = A B^T [M, N = n_split] is d(hidden); aux_in [M, 2 N] holds gate | up; C [M, 2 N] = d(gate) | d(up)
 };
 
@@ -56,7 +57,14 @@ struct GemmArgs {
   int glu_act;                  // GF_SWIGLU: activation of the gate, 0 silu, 1 relu, 2 clamped: g sigmoid(alpha g) (u + 1)
   float glu_limit, glu_alpha;   //   with g at most `limit` and u within +- `limit`
   const float* glu_bias;        // GF_SWIGLU: [2 N], of the gate, then of the up rows; or null
+  float* split_ws;              // optional: fp32 [tc_gemm_split_floats(args)], lets a product with few tiles split its reduction
+  int splits;                   // GF_SPLIT_SLICES: number of parts
 };
+
+// Floats of workspace with which launch_tc_gemm spreads this product's reduction over idle SMs; 0 where it would not.
+long long tc_gemm_split_floats(const GemmArgs& args);
+// Accumulator columns of the CTA-pair configuration that would take this product, 0 if none would.
+int tc_gemm_pair_config(const GemmArgs& args);
 
 // Launches on `stream`. Throws std::runtime_error on invalid arguments.
 void launch_tc_gemm(const GemmArgs& args, cudaStream_t stream);

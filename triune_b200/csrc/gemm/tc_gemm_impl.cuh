@@ -45,7 +45,7 @@ struct KParams {
   long long* dbg;       // optional phase timers (clock ticks summed over one warp's chunks), null in normal runs
   int total_tiles;
   int group_m;          // tile order: blocks of group_m row tiles x all column tiles (see raster)
-  int splits;           // split-K factor (dense mode, fp32 accumulate only)
+  int splits;           // split-K factor (dense mode, fp32 output: added into one matrix, or GF_SPLIT_SLICES)
   int iters_per_split;  // K iterations (of 64) handled by one split
   int n_split;          // SwiGLU epilogues: column offset of the "up" half (= FFN hidden width)
   float beta;           // EPI_ADDAUX: weight of the added rows
@@ -53,6 +53,13 @@ struct KParams {
   float glu_limit, glu_alpha;
   const float* glu_bias;  // EPI_SWIGLU: [2 n_split] or null
 };
+
+// Parts of whole 64-deep iterations, none of them empty.
+__host__ inline void set_split_slices(KParams& kp, int splits) {
+  const int iters = (kp.K + BK - 1) / BK;
+  kp.iters_per_split = (iters + splits - 1) / splits;
+  kp.splits = (iters + kp.iters_per_split - 1) / kp.iters_per_split;
+}
 
 struct Tile {
   int m0, n0, ba, bb, g, k_begin, k_iters;
@@ -142,6 +149,7 @@ __device__ __forceinline__ Tile decode_tile(const KParams& p, int t) {
       tl.bb = p.b_batched ? b : 0;
       const int total_iters = (p.K + BK - 1) / BK;
       if (p.splits > 1) {
+        if (p.flags & GF_SPLIT_SLICES) tl.g = split;
         tl.k_begin = split * p.iters_per_split * BK;
         const int left = total_iters - split * p.iters_per_split;
         tl.k_iters = left < p.iters_per_split ? (left < 0 ? 0 : left) : p.iters_per_split;
@@ -201,7 +209,7 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, 
   constexpr bool out_f32 = (EPI == EPI_PLAIN_F32);
   constexpr int CW = out_f32 ? 16 : 32;  // columns per staged chunk (64 bytes)
   constexpr int NP = CW / 2;             // packed fp32 pairs per lane and chunk
-  const bool reduce_add = ((p.flags & GF_ACCUMULATE) != 0) || p.splits > 1;
+  const bool reduce_add = ((p.flags & GF_ACCUMULATE) != 0) || (p.splits > 1 && !(p.flags & GF_SPLIT_SLICES));
   const uint64_t alpha2 = pack_f2(p.alpha, p.alpha);
   const int gm = m_base + lane_base + lane;
   const bool row_ok = gm < p.M;

@@ -70,6 +70,7 @@ __device__ __forceinline__ Tile decode_pair_tile(const KParams& p, int t, int nu
     tl.k_end = k1;
     tl.k_iters = p.k_runs ? run_list_blocks(p.k_runs, k0, k1) : (k1 - k0 + BK - 1) / BK;
   } else if (p.splits > 1) {
+    if (p.flags & GF_SPLIT_SLICES) tl.g = split;
     tl.k_begin = split * p.iters_per_split * BK;
     const int left = total_iters - split * p.iters_per_split;
     tl.k_iters = left < p.iters_per_split ? (left < 0 ? 0 : left) : p.iters_per_split;
@@ -370,37 +371,41 @@ int pair_sm_count() {
 
 }  // namespace
 
-// Runs the product on CTA pairs when the shape suits them; returns false (nothing launched) otherwise.
-bool launch_tc_gemm_pair(const GemmArgs& a, cudaStream_t stream) {
+int tc_gemm_pair_config(const GemmArgs& a) {
   const bool grouped_k = a.mode == GEMM_GROUPED_K;
   const bool grouped_m = a.mode == GEMM_GROUPED_M;
   const int groups = grouped_k ? (a.batch < 1 ? 1 : a.batch) : 1;
   if (grouped_k) {
-    if (a.group_offsets == nullptr || !a.a_mn_major || !a.b_mn_major) return false;
+    if (a.group_offsets == nullptr || !a.a_mn_major || !a.b_mn_major) return 0;
   } else if (grouped_m) {
-    if (!(a.flags & GF_PAIRED_GROUPS) || a.tile_group == nullptr || a.strideA != 0 || (a.M % (2 * BM)) != 0) return false;
+    if (!(a.flags & GF_PAIRED_GROUPS) || a.tile_group == nullptr || a.strideA != 0 || (a.M % (2 * BM)) != 0) return 0;
   } else if (a.mode != GEMM_DENSE || a.batch > 1 || a.strideA != 0 || a.strideB != 0) {
-    return false;
+    return 0;
   }
-  if (a.flags & (GF_GELU | GF_DGELU | GF_ADDAUX)) return false;
-  if (a.M < 2 * BM) return false;
+  if (a.flags & (GF_GELU | GF_DGELU | GF_ADDAUX)) return 0;
+  if (a.M < 2 * BM) return 0;
   const int num_m_tiles = (a.M + BM - 1) / BM;
-  if ((num_m_tiles & 1) && num_m_tiles < 9) return false;  // an odd tile leaves half a pair idle: too costly when few
-  const long long k_each = (long long)a.K / groups;       // grouped-K: K is the total over the groups
+  if ((num_m_tiles & 1) && num_m_tiles < 9) return 0;  // an odd tile leaves half a pair idle: too costly when few
+  const long long k_each = (long long)a.K / groups;    // grouped-K: K is the total over the groups
   static const long long min_k = [] {
     const char* e = std::getenv("TRIUNE_GEMM_PAIR_MIN_K");  // tuning knob: shortest reduction handed to CTA pairs
     return e ? std::atoll(e) : 768ll;
   }();
-  const bool swiglu = (a.flags & GF_SWIGLU) != 0, dswiglu = (a.flags & GF_DSWIGLU) != 0;
-  int ncfg = 0;
-  if (swiglu) {
-    // 256 accumulator columns = 128 gate + 128 up columns of 128 outputs
-    if (a.N % 128 == 0 && k_each >= min_k && !a.a_mn_major && !a.b_mn_major) ncfg = 256;
-  } else if (dswiglu) {
-    if (a.N % 256 == 0 && k_each >= min_k && !a.a_mn_major) ncfg = 256;
-  } else if (a.N % 384 == 0 && k_each >= (min_k < 1024 ? 1024 : min_k)) ncfg = 384;  // single-buffered: long reductions only
-  else if (a.N % 256 == 0 && k_each >= min_k) ncfg = 256;
+  if (a.flags & GF_SWIGLU)  // 256 accumulator columns = 128 gate + 128 up columns of 128 outputs
+    return (a.N % 128 == 0 && k_each >= min_k && !a.a_mn_major && !a.b_mn_major) ? 256 : 0;
+  if (a.flags & GF_DSWIGLU) return (a.N % 256 == 0 && k_each >= min_k && !a.a_mn_major) ? 256 : 0;
+  if (a.N % 384 == 0 && k_each >= (min_k < 1024 ? 1024 : min_k)) return 384;  // single-buffered: long reductions only
+  return (a.N % 256 == 0 && k_each >= min_k) ? 256 : 0;
+}
+
+// Runs the product on CTA pairs when the shape suits them; returns false (nothing launched) otherwise.
+bool launch_tc_gemm_pair(const GemmArgs& a, cudaStream_t stream) {
+  const int ncfg = tc_gemm_pair_config(a);
   if (ncfg == 0) return false;
+  const bool grouped_k = a.mode == GEMM_GROUPED_K;
+  const bool grouped_m = a.mode == GEMM_GROUPED_M;
+  const int groups = grouped_k ? (a.batch < 1 ? 1 : a.batch) : 1;
+  const bool swiglu = (a.flags & GF_SWIGLU) != 0, dswiglu = (a.flags & GF_DSWIGLU) != 0;
   const int n_out = swiglu ? ncfg / 2 : ncfg;
 
   KParams kp;
@@ -428,8 +433,11 @@ bool launch_tc_gemm_pair(const GemmArgs& a, cudaStream_t stream) {
   kp.group_m = raster_group_m(num_mp, kp.num_n, pair_sm_count() / 2);
   int pair_tiles = num_mp * kp.num_n * groups;
   const int max_clusters = pair_sm_count() / 2;
-  // Split-K exactly as in the one-CTA kernel: only into an fp32 accumulator, when the tiles leave most SMs idle.
-  if (!grouped_k && !grouped_m && (kp.flags & GF_OUT_F32) && (kp.flags & GF_ACCUMULATE) && a.bias == nullptr && a.row_scale == nullptr) {
+  // Split-K exactly as in the one-CTA kernel: into an fp32 accumulator or separate slices, when the tiles leave most SMs idle.
+  if (kp.flags & GF_SPLIT_SLICES) {
+    set_split_slices(kp, a.splits);
+    pair_tiles *= kp.splits;
+  } else if (!grouped_k && !grouped_m && (kp.flags & GF_OUT_F32) && (kp.flags & GF_ACCUMULATE) && a.bias == nullptr && a.row_scale == nullptr) {
     const int total_iters = (a.K + BK - 1) / BK;
     if (pair_tiles * 2 <= max_clusters && total_iters >= 16) {
       int splits = max_clusters / pair_tiles;
@@ -461,9 +469,10 @@ bool launch_tc_gemm_pair(const GemmArgs& a, cudaStream_t stream) {
                        (uint64_t)a.ldb * 2ull, sB, BK, 64);
   const bool c_f32 = (kp.flags & GF_OUT_F32) != 0;
   const int c_elem = c_f32 ? 4 : 2;
-  const uint64_t c_bstride = (groups > 1 ? (uint64_t)a.strideC : (uint64_t)a.ldc * (uint64_t)a.M) * c_elem;
+  const uint64_t c_parts = (kp.flags & GF_SPLIT_SLICES) ? (uint64_t)kp.splits : (uint64_t)groups;
+  const uint64_t c_bstride = (c_parts > 1 ? (uint64_t)a.strideC : (uint64_t)a.ldc * (uint64_t)a.M) * c_elem;
   CUtensorMap tmC = make_tmap_3d(a.C, c_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, c_elem,
-                                 dswiglu ? 2ull * (uint64_t)a.N : (uint64_t)a.N, (uint64_t)a.M, (uint64_t)groups,
+                                 dswiglu ? 2ull * (uint64_t)a.N : (uint64_t)a.N, (uint64_t)a.M, c_parts,
                                  (uint64_t)a.ldc * c_elem, c_bstride, c_f32 ? 16 : 32, 32);
   CUtensorMap tmAux = tmC;
   if (swiglu && a.aux_out != nullptr)  // gate | up pre-activations, [M, 2 N] contiguous
