@@ -90,3 +90,23 @@ def test_products_of_few_tiles_against_fp32(M, N, K, a_mn, b_mn, what):
         got = ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, alpha=alpha, **kw)
         assert _rel(got, want) < (2e-5 if what == "f32" else bf16)
     assert torch.isfinite(got.float()).all()
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("N,K", [(8, 8), (24, 72), (200, 384), (4760, 264), (2048, 5632), (19008, 520)])
+def test_products_of_a_few_rows_against_fp32(M, N, K):
+    from triune_b200 import _ext, ops
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    wide = rnd(M, K + 16)
+    a, b, bias = wide[:, 8 : K + 8], rnd(N, K), rnd(N)  # rows of a wider matrix
+    want = K ** -0.5 * a.float() @ b.float().t() + bias.float()
+    assert _rel(ops.gemm(a, b, bias=bias, alpha=K ** -0.5), want) < 2.0 ** -8
+    assert _rel(ops.gemm(a, b, bias=bias, alpha=K ** -0.5, gelu=True), F.gelu(want, approximate="tanh")) < 2.0 ** -8
+    if N % 64 == 0:  # gate rows, then up rows
+        h = torch.empty(M, N // 2, device="cuda", dtype=torch.bfloat16)
+        b = b * K ** -0.5
+        _ext.serving().tc_gemm_swiglu(a, b, h, None)
+        gate, up = (a.float() @ b.float().t()).chunk(2, dim=1)
+        assert _rel(h, F.silu(gate) * up) < 2.0 ** -8

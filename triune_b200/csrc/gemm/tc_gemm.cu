@@ -327,6 +327,7 @@ struct SplitPlan {
 };
 SplitPlan split_plan(const GemmArgs& a) {
   SplitPlan p{1, 0};
+  if (a.M <= SKINNY_MAX_M && !a.a_mn_major && !a.b_mn_major && !(a.flags & GF_OUT_F32) && a.aux_in == nullptr && a.aux_out == nullptr) return p;
   if (a.mode != GEMM_DENSE || a.batch > 1 || a.strideA != 0 || a.strideB != 0 || a.row_scale != nullptr ||
       (a.flags & (GF_ACCUMULATE | GF_SWIGLU | GF_DSWIGLU | GF_ADDAUX | GF_SPLIT_SLICES)))
     return p;
@@ -461,6 +462,7 @@ void launch_tc_gemm(const GemmArgs& a, cudaStream_t stream) {
     if (dswiglu && a.aux_in == nullptr) throw std::runtime_error("tc_gemm: gate/up rows missing");
   }
 
+  if (launch_skinny_gemm(a, stream)) return;
   const SplitPlan plan = (a.flags & GF_SPLIT_SLICES) ? SplitPlan{a.splits, 0} : split_plan(a);
   if (!(a.flags & GF_SPLIT_SLICES) && a.split_ws != nullptr && plan.splits > 1) {
     GemmArgs part = a;  // bare fp32 products of the parts, then their sum through the epilogue that was asked for

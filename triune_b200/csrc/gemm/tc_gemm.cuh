@@ -69,6 +69,11 @@ int tc_gemm_pair_config(const GemmArgs& args);
 // Launches on `stream`. Throws std::runtime_error on invalid arguments.
 void launch_tc_gemm(const GemmArgs& args, cudaStream_t stream);
 
+// Products of at most SKINNY_MAX_M rows with a K-major weight (plain, bias, GELU or SwiGLU, bf16 output): streams the weight
+// through warp-level matrix instructions (skinny_gemm.cu). Returns false, launching nothing, for every other call.
+constexpr int SKINNY_MAX_M = 16;
+bool launch_skinny_gemm(const GemmArgs& args, cudaStream_t stream);
+
 // CTA-pair (tcgen05 cta_group::2) variant for dense products with long reductions; returns false, launching
 // nothing, when the shape does not suit it. launch_tc_gemm tries it first.
 bool launch_tc_gemm_pair(const GemmArgs& args, cudaStream_t stream);
