@@ -110,3 +110,42 @@ def test_products_of_a_few_rows_against_fp32(M, N, K):
         _ext.serving().tc_gemm_swiglu(a, b, h, None)
         gate, up = (a.float() @ b.float().t()).chunk(2, dim=1)
         assert _rel(h, F.silu(gate) * up) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("B,H,D,delta,learn_beta,rope,on_device", [
+    (1, 1, 64, False, False, True, False), (3, 2, 64, False, False, False, True), (2, 3, 128, False, False, True, True),
+    (1, 2, 128, True, True, True, False), (5, 1, 64, True, False, True, True), (2, 4, 64, True, True, False, False),
+])
+def test_mixer_step_against_a_64_bit_statement(B, H, D, delta, learn_beta, rope, on_device):
+    from triune_b200.models.attention import VectorisedGLA
+
+    torch.manual_seed(B * 100 + H * 10 + D)
+    dim = H * D
+    m = VectorisedGLA(dim, H, D, use_delta_rule=delta, use_rope=rope, learn_beta=learn_beta, rope_max_seq_len=64).cuda().bfloat16().eval()
+    x = torch.randn(B, 1, dim, device="cuda").bfloat16()
+    s0 = torch.randn(B, H, D, D, device="cuda")
+    at = 77  # past the first size of the rotary tables
+    if on_device and rope:
+        m.rope(1, "cuda:0", offset=at)  # a position on the device relies on tables that cover it
+    with torch.no_grad():
+        y, (s1, after) = m(x, cache=(s0.clone(), torch.tensor([at], device="cuda") if on_device else at))
+    assert int(after) == at + 1
+    # from the projection rows as the model rounds them, so that only the step itself is compared
+    from triune_b200 import ops
+
+    with torch.no_grad():
+        qkvg = ops.linear(x.reshape(B, dim), m.qkvg_weight).double()
+    q, k, v, g = (t.reshape(B, H, D) for t in qkvg.chunk(4, dim=1))
+    q, k = (F.normalize(F.elu(t) + 1, dim=-1) for t in (q, k))
+    if rope:
+        c, s = (t[at].double().cuda() for t in (m.rope._cos, m.rope._sin))
+        q, k = (t * c + torch.cat((-t[..., D // 2:], t[..., : D // 2]), -1) * s for t in (q, k))
+    u, st = v, s0.double()
+    if delta:
+        u = v - torch.einsum("bhk,bhkv->bhv", k, st)
+        if learn_beta:
+            u = u * torch.sigmoid(x.reshape(B, dim).double() @ m.beta_proj.weight.double().t()).unsqueeze(-1)
+    st = st * torch.exp(F.logsigmoid(g)).unsqueeze(-1) + k.unsqueeze(-1) * u.unsqueeze(-2)
+    o = torch.einsum("bhk,bhkv->bhv", q, st).reshape(B, dim)
+    assert _rel(s1, st) < 2e-6                                              # fp32 throughout
+    assert _rel(y.reshape(B, dim), o @ m.out_proj.weight.double().t()) < 2.0 ** -7  # two bf16 roundings

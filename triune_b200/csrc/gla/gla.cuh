@@ -48,6 +48,24 @@ void gla_set_debug_buffer(long long* counters);
 // One decode step for B*H heads: state [BH,64,64] fp32 in place; q,k,v,g rows of 64 bf16; out bf16.
 void launch_gla_decode_step(GlaMat Q, GlaMat K, GlaMat V, GlaMat G, float* state, GlaMat O, int B, int H,
                             bool gate_logits, cudaStream_t s);
+// One decoding step from the fused projection rows [B, ld] = [q | k | v | gate logits] (mixer_step.cu).
+struct MixerStep {
+  const __nv_bfloat16* qkvg;
+  long long ld;
+  int H;
+  const float *cos, *sin;  // fp32 [table_rows, D], or null: no rotation
+  long long table_rows;
+  const long long* pos;    // position on the device, or null: pos_host
+  long long pos_host;
+  const float* state_in;   // fp32 [B, H, D, D]
+  float* state_out;        // may be state_in
+  __nv_bfloat16* out;      // [B, H * D]
+  const __nv_bfloat16* x;  // delta rule with beta_w: the projection's input rows [B, dim]
+  long long ldx;
+  const __nv_bfloat16* beta_w;  // [H, dim], or null: write strength 1
+  int dim;
+};
+void launch_mixer_step(const MixerStep& p, int B, int D, bool delta, cudaStream_t s);
 // Gated DeltaNet token recurrence over T tokens (T = 1: one decode step) for B*H heads of dimension D (64 or 128):
 // state [BH,D,D] fp32 in place; beta: null (1), fp32 [B*T,H] (beta_mode 1) or fp32 [B*T,H*D] (beta_mode 2).
 void launch_gdn_recurrent(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta,

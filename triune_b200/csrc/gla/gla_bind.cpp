@@ -95,6 +95,54 @@ void gla_decode(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, co
                              (int)B, (int)H, gate_logits, cur_stream());
 }
 
+// One decoding step: qkvg [B, 4 H D] -> (out [B, H D], state after the step). `inplace`: the state is updated where it is.
+std::vector<Tensor> mixer_step(const Tensor& qkvg, const c10::optional<Tensor>& cos, const c10::optional<Tensor>& sin,
+                               const c10::optional<Tensor>& pos, int64_t pos_host, const Tensor& state, bool inplace, bool delta,
+                               const c10::optional<Tensor>& x, const c10::optional<Tensor>& beta_w) {
+  c10::cuda::CUDAGuard guard(qkvg.device());
+  const auto m = mat(qkvg, 0);
+  TORCH_CHECK(state.is_cuda() && state.scalar_type() == at::kFloat && state.is_contiguous() && state.dim() == 4 &&
+                  state.size(2) == state.size(3) && state.size(0) == qkvg.size(0) && state.get_device() == qkvg.get_device() &&
+                  4 * state.size(1) * state.size(2) == qkvg.size(1),
+              "mixer_step: state [B, H, D, D] fp32 contiguous for qkvg [B, 4 H D]");
+  const int64_t B = state.size(0), H = state.size(1), D = state.size(2);
+  tb::MixerStep p{};
+  p.qkvg = reinterpret_cast<const __nv_bfloat16*>(m.ptr);
+  p.ld = m.ld;
+  p.H = (int)H;
+  if (cos.has_value() && cos->defined()) {
+    for (const Tensor& t : {*cos, *sin})
+      TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.dim() == 2 && t.size(1) == D && t.size(0) > 0 &&
+                      t.size(0) == cos->size(0),
+                  "mixer_step: rotary tables [rows, D] fp32");
+    p.cos = cos->data_ptr<float>();
+    p.sin = sin->data_ptr<float>();
+    p.table_rows = cos->size(0);
+  }
+  if (pos.has_value() && pos->defined()) {
+    TORCH_CHECK(pos->is_cuda() && pos->scalar_type() == at::kLong && pos->numel() >= 1, "mixer_step: position int64 on the device");
+    p.pos = reinterpret_cast<const long long*>(pos->data_ptr<int64_t>());
+  }
+  p.pos_host = pos_host;
+  if (beta_w.has_value() && beta_w->defined()) {
+    TORCH_CHECK(x.has_value() && x->defined(), "mixer_step: the write strength needs the input rows");
+    const auto xm = mat(*x, 0), wm = mat(*beta_w, 0);
+    TORCH_CHECK(beta_w->is_contiguous() && beta_w->size(0) == H && beta_w->size(1) == x->size(1) && x->size(0) == B && x->size(1) % 8 == 0,
+                "mixer_step: beta weight [H, dim] for input rows [B, dim]");
+    p.x = reinterpret_cast<const __nv_bfloat16*>(xm.ptr);
+    p.ldx = xm.ld;
+    p.beta_w = reinterpret_cast<const __nv_bfloat16*>(wm.ptr);
+    p.dim = (int)x->size(1);
+  }
+  Tensor out = torch::empty({B, H * D}, qkvg.options());
+  Tensor next = inplace ? state : torch::empty_like(state);
+  p.state_in = state.data_ptr<float>();
+  p.state_out = next.data_ptr<float>();
+  p.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+  tb::launch_mixer_step(p, (int)B, (int)D, delta, cur_stream());
+  return {out, next};
+}
+
 // Gated DeltaNet recurrence (no gradient): q,k,v,g as [B*T, ld] matrices whose columns col0 + h*D.. hold head h.
 void gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol,
                    const Tensor& g, int64_t gcol, const c10::optional<Tensor>& beta, Tensor& state, Tensor& out,
@@ -223,6 +271,7 @@ void register_gla(pybind11::module& m) {
     TORCH_CHECK(!t.has_value() || !t->defined() || (t->scalar_type() == at::kLong && t->numel() >= 8), "int64[8] expected");
     tb::gla_set_debug_buffer(t.has_value() && t->defined() ? (long long*)t->data_ptr<int64_t>() : nullptr);
   });
+  m.def("mixer_step", &mixer_step);
   m.def("gdn_recurrent", &gdn_recurrent);
   m.def("gdn_chunk_fwd", &gdn_chunk_fwd);
   m.def("gdn_chunk_bwd", &gdn_chunk_bwd);

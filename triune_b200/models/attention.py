@@ -152,6 +152,13 @@ class VectorisedGLA(nn.Module):
         lora = getattr(self, "qkvg_lora", None)  # set by the fine-tuner (FusedProjectionLoRA)
         x2 = x.reshape(B * T, self.dim)
         qkvg = lora(x2) if lora is not None else ops.linear(x2, self.qkvg_weight)
+        plain_beta = self.beta_proj is None or type(self.beta_proj) is nn.Linear  # wrapped ones run their own forward below
+        beta_w = self.beta_proj.weight if plain_beta and self.beta_proj is not None else None
+        if T == 1 and plain_beta and gla_cuda.step_supported(qkvg, state, H, D, x2, beta_w):
+            rope = self.rope.tables(1, x.device, offset) if self.use_rope else None
+            out, new_state = gla_cuda.mixer_step(qkvg, rope, offset, state, self.use_delta_rule, x2, beta_w)
+            y = _project(self.out_proj, out.view(B, 1, self.hidden_dim), 1.0 if self.use_delta_rule else self.out_scale)
+            return y, format_cache(new_state if cache is not None else None, cache, fmt, offset, T)
         cos = sin = None
         if self.use_rope:
             cos, sin = self.rope(T, x.device, offset=offset)

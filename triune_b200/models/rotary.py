@@ -62,17 +62,23 @@ class RotaryEmbedding(nn.Module):
         cos, sin = ops.rope_tables(length, self.head_dim, self.base, 0, device)
         self._cos, self._sin = cos, sin
 
+    def tables(self, seq_len: int, device, offset=0):
+        """The whole tables [rows, head_dim], grown to cover ``offset + seq_len`` positions where ``offset`` is a number (a
+        position on the device relies on the caller having sized them)."""
+        device = torch.device(device)
+        length = max(self.max_seq_len, 1)
+        if not torch.is_tensor(offset):
+            while length < offset + seq_len:
+                length *= 2
+        if self._cos is None or self._cos.device != device or (not torch.is_tensor(offset) and self._cos.shape[0] < offset + seq_len):
+            self._build(length, device)
+        return self._cos, self._sin
+
     def forward(self, seq_len: int, device, offset=0):
         if torch.is_tensor(offset):
             # position lives on the device (CUDA-graph decoding): gather rows; the caller sized the table beforehand
-            if self._cos is None or self._cos.device != torch.device(device):
-                self._build(max(self.max_seq_len, 1), device)
+            self.tables(seq_len, device, offset)
             pos = offset.reshape(-1)[:1].long() + torch.arange(seq_len, device=offset.device)
             return self._cos.index_select(0, pos), self._sin.index_select(0, pos)
-        need = offset + seq_len
-        if self._cos is None or self._cos.device != torch.device(device) or self._cos.shape[0] < need:
-            length = max(self.max_seq_len, 1)
-            while length < need:
-                length *= 2
-            self._build(length, device)
-        return self._cos[offset:need], self._sin[offset:need]
+        cos, sin = self.tables(seq_len, device, offset)
+        return cos[offset : offset + seq_len], sin[offset : offset + seq_len]

@@ -158,6 +158,31 @@ def decode_step(q, k, v, g, state, gate_logits):
     return out.view(B, 1, H, D), st
 
 
+def _aligned_rows(t) -> bool:
+    return t.dtype == torch.bfloat16 and t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
+def step_supported(qkvg, state, H: int, D: int, x=None, beta_w=None) -> bool:
+    """True when :func:`mixer_step` covers a single token: bf16 projection rows, head dim 64 or 128, fp32 state, no gradient."""
+    if beta_w is not None and not (beta_w.is_cuda and beta_w.is_contiguous() and _aligned_rows(beta_w) and _aligned_rows(x)):
+        return False
+    return (_ext.use_kernels(qkvg, state) and not torch.is_grad_enabled() and torch.is_tensor(state) and D in (64, 128)
+            and _aligned_rows(qkvg) and state.dtype == torch.float32 and state.is_contiguous()
+            and state.shape == (qkvg.shape[0], H, D, D))
+
+
+def mixer_step(qkvg, rope, offset, state, delta: bool, x=None, beta_w=None):
+    """One decoding step from the fused projection rows in one launch -> (out [B, H*D] bf16, state after the step).
+    ``rope``: (cos, sin) tables [rows, D] or None; ``offset``: position, an int or a device tensor. The 64-wide GLA state is
+    updated in place, as :func:`decode_step` does; the others come back as a new tensor."""
+    cos, sin = rope if rope is not None else (None, None)
+    dev_pos = offset if torch.is_tensor(offset) else None
+    inplace = not delta and state.shape[-1] == 64
+    out, new = _ext.ext().mixer_step(qkvg, cos, sin, dev_pos, 0 if dev_pos is not None else int(offset), state, inplace, delta, x, beta_w)
+    _tick(1)
+    return out, new
+
+
 def gdn_supported(q, k, v, g, beta) -> bool:
     """True when the recurrent Gated DeltaNet kernel covers this call: bf16, head dim 64 or 128 (keys = values), no
     gradient wanted."""
