@@ -149,3 +149,44 @@ def test_mixer_step_against_a_64_bit_statement(B, H, D, delta, learn_beta, rope,
     o = torch.einsum("bhk,bhkv->bhv", q, st).reshape(B, dim)
     assert _rel(s1, st) < 2e-6                                              # fp32 throughout
     assert _rel(y.reshape(B, dim), o @ m.out_proj.weight.double().t()) < 2.0 ** -7  # two bf16 roundings
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [2, 16, 17, 63, 64, 65, 191, 256])
+def test_gated_attention_of_any_length_against_fp64(T, D):
+    B, H = 2, 3
+    q, k, v, g, s0 = (t.requires_grad_(True) for t in _mixer_inputs(B, T, H, D, seed=T))
+    o, s = gla_cuda._GLAFn.apply(q, k, v, g, s0, True)
+    wo, ws = torch.randn_like(o), torch.randn_like(s) * 0.1
+    got = (o, s, *torch.autograd.grad((o.float() * wo).sum() + (s * ws).sum(), (q, k, v, g, s0)))
+    x = [t.detach().double().requires_grad_(True) for t in (q, k, v, g, s0)]
+    gl = F.logsigmoid(x[3])
+    if T >= 64:
+        gl = gl.clamp(min=gla_cuda.GLA_MIN_LOG_DECAY)
+    oo, ss = ref.gla_chunk(*x[:3], gl, x[4])
+    want = (oo, ss, *torch.autograd.grad((oo * wo.double()).sum() + (ss * ws.double()).sum(), x))
+    # under 64 tokens everything is fp32 and bf16 results round by at most 2^-9; whole chunks have bf16 operands (states,
+    # weighted keys and scores, 2^-9 each) in two products that follow one another. A gate gradient is the sum over the
+    # later tokens of q dq - k dk: up to T independent errors of 2^-8 of such terms, whose sum itself stays about as large as one
+    rounding = 2.0 ** -8
+    for n, a, b in zip(("o", "s", "dq", "dk", "dv", "dg", "ds0"), got, want):
+        limit = (1e-5 if a.dtype == torch.float32 else rounding) if T < 64 else (2 * T ** 0.5 if n == "dg" else 4) * rounding
+        assert _rel(a, b) < limit, (n, _rel(a, b))
+
+
+@pytest.mark.parametrize("T,D", [(21, 128), (150, 64), (150, 128)])
+def test_fused_projection_rows_match_separate_tensors(T, D):
+    B, H = 2, 2
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(B * T, 4 * H * D, device="cuda", generator=gen).bfloat16().requires_grad_(True)
+    s0 = torch.randn(1, H, D, D, device="cuda", generator=gen).requires_grad_(True)  # one state for every sequence
+    w = torch.randn(B * T, H * D, device="cuda", generator=gen)
+    o, s = gla_cuda.gla_attention_core(x, None, None, s0, B, T, H)
+    got = torch.autograd.grad((o.float() * w).sum() + s.sum(), (x, s0))
+    from triune_b200 import ops
+
+    q, k, v, g = ops.qk_feature_map(x, None, None, B, T, H, D)
+    oo, ss = gla_cuda._GLAFn.apply(q, k, v, g, s0.expand(B, H, D, D), True)
+    want = torch.autograd.grad((oo.reshape(B * T, H * D).float() * w).sum() + ss.sum(), (x, s0))
+    assert torch.equal(o, oo.reshape(B * T, H * D)) and torch.equal(s, ss)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])

@@ -1,4 +1,4 @@
-// Launchers of the gated-linear-attention kernels (head_dim 64, chunk 64, bf16 in, fp32 state).
+// Launchers of the gated-linear-attention kernels (head_dim 64 or 128, chunk 64, bf16 in, fp32 state).
 //
 // The sequence is processed in three phases, forward and backward alike:
 //   1. per chunk, in parallel:   local state contribution (K~^T V, or Q~^T dO going backward)
@@ -16,7 +16,7 @@ namespace tb {
 
 constexpr float GLA_MIN_LOG_DECAY = -5.0f;
 
-// A [B*T rows] x [64 cols] bf16 slice of a wider row-major matrix: element (row, c) = ptr[row*ld + col0 + h*64 + c].
+// A [B*T rows] x [D cols] bf16 slice of a wider row-major matrix: element (row, c) = ptr[row*ld + col0 + h*D + c].
 struct GlaMat {
   const void* ptr;
   long long ld;
@@ -24,8 +24,10 @@ struct GlaMat {
 };
 
 struct GlaDims {
-  int B, T, H;
+  int B, T, H;       // T: tokens per sequence taken by the call, a multiple of 64
   bool gate_logits;  // g holds raw logits (log-sigmoid applied in-kernel) instead of log decays
+  int D = 64;        // head dimension (keys and values): 64 or 128
+  int rows = 0;      // rows per sequence in the matrices where that is more than T, else 0
 };
 
 // mode 0: kv[bh,c] = (k * exp(b_last - b))^T v and decay[bh,c] = exp(b_last);  mode 1: kv = (q * exp(b))^T dO.
@@ -33,16 +35,30 @@ void launch_gla_chunk_outer(int mode, GlaMat X, GlaMat Y, GlaMat G, float* out_k
                             int* status, cudaStream_t s);
 // forward: states[c] = S before chunk c, S <- decay[c] * S + kv[c];  reverse: states[c] = dS after chunk c.
 void launch_gla_scan(const float* kv, const float* decay, const float* init, __nv_bfloat16* states, float* final_state,
-                     int BH, int NT, bool reverse, cudaStream_t s);
+                     int BH, int NT, int D, bool reverse, cudaStream_t s);
 void launch_gla_fwd_out(GlaMat Q, GlaMat K, GlaMat V, GlaMat G, const __nv_bfloat16* states, GlaMat O, GlaDims d,
                         int* status, cudaStream_t s);
 void launch_gla_bwd_main(GlaMat Q, GlaMat K, GlaMat V, GlaMat G, GlaMat dO, const __nv_bfloat16* states,
                          const __nv_bfloat16* dstates, GlaMat dQ, GlaMat dK, GlaMat dV, float* dgl_local,
                          float* chunk_tot, GlaDims d, int* status, cudaStream_t s);
-// end_term (optional, fp32 [B*H, 64]): rowsum(dS_T * S_T), the gate gradient that reaches every token through a
+// end_term (optional, fp32 [B*H, D]): rowsum(dS_T * S_T), the gate gradient that reaches every token through a
 // differentiated final state.
 void launch_gla_dg_finalize(const float* dgl_local, const float* chunk_tot, GlaMat G, GlaMat dG, GlaDims d,
                             cudaStream_t s, const float* end_term = nullptr);
+// Fewer than 64 tokens, fp32 throughout (gla_tail.cu): rows [t0, t0 + n) of every sequence of `rows` rows.
+struct GlaTail {
+  int B, H, D, rows, t0, n;
+  bool gate_logits;
+  float floor;  // least log decay of a token
+};
+// state0 / state1: fp32 [B*H, D, D] before (null: zero) and after the tokens; outputs are written to the same rows of O.
+void launch_gla_tail_fwd(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const GlaMat& O, const float* state0,
+                         float* state1, const GlaTail& t, cudaStream_t s);
+// dstate1, end1 (rowsum(dstate1 * state1), fp32 [B*H, D]): null where the state after the tokens has no gradient. Writes the
+// tokens' rows of dQ, dK, dV, dG, the gradient of state0 and its rowsum with state0.
+void launch_gla_tail_bwd(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const GlaMat& dO, const GlaMat& dQ,
+                         const GlaMat& dK, const GlaMat& dV, const GlaMat& dG, const float* state0, const float* dstate1,
+                         const float* end1, float* dstate0, float* end0, const GlaTail& t, cudaStream_t s);
 // Developer aid: eight int64 counters (device memory) receiving the backward kernel's phase clocks; null disables.
 void gla_set_debug_buffer(long long* counters);
 // One decode step for B*H heads: state [BH,64,64] fp32 in place; q,k,v,g rows of 64 bf16; out bf16.

@@ -3,6 +3,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <cmath>
+
 #include "gla.cuh"
 
 namespace {
@@ -18,72 +20,103 @@ tb::GlaMat mat(const Tensor& t, int64_t col0) {
   return tb::GlaMat{t.data_ptr(), t.stride(0), (int)col0};
 }
 
-// Forward: returns (states bf16 [BH*NT,64,64], decay fp32 [BH*NT,64], final_state fp32 [BH,64,64]); writes out.
+// Forward over [B*T] rows: whole chunks of 64 tokens on the chunk kernels, the T % 64 tokens after them one by one in fp32
+// (all of them where T < 64, and then without the chunk kernels' clamp of the log decay, which that case never had).
+// Returns (states bf16 [BH*NT,D,D], decay fp32 [BH*NT,D], final_state fp32 [BH,D,D], status) and, where there are both
+// chunks and further tokens, the state between them (fp32 [BH,D,D]); writes out.
 std::vector<Tensor> gla_fwd(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol,
                             const Tensor& g, int64_t gcol, Tensor& out, int64_t ocol, const c10::optional<Tensor>& init,
-                            int64_t B, int64_t T, int64_t H, bool gate_logits) {
+                            int64_t B, int64_t T, int64_t H, bool gate_logits, int64_t D) {
   c10::cuda::CUDAGuard guard(q.device());
-  const int64_t NT = T / 64, BH = B * H;
+  TORCH_CHECK(D == 64 || D == 128, "gla_fwd: head dimension 64 or 128");
+  const int64_t NT = T / 64, BH = B * H, rest = T % 64;
   auto f32 = q.options().dtype(at::kFloat);
-  Tensor kv = torch::empty({BH * NT, 64, 64}, f32);
-  Tensor decay = torch::empty({BH * NT, 64}, f32);
-  Tensor states = torch::empty({BH * NT, 64, 64}, q.options());
-  Tensor fin = torch::empty({BH, 64, 64}, f32);
-  Tensor status = torch::zeros({1}, q.options().dtype(at::kInt));
-  tb::GlaDims d{(int)B, (int)T, (int)H, gate_logits};
+  Tensor decay = torch::empty({BH * NT, D}, f32);
+  Tensor states = torch::empty({BH * NT, D, D}, q.options());
+  Tensor fin = torch::empty({BH, D, D}, f32);
+  Tensor status = NT > 0 ? torch::zeros({1}, q.options().dtype(at::kInt)) : torch::empty({0}, q.options().dtype(at::kInt));
   auto s = cur_stream();
-  tb::launch_gla_chunk_outer(0, mat(k, kcol), mat(v, vcol), mat(g, gcol), kv.data_ptr<float>(), decay.data_ptr<float>(), d,
-                             status.data_ptr<int>(), s);
   const float* ip = nullptr;
-  Tensor initc;
+  Tensor initc, mid;
   if (init.has_value() && init->defined()) {
     initc = init->to(at::kFloat).contiguous();
+    TORCH_CHECK(initc.numel() == BH * D * D, "gla_fwd: initial state [B, H, D, D]");
     ip = initc.data_ptr<float>();
   }
-  tb::launch_gla_scan(kv.data_ptr<float>(), decay.data_ptr<float>(), ip,
-                      reinterpret_cast<__nv_bfloat16*>(states.data_ptr()), fin.data_ptr<float>(), (int)BH, (int)NT, false, s);
-  tb::launch_gla_fwd_out(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol),
-                         reinterpret_cast<const __nv_bfloat16*>(states.data_ptr()), mat(out, ocol), d,
-                         status.data_ptr<int>(), s);
-  return {states, decay, fin, status};
+  if (NT > 0) {
+    Tensor kv = torch::empty({BH * NT, D, D}, f32);
+    Tensor after = rest > 0 ? (mid = torch::empty({BH, D, D}, f32)) : fin;
+    const tb::GlaDims d{(int)B, (int)(NT * 64), (int)H, gate_logits, (int)D, (int)T};
+    tb::launch_gla_chunk_outer(0, mat(k, kcol), mat(v, vcol), mat(g, gcol), kv.data_ptr<float>(), decay.data_ptr<float>(), d,
+                               status.data_ptr<int>(), s);
+    tb::launch_gla_scan(kv.data_ptr<float>(), decay.data_ptr<float>(), ip, reinterpret_cast<__nv_bfloat16*>(states.data_ptr()),
+                        after.data_ptr<float>(), (int)BH, (int)NT, (int)D, false, s);
+    tb::launch_gla_fwd_out(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol),
+                           reinterpret_cast<const __nv_bfloat16*>(states.data_ptr()), mat(out, ocol), d,
+                           status.data_ptr<int>(), s);
+    ip = after.data_ptr<float>();
+  }
+  if (rest > 0) {
+    const tb::GlaTail t{(int)B, (int)H, (int)D, (int)T, (int)(NT * 64), (int)rest, gate_logits, NT > 0 ? tb::GLA_MIN_LOG_DECAY : -INFINITY};
+    tb::launch_gla_tail_fwd(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), mat(out, ocol), ip, fin.data_ptr<float>(), t, s);
+  }
+  std::vector<Tensor> r{states, decay, fin, status};
+  if (NT > 0 && rest > 0) r.push_back(mid);
+  return r;
 }
 
 // Backward: writes dq, dk, dv, dg into the given matrices. With `dfin` (gradient of the final state, fp32
-// [BH,64,64]) and `fin` (the final state itself) the reverse scan starts from dfin instead of zero and the gate
-// gradient receives rowsum(dfin * fin). Returns (status, gradient of the initial state [BH,64,64] fp32).
+// [BH,D,D]) and `fin` (the final state itself) the reverse scan starts from dfin instead of zero and the gate
+// gradient receives rowsum(dfin * fin). `before_rest`: the state before the T % 64 last tokens (the initial state where
+// T < 64; none: zero). Returns (status, gradient of the initial state [BH,D,D] fp32).
 std::vector<Tensor> gla_bwd(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol, const Tensor& g,
                int64_t gcol, const Tensor& dout, int64_t docol, const Tensor& states, const Tensor& decay, Tensor& dq,
                int64_t dqcol, Tensor& dk, int64_t dkcol, Tensor& dv, int64_t dvcol, Tensor& dg, int64_t dgcol, int64_t B,
                int64_t T, int64_t H, bool gate_logits, const c10::optional<Tensor>& dfin,
-               const c10::optional<Tensor>& fin) {
+               const c10::optional<Tensor>& fin, int64_t D, const c10::optional<Tensor>& before_rest) {
   c10::cuda::CUDAGuard guard(q.device());
-  const int64_t NT = T / 64, BH = B * H;
+  TORCH_CHECK(D == 64 || D == 128, "gla_bwd: head dimension 64 or 128");
+  const int64_t NT = T / 64, BH = B * H, rest = T % 64;
   auto f32 = q.options().dtype(at::kFloat);
-  Tensor dfinc, end_term;
-  Tensor dinit = torch::empty({BH, 64, 64}, f32);
+  Tensor dnext, end_term;  // gradient of the state after the tokens in hand, its rowsum with that state
+  Tensor dinit = torch::empty({BH, D, D}, f32);
   if (dfin.has_value() && dfin->defined()) {
     TORCH_CHECK(fin.has_value() && fin->defined(), "the final state is needed with its gradient");
-    dfinc = dfin->to(at::kFloat).reshape({BH, 64, 64}).contiguous();
-    end_term = (dfinc * fin->to(at::kFloat).reshape({BH, 64, 64})).sum(-1).contiguous();
+    dnext = dfin->to(at::kFloat).reshape({BH, D, D}).contiguous();
+    end_term = (dnext * fin->to(at::kFloat).reshape({BH, D, D})).sum(-1).contiguous();
   }
-  Tensor m = torch::empty({BH * NT, 64, 64}, f32);
-  Tensor dstates = torch::empty({BH * NT, 64, 64}, q.options());
-  Tensor dgl = torch::empty({B * T, H * 64}, f32);
-  Tensor tot = torch::empty({BH * NT, 64}, f32);
-  Tensor status = torch::zeros({1}, q.options().dtype(at::kInt));
-  tb::GlaDims d{(int)B, (int)T, (int)H, gate_logits};
+  auto fp = [](const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; };
   auto s = cur_stream();
+  if (rest > 0) {
+    const tb::GlaTail t{(int)B, (int)H, (int)D, (int)T, (int)(NT * 64), (int)rest, gate_logits, NT > 0 ? tb::GLA_MIN_LOG_DECAY : -INFINITY};
+    Tensor from, dmid = NT > 0 ? torch::empty({BH, D, D}, f32) : dinit, emid = torch::empty({BH, D}, f32);
+    if (before_rest.has_value() && before_rest->defined()) {
+      from = before_rest->to(at::kFloat).contiguous();
+      TORCH_CHECK(from.numel() == BH * D * D, "gla_bwd: state [B, H, D, D] before the last tokens");
+    }
+    TORCH_CHECK(NT == 0 || from.defined(), "gla_bwd: the state after the whole chunks is needed");
+    tb::launch_gla_tail_bwd(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), mat(dout, docol), mat(dq, dqcol), mat(dk, dkcol),
+                            mat(dv, dvcol), mat(dg, dgcol), fp(from), fp(dnext), fp(end_term), dmid.data_ptr<float>(),
+                            emid.data_ptr<float>(), t, s);
+    dnext = dmid;
+    end_term = emid;
+  }
+  Tensor status = NT > 0 ? torch::zeros({1}, q.options().dtype(at::kInt)) : torch::empty({0}, q.options().dtype(at::kInt));
+  if (NT == 0) return {status, dinit};
+  Tensor m = torch::empty({BH * NT, D, D}, f32);
+  Tensor dstates = torch::empty({BH * NT, D, D}, q.options());
+  Tensor dgl = torch::empty({B * T, H * D}, f32);
+  Tensor tot = torch::empty({BH * (D / 64) * NT, 64}, f32);
+  const tb::GlaDims d{(int)B, (int)(NT * 64), (int)H, gate_logits, (int)D, (int)T};
   tb::launch_gla_chunk_outer(1, mat(q, qcol), mat(dout, docol), mat(g, gcol), m.data_ptr<float>(), nullptr, d,
                              status.data_ptr<int>(), s);
-  tb::launch_gla_scan(m.data_ptr<float>(), decay.data_ptr<float>(), dfinc.defined() ? dfinc.data_ptr<float>() : nullptr,
-                      reinterpret_cast<__nv_bfloat16*>(dstates.data_ptr()), dinit.data_ptr<float>(), (int)BH, (int)NT,
-                      true, s);
+  tb::launch_gla_scan(m.data_ptr<float>(), decay.data_ptr<float>(), fp(dnext), reinterpret_cast<__nv_bfloat16*>(dstates.data_ptr()),
+                      dinit.data_ptr<float>(), (int)BH, (int)NT, (int)D, true, s);
   tb::launch_gla_bwd_main(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), mat(dout, docol),
                           reinterpret_cast<const __nv_bfloat16*>(states.data_ptr()),
                           reinterpret_cast<const __nv_bfloat16*>(dstates.data_ptr()), mat(dq, dqcol), mat(dk, dkcol),
                           mat(dv, dvcol), dgl.data_ptr<float>(), tot.data_ptr<float>(), d, status.data_ptr<int>(), s);
-  tb::launch_gla_dg_finalize(dgl.data_ptr<float>(), tot.data_ptr<float>(), mat(g, gcol), mat(dg, dgcol), d, s,
-                             end_term.defined() ? end_term.data_ptr<float>() : nullptr);
+  tb::launch_gla_dg_finalize(dgl.data_ptr<float>(), tot.data_ptr<float>(), mat(g, gcol), mat(dg, dgcol), d, s, fp(end_term));
   return {status, dinit};
 }
 
@@ -264,8 +297,14 @@ std::vector<Tensor> gdn_chunk_bwd(const Tensor& q, int64_t qcol, const Tensor& k
 }  // namespace
 
 void register_gla(pybind11::module& m) {
-  m.def("gla_fwd", &gla_fwd);
-  m.def("gla_bwd", &gla_bwd);
+  namespace py = pybind11;
+  m.def("gla_fwd", &gla_fwd, py::arg("q"), py::arg("qcol"), py::arg("k"), py::arg("kcol"), py::arg("v"), py::arg("vcol"), py::arg("g"),
+        py::arg("gcol"), py::arg("out"), py::arg("ocol"), py::arg("init"), py::arg("B"), py::arg("T"), py::arg("H"),
+        py::arg("gate_logits"), py::arg("D") = 64);
+  m.def("gla_bwd", &gla_bwd, py::arg("q"), py::arg("qcol"), py::arg("k"), py::arg("kcol"), py::arg("v"), py::arg("vcol"), py::arg("g"),
+        py::arg("gcol"), py::arg("dout"), py::arg("docol"), py::arg("states"), py::arg("decay"), py::arg("dq"), py::arg("dqcol"),
+        py::arg("dk"), py::arg("dkcol"), py::arg("dv"), py::arg("dvcol"), py::arg("dg"), py::arg("dgcol"), py::arg("B"), py::arg("T"),
+        py::arg("H"), py::arg("gate_logits"), py::arg("dfin"), py::arg("fin"), py::arg("D") = 64, py::arg("before_rest") = py::none());
   m.def("gla_decode", &gla_decode);
   m.def("gla_debug_buffer", [](const c10::optional<Tensor>& t) {
     TORCH_CHECK(!t.has_value() || !t->defined() || (t->scalar_type() == at::kLong && t->numel() >= 8), "int64[8] expected");

@@ -66,7 +66,7 @@ extern "C" int triune_gla_forward_noalloc(const void* q, const void* k, const vo
   tb::GlaDims d{B, T, H, gate_logits != 0};
   try {
     tb::launch_gla_chunk_outer(0, K, V, G, kv, decay, d, status, stream);
-    tb::launch_gla_scan(kv, decay, init_state, states, final_state, B * H, T / 64, false, stream);
+    tb::launch_gla_scan(kv, decay, init_state, states, final_state, B * H, T / 64, 64, false, stream);
     tb::launch_gla_fwd_out(Q, K, V, G, states, O, d, status, stream);
   } catch (...) {
     return -3;

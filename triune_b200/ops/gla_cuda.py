@@ -1,8 +1,8 @@
 """Dispatch to the sm_100a chunked GLA kernels (forward, backward, decode step).
 
 Two entry points:
-  * :func:`gla_chunk` for separate ``[B,T,H,64]`` tensors (the public ``ops.gla`` signature);
-  * :func:`gla_attention_core` for the model: it consumes the fused projection output ``qkvg [B*T, 4*H*64]``
+  * :func:`gla_chunk` for separate ``[B,T,H,D]`` tensors (the public ``ops.gla`` signature);
+  * :func:`gla_attention_core` for the model: it consumes the fused projection output ``qkvg [B*T, 4*H*D]``
     directly (feature map + RoPE kernel, then the chunk kernels read v and the gate logits in place through
     strided TMA maps) and its backward writes all four gradients into one ``d qkvg`` buffer.
 
@@ -50,7 +50,7 @@ def supported(q, k, v, g, initial_state) -> bool:
 
 
 def _as_matrix(x: torch.Tensor) -> torch.Tensor:
-    """[B,T,H,64] -> a 2-D [B*T, ld] matrix view whose columns h*64.. hold head h (copying only if needed)."""
+    """[B,T,H,D] -> a 2-D [B*T, ld] matrix view whose columns h*D.. hold head h (copying only if needed)."""
     B, T, H, D = x.shape
     if x.stride(3) == 1 and x.stride(2) == D and x.stride(0) == T * x.stride(1) and x.stride(1) % 8 == 0 \
             and x.data_ptr() % 16 == 0:
@@ -65,10 +65,11 @@ class _GLAFn(torch.autograd.Function):
         e = _ext.ext()
         qm, km, vm, gm = (_as_matrix(t.to(torch.bfloat16)) for t in (q, k, v, g))
         out = torch.empty(B * T, H * D, device=q.device, dtype=torch.bfloat16)
-        states, decay, fin, status = e.gla_fwd(qm, 0, km, 0, vm, 0, gm, 0, out, 0, init, B, T, H, gate_logits)
-        _tick(3)
-        _note(status)
-        ctx.save_for_backward(qm, km, vm, gm, states, decay, fin)
+        states, decay, fin, status, *mid = e.gla_fwd(qm, 0, km, 0, vm, 0, gm, 0, out, 0, init, B, T, H, gate_logits, D)
+        _tick(3 * (T >= 64) + (T % 64 != 0))
+        if T >= 64:
+            _note(status)
+        ctx.save_for_backward(qm, km, vm, gm, states, decay, fin, mid[0] if mid else (init if T < 64 else None))
         ctx.dims = (B, T, H, D, gate_logits, init is not None)
         ctx.set_materialize_grads(False)
         return out.view(B, T, H, D), fin.view(B, H, D, D)
@@ -78,7 +79,7 @@ class _GLAFn(torch.autograd.Function):
         # The final state is differentiable: its gradient seeds the reverse inter-chunk scan (it is the state
         # gradient after the last chunk), adds rowsum(dS_T * S_T) to every token's gate gradient, and the scan's
         # last value is the gradient of the initial state.
-        qm, km, vm, gm, states, decay, fin = ctx.saved_tensors
+        qm, km, vm, gm, states, decay, fin, before = ctx.saved_tensors
         B, T, H, D, gate_logits, has_init = ctx.dims
         e = _ext.ext()
         if dout is None:
@@ -86,39 +87,32 @@ class _GLAFn(torch.autograd.Function):
         dom = _as_matrix(dout.to(torch.bfloat16))
         dq, dk, dv, dg = (torch.empty(B * T, H * D, device=dom.device, dtype=torch.bfloat16) for _ in range(4))
         status, dinit = e.gla_bwd(qm, 0, km, 0, vm, 0, gm, 0, dom, 0, states, decay, dq, 0, dk, 0, dv, 0, dg, 0, B, T, H,
-                                  gate_logits, dfin, fin if dfin is not None else None)
-        _tick(4)
-        _note(status)
+                                  gate_logits, dfin, fin if dfin is not None else None, D, before)
+        _tick(4 * (T >= 64) + 2 * (T % 64 != 0))
+        if T >= 64:
+            _note(status)
         sh = (B, T, H, D)
         dinit = dinit.view(B, H, D, D) if (has_init and ctx.needs_input_grad[4]) else None
         return dq.view(sh), dk.view(sh), dv.view(sh), dg.view(sh), dinit, None
 
 
 def gla_chunk(q, k, v, g, initial_state, scale, gate_logits):
-    """Kernel path of ``ops.gla``. Ragged tails (T % 64) are finished by the reference op with state carry."""
-    from . import reference as ref
-
+    """Kernel path of ``ops.gla`` for T >= 64, or one token with a state. The last T % 64 tokens are walked in fp32."""
     B, T, H, D = q.shape
-    if D != 64 or v.shape[-1] != 64:
+    square = D == v.shape[-1]
+    if not (square and (D == 64 or (D == 128 and T > 1))):
         return _gla_wide_heads(q, k, v, g, initial_state, scale, gate_logits)
     if T == 1:
         return decode_step(q, k, v, g, initial_state, gate_logits)
-    Tm = (T // 64) * 64
-    out, state = _GLAFn.apply(q[:, :Tm], k[:, :Tm], v[:, :Tm], g[:, :Tm], initial_state, gate_logits)
-    if Tm < T:
-        # ragged tail: the reference op continues from the kernels' final state (which carries its gradient back into
-        # the first Tm tokens) with the kernels' clamp of the per-token log decay
-        gl = torch.nn.functional.logsigmoid(g[:, Tm:].float()) if gate_logits else g[:, Tm:].float()
-        gl = gl.clamp(min=GLA_MIN_LOG_DECAY, max=0.0)
-        o2, state = ref.gla_chunk(q[:, Tm:], k[:, Tm:], v[:, Tm:], gl, state, 1.0)
-        out = torch.cat((out, o2.to(out.dtype)), dim=1)
+    out, state = _GLAFn.apply(q, k, v, g, initial_state, gate_logits)
     if scale != 1.0:
         out = out * scale
     return out, state
 
 
 def _gla_wide_heads(q, k, v, g, initial_state, scale, gate_logits):
-    """Heads wider than 64 on the 64-wide kernels.
+    """Heads of 192 or 256 dimensions, heads with keys and values of different widths and single tokens of wide heads on the
+    64-wide kernels.
 
     The decay is diagonal over key dimensions, so the state rows of different key dimensions never mix:
     S[d, :] only sees q_d, k_d, g_d. A head with dk = 64 a, dv = 64 c is therefore exactly the sum over the ``a``
@@ -289,56 +283,57 @@ def gdn_recurrent(q, k, v, g, beta, initial_state, scale, gate_logits):
 
 
 class _GLACoreFn(torch.autograd.Function):
-    """qkvg [B*T, 4*H*64] -> attention output [B*T, H*64] (feature map, RoPE and the chunk scan fused)."""
+    """qkvg [B*T, 4*H*D] -> attention output [B*T, H*D] (feature map, RoPE and the chunk scan fused), any T > 1."""
 
     @staticmethod
     def forward(ctx, qkvg, cos_half, sin_half, init, B, T, H):
-        D = 64
+        D = qkvg.shape[1] // (4 * H)
         HD = H * D
         e = _ext.ext()
         qk = e.qk_prep_fwd(qkvg, HD, cos_half, sin_half, T, H, D).view(B * T, 2 * HD)
         out = torch.empty(B * T, HD, device=qkvg.device, dtype=torch.bfloat16)
-        states, decay, fin, status = e.gla_fwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, out, 0, init, B, T, H, True)
-        _tick(4)
-        _note(status)
-        none = torch.empty(0, device=qkvg.device)
-        ctx.save_for_backward(qkvg, qk, states, decay, cos_half if cos_half is not None else none,
-                              sin_half if sin_half is not None else none)
-        ctx.dims = (B, T, H, cos_half is not None)
+        states, decay, fin, status, *mid = e.gla_fwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, out, 0, init, B, T, H, True, D)
+        _tick(1 + 3 * (T >= 64) + (T % 64 != 0))
+        if T >= 64:
+            _note(status)
+        # whole chunks of 64-wide heads: the state is carried, not trained through (a caller that keeps it across steps does
+        # not detach it); elsewhere it has a gradient, and so has the initial state
+        train_state = D == 128 or T % 64 != 0
+        before = mid[0] if mid else (init if T < 64 else None)
+        ctx.save_for_backward(qkvg, qk, states, decay, cos_half, sin_half, before, fin if train_state else None)
+        ctx.dims = (B, T, H, D, init is not None and train_state)
+        ctx.set_materialize_grads(False)
         fin = fin.view(B, H, D, D)
-        ctx.mark_non_differentiable(fin)
+        if not train_state:
+            ctx.mark_non_differentiable(fin)
         return out, fin
 
     @staticmethod
     def backward(ctx, dout, dfin):
-        qkvg, qk, states, decay, cs, sn = ctx.saved_tensors
-        B, T, H, rope = ctx.dims
-        D = 64
+        qkvg, qk, states, decay, cs, sn, before, fin = ctx.saved_tensors
+        B, T, H, D, grad_init = ctx.dims
         HD = H * D
         e = _ext.ext()
-        dout = dout.contiguous()
+        dout = qkvg.new_zeros(B * T, HD) if dout is None else dout.contiguous()
         dqk = torch.empty_like(qk)
         dqkvg = torch.empty_like(qkvg)
-        status, _ = e.gla_bwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, dout, 0, states, decay, dqk, 0, dqk, HD, dqkvg,
-                              2 * HD, dqkvg, 3 * HD, B, T, H, True, None, None)
-        e.qk_prep_bwd(qkvg, HD, dqk.view(B * T, 2, H, D), dqkvg, cs if rope else None, sn if rope else None, T, H, D)
-        _tick(5)
-        _note(status)
-        return dqkvg, None, None, None, None, None, None
+        status, dinit = e.gla_bwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, dout, 0, states, decay, dqk, 0, dqk, HD, dqkvg,
+                                  2 * HD, dqkvg, 3 * HD, B, T, H, True, dfin, fin if dfin is not None else None, D, before)
+        e.qk_prep_bwd(qkvg, HD, dqk.view(B * T, 2, H, D), dqkvg, cs, sn, T, H, D)
+        _tick(1 + 4 * (T >= 64) + 2 * (T % 64 != 0))
+        if T >= 64:
+            _note(status)
+        return dqkvg, None, None, dinit.view(B, H, D, D) if grad_init and ctx.needs_input_grad[3] else None, None, None, None
 
 
 def core_supported(qkvg: torch.Tensor, T: int, D: int) -> bool:
-    return (
-        _ext.use_kernels(qkvg)
-        and qkvg.dtype == torch.bfloat16
-        and D == 64
-        and T % 64 == 0
-        and T >= 64
-        and qkvg.is_contiguous()
-    )
+    return _ext.use_kernels(qkvg) and qkvg.dtype == torch.bfloat16 and D in (64, 128) and T > 1 and qkvg.is_contiguous()
 
 
 def gla_attention_core(qkvg, cos, sin, init, B, T, H):
-    ch = cos[:, :32].float().contiguous() if cos is not None else None
-    sh = sin[:, :32].float().contiguous() if sin is not None else None
+    D = qkvg.shape[1] // (4 * H)
+    ch = cos[:, : D // 2].float().contiguous() if cos is not None else None
+    sh = sin[:, : D // 2].float().contiguous() if sin is not None else None
+    if init is not None and init.shape != (B, H, D, D):
+        init = init.expand(B, H, D, D)  # one state for every sequence
     return _GLACoreFn.apply(qkvg, ch, sh, init, B, T, H)
