@@ -190,3 +190,35 @@ def test_fused_projection_rows_match_separate_tensors(T, D):
     want = torch.autograd.grad((oo.reshape(B * T, H * D).float() * w).sum() + ss.sum(), (x, s0))
     assert torch.equal(o, oo.reshape(B * T, H * D)) and torch.equal(s, ss)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (1, 2048), (7, 264), (37, 1536), (1185, 384), (1184, 776), (2375, 2040), (9480, 512), (5000, 1032)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norm_rows_against_fp64(rows, d, residual):
+    from triune_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(rows + d)
+    x, r, dy, ds = (torch.randn(rows, d, device="cuda", generator=g).bfloat16().requires_grad_(i < 2) for i in range(4))
+    w = (1 + 0.1 * torch.randn(d, device="cuda", generator=g)).bfloat16().requires_grad_(True)
+    if residual:
+        outs, seeds = ops.add_rmsnorm(x, r, w, 1e-6), (dy, ds)
+    else:
+        outs, seeds = (ops.rmsnorm(x, w, 1e-6),), (dy,)
+    got = torch.autograd.grad(outs, (x, w), seeds)
+    s = (x.detach() + r.detach() if residual else x.detach()).double().requires_grad_(True)
+    w64 = w.detach().double().requires_grad_(True)
+    y = s * torch.rsqrt(s.pow(2).mean(-1, keepdim=True) + 1e-6) * w64
+    want = torch.autograd.grad((y, s * 1.0) if residual else (y,), (s, w64), tuple(t.double() for t in seeds))
+    for a, b in zip((*outs, *got), (y, *((s,) if residual else ()), *want)):
+        assert _rel(a, b) < 2.0 ** -8  # fp32 sums, results rounded to bf16: at most 2^-9 each
+
+
+def test_weight_gradients_add_to_an_fp32_arena():
+    from triune_b200 import ops
+
+    x = torch.randn(700, 384, device="cuda").bfloat16().requires_grad_(True)
+    w = torch.ones(384, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    plain, = torch.autograd.grad(ops.rmsnorm(x, w).float().square().sum(), w)
+    w.main_grad = torch.full((384,), 3.0, device="cuda")
+    ops.rmsnorm(x, w).float().square().sum().backward()
+    assert w.grad is None and _rel(w.main_grad - 3.0, plain) < 2.0 ** -8

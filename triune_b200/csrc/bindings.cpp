@@ -49,20 +49,32 @@ std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& re
   return {y, rstd, has_res ? sum_out : Tensor()};
 }
 
+// Where a gradient's column sums go: into `into` (fp32, added), or a new tensor, bf16 on request and else fp32.
+tb::ColumnSum column_sum(const c10::optional<Tensor>& into, bool bf16, int64_t n, const Tensor& like, Tensor& res) {
+  const bool add = into.has_value() && into->defined();
+  if (add)
+    TORCH_CHECK(into->is_cuda() && into->scalar_type() == at::kFloat && into->is_contiguous() && into->numel() == n, "out must be fp32 [N]");
+  res = add ? *into : torch::empty({n}, like.options().dtype(bf16 ? at::kBFloat16 : at::kFloat));
+  if (!add && bf16) return {nullptr, bfm(res), false};
+  return {res.data_ptr<float>(), nullptr, add};
+}
+
+// Returns (dx, dw): dw as column_sum says.
 std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& dy, const Tensor& rstd,
-                                const c10::optional<Tensor>& dres) {
+                                const c10::optional<Tensor>& dres, const c10::optional<Tensor>& dw_into, bool dw_bf16) {
   check_bf16_cuda(x, "x");
   check_bf16_cuda(w, "w");
   const int d = (int)x.size(-1);
   const int rows = (int)(x.numel() / d);
   c10::cuda::CUDAGuard guard(x.device());
-  Tensor dx = torch::empty_like(x);
-  Tensor dw = torch::zeros({d}, x.options().dtype(at::kFloat));
+  Tensor dx = torch::empty_like(x), dw;
+  const tb::ColumnSum to = column_sum(dw_into, dw_bf16, d, x, dw);
+  Tensor partial = torch::empty({tb::rmsnorm_bwd_parts(rows, d), d}, x.options().dtype(at::kFloat));
   Tensor dyc = dy.contiguous();
   const bool has = dres.has_value() && dres->defined();
   Tensor drc = has ? dres->contiguous() : Tensor();
   tb::launch_rmsnorm_bwd(bf(x), bf(w), bf(dyc), rstd.data_ptr<float>(), has ? bf(drc) : nullptr, bfm(dx),
-                         dw.data_ptr<float>(), rows, d, cur_stream());
+                         partial.data_ptr<float>(), to, rows, d, cur_stream());
   return {dx, dw};
 }
 
@@ -188,21 +200,19 @@ Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, int64_t ignore_index, d
   return loss;
 }
 
-// Column sums of a bf16 [M, N] matrix in fp32: returns a new [N] tensor, or adds into `out` when given.
-Tensor colsum(const Tensor& x, const c10::optional<Tensor>& out) {
+// Column sums of a bf16 [M, N] matrix in fp32: returns a new [N] tensor (rounded to bf16 on request), or adds into `out`.
+Tensor colsum(const Tensor& x, const c10::optional<Tensor>& out, bool bf16) {
   check_bf16_cuda(x, "x");
   TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && x.size(1) % 8 == 0 && x.stride(0) % 8 == 0,
               "x must be [M, N] with N and the row pitch multiples of 8");
   TORCH_CHECK((reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0, "x must be 16-byte aligned");
   c10::cuda::CUDAGuard guard(x.device());
   const int M = (int)x.size(0), N = (int)x.size(1);
-  const bool acc = out.has_value() && out->defined();
-  if (acc)
-    TORCH_CHECK(out->scalar_type() == at::kFloat && out->is_contiguous() && out->numel() == N, "out must be fp32 [N]");
-  Tensor res = acc ? *out : torch::empty({N}, x.options().dtype(at::kFloat));
+  Tensor res;
+  const tb::ColumnSum to = column_sum(out, bf16, N, x, res);
   const int parts = tb::colsum_parts(M, N);
   Tensor partial = torch::empty({parts, N}, x.options().dtype(at::kFloat));
-  tb::launch_colsum(bf(x), x.stride(0), M, N, partial.data_ptr<float>(), parts, res.data_ptr<float>(), acc, cur_stream());
+  tb::launch_colsum(bf(x), x.stride(0), M, N, partial.data_ptr<float>(), parts, to, cur_stream());
   return res;
 }
 
@@ -423,7 +433,8 @@ void register_comm(pybind11::module& m);
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   register_gemm(m);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("rmsnorm_bwd", &rmsnorm_bwd, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("dy"), pybind11::arg("rstd"),
+        pybind11::arg("dres"), pybind11::arg("dw_into") = pybind11::none(), pybind11::arg("dw_bf16") = false);
   m.def("qk_prep_fwd", &qk_prep_fwd);
   m.def("qk_prep_bwd", &qk_prep_bwd);
   m.def("ce_fwd_bwd", &ce_fwd_bwd);
@@ -432,7 +443,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("rope_apply", &rope_apply);
   m.def("embedding_bwd", &embedding_bwd);
-  m.def("colsum", &colsum);
+  m.def("colsum", &colsum, pybind11::arg("x"), pybind11::arg("out"), pybind11::arg("bf16") = false);
   m.def("gather_rows", &gather_rows);
   m.def("combine_rows", &combine_rows);
   m.def("index_error_word", &index_error_word, "first out-of-table index seen by the row-movement kernels: [kernel, row, index, limit]");

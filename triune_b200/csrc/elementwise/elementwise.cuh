@@ -11,14 +11,20 @@ namespace tb {
 // y = rmsnorm(x [+ res]) * w ; if res != null also writes sum_out = x + res. d % 8 == 0, d <= 2048.
 void launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
                         __nv_bfloat16* sum_out, float* rstd, int rows, int d, float eps, cudaStream_t s);
-// dx = d(rmsnorm)/dx * dy [+ dres]; dw (fp32, pre-zeroed or accumulating) += sum_rows dy * xhat.
+// Where column sums go: fp32 (added to what is there with `add`), or bf16.
+struct ColumnSum {
+  float* out;
+  __nv_bfloat16* out16;
+  bool add;
+};
+int rmsnorm_bwd_parts(int rows, int d);
+// dx = d(rmsnorm)/dx * dy [+ dres]; dw = sum_rows dy * xhat. `partial` holds rmsnorm_bwd_parts(rows, d) x d floats.
 void launch_rmsnorm_bwd(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* dy, const float* rstd,
-                        const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw, int rows, int d, cudaStream_t s);
+                        const __nv_bfloat16* dres, __nv_bfloat16* dx, float* partial, const ColumnSum& dw, int rows, int d, cudaStream_t s);
 
-// out[n] (+)= sum over rows of x[m, n] (bf16 in, fp32 out); `partial` holds colsum_parts(M, N) x N floats.
+// out[n] (+)= sum over rows of x[m, n] (bf16 in, fp32 sums); `partial` holds colsum_parts(M, N) x N floats.
 int colsum_parts(int M, int N);
-void launch_colsum(const __nv_bfloat16* x, long long ld, int M, int N, float* partial, int parts, float* out,
-                   bool accumulate, cudaStream_t s);
+void launch_colsum(const __nv_bfloat16* x, long long ld, int M, int N, float* partial, int parts, const ColumnSum& out, cudaStream_t s);
 
 void launch_qk_prep_fwd(const __nv_bfloat16* in, long long in_ld, int k_col_offset, __nv_bfloat16* out, const float* cs,
                         const float* sn, long long tokens, int T, int H, int D, cudaStream_t s);

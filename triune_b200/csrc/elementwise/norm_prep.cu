@@ -16,10 +16,24 @@ namespace tb {
 
 namespace {
 
+constexpr int NORM_PARTS = 148 * 2;  // blocks of the backward kernel: two per SM are resident
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+__device__ __forceinline__ void unpack_row8(const uint4& u, float (&f)[8]) {
+  const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(x[i] << 16);
+    f[2 * i + 1] = __uint_as_float(x[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ uint4 pack_row8(const float (&f)[8]) {
+  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
 }
 
 // Each lane holds up to MAXV 8-element vectors of its row (d <= 32*8*MAXV); MAXV is a template parameter so
@@ -95,93 +109,186 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
   }
 }
 
-// dx = rstd * (w*dy - xhat * mean(w*dy*xhat)) [+ dres_in]; dw += sum_rows dy * xhat (fp32 atomics,
-// one atomic per column per block after an in-block reduction).
-template <bool HAS_DRES, int MAXV>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                          const __nv_bfloat16* __restrict__ w,
-                                                          const __nv_bfloat16* __restrict__ dy,
-                                                          const float* __restrict__ rstd,
-                                                          const __nv_bfloat16* __restrict__ dres,
-                                                          __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
-                                                          int rows, int d) {
-  extern __shared__ float dw_smem[];  // [d]
-  const int warps_per_block = blockDim.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nvec = d >> 3;
-  for (int i = threadIdx.x; i < d; i += blockDim.x) dw_smem[i] = 0.f;
-  __syncthreads();
-  float dwacc[MAXV][8];
+// The same with a row spread over the warps of a block, eight columns a thread and R rows in flight, for rows wider than 512
+// (a warp that holds 1536 columns has little else in flight) and for few rows (decoding: one row is a chain of latencies, and a
+// warp alone walks eight loads before it can sum). Measured against the kernel above, with the residual: NUMBERS_FWD
+// `wpr` warps per row; the block's warps / wpr rows side by side.
+template <bool HAS_RES, int R>
+__global__ void __launch_bounds__(256) rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
+                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                                               __nv_bfloat16* __restrict__ sum_out, float* __restrict__ rstd, int rows,
+                                                               int d, float eps, int wpr) {
+  __shared__ float red[2][8][R];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slots = (blockDim.x >> 5) / wpr;
+  const int slot = warp / wpr, col = ((warp % wpr) * 32 + lane) * 8;
+  const bool live = col < d;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const uint4 wv = live ? *reinterpret_cast<const uint4*>(w + col) : zero;
+  int buf = 0;
+  for (long long base = (long long)blockIdx.x * slots * R; base < rows; base += (long long)gridDim.x * slots * R, buf ^= 1) {
+    const long long row0 = base + slot * R;
+    uint4 xv[R];
+    float ss[R];
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i)
+    for (int i = 0; i < R; ++i) xv[i] = (live && row0 + i < rows) ? *reinterpret_cast<const uint4*>(x + (row0 + i) * d + col) : zero;
+    if (HAS_RES) {
+      uint4 rv[R];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
+      for (int i = 0; i < R; ++i) rv[i] = (live && row0 + i < rows) ? *reinterpret_cast<const uint4*>(res + (row0 + i) * d + col) : zero;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        float a[8], b[8];
+        unpack_row8(xv[i], a);
+        unpack_row8(rv[i], b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] += b[j];
+        xv[i] = pack_row8(a);
+        if (live && row0 + i < rows) *reinterpret_cast<uint4*>(sum_out + (row0 + i) * d + col) = xv[i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float a[8];
+      unpack_row8(xv[i], a);
+      ss[i] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss[i] += a[j] * a[j];
+      ss[i] = warp_sum(ss[i]);
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) red[buf][warp][i] = ss[i];
+    }
+    __syncthreads();  // the other buffer's readers are past the barrier before this one
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float sum = 0.f;
+      for (int p = 0; p < wpr; ++p) sum += red[buf][slot * wpr + p][i];
+      const float inv = rsqrtf(sum / (float)d + eps);
+      if (row0 + i < rows) {
+        if (rstd && warp % wpr == 0 && lane == 0) rstd[row0 + i] = inv;
+        if (live) {
+          float a[8], wf[8];
+          unpack_row8(xv[i], a);
+          unpack_row8(wv, wf);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) a[j] = a[j] * inv * wf[j];
+          *reinterpret_cast<uint4*>(y + (row0 + i) * d + col) = pack_row8(a);
+        }
+      }
+    }
+  }
+}
 
-  for (long long row = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < rows;
-       row += (long long)gridDim.x * warps_per_block) {
-    const float inv = rstd[row];
-    float xh[MAXV][8], wdy[MAXV][8];
-    float dot = 0.f;
+// dx = rstd * (w*dy - xhat * mean(w*dy*xhat)) [+ dres_in]; partial[block][d] = the block's sum over rows of dy * xhat.
+// Eight columns a thread, a row spread over `wpr` warps, R rows in flight. One warp per row before, with the row, its gradient
+// and the weight gradient's sums in 220 registers and one block per 64 rows, was bound by latency; so were the atomics at its
+// end. With the sum over blocks, the residual's gradient and the conversion of dw, cold: 8192 x 2048 101 -> 46 us (2.9 TB/s),
+// 8192 x 1536 81 -> 43, 16384 x 512 40 -> 32, 32768 x 384 47 -> 43; in a replayed graph 2331 x 2048 44 -> 11.6, 600 x 384 14.6 -> 5.9.
+template <bool HAS_DRES, int R>
+__global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                             const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd,
+                                                             const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                                                             float* __restrict__ partial, int rows, int d, int wpr) {
+  __shared__ float red[2][8][R];
+  __shared__ float cols[8][256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slots = (blockDim.x >> 5) / wpr;
+  const int slot = warp / wpr, col = ((warp % wpr) * 32 + lane) * 8;
+  const bool live = col < d;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  float wf[8], dw[8];
+  unpack_row8(live ? *reinterpret_cast<const uint4*>(w + col) : zero, wf);
 #pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = lane + i * 32;
-      if (v < nvec) {
-        uint4 xv = reinterpret_cast<const uint4*>(x + row * d)[v];
-        uint4 gv = reinterpret_cast<const uint4*>(dy + row * d)[v];
-        uint4 wv = reinterpret_cast<const uint4*>(w)[v];
-        const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&xv);
-        const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gv);
-        const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wv);
+  for (int j = 0; j < 8; ++j) dw[j] = 0.f;
+  int buf = 0;
+  for (long long base = (long long)blockIdx.x * slots * R; base < rows; base += (long long)gridDim.x * slots * R, buf ^= 1) {
+    const long long row0 = base + slot * R;
+    uint4 xv[R], gv[R], rv[R];
+    float inv[R], dot[R];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 xf = __bfloat1622float2(x2[j]), gf = __bfloat1622float2(g2[j]), wf = __bfloat1622float2(w2[j]);
-          xh[i][2 * j] = xf.x * inv;
-          xh[i][2 * j + 1] = xf.y * inv;
-          wdy[i][2 * j] = gf.x * wf.x;
-          wdy[i][2 * j + 1] = gf.y * wf.y;
-          dwacc[i][2 * j] += gf.x * xh[i][2 * j];
-          dwacc[i][2 * j + 1] += gf.y * xh[i][2 * j + 1];
-          dot += wdy[i][2 * j] * xh[i][2 * j] + wdy[i][2 * j + 1] * xh[i][2 * j + 1];
-        }
-      }
+    for (int i = 0; i < R; ++i) {
+      const bool in = row0 + i < rows;
+      const long long at = (row0 + i) * d + col;
+      inv[i] = in ? rstd[row0 + i] : 0.f;
+      xv[i] = (live && in) ? *reinterpret_cast<const uint4*>(x + at) : zero;
+      gv[i] = (live && in) ? *reinterpret_cast<const uint4*>(dy + at) : zero;
+      if (HAS_DRES) rv[i] = (live && in) ? *reinterpret_cast<const uint4*>(dres + at) : zero;
     }
-    dot = warp_sum(dot) / (float)d;
 #pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = lane + i * 32;
-      if (v < nvec) {
-        float o[8];
+    for (int i = 0; i < R; ++i) {
+      float a[8], g[8];
+      unpack_row8(xv[i], a);
+      unpack_row8(gv[i], g);
+      dot[i] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = inv * (wdy[i][j] - xh[i][j] * dot);
+      for (int j = 0; j < 8; ++j) {
+        const float gx = g[j] * (a[j] * inv[i]);
+        dw[j] += gx;
+        dot[i] += gx * wf[j];
+      }
+      dot[i] = warp_sum(dot[i]);
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) red[buf][warp][i] = dot[i];
+    }
+    __syncthreads();  // the other buffer's readers are past the barrier before this one
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float sum = 0.f;
+      for (int p = 0; p < wpr; ++p) sum += red[buf][slot * wpr + p][i];
+      sum /= (float)d;
+      if (live && row0 + i < rows) {
+        float a[8], g[8];
+        unpack_row8(xv[i], a);
+        unpack_row8(gv[i], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = inv[i] * (g[j] * wf[j] - a[j] * inv[i] * sum);
         if (HAS_DRES) {
-          uint4 rv = reinterpret_cast<const uint4*>(dres + row * d)[v];
-          const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
+          float r[8];
+          unpack_row8(rv[i], r);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float2 rf = __bfloat1622float2(r2[j]);
-            o[2 * j] += rf.x;
-            o[2 * j + 1] += rf.y;
-          }
+          for (int j = 0; j < 8; ++j) a[j] += r[j];
         }
-        uint4 ov;
-        ov.x = pack_bf16x2(o[0], o[1]);
-        ov.y = pack_bf16x2(o[2], o[3]);
-        ov.z = pack_bf16x2(o[4], o[5]);
-        ov.w = pack_bf16x2(o[6], o[7]);
-        reinterpret_cast<uint4*>(dx + row * d)[v] = ov;
+        *reinterpret_cast<uint4*>(dx + (row0 + i) * d + col) = pack_row8(a);
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int v = lane + i * 32;
-    if (v < nvec) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) atomicAdd(&dw_smem[v * 8 + j], dwacc[i][j]);
-    }
-  }
+  for (int j = 0; j < 8; ++j) cols[warp][j * 32 + lane] = dw[j];
   __syncthreads();
-  for (int i = threadIdx.x; i < d; i += blockDim.x) atomicAdd(&dw[i], dw_smem[i]);
+  if (slot == 0 && live) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float sum = dw[j];
+      for (int o = 1; o < slots; ++o) sum += cols[warp + o * wpr][j * 32 + lane];
+      dw[j] = sum;
+    }
+    float4* out = reinterpret_cast<float4*>(partial + (long long)blockIdx.x * d + col);
+    out[0] = make_float4(dw[0], dw[1], dw[2], dw[3]);
+    out[1] = make_float4(dw[4], dw[5], dw[6], dw[7]);
+  }
+}
+
+// Sums `parts` partial rows of N columns in a fixed order: 32 columns a block, eight groups of rows (one thread per column over all
+// parts took 10 us for 296 x 384; now 2.5). Writes fp32 (added to what is there with `accumulate`) or bf16.
+__global__ void __launch_bounds__(256) column_parts_kernel(const float* __restrict__ partial, int parts, int N, float* __restrict__ out,
+                                                           __nv_bfloat16* __restrict__ out16, int accumulate) {
+  __shared__ float red[8][33];
+  const int group = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (c < N) {
+#pragma unroll 8
+    for (int p = group; p < parts; p += 8) s += partial[(long long)p * N + c];
+  }
+  red[group][lane] = s;
+  __syncthreads();
+  if (group == 0 && c < N) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) s += red[i][lane];
+    if (out16 != nullptr) out16[c] = __float2bfloat16(s);
+    else out[c] = accumulate ? out[c] + s : s;
+  }
 }
 
 // ---------------------------------------------------------------- q/k feature map + RoPE
@@ -331,23 +438,42 @@ inline int row_grid(long long work_items, int per_block) {
 }
 
 
-template <int MAXV>
-void rmsnorm_fwd_dispatch(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
-                          __nv_bfloat16* sum_out, float* rstd, int rows, int d, float eps, int grid, cudaStream_t s) {
-  if (res)
-    rmsnorm_fwd_kernel<true, MAXV><<<grid, 256, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps);
-  else
-    rmsnorm_fwd_kernel<false, MAXV><<<grid, 256, 0, s>>>(x, nullptr, w, y, nullptr, rstd, rows, d, eps);
+// Warps per row and threads of a block of whole rows, rows in flight, blocks (at most `cap`) of the kernels that spread a row.
+struct WideGeom {
+  int wpr, threads, blocks;
+  bool four;  // four rows in flight, where that leaves every SM two blocks; else one
+};
+WideGeom wide_geom(int rows, int d, int cap) {
+  WideGeom g;
+  g.wpr = (d + 255) / 256;
+  const int slots = 8 / g.wpr;
+  g.threads = slots * g.wpr * 32;
+  g.four = rows >= 148 * 2 * slots * 4;
+  const int per = slots * (g.four ? 4 : 1), need = (rows + per - 1) / per;
+  g.blocks = need < cap ? need : cap;
+  return g;
 }
 
-template <int MAXV>
-void rmsnorm_bwd_dispatch(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* dy, const float* rstd,
-                          const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw, int rows, int d, int grid,
-                          cudaStream_t s) {
-  if (dres)
-    rmsnorm_bwd_kernel<true, MAXV><<<grid, 256, d * sizeof(float), s>>>(x, w, dy, rstd, dres, dx, dw, rows, d);
-  else
-    rmsnorm_bwd_kernel<false, MAXV><<<grid, 256, d * sizeof(float), s>>>(x, w, dy, rstd, nullptr, dx, dw, rows, d);
+template <bool HAS_RES>
+void rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y, __nv_bfloat16* sum_out,
+                 float* rstd, int rows, int d, float eps, cudaStream_t s) {
+  if (rows > 148 * 8 && d <= (HAS_RES ? 512 : 1024)) {
+    const int grid = row_grid(rows, 8);
+    if (d <= 512) rmsnorm_fwd_kernel<HAS_RES, 2><<<grid, 256, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps);
+    else if constexpr (!HAS_RES) rmsnorm_fwd_kernel<false, 4><<<grid, 256, 0, s>>>(x, nullptr, w, y, nullptr, rstd, rows, d, eps);
+    return;
+  }
+  const WideGeom g = wide_geom(rows, d, 148 * 8);
+  if (g.four) rmsnorm_fwd_wide_kernel<HAS_RES, 4><<<g.blocks, g.threads, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps, g.wpr);
+  else rmsnorm_fwd_wide_kernel<HAS_RES, 1><<<g.blocks, g.threads, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps, g.wpr);
+}
+
+template <bool HAS_DRES>
+void rmsnorm_bwd(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* dy, const float* rstd, const __nv_bfloat16* dres,
+                 __nv_bfloat16* dx, float* partial, int rows, int d, cudaStream_t s) {
+  const WideGeom g = wide_geom(rows, d, NORM_PARTS);
+  if (g.four) rmsnorm_bwd_kernel<HAS_DRES, 4><<<g.blocks, g.threads, 0, s>>>(x, w, dy, rstd, dres, dx, partial, rows, d, g.wpr);
+  else rmsnorm_bwd_kernel<HAS_DRES, 1><<<g.blocks, g.threads, 0, s>>>(x, w, dy, rstd, dres, dx, partial, rows, d, g.wpr);
 }
 
 }  // namespace
@@ -355,21 +481,20 @@ void rmsnorm_bwd_dispatch(const __nv_bfloat16* x, const __nv_bfloat16* w, const 
 void launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
                         __nv_bfloat16* sum_out, float* rstd, int rows, int d, float eps, cudaStream_t s) {
   if (rows == 0) return;
-  const int grid = row_grid(rows, 8);
-  if (d <= 512) rmsnorm_fwd_dispatch<2>(x, res, w, y, sum_out, rstd, rows, d, eps, grid, s);
-  else if (d <= 1024) rmsnorm_fwd_dispatch<4>(x, res, w, y, sum_out, rstd, rows, d, eps, grid, s);
-  else rmsnorm_fwd_dispatch<8>(x, res, w, y, sum_out, rstd, rows, d, eps, grid, s);
+  if (res != nullptr) rmsnorm_fwd<true>(x, res, w, y, sum_out, rstd, rows, d, eps, s);
+  else rmsnorm_fwd<false>(x, nullptr, w, y, nullptr, rstd, rows, d, eps, s);
 }
 
+int rmsnorm_bwd_parts(int rows, int d) { return wide_geom(rows, d, NORM_PARTS).blocks; }
+
 void launch_rmsnorm_bwd(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* dy, const float* rstd,
-                        const __nv_bfloat16* dres, __nv_bfloat16* dx, float* dw, int rows, int d, cudaStream_t s) {
-  if (rows == 0) return;
-  // few, fat blocks: every block ends with d global atomics into dw, so the block count bounds the contention
-  long long b = ((long long)rows + 8 * 8 - 1) / (8 * 8);
-  const int grid = (int)(b < 1 ? 1 : (b > 148 * 3 ? 148 * 3 : b));
-  if (d <= 512) rmsnorm_bwd_dispatch<2>(x, w, dy, rstd, dres, dx, dw, rows, d, grid, s);
-  else if (d <= 1024) rmsnorm_bwd_dispatch<4>(x, w, dy, rstd, dres, dx, dw, rows, d, grid, s);
-  else rmsnorm_bwd_dispatch<8>(x, w, dy, rstd, dres, dx, dw, rows, d, grid, s);
+                        const __nv_bfloat16* dres, __nv_bfloat16* dx, float* partial, const ColumnSum& dw, int rows, int d,
+                        cudaStream_t s) {
+  if (rows > 0) {
+    if (dres != nullptr) rmsnorm_bwd<true>(x, w, dy, rstd, dres, dx, partial, rows, d, s);
+    else rmsnorm_bwd<false>(x, w, dy, rstd, nullptr, dx, partial, rows, d, s);
+  }
+  column_parts_kernel<<<(d + 31) / 32, 256, 0, s>>>(partial, rows > 0 ? rmsnorm_bwd_parts(rows, d) : 0, d, dw.out, dw.out16, dw.add ? 1 : 0);
 }
 
 void launch_qk_prep_fwd(const __nv_bfloat16* in, long long in_ld, int k_col_offset, __nv_bfloat16* out, const float* cs,
@@ -411,6 +536,7 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
   if (col < N) {
+#pragma unroll 4
     for (int m = blockIdx.y * 8 + warp; m < M; m += gridDim.y * 8) {
       const uint4 u = *reinterpret_cast<const uint4*>(x + (long long)m * ld + col);
       const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
@@ -434,15 +560,6 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
   }
 }
 
-__global__ void colsum_finalize_kernel(const float* __restrict__ partial, int parts, int N, float* __restrict__ out,
-                                       int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
-  float s = 0.f;
-  for (int p = 0; p < parts; ++p) s += partial[(long long)p * N + c];
-  out[c] = accumulate ? out[c] + s : s;
-}
-
 }  // namespace
 
 int colsum_parts(int M, int N) {
@@ -453,11 +570,11 @@ int colsum_parts(int M, int N) {
   return parts < 1 ? 1 : parts;
 }
 
-void launch_colsum(const __nv_bfloat16* x, long long ld, int M, int N, float* partial, int parts, float* out,
-                   bool accumulate, cudaStream_t s) {
+void launch_colsum(const __nv_bfloat16* x, long long ld, int M, int N, float* partial, int parts,
+                   const ColumnSum& out, cudaStream_t s) {
   dim3 grid((N + 255) / 256, parts);
   colsum_partial_kernel<<<grid, 256, 0, s>>>(x, ld, M, N, partial);
-  colsum_finalize_kernel<<<(N + 255) / 256, 256, 0, s>>>(partial, parts, N, out, accumulate ? 1 : 0);
+  column_parts_kernel<<<(N + 31) / 32, 256, 0, s>>>(partial, parts, N, out.out, out.out16, out.add ? 1 : 0);
 }
 
 }  // namespace tb

@@ -141,7 +141,7 @@ def _accumulate_bias_grad(b: Optional[torch.Tensor], dy2: torch.Tensor):
             mg.add_(dy2.sum(0, dtype=torch.float32))
         return None
     if fast:
-        db = _ext.ext().colsum(dy2, None)
+        db = _ext.ext().colsum(dy2, None, b.dtype == torch.bfloat16)
         _tick(2)
         return db.to(b.dtype)
     return dy2.sum(0, dtype=torch.float32).to(b.dtype)
@@ -333,6 +333,21 @@ def swiglu_mlp(x, w13, w2):
 # ----------------------------------------------------------------------------
 # RMSNorm
 # ----------------------------------------------------------------------------
+def _rmsnorm_bwd(x, w, dy, rstd, dres):
+    """(dx, dw); the weight's gradient goes into its ``main_grad`` where it has one (then None)."""
+    mg = getattr(w, "main_grad", None)
+    if mg is None:
+        dx, dw = _ext.ext().rmsnorm_bwd(x, w, dy, rstd, dres, None, w.dtype == torch.bfloat16)
+        _tick(2)
+        return dx, dw.to(w.dtype)
+    into = mg if mg.is_cuda and mg.dtype == torch.float32 and mg.is_contiguous() else None
+    dx, dw = _ext.ext().rmsnorm_bwd(x, w, dy, rstd, dres, into)
+    _tick(2)
+    if into is None:
+        mg.add_(dw)
+    return dx, None
+
+
 class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps):
@@ -345,14 +360,7 @@ class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd = ctx.saved_tensors
-        dx, dw = _ext.ext().rmsnorm_bwd(x, w, dy, rstd, None)
-        _tick()
-        mg = getattr(w, "main_grad", None)
-        if mg is not None:
-            mg.add_(dw)
-            dw = None
-        else:
-            dw = dw.to(w.dtype)
+        dx, dw = _rmsnorm_bwd(x, w, dy, rstd, None)
         return dx, dw, None
 
 
@@ -371,14 +379,7 @@ class _AddRMSNormFn(torch.autograd.Function):
         s, w, rstd = ctx.saved_tensors
         if dy is None:
             dy = torch.zeros_like(s)
-        dx, dw = _ext.ext().rmsnorm_bwd(s, w, dy, rstd, ds)
-        _tick()
-        mg = getattr(w, "main_grad", None)
-        if mg is not None:
-            mg.add_(dw)
-            dw = None
-        else:
-            dw = dw.to(w.dtype)
+        dx, dw = _rmsnorm_bwd(s, w, dy, rstd, ds)
         return dx, dx, dw, None
 
 
