@@ -325,6 +325,15 @@ def swiglu_mlp(x, w13, w2):
     H = w13.shape[0] // 2
     if (_ext.use_kernels(x, w13, w2) and x.dtype == torch.bfloat16 and H % 32 == 0 and w13.shape[1] % 8 == 0
             and w2.shape[0] % 8 == 0 and w13.is_contiguous() and w2.is_contiguous()):
+        if not _wants_grad(x, w13, w2):
+            # inference: the pre-activations of the backward pass are not written, and few rows take the streaming product
+            x2 = x.reshape(-1, x.shape[-1])
+            if not _tma_ok(x2):
+                x2 = x2.contiguous()
+            h = torch.empty(x2.shape[0], H, device=x.device, dtype=x.dtype)
+            _ext.serving().tc_gemm_swiglu(x2, w13, h, None)
+            _tick()
+            return gemm(h, w2).view(*x.shape[:-1], w2.shape[0])
         return _SwiGLUMLPFn.apply(x, w13, w2)
     gu = F.linear(x, w13)
     return F.linear(ref.swiglu(gu[..., :H], gu[..., H:]), w2)
