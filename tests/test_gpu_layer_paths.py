@@ -222,3 +222,63 @@ def test_weight_gradients_add_to_an_fp32_arena():
     w.main_grad = torch.full((384,), 3.0, device="cuda")
     ops.rmsnorm(x, w).float().square().sum().backward()
     assert w.grad is None and _rel(w.main_grad - 3.0, plain) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T", [2, 63, 64, 65, 130])
+@pytest.mark.parametrize("with_beta", [False, True])
+def test_delta_rule_training_of_any_length_against_fp64(T, D, with_beta):
+    from triune_b200 import ops
+
+    B, H = 2, 3
+    q, k, v, g, s0 = _mixer_inputs(B, T, H, D, seed=T)
+    ins = [q, k, v, g, s0] + ([torch.rand(B, T, H, device="cuda")] if with_beta else [])
+    ins = [t.requires_grad_(True) for t in ins]
+    o, s = ops.gated_deltanet(*ins[:4], beta=ins[5] if with_beta else None, initial_state=ins[4], gate_logits=True)
+    wo, ws = torch.randn_like(o), torch.randn_like(s) * 0.1
+    got = (o, s, *torch.autograd.grad((o.float() * wo).sum() + (s * ws).sum(), ins))
+    x = [t.detach().double().requires_grad_(True) for t in ins]
+    gl = F.logsigmoid(x[3]).clamp(min=gla_cuda.GLA_MIN_LOG_DECAY)
+    oo, ss = ref.gated_deltanet_recurrent(*x[:3], gl, x[5] if with_beta else None, x[4])
+    want = (oo, ss, *torch.autograd.grad((oo * wo.double()).sum() + (ss * ws.double()).sum(), x))
+    # bf16 operands (2^-9 each) in the chunk's inverse, the effective values, states and scores: up to four products that follow
+    # one another, twice that backward; gate gradients add the errors of up to T later tokens
+    for n, a, b in zip(("o", "s", "dq", "dk", "dv", "dg", "ds0", "dbeta"), got, want):
+        limit = 2.0 ** -8 * (2 * T ** 0.5 + 8 if n == "dg" else 4 if n in ("o", "s") else 8)
+        assert _rel(a, b) < limit, (n, _rel(a, b))
+
+
+@pytest.mark.parametrize("T,D", [(21, 128), (150, 64), (128, 128)])
+def test_fused_delta_rule_rows_match_separate_tensors(T, D):
+    from triune_b200 import ops
+
+    B, H = 2, 2
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(B * T, 4 * H * D, device="cuda", generator=gen).bfloat16().requires_grad_(True)
+    beta = torch.rand(B * T, H, device="cuda", generator=gen).requires_grad_(True)
+    s0 = torch.randn(B, H, D, D, device="cuda", generator=gen).requires_grad_(True)
+    w = torch.randn(B * T, H * D, device="cuda", generator=gen)
+    cos, sin = ops.rope_tables(T + 3, D, 10000.0, 0, x.device)
+    cos, sin = cos[3:], sin[3:]
+    o, s = gla_cuda.gdn_attention_core(x, cos, sin, beta, s0, B, T, H)
+    got = torch.autograd.grad((o.float() * w).sum() + s.sum(), (x, beta, s0))
+    q, k, v, g = ops.qk_feature_map(x, cos, sin, B, T, H, D)
+    oo, ss = ops.gated_deltanet(q, k, v, g, beta=beta.view(B, T, H), initial_state=s0, gate_logits=True)
+    want = torch.autograd.grad((oo.reshape(B * T, H * D).float() * w).sum() + ss.sum(), (x, beta, s0))
+    assert torch.equal(o, oo.reshape(B * T, H * D)) and torch.equal(s, ss)
+    # dbeta sums a row's parts with shared-memory atomics: the order of fp32 additions may differ between runs
+    assert torch.equal(got[0], want[0]) and _rel(got[1], want[1]) < 1e-6 and torch.equal(got[2], want[2])
+
+
+@pytest.mark.parametrize("rows,dim,H", [(1, 8, 1), (15, 264, 6), (16, 384, 8), (33, 520, 9), (600, 2048, 16), (9000, 1024, 8)])
+def test_write_strengths_against_fp64(rows, dim, H):
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, dim, device="cuda", generator=gen).bfloat16().requires_grad_(True)
+    w = (torch.randn(H, dim, device="cuda", generator=gen) * dim ** -0.5).bfloat16().requires_grad_(True)
+    db = torch.randn(rows, H, device="cuda", generator=gen)
+    beta = gla_cuda.write_strength(x, w)
+    dx, dw = torch.autograd.grad(beta, (x, w), db)
+    x64, w64 = (t.detach().double().requires_grad_(True) for t in (x, w))
+    b64 = torch.sigmoid(x64 @ w64.t())
+    dx64, dw64 = torch.autograd.grad(b64, (x64, w64), db.double())
+    assert _rel(beta, b64) < 2e-6 and _rel(dx, dx64) < 2.0 ** -8 and _rel(dw, dw64) < 2.0 ** -8  # fp32 sums; bf16 gradients

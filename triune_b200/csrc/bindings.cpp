@@ -78,6 +78,16 @@ std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& 
   return {dx, dw};
 }
 
+// Row pitch of rotary tables: fp32 rows that the kernels read in 16-byte vectors.
+int table_pitch(const Tensor& cs, const Tensor& sn, int64_t T, int64_t D) {
+  for (const Tensor* t : {&cs, &sn})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 2 && t->stride(1) == 1 && t->stride(0) % 4 == 0 &&
+                    t->size(0) >= T && t->size(1) >= D / 2 && t->stride(0) == cs.stride(0) &&
+                    (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0,
+                "rotary tables: fp32 [T, D / 2] with 16-byte rows of one pitch");
+  return (int)cs.stride(0);
+}
+
 // in: [tokens, ld] with q at col 0 and k at col k_off; returns [tokens, 2, H, D].
 Tensor qk_prep_fwd(const Tensor& in, int64_t k_off, const c10::optional<Tensor>& cs, const c10::optional<Tensor>& sn,
                    int64_t T, int64_t H, int64_t D) {
@@ -89,7 +99,7 @@ Tensor qk_prep_fwd(const Tensor& in, int64_t k_off, const c10::optional<Tensor>&
   Tensor out = torch::empty({tokens, 2, H, D}, in.options());
   const bool rope = cs.has_value() && cs->defined();
   tb::launch_qk_prep_fwd(bf(in), in.stride(0), (int)k_off, bfm(out), rope ? cs->data_ptr<float>() : nullptr,
-                         rope ? sn->data_ptr<float>() : nullptr, tokens, (int)T, (int)H, (int)D, cur_stream());
+                         rope ? sn->data_ptr<float>() : nullptr, rope ? table_pitch(*cs, *sn, T, D) : 0, tokens, (int)T, (int)H, (int)D, cur_stream());
   return out;
 }
 
@@ -101,7 +111,7 @@ void qk_prep_bwd(const Tensor& in, int64_t k_off, const Tensor& dout, Tensor& d_
   c10::cuda::CUDAGuard guard(in.device());
   const bool rope = cs.has_value() && cs->defined();
   tb::launch_qk_prep_bwd(bf(in), in.stride(0), (int)k_off, bf(dout), bfm(d_in), d_in.stride(0),
-                         rope ? cs->data_ptr<float>() : nullptr, rope ? sn->data_ptr<float>() : nullptr, in.size(0),
+                         rope ? cs->data_ptr<float>() : nullptr, rope ? sn->data_ptr<float>() : nullptr, rope ? table_pitch(*cs, *sn, T, D) : 0, in.size(0),
                          (int)T, (int)H, (int)D, cur_stream());
 }
 

@@ -17,6 +17,8 @@ struct ColumnSum {
   __nv_bfloat16* out16;
   bool add;
 };
+// Sum of `parts` rows of N partial sums, in a fixed order.
+void launch_column_parts(const float* partial, int parts, int N, const ColumnSum& out, cudaStream_t s);
 int rmsnorm_bwd_parts(int rows, int d);
 // dx = d(rmsnorm)/dx * dy [+ dres]; dw = sum_rows dy * xhat. `partial` holds rmsnorm_bwd_parts(rows, d) x d floats.
 void launch_rmsnorm_bwd(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* dy, const float* rstd,
@@ -26,10 +28,11 @@ void launch_rmsnorm_bwd(const __nv_bfloat16* x, const __nv_bfloat16* w, const __
 int colsum_parts(int M, int N);
 void launch_colsum(const __nv_bfloat16* x, long long ld, int M, int N, float* partial, int parts, const ColumnSum& out, cudaStream_t s);
 
+// cs, sn: fp32 tables with rows of `table_ld` floats (a multiple of four, 16-byte aligned), D / 2 of each used, or null
 void launch_qk_prep_fwd(const __nv_bfloat16* in, long long in_ld, int k_col_offset, __nv_bfloat16* out, const float* cs,
-                        const float* sn, long long tokens, int T, int H, int D, cudaStream_t s);
+                        const float* sn, int table_ld, long long tokens, int T, int H, int D, cudaStream_t s);
 void launch_qk_prep_bwd(const __nv_bfloat16* in, long long in_ld, int k_col_offset, const __nv_bfloat16* dout,
-                        __nv_bfloat16* d_in, long long d_in_ld, const float* cs, const float* sn, long long tokens,
+                        __nv_bfloat16* d_in, long long d_in_ld, const float* cs, const float* sn, int table_ld, long long tokens,
                         int T, int H, int D, cudaStream_t s);
 
 // Row-wise cross entropy over bf16 logits [rows, V] (row stride ld). Writes per-row loss (0 for ignored

@@ -103,9 +103,10 @@ __device__ __forceinline__ bool phase_sync(GBars* bars) {
   return bars->failed == 0;
 }
 
-// bmat[t][d] (fp32, row pitch D + 4) = inclusive cumulative clamped log decay of the gate tiles (D / 64 tiles side by side).
+// bmat[t][d] (fp32, row pitch D + 4) = inclusive cumulative clamped log decay of the gate tiles (D / 64 tiles side by side). Rows
+// from `left` on are past the sequence's end: no decay there (and, the tiles being filled with zeros, no key and no value).
 template <int D>
-__device__ __forceinline__ void cumsum_d(const uint8_t* sG, float* bmat, bool logits) {
+__device__ __forceinline__ void cumsum_d(const uint8_t* sG, float* bmat, bool logits, int left) {
   constexpr int PARTS = GDN_THREADS / D, LEN = C / PARTS, BST = D + 4;
   __shared__ float totals[GDN_THREADS];
   const int tid = threadIdx.x, d = tid % D, part = tid / D;
@@ -117,7 +118,7 @@ __device__ __forceinline__ void cumsum_d(const uint8_t* sG, float* bmat, bool lo
   for (int i = 0; i < LEN; ++i) {
     const int r = part * LEN + i;
     const __nv_bfloat16 x = *reinterpret_cast<const __nv_bfloat16*>(tile + sw_off(r, dc >> 3) + (dc & 7) * 2);
-    run += log_decay(__bfloat162float(x), logits);
+    run += r < left ? log_decay(__bfloat162float(x), logits) : 0.f;
     c[i] = run;
   }
   totals[part * D + d] = run;
@@ -290,9 +291,10 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_wy_kernel(
   float* Lm = ftab + 16 * D;
   GBars* bars = reinterpret_cast<GBars*>(Lm + C * LP);
   const int tid = threadIdx.x;
-  const int NT = T / C;
+  const int NT = (T + C - 1) / C;
   const int cidx = blockIdx.x, chunk = cidx % NT, bh = cidx / NT, h = bh % H, b = bh / H;
-  const int row0 = b * T + chunk * C;
+  const int row0 = b * T + chunk * C, left = T - chunk * C;  // first row; rows of the sequence from there on
+  auto strength = [&](const float* be, int r) { return be == nullptr ? 1.f : (r < left ? be[(long long)(row0 + r) * H + h] : 0.f); };
 
   cta_setup(bars, 2, Cfg::TMEM_COLS);
   const uint32_t tmem = bars->tmem_slot;
@@ -300,9 +302,9 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_wy_kernel(
     mbar_expect_tx(&bars->tma, 3 * NH * TILE);
 #pragma unroll
     for (int n = 0; n < NH; ++n) {
-      tma_load_3d(sK + n * TILE, &tmK, &bars->tma, kcol + h * D + n * 64, row0, 0);
-      tma_load_3d(sV + n * TILE, &tmV, &bars->tma, vcol + h * D + n * 64, row0, 0);
-      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, row0, 0);
+      tma_load_3d(sK + n * TILE, &tmK, &bars->tma, kcol + h * D + n * 64, chunk * C, b);
+      tma_load_3d(sV + n * TILE, &tmV, &bars->tma, vcol + h * D + n * 64, chunk * C, b);
+      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, chunk * C, b);
     }
   }
   bool ok = wait_inputs(bars);
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_wy_kernel(
   // the first 2 * NH tiles with Kbar scaled in place.
   uint8_t* const kh[4] = {sR + 1 * NH * TILE, sR + 0 * NH * TILE, sR + 2 * NH * TILE, sR + 3 * NH * TILE};
   if (ok) {
-    cumsum_d<D>(sG, bmat, logits != 0);
+    cumsum_d<D>(sG, bmat, logits != 0, left);
     factor_tables_d<D>(bmat, ftab);
     build_row_operands<D, true>(sK, kh, bmat, ftab);
     build_key_operand<D>(sK, sKt, bmat);
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_wy_kernel(
       float v[32];
       load_acc_cols<32>(tmem, me.chalf * 32, me.quarter, v);
       if (me.active) {
-        const float bt = beta != nullptr ? beta[(long long)(row0 + me.row) * H + h] : 1.f;
+        const float bt = strength(beta, me.row);
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const int s = me.chalf * 32 + i;
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_wy_kernel(
       for (int idx = tid; idx < C * CH; idx += GDN_THREADS) {
         const int row = idx / CH, ch = idx % CH, half = ch >> 3, cc = ch & 7;
         const uint32_t off = half * TILE + sw_off(row, cc);
-        const float bt = beta != nullptr ? beta[(long long)(row0 + row) * H + h] : 1.f;
+        const float bt = strength(beta, row);
         float x[8];
         unpack8(*reinterpret_cast<const uint4*>(sV + off), x);
 #pragma unroll
@@ -688,9 +690,9 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_scores_kernel(
   float* ftab = bmat + C * BST;
   GBars* bars = reinterpret_cast<GBars*>(ftab + 16 * D);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int NT = T / C;
+  const int NT = (T + C - 1) / C;
   const int cidx = blockIdx.x, chunk = cidx % NT, bh = cidx / NT, h = bh % H, b = bh / H;
-  const int row0 = b * T + chunk * C;
+  const int row0 = b * T + chunk * C, left = T - chunk * C;  // first row; rows of the sequence from there on
 
   cta_setup(bars, 2, Cfg::TMEM_COLS);
   const uint32_t tmem = bars->tmem_slot;
@@ -698,13 +700,13 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_scores_kernel(
     mbar_expect_tx(&bars->tma, (4 * NH + (B1 ? 0 : NH * NH)) * TILE);
 #pragma unroll
     for (int n = 0; n < NH; ++n) {
-      tma_load_3d(sQ + n * TILE, &tmQ, &bars->tma, qcol + h * D + n * 64, row0, 0);
-      tma_load_3d(sK + n * TILE, &tmK, &bars->tma, kcol + h * D + n * 64, row0, 0);
-      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, row0, 0);
+      tma_load_3d(sQ + n * TILE, &tmQ, &bars->tma, qcol + h * D + n * 64, chunk * C, b);
+      tma_load_3d(sK + n * TILE, &tmK, &bars->tma, kcol + h * D + n * 64, chunk * C, b);
+      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, chunk * C, b);
       if (y_is_chunked)
         tma_load_3d(sY + n * TILE, &tmY, &bars->tma, n * 64, cidx * C, 0);
       else
-        tma_load_3d(sY + n * TILE, &tmY, &bars->tma, ycol + h * D + n * 64, row0, 0);
+        tma_load_3d(sY + n * TILE, &tmY, &bars->tma, ycol + h * D + n * 64, chunk * C, b);
     }
     if (!B1) {
 #pragma unroll
@@ -719,7 +721,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_scores_kernel(
   uint8_t* const qj[4] = {sA, sA + NH * TILE, sA + 2 * NH * TILE, sG};  // Q~(3) overwrites the gate tiles
   constexpr int COL_P = 0, COL_O = 64, COL_H = 64 + D;
   if (ok) {
-    cumsum_d<D>(sG, bmat, logits != 0);
+    cumsum_d<D>(sG, bmat, logits != 0, left);
     factor_tables_d<D>(bmat, ftab);
     build_row_operands<D, false>(sQ, qj, bmat, ftab);
     build_key_operand<D>(sK, sKt, bmat);
@@ -790,8 +792,10 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_scores_kernel(
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] *= scale;
             __nv_bfloat16* dst = out + (long long)(row0 + me.row) * out_ld + ocol + h * D + c0;
+            if (me.row < left) {
 #pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, v + c8 * 8);
+              for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, v + c8 * 8);
+            }
           }
         }
       }
@@ -862,9 +866,9 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_state_terms_kernel(
   float* bmat = reinterpret_cast<float*>(sdS + NH * SB);
   GBars* bars = reinterpret_cast<GBars*>(bmat + C * BST);
   const int tid = threadIdx.x;
-  const int NT = T / C;
+  const int NT = (T + C - 1) / C;
   const int cidx = blockIdx.x, chunk = cidx % NT, bh = cidx / NT, h = bh % H, b = bh / H;
-  const int row0 = b * T + chunk * C;
+  const int row0 = b * T + chunk * C, left = T - chunk * C;  // first row; rows of the sequence from there on
 
   cta_setup(bars, 1, Cfg::TMEM_COLS);
   const uint32_t tmem = bars->tmem_slot;
@@ -872,10 +876,10 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_state_terms_kernel(
     mbar_expect_tx(&bars->tma, (4 * NH + 2 * NH * NH) * TILE);
 #pragma unroll
     for (int n = 0; n < NH; ++n) {
-      tma_load_3d(sdO + n * TILE, &tmdO, &bars->tma, docol + h * D + n * 64, row0, 0);
+      tma_load_3d(sdO + n * TILE, &tmdO, &bars->tma, docol + h * D + n * 64, chunk * C, b);
       tma_load_3d(sU + n * TILE, &tmU, &bars->tma, n * 64, cidx * C, 0);
       tma_load_3d(sdU + n * TILE, &tmdU, &bars->tma, n * 64, cidx * C, 0);
-      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, row0, 0);
+      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, chunk * C, b);
       // states as K-major B operands: [dv half n][D key rows][64 value columns]
       tma_load_3d(sS + n * SB, &tmS, &bars->tma, n * 64, cidx * D, 0);
       tma_load_3d(sdS + n * SB, &tmdS, &bars->tma, n * 64, cidx * D, 0);
@@ -899,7 +903,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_state_terms_kernel(
         }
       umma_commit(&bars->mma[0]);
     }
-    cumsum_d<D>(sG, bmat, logits != 0);
+    cumsum_d<D>(sG, bmat, logits != 0, left);
     ok = wait_mma(bars, 0);
     if (ok) {
 #pragma unroll 1
@@ -979,9 +983,10 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_wy_kernel(
   float* dbs = bmat + C * BST;  // per-row dbeta partial sums
   GBars* bars = reinterpret_cast<GBars*>(dbs + C);
   const int tid = threadIdx.x;
-  const int NT = T / C;
+  const int NT = (T + C - 1) / C;
   const int cidx = blockIdx.x, chunk = cidx % NT, bh = cidx / NT, h = bh % H, b = bh / H;
-  const int row0 = b * T + chunk * C;
+  const int row0 = b * T + chunk * C, left = T - chunk * C;  // first row; rows of the sequence from there on
+  auto strength = [&](const float* be, int r) { return be == nullptr ? 1.f : (r < left ? be[(long long)(row0 + r) * H + h] : 0.f); };
 
   cta_setup(bars, 2, Cfg::TMEM_COLS);
   const uint32_t tmem = bars->tmem_slot;
@@ -994,9 +999,9 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_wy_kernel(
       tma_load_3d(sdUW + (NH + n) * TILE, &tmdW, &bars->tma, n * 64, cidx * C, 0);
       tma_load_3d(sU0 + n * TILE, &tmU0, &bars->tma, n * 64, cidx * C, 0);
       tma_load_3d(sW + n * TILE, &tmW, &bars->tma, n * 64, cidx * C, 0);
-      tma_load_3d(sV + n * TILE, &tmV, &bars->tma, vcol + h * D + n * 64, row0, 0);
-      tma_load_3d(sK + n * TILE, &tmK, &bars->tma, kcol + h * D + n * 64, row0, 0);
-      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, row0, 0);
+      tma_load_3d(sV + n * TILE, &tmV, &bars->tma, vcol + h * D + n * 64, chunk * C, b);
+      tma_load_3d(sK + n * TILE, &tmK, &bars->tma, kcol + h * D + n * 64, chunk * C, b);
+      tma_load_3d(sG + n * TILE, &tmG, &bars->tma, gcol + h * D + n * 64, chunk * C, b);
     }
   }
   bool ok = wait_inputs(bars);
@@ -1011,11 +1016,11 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_wy_kernel(
       umma_commit(&bars->mma[0]);
     }
     if (tid < C) dbs[tid] = 0.f;
-    cumsum_d<D>(sG, bmat, logits != 0);
+    cumsum_d<D>(sG, bmat, logits != 0, left);
     ok = wait_mma(bars, 0);
     if (ok) {
       // warps 0-3 (chalf 0) own the dVb row, warps 4-7 (chalf 1) the dKb row of their token s = me.row
-      const float bt = (me.active && beta != nullptr) ? beta[(long long)(row0 + me.row) * H + h] : 1.f;
+      const float bt = me.active ? strength(beta, me.row) : 1.f;
       float part = 0.f;
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
@@ -1037,8 +1042,10 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_wy_kernel(
               }
             }
             __nv_bfloat16* dst = dv + (long long)(row0 + me.row) * dv_ld + dvcol + h * D + c0;
+            if (me.row < left) {
 #pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, o + c8 * 8);
+              for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, o + c8 * 8);
+            }
             store_row_cols<32>(sdVb + half * TILE, me.row, cin, v, 1 << 30);
           } else {
             // dkr1 = beta e^{bp} dKb, <dKb, Kbar>
@@ -1095,7 +1102,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_wy_kernel(
       float v[32];
       load_acc_cols<32>(tmem, 2 * D + me.chalf * 32, me.quarter, v);
       if (me.active) {
-        const float bt = beta != nullptr ? beta[(long long)(row0 + me.row) * H + h] : 1.f;
+        const float bt = strength(beta, me.row);
         const float* lr = Lraw + ((long long)cidx * C + me.row) * C + me.chalf * 32;
         float part = 0.f, o[32];
 #pragma unroll
@@ -1113,7 +1120,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_wy_kernel(
     }
   }
   __syncthreads();
-  if (ok && dbeta != nullptr && tid < C) dbeta[(long long)(row0 + tid) * H + h] = dbs[tid];
+  if (ok && dbeta != nullptr && tid < C && tid < left) dbeta[(long long)(row0 + tid) * H + h] = dbs[tid];
   cta_teardown(bars, tmem, Cfg::TMEM_COLS, status);
 }
 
@@ -1161,23 +1168,23 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_scores_kernel(
   GBars* bars = reinterpret_cast<GBars*>(ftab + 16 * 64);
   static_assert(BST == LP, "the 64-wide decay matrix uses the common 68-float pitch");
   const int tid = threadIdx.x;
-  const int NT = T / C;
+  const int NT = (T + C - 1) / C;
   const int dh = blockIdx.x % NH, cidx = blockIdx.x / NH;
   const int chunk = cidx % NT, bh = cidx / NT, h = bh % H, b = bh / H;
-  const int row0 = b * T + chunk * C;
+  const int row0 = b * T + chunk * C, left = T - chunk * C;  // first row; rows of the sequence from there on
   const int dcol = h * D + dh * DH;  // first column of this slice inside a [rows, H * D] matrix
 
   cta_setup(bars, 3, 512);
   const uint32_t tmem = bars->tmem_slot;
   if (tid == 0) {
     mbar_expect_tx(&bars->tma, (4 + 2 * NH) * TILE);
-    tma_load_3d(sQ, &tmQ, &bars->tma, qcol + dcol, row0, 0);
-    tma_load_3d(sK, &tmK, &bars->tma, kcol + dcol, row0, 0);
-    tma_load_3d(sG, &tmG, &bars->tma, gcol + dcol, row0, 0);
+    tma_load_3d(sQ, &tmQ, &bars->tma, qcol + dcol, chunk * C, b);
+    tma_load_3d(sK, &tmK, &bars->tma, kcol + dcol, chunk * C, b);
+    tma_load_3d(sG, &tmG, &bars->tma, gcol + dcol, chunk * C, b);
     tma_load_3d(sdL, &tmdL, &bars->tma, 0, cidx * C, 0);
 #pragma unroll
     for (int n = 0; n < NH; ++n) {
-      tma_load_3d(sdO + n * TILE, &tmdO, &bars->tma, docol + h * D + n * 64, row0, 0);
+      tma_load_3d(sdO + n * TILE, &tmdO, &bars->tma, docol + h * D + n * 64, chunk * C, b);
       tma_load_3d(sU + n * TILE, &tmU, &bars->tma, n * 64, cidx * C, 0);
     }
   }
@@ -1198,7 +1205,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_scores_kernel(
           umma_bf16(tmem, desc_k(ado + n * TILE, k), desc_k(au + n * TILE, k), id, (n > 0 || k > 0) ? 1u : 0u);
       umma_commit(&bars->mma[0]);
     }
-    cumsum_d<64>(sG, bmat, logits != 0);
+    cumsum_d<64>(sG, bmat, logits != 0, left);
     factor_tables_d<64>(bmat, ftab);
     build_row_operands<64, false>(sQ, qj, bmat, ftab);
     build_row_operands<64, true>(sK, kj, bmat, ftab);
@@ -1297,8 +1304,10 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_scores_kernel(
           t2[i] = kv[i] * dkrv[i];
         }
         __nv_bfloat16* dst = dq + (long long)(row0 + me.row) * dq_ld + dqcol + dcol + c0;
+        if (me.row < left) {
 #pragma unroll
-        for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, dqv + c8 * 8);
+          for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, dqv + c8 * 8);
+        }
 #pragma unroll
         for (int c4 = 0; c4 < 8; ++c4) {
           *reinterpret_cast<float4*>(e1 + me.row * LP + c0 + c4 * 4) = make_float4(t1[c4 * 4], t1[c4 * 4 + 1], t1[c4 * 4 + 2], t1[c4 * 4 + 3]);
@@ -1367,8 +1376,10 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_scores_kernel(
           t1[i] = t1[i] - kv[i] * dkw + t2[i];  // E1 + E2: what the suffix sums run over
         }
         __nv_bfloat16* dst = dk + (long long)(row0 + me.row) * dk_ld + dkcol + dcol + c0;
+        if (me.row < left) {
 #pragma unroll
-        for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, dkv + c8 * 8);
+          for (int c8 = 0; c8 < 4; ++c8) store8_bf16(dst + c8 * 8, dkv + c8 * 8);
+        }
 #pragma unroll
         for (int c4 = 0; c4 < 8; ++c4)
           *reinterpret_cast<float4*>(e1 + me.row * LP + c0 + c4 * 4) = make_float4(t1[c4 * 4], t1[c4 * 4 + 1], t1[c4 * 4 + 2], t1[c4 * 4 + 3]);
@@ -1390,16 +1401,17 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_bwd_scores_kernel(
     float base = 0.f;
     for (int pp = part + 1; pp < NPARTS; ++pp) base += e1[(PR * pp) * LP + d];
     float* dst = dgl_local + (long long)row0 * (H * D) + dcol + d;
-    for (int t = PR * part; t < PR * part + PR; ++t) dst[(long long)t * (H * D)] = e1[t * LP + d] + base - e2[t * LP + d];
+    for (int t = PR * part; t < PR * part + PR && t < left; ++t) dst[(long long)t * (H * D)] = e1[t * LP + d] + base - e2[t * LP + d];
     if (part == 0) chunk_tot[(((long long)bh * NH + dh) * NT + chunk) * 64 + d] = e1[d] + base;
   }
   cta_teardown(bars, tmem, 512, status);
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-CUtensorMap user_map(const GlaMat& m, long long rows) {
-  return make_tmap_3d(m.ptr, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)m.ld, (uint64_t)rows, 1, (uint64_t)m.ld * 2ull,
-                      (uint64_t)m.ld * 2ull * (uint64_t)rows, 64, 64);
+// {columns of the wide matrix, rows of one sequence, sequences}: a box past a sequence's end is filled with zeros
+CUtensorMap user_map(const GlaMat& m, const GdnDims& d) {
+  return make_tmap_3d(m.ptr, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)m.ld, (uint64_t)d.T, (uint64_t)d.B, (uint64_t)m.ld * 2ull,
+                      (uint64_t)m.ld * 2ull * (uint64_t)d.T, 64, 64);
 }
 // [rows, width] contiguous bf16 scratch; box 64 columns x box_rows rows
 CUtensorMap scratch_map(const void* p, long long rows, int width, int box_rows) {
@@ -1417,16 +1429,15 @@ void smem_attr(K kern, int bytes) {
   if (e != cudaSuccess) throw std::runtime_error(std::string("cannot set shared memory size: ") + cudaGetErrorString(e));
 }
 void check_dims(const GdnDims& d) {
-  if (d.T <= 0 || d.T % C != 0) throw std::runtime_error("gdn chunk kernels need T to be a positive multiple of 64");
+  if (d.T <= 0) throw std::runtime_error("gdn chunk kernels need tokens");
   if (d.D != 64 && d.D != 128) throw std::runtime_error("gdn chunk kernels support head_dim 64 and 128");
 }
 
 template <int D>
 void fwd_impl(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, const float* init,
               const GlaMat& O, const GdnScratch& w, const GdnDims& d, float scale, int* status, cudaStream_t s) {
-  const long long rows = (long long)d.B * d.T;
-  const int NT = d.T / C, BH = d.B * d.H, nchunks = BH * NT;
-  CUtensorMap tk = user_map(K, rows), tv = user_map(V, rows), tg = user_map(G, rows), tq = user_map(Q, rows);
+  const int NT = (d.T + C - 1) / C, BH = d.B * d.H, nchunks = BH * NT;
+  CUtensorMap tk = user_map(K, d), tv = user_map(V, d), tg = user_map(G, d), tq = user_map(Q, d);
   {
     auto kern = gdn_wy_kernel<D>;
     static PerDeviceOnce once;
@@ -1460,11 +1471,10 @@ void bwd_impl(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G
               const float* dfin, const GlaMat& dQ, const GlaMat& dK, const GlaMat& dV, const GdnScratch& w,
               const GdnBwdScratch& x, const GdnDims& d, float scale, int* status, cudaStream_t s) {
   constexpr int NH = D / 64;
-  const long long rows = (long long)d.B * d.T;
-  const int NT = d.T / C, BH = d.B * d.H, nchunks = BH * NT;
+  const int NT = (d.T + C - 1) / C, BH = d.B * d.H, nchunks = BH * NT;
   const long long crow = (long long)nchunks * C, srow = (long long)nchunks * D;
-  CUtensorMap tq = user_map(Q, rows), tk = user_map(K, rows), tv = user_map(V, rows), tg = user_map(G, rows),
-              tdo = user_map(dO, rows);
+  CUtensorMap tq = user_map(Q, d), tk = user_map(K, d), tv = user_map(V, d), tg = user_map(G, d),
+              tdo = user_map(dO, d);
   CUtensorMap tu = scratch_map(w.U, crow, D, 64), tu0 = scratch_map(w.U0, crow, D, 64), tw = scratch_map(w.W, crow, D, 64),
               tt = scratch_map(w.Tm, crow, C, 64), tdu = scratch_map(x.dU, crow, D, 64),
               tdw = scratch_map(x.dW, crow, D, 64), tdl = scratch_map(x.dLraw, crow, C, 64);

@@ -82,6 +82,14 @@ struct MixerStep {
   int dim;
 };
 void launch_mixer_step(const MixerStep& p, int B, int D, bool delta, cudaStream_t s);
+// Write strengths of the delta rule (write_strength.cu): beta [rows, H] = sigmoid(x w^T), x rows of `dim` with pitch ldx, w [H, dim].
+constexpr int STRENGTH_MAX_HEADS = 16;
+void launch_strength_fwd(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, float* beta, int rows, int dim, int H,
+                         cudaStream_t s);
+// dx [rows, dim] and partial [strength_bwd_parts(rows, dim)][H * dim], whose sum over blocks is the gradient of w.
+int strength_bwd_parts(int rows, int dim);
+void launch_strength_bwd(const float* dbeta, const float* beta, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w,
+                         __nv_bfloat16* dx, float* partial, int rows, int dim, int H, cudaStream_t s);
 // Gated DeltaNet token recurrence over T tokens (T = 1: one decode step) for B*H heads of dimension D (64 or 128):
 // state [BH,D,D] fp32 in place; beta: null (1), fp32 [B*T,H] (beta_mode 1) or fp32 [B*T,H*D] (beta_mode 2).
 void launch_gdn_recurrent(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta,
@@ -98,10 +106,10 @@ void launch_gdn_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const 
 
 // ---- Gated DeltaNet, chunk-parallel training path (gdn_chunk_kernels.cu) ----
 struct GdnDims {
-  int B, T, H, D;    // T a multiple of 64, D = 64 or 128 (keys and values)
+  int B, T, H, D;    // D = 64 or 128 (keys and values)
   bool gate_logits;
 };
-// Per-chunk tensors produced by the forward pass and kept for the backward pass. nchunks = B * H * T / 64.
+// Per-chunk tensors produced by the forward pass and kept for the backward pass. nchunks = B * H * ceil(T / 64).
 struct GdnScratch {
   __nv_bfloat16* U0;      // [nchunks, 64, D]   T (beta V)
   __nv_bfloat16* W;       // [nchunks, 64, D]   T (beta Kbar)
@@ -126,7 +134,7 @@ struct GdnBwdScratch {
   __nv_bfloat16* dLraw;   // [nchunks, 64, 64]
   float* dbeta;           // [B * T, H] (null without beta)
   float* dgl_local;       // [B * T, H * D]     in-chunk part of the gate gradient
-  float* chunk_tot;       // [B * H * D / 64, T / 64, 64] chunk totals (the layout gla_dg_finalize reads with H * D / 64 heads)
+  float* chunk_tot;       // [B * H * D / 64, ceil(T / 64), 64] chunk totals (the layout gla_dg_finalize reads with H * D / 64 heads)
 };
 // out = scale * GatedDeltaNet(q, k, v, g, beta); beta fp32 [B*T, H] or null; init fp32 [B*H, D, D] or null.
 void launch_gdn_chunk_fwd(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta,

@@ -5,6 +5,7 @@
 
 #include <cmath>
 
+#include "../elementwise/elementwise.cuh"
 #include "gla.cuh"
 
 namespace {
@@ -202,6 +203,7 @@ void gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol,
   tb::launch_gdn_recurrent(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), bp, mode, state.data_ptr<float>(),
                            mat(out, ocol), (int)B, (int)T, (int)H, (int)D, gate_logits, (float)scale, cur_stream());
 }
+inline const __nv_bfloat16* bfc(const Tensor& t) { return reinterpret_cast<const __nv_bfloat16*>(t.data_ptr()); }
 inline __nv_bfloat16* bfp(Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); }
 
 // Chunk-parallel Gated DeltaNet forward. q, k, v, g: [B*T, ld] bf16 matrices with head h at columns col + h*D;
@@ -212,8 +214,8 @@ std::vector<Tensor> gdn_chunk_fwd(const Tensor& q, int64_t qcol, const Tensor& k
                                   const c10::optional<Tensor>& init, Tensor& out, int64_t ocol, int64_t B, int64_t T,
                                   int64_t H, int64_t D, bool gate_logits, double scale, bool keep_scores) {
   c10::cuda::CUDAGuard guard(q.device());
-  TORCH_CHECK(T % 64 == 0 && (D == 64 || D == 128), "gdn_chunk_fwd: T % 64 == 0 and D in {64, 128}");
-  const int64_t NT = T / 64, BH = B * H, n = BH * NT;
+  TORCH_CHECK(T > 0 && (D == 64 || D == 128), "gdn_chunk_fwd: tokens and D in {64, 128}");
+  const int64_t NT = (T + 63) / 64, BH = B * H, n = BH * NT;
   auto bf = q.options();
   auto f32 = q.options().dtype(at::kFloat);
   Tensor U0 = torch::empty({n, 64, D}, bf), W = torch::empty({n, 64, D}, bf), Tm = torch::empty({n, 64, 64}, bf),
@@ -252,7 +254,7 @@ std::vector<Tensor> gdn_chunk_bwd(const Tensor& q, int64_t qcol, const Tensor& k
                                   int64_t D, bool gate_logits, double scale) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(saved.size() >= 9, "gdn_chunk_bwd: the forward's saved tensors are missing");
-  const int64_t NT = T / 64, BH = B * H, n = BH * NT, NH = D / 64;
+  const int64_t NT = (T + 63) / 64, BH = B * H, n = BH * NT, NH = D / 64;
   auto bf = q.options();
   auto f32 = q.options().dtype(at::kFloat);
   Tensor G1 = torch::empty({n, 64, D}, f32), H1 = torch::empty({n, D, D}, f32), dU = torch::empty({n, 64, D}, bf),
@@ -288,11 +290,44 @@ std::vector<Tensor> gdn_chunk_bwd(const Tensor& q, int64_t qcol, const Tensor& k
   // 64-wide slice of a head counted as a head of its own
   Tensor end_term;
   if (dfp != nullptr) end_term = (dfinc.reshape({BH, D, D}) * saved[8].reshape({BH, D, D})).sum(-1).reshape({BH * NH, 64}).contiguous();
-  tb::GlaDims gd{(int)B, (int)T, (int)(H * NH), gate_logits};
+  tb::GlaDims gd{(int)B, (int)(NT * 64), (int)(H * NH), gate_logits, 64, (int)T};
   tb::launch_gla_dg_finalize(dgl.data_ptr<float>(), tot.data_ptr<float>(), mat(g, gcol), mat(dg, dgcol), gd, s,
                              end_term.defined() ? end_term.data_ptr<float>() : nullptr);
   // the per-chunk intermediates follow for inspection (stage-by-stage comparison against the PyTorch oracle)
   return {dbeta, dS0, status, G1, H1, dU, dSend, dq1, dkw1, dkr1, dW, dLraw, dgl, tot};
+}
+
+void strength_operands(const Tensor& x, const Tensor& w) {
+  (void)mat(x, 0);
+  (void)mat(w, 0);
+  TORCH_CHECK(w.is_contiguous() && w.size(1) == x.size(1) && w.size(0) <= tb::STRENGTH_MAX_HEADS && x.get_device() == w.get_device(),
+              "write strengths: x [rows, dim], w [heads, dim] contiguous, up to 16 heads");
+}
+
+// beta [rows, H] fp32 = sigmoid(x w^T)
+Tensor strength_fwd(const Tensor& x, const Tensor& w) {
+  strength_operands(x, w);
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor beta = torch::empty({x.size(0), w.size(0)}, x.options().dtype(at::kFloat));
+  tb::launch_strength_fwd(bfc(x), x.stride(0), bfc(w), beta.data_ptr<float>(), (int)x.size(0), (int)x.size(1), (int)w.size(0), cur_stream());
+  return beta;
+}
+
+// (dx bf16 [rows, dim], dw bf16 [H, dim]) from the gradient of beta (fp32 [rows, H])
+std::vector<Tensor> strength_bwd(const Tensor& dbeta, const Tensor& beta, const Tensor& x, const Tensor& w) {
+  strength_operands(x, w);
+  const int64_t rows = x.size(0), dim = x.size(1), H = w.size(0);
+  for (const Tensor* t : {&dbeta, &beta})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == rows * H, "write strengths: fp32 [rows, H]");
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor dx = torch::empty({rows, dim}, x.options()), dw = torch::empty({H, dim}, w.options());
+  const int parts = tb::strength_bwd_parts((int)rows, (int)dim);
+  Tensor partial = torch::empty({parts, H * dim}, x.options().dtype(at::kFloat));
+  auto s = cur_stream();
+  tb::launch_strength_bwd(dbeta.data_ptr<float>(), beta.data_ptr<float>(), bfc(x), x.stride(0), bfc(w), bfp(dx), partial.data_ptr<float>(),
+                          (int)rows, (int)dim, (int)H, s);
+  tb::launch_column_parts(partial.data_ptr<float>(), parts, (int)(H * dim), {nullptr, bfp(dw), false}, s);
+  return {dx, dw};
 }
 }  // namespace
 
@@ -311,6 +346,8 @@ void register_gla(pybind11::module& m) {
     tb::gla_set_debug_buffer(t.has_value() && t->defined() ? (long long*)t->data_ptr<int64_t>() : nullptr);
   });
   m.def("mixer_step", &mixer_step);
+  m.def("strength_fwd", &strength_fwd);
+  m.def("strength_bwd", &strength_bwd);
   m.def("gdn_recurrent", &gdn_recurrent);
   m.def("gdn_chunk_fwd", &gdn_chunk_fwd);
   m.def("gdn_chunk_bwd", &gdn_chunk_bwd);

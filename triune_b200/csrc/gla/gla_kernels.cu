@@ -903,7 +903,7 @@ __global__ void __launch_bounds__(BWD_THREADS) gla_bwd_main_kernel(
   }
 }
 
-// dg[t] = (local suffix + totals of later chunks) * d(log decay)/d(gate input). Heads are 64-wide slices here. Bound by
+// dg[t] = (local suffix + totals of later chunks) * d(log decay)/d(gate input). Heads are 64-wide slices here; rows past a sequence's end are left out. Bound by
 // memory: eight columns a thread in 16-byte accesses, the later chunks' totals summed by four groups of threads (8 x 1024 tokens,
 // 24 slices: 79 -> 32 us, 3.2 TB/s).
 __global__ void __launch_bounds__(256) gla_dg_finalize_kernel(const float* __restrict__ dgl_local,
@@ -916,12 +916,13 @@ __global__ void __launch_bounds__(256) gla_dg_finalize_kernel(const float* __res
   const int chunk = blockIdx.x % NT, bh = blockIdx.x / NT, h = bh % H, b = bh / H;
   const int tid = threadIdx.x;
   const long long row0 = (long long)b * rows + chunk * C;
-  const int ch = (tid & 7) * 8;
+  const int ch = (tid & 7) * 8, left = rows - chunk * C;  // rows of the sequence from row0 on
   // both rows of a thread are read ahead of the barrier
   uint4 gu[2];
   float loc[2][8];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
+    if ((tid >> 3) + 32 * i >= left) continue;
     const long long r = row0 + (tid >> 3) + 32 * i;
     gu[i] = *reinterpret_cast<const uint4*>(g + r * g_ld + gcol + h * D + ch);
     ld8(dgl_local + r * (H * D) + h * D + ch, loc[i]);
@@ -940,6 +941,7 @@ __global__ void __launch_bounds__(256) gla_dg_finalize_kernel(const float* __res
   for (int j = 0; j < 8; ++j) later[j] = (carry[0][ch + j] + carry[1][ch + j]) + (carry[2][ch + j] + carry[3][ch + j]);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
+    if ((tid >> 3) + 32 * i >= left) continue;
     float x[8], o[8];
     unpack8(gu[i], x);
 #pragma unroll
@@ -1103,7 +1105,7 @@ void launch_gla_bwd_main(GlaMat Q, GlaMat K, GlaMat V, GlaMat G, GlaMat dO, cons
 
 void launch_gla_dg_finalize(const float* dgl_local, const float* chunk_tot, GlaMat G, GlaMat dG, GlaDims d,
                             cudaStream_t s, const float* end_term) {
-  check_dims(d);
+  if (d.T % C != 0 || d.T <= 0) throw std::runtime_error("gla_dg_finalize: whole chunks of 64 tokens (of which `rows` are there)");
   const int slices = d.H * (d.D / 64), grid = d.B * slices * (d.T / C);
   gla_dg_finalize_kernel<<<grid, 256, 0, s>>>(dgl_local, chunk_tot, reinterpret_cast<const __nv_bfloat16*>(G.ptr), G.ld,
                                               G.col0, reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(dG.ptr)), dG.ld,

@@ -166,9 +166,19 @@ class VectorisedGLA(nn.Module):
             out, new_state = gla_cuda.gla_attention_core(qkvg, cos, sin, state, B, T, H)
             y = _project(self.out_proj, out.view(B, T, self.hidden_dim), self.out_scale)
             return y, format_cache(new_state if cache is not None else None, cache, fmt, offset, T)
+        beta = None
+        if self.use_delta_rule and self.beta_proj is not None:
+            if plain_beta and gla_cuda.strength_supported(x2, beta_w):
+                beta = gla_cuda.write_strength(x2, beta_w)
+            else:
+                beta = torch.sigmoid(self.beta_proj(x)).view(B * T, H)
+        if self.use_delta_rule and (beta is None or beta.dtype == torch.float32) and gla_cuda.gdn_core_supported(qkvg, T, D, beta):
+            out, new_state = gla_cuda.gdn_attention_core(qkvg, cos, sin, beta, state, B, T, H)
+            y = _project(self.out_proj, out.view(B, T, self.hidden_dim))
+            return y, format_cache(new_state if cache is not None else None, cache, fmt, offset, T)
         q, k, v, g = ops.qk_feature_map(qkvg, cos, sin, B, T, H, D)
         if self.use_delta_rule:
-            beta = torch.sigmoid(self.beta_proj(x)).view(B, T, H) if self.beta_proj is not None else None
+            beta = None if beta is None else beta.view(B, T, H)
             out, new_state = ops.gated_deltanet(q, k, v, g, beta=beta, initial_state=state, gate_logits=True)
         else:
             out, new_state = ops.gla(q, k, v, g, initial_state=state, gate_logits=True)

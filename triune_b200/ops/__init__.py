@@ -497,6 +497,16 @@ def embedding(ids, weight):
     return F.embedding(ids, weight)
 
 
+def half_tables(cos, sin, D: int):
+    """The first D / 2 columns of rotary tables as the feature-map kernels read them: in place where rows are 16-byte aligned."""
+    if cos is None:
+        return None, None
+    cs, sn = (t[:, : D // 2].float() for t in (cos, sin))
+    if any(t.stride(1) != 1 or t.stride(0) % 4 != 0 or t.stride(0) != cs.stride(0) or t.data_ptr() % 16 != 0 for t in (cs, sn)):
+        cs, sn = cs.contiguous(), sn.contiguous()
+    return cs, sn
+
+
 class _QKPrepFn(torch.autograd.Function):
     """qkvg [tokens, 4*H*D] -> (q~, k~) = rope(normalize(elu(.)+1)); reads the q and k column blocks in place."""
 
@@ -529,8 +539,7 @@ def qk_feature_map(qkvg: torch.Tensor, cos: Optional[torch.Tensor], sin: Optiona
     """
     HD = H * D
     if _ext.use_kernels(qkvg) and qkvg.dtype == torch.bfloat16 and D in (64, 128):
-        ch = cos[:, : D // 2].float().contiguous() if cos is not None else None
-        sh = sin[:, : D // 2].float().contiguous() if sin is not None else None
+        ch, sh = half_tables(cos, sin, D)
         qk = _QKPrepFn.apply(qkvg, ch, sh, T, H, D)  # [tokens, 2, H, D]
         qk = qk.view(B, T, 2, H, D)
         q, k = qk[:, :, 0], qk[:, :, 1]

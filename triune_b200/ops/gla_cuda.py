@@ -210,50 +210,112 @@ class _GDNChunkFn(torch.autograd.Function):
     def forward(ctx, q, k, v, g, beta, init, scale, gate_logits):
         B, T, H, D = q.shape
         e = _ext.ext()
-        pad = (-T) % 64
-        if pad:
-            # appended tokens with no key, no value and no decay leave the state and the real outputs untouched
-            zeros = q.new_zeros(B, pad, H, D)
-            q, k, v = (torch.cat((t, zeros), dim=1) for t in (q, k, v))
-            g = torch.cat((g, g.new_full((B, pad, H, D), 30.0 if gate_logits else 0.0)), dim=1)
-            if beta is not None:
-                beta = torch.cat((beta, beta.new_zeros(B, pad, H)), dim=1)
-        Tp = T + pad
         qm, km, vm, gm = (_as_matrix(t.to(torch.bfloat16)) for t in (q, k, v, g))
-        out = torch.empty(B * Tp, H * D, device=q.device, dtype=torch.bfloat16)
-        bt = beta.float().reshape(B * Tp, H).contiguous() if beta is not None else None
+        out = torch.empty(B * T, H * D, device=q.device, dtype=torch.bfloat16)
+        bt = beta.float().reshape(B * T, H).contiguous() if beta is not None else None
         ini = init.float().reshape(B * H, D, D).contiguous() if init is not None else None
         need = any(ctx.needs_input_grad[:6])
-        res = e.gdn_chunk_fwd(qm, 0, km, 0, vm, 0, gm, 0, bt, ini, out, 0, B, Tp, H, D, bool(gate_logits), float(scale),
+        res = e.gdn_chunk_fwd(qm, 0, km, 0, vm, 0, gm, 0, bt, ini, out, 0, B, T, H, D, bool(gate_logits), float(scale),
                               need and bt is not None)
         _tick(3)
         _note(res[9])
         if need:
-            ctx.save_for_backward(qm, km, vm, gm, bt if bt is not None else torch.empty(0, device=q.device), *res[:9])
-        ctx.dims = (B, T, Tp, H, D, float(scale), bool(gate_logits), beta is not None, init is not None,
-                    None if beta is None else beta.dtype)
+            ctx.save_for_backward(qm, km, vm, gm, bt, *res[:9])
+        ctx.dims = (B, T, H, D, float(scale), bool(gate_logits), None if beta is None else beta.dtype, init is not None)
         ctx.set_materialize_grads(False)
-        return out.view(B, Tp, H, D)[:, :T], res[8].view(B, H, D, D)
+        return out.view(B, T, H, D), res[8].view(B, H, D, D)
 
     @staticmethod
     def backward(ctx, dout, dfin):
         qm, km, vm, gm, bt, *saved = ctx.saved_tensors
-        B, T, Tp, H, D, scale, gate_logits, has_beta, has_init, beta_dtype = ctx.dims
-        e = _ext.ext()
-        dom = torch.zeros(B, Tp, H, D, device=qm.device, dtype=torch.bfloat16)
-        if dout is not None:
-            dom[:, :T] = dout
-        dom = dom.view(B * Tp, H * D)
-        dq, dk, dv, dg = (torch.empty(B * Tp, H * D, device=qm.device, dtype=torch.bfloat16) for _ in range(4))
+        B, T, H, D, scale, gate_logits, beta_dtype, has_init = ctx.dims
+        dom = qm.new_zeros(B * T, H * D) if dout is None else _as_matrix(dout.to(torch.bfloat16))
+        dq, dk, dv, dg = (torch.empty(B * T, H * D, device=qm.device, dtype=torch.bfloat16) for _ in range(4))
         dfl = dfin.float().reshape(B * H, D, D).contiguous() if dfin is not None else None
-        dbeta, ds0, status = e.gdn_chunk_bwd(qm, 0, km, 0, vm, 0, gm, 0, dom, 0, bt if has_beta else None, dfl, list(saved),
-                                             dq, 0, dk, 0, dv, 0, dg, 0, B, Tp, H, D, gate_logits, scale)[:3]
+        dbeta, ds0, status = _ext.ext().gdn_chunk_bwd(qm, 0, km, 0, vm, 0, gm, 0, dom, 0, bt, dfl, list(saved), dq, 0, dk, 0, dv, 0, dg, 0,
+                                                      B, T, H, D, gate_logits, scale)[:3]
         _tick(6)
         _note(status)
-        sh = (B, Tp, H, D)
-        cut = lambda t: t.view(sh)[:, :T]
-        db = dbeta.view(B, Tp, H)[:, :T].to(beta_dtype) if has_beta else None
-        return cut(dq), cut(dk), cut(dv), cut(dg), db, ds0.view(B, H, D, D) if has_init else None, None, None
+        sh = (B, T, H, D)
+        db = dbeta.view(B, T, H).to(beta_dtype) if bt is not None else None
+        return dq.view(sh), dk.view(sh), dv.view(sh), dg.view(sh), db, ds0.view(B, H, D, D) if has_init else None, None, None
+
+
+class _GDNCoreFn(torch.autograd.Function):
+    """qkvg [B*T, 4*H*D], write strengths [B*T, H] fp32 (or None: 1) -> (mixer output [B*T, H*D], final state): feature map, rotation
+    and the chunk kernels on the projection rows in place; the backward pass writes all four gradients into one buffer."""
+
+    @staticmethod
+    def forward(ctx, qkvg, cos_half, sin_half, beta, init, B, T, H):
+        D = qkvg.shape[1] // (4 * H)
+        HD = H * D
+        e = _ext.ext()
+        qk = e.qk_prep_fwd(qkvg, HD, cos_half, sin_half, T, H, D).view(B * T, 2 * HD)
+        out = torch.empty(B * T, HD, device=qkvg.device, dtype=torch.bfloat16)
+        ini = init.float().reshape(B * H, D, D).contiguous() if init is not None else None
+        res = e.gdn_chunk_fwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, beta, ini, out, 0, B, T, H, D, True, 1.0, beta is not None)
+        _tick(4)
+        _note(res[9])
+        ctx.save_for_backward(qkvg, qk, cos_half, sin_half, beta, *res[:9])
+        ctx.dims = (B, T, H, D, init is not None)
+        ctx.set_materialize_grads(False)
+        return out, res[8].view(B, H, D, D)
+
+    @staticmethod
+    def backward(ctx, dout, dfin):
+        qkvg, qk, cs, sn, beta, *saved = ctx.saved_tensors
+        B, T, H, D, has_init = ctx.dims
+        HD = H * D
+        e = _ext.ext()
+        dout = qkvg.new_zeros(B * T, HD) if dout is None else dout.contiguous()
+        dqk, dqkvg = torch.empty_like(qk), torch.empty_like(qkvg)
+        dfl = dfin.float().reshape(B * H, D, D).contiguous() if dfin is not None else None
+        dbeta, ds0, status = e.gdn_chunk_bwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, dout, 0, beta, dfl, list(saved), dqk, 0, dqk, HD,
+                                             dqkvg, 2 * HD, dqkvg, 3 * HD, B, T, H, D, True, 1.0)[:3]
+        e.qk_prep_bwd(qkvg, HD, dqk.view(B * T, 2, H, D), dqkvg, cs, sn, T, H, D)
+        _tick(7)
+        _note(status)
+        return (dqkvg, None, None, dbeta if beta is not None else None, ds0.view(B, H, D, D) if has_init else None, None, None, None)
+
+
+def gdn_core_supported(qkvg: torch.Tensor, T: int, D: int, beta) -> bool:
+    """True when :func:`gdn_attention_core` covers a training pass; without gradients the fp32 recurrence is taken."""
+    return (core_supported(qkvg, T, D) and torch.is_grad_enabled()
+            and (qkvg.requires_grad or (beta is not None and beta.requires_grad)))
+
+
+def gdn_attention_core(qkvg, cos, sin, beta, init, B, T, H):
+    from . import half_tables
+
+    return _GDNCoreFn.apply(qkvg, *half_tables(cos, sin, qkvg.shape[1] // (4 * H)), beta, init, B, T, H)
+
+
+class _StrengthFn(torch.autograd.Function):
+    """sigmoid(x w^T) in fp32 for x [rows, dim], w [heads, dim]."""
+
+    @staticmethod
+    def forward(ctx, x2, w):
+        beta = _ext.ext().strength_fwd(x2, w)
+        _tick(1)
+        ctx.save_for_backward(x2, w, beta)
+        return beta
+
+    @staticmethod
+    def backward(ctx, dbeta):
+        x2, w, beta = ctx.saved_tensors
+        dx, dw = _ext.ext().strength_bwd(dbeta.contiguous(), beta, x2, w)
+        _tick(2)
+        return dx, dw
+
+
+def strength_supported(x2, w) -> bool:
+    return (_ext.use_kernels(x2, w) and w.is_contiguous() and w.shape[0] <= 16 and w.shape[1] % 8 == 0 and _aligned_rows(x2)
+            and _aligned_rows(w))
+
+
+def write_strength(x2, w):
+    """Write strengths of the delta rule, fp32 [rows, heads]."""
+    return _StrengthFn.apply(x2, w)
 
 
 def gdn_chunk(q, k, v, g, beta, initial_state, scale, gate_logits):
@@ -332,8 +394,9 @@ def core_supported(qkvg: torch.Tensor, T: int, D: int) -> bool:
 
 def gla_attention_core(qkvg, cos, sin, init, B, T, H):
     D = qkvg.shape[1] // (4 * H)
-    ch = cos[:, : D // 2].float().contiguous() if cos is not None else None
-    sh = sin[:, : D // 2].float().contiguous() if sin is not None else None
+    from . import half_tables
+
+    ch, sh = half_tables(cos, sin, D)
     if init is not None and init.shape != (B, H, D, D):
         init = init.expand(B, H, D, D)  # one state for every sequence
     return _GLACoreFn.apply(qkvg, ch, sh, init, B, T, H)
