@@ -10,7 +10,9 @@
 #include <stdint.h>
 
 #include <stdexcept>
+#include <string>
 
+#include "../common/dependent_launch.cuh"
 #include "../common/ptx.cuh"
 #include "elementwise.cuh"
 
@@ -125,6 +127,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_wide_kernel(const __nv_bfloat
   const int slot = warp / wpr, col = ((warp % wpr) * 32 + lane) * 8;
   const bool live = col < d;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  allow_dependents();
+  wait_predecessors();  // launched over the end of the kernel before it
   const uint4 wv = live ? *reinterpret_cast<const uint4*>(w + col) : zero;
   int buf = 0;
   for (long long base = (long long)blockIdx.x * slots * R; base < rows; base += (long long)gridDim.x * slots * R, buf ^= 1) {
@@ -474,8 +478,9 @@ void rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bf
     return;
   }
   const WideGeom g = wide_geom(rows, d, 148 * 8);
-  if (g.four) rmsnorm_fwd_wide_kernel<HAS_RES, 4><<<g.blocks, g.threads, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps, g.wpr);
-  else rmsnorm_fwd_wide_kernel<HAS_RES, 1><<<g.blocks, g.threads, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps, g.wpr);
+  const cudaError_t e = launch_dependent(g.four ? rmsnorm_fwd_wide_kernel<HAS_RES, 4> : rmsnorm_fwd_wide_kernel<HAS_RES, 1>, dim3(g.blocks),
+                                         dim3(g.threads), s, x, res, w, y, sum_out, rstd, rows, d, eps, g.wpr);
+  if (e != cudaSuccess) throw std::runtime_error(std::string("rmsnorm launch failed: ") + cudaGetErrorString(e));
 }
 
 template <bool HAS_DRES>

@@ -8,6 +8,7 @@
 // eight contiguous weights (one 16-byte load) are the k pairs {2 t, 2 t + 1, 2 t + 8, 2 t + 9} of two steps, and the four
 // lanes of a row read a whole 128-byte line in two loads. The W warps of a CTA split K and their partial sums meet in
 // shared memory; W is chosen so that about 16 warps per SM stream (16 KB in flight each SM at four loads a lane and more).
+// Four steps of loads are kept in flight, and the kernel is launched over the end of the one before it (dependent_launch.cuh).
 // Nothing is staged: a slice of A is read by one warp of the CTA only. Measured with the weight in DRAM (M = 1 to 8, before ->
 // after): 8192 x 2048 20.2 -> 11.7 us, 2048 x 2048 18.6 -> 5.4, 2048 x 5632 39.0 -> 10.4, 32000 x 2048 36 -> 30, gated 5632 x
 // 2048 23.2 -> 14.3; at 16 rows 20.1 -> 12.0, 18.5 -> 6.5, 39.0 -> 12.2, 34.6 -> 32.9, 23.3 -> 16.1.
@@ -16,6 +17,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "../common/dependent_launch.cuh"
 #include "../common/ptx.cuh"
 #include "tc_gemm.cuh"
 
@@ -45,6 +47,7 @@ __global__ void __launch_bounds__(W * 32) skinny_kernel(const __nv_bfloat16* __r
   __shared__ float sums[W][PARTS][NT * 8][SK_ROWS + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = blockIdx.x * SK_ROWS;
+  wait_predecessors();
   const int steps = (K + 63) / 64, s0 = (int)((long long)warp * steps / W), s1 = (int)((long long)(warp + 1) * steps / W);
   float acc[PARTS][NT][4];
 #pragma unroll
@@ -55,7 +58,7 @@ __global__ void __launch_bounds__(W * 32) skinny_kernel(const __nv_bfloat16* __r
       for (int i = 0; i < 4; ++i) acc[p][j][i] = 0.f;
   const bool r0 = n0 + g < N, r1 = n0 + g + 8 < N;
   const __nv_bfloat16* w0 = B + (long long)(n0 + g) * ldb + t * 8;
-#pragma unroll 2
+#pragma unroll 4
   for (int s = s0; s < s1; ++s) {
     const int k = s * 64;
     const bool lo = k + t * 8 < K, hi = k + 32 + t * 8 < K;
@@ -85,6 +88,7 @@ __global__ void __launch_bounds__(W * 32) skinny_kernel(const __nv_bfloat16* __r
           mma_16x8x16(acc[p][j], a[p][2 * h].z, a[p][2 * h + 1].z, a[p][2 * h].w, a[p][2 * h + 1].w, b[j][h].z, b[j][h].w);
         }
   }
+  allow_dependents();  // the loads are in: the next kernel's blocks may come while sums meet and are written
 #pragma unroll
   for (int p = 0; p < PARTS; ++p)
 #pragma unroll
@@ -117,11 +121,11 @@ __global__ void __launch_bounds__(W * 32) skinny_kernel(const __nv_bfloat16* __r
 template <int W, int NT>
 void run(const GemmArgs& a, int blocks, cudaStream_t s) {
   auto c = reinterpret_cast<__nv_bfloat16*>(a.C);
-  if (a.flags & GF_SWIGLU)
-    skinny_kernel<W, NT, true><<<blocks, W * 32, 0, s>>>(a.A, a.lda, a.B, a.ldb, c, a.ldc, a.M, a.N, a.K, 1.f, nullptr, 0);
-  else
-    skinny_kernel<W, NT, false><<<blocks, W * 32, 0, s>>>(a.A, a.lda, a.B, a.ldb, c, a.ldc, a.M, a.N, a.K, a.alpha, a.bias,
-                                                         (a.flags & GF_GELU) != 0);
+  const bool glu = (a.flags & GF_SWIGLU) != 0;
+  const cudaError_t e = launch_dependent(glu ? skinny_kernel<W, NT, true> : skinny_kernel<W, NT, false>, dim3(blocks), dim3(W * 32), s, a.A, a.lda,
+                                         a.B, a.ldb, c, a.ldc, a.M, a.N, a.K, glu ? 1.f : a.alpha, glu ? nullptr : a.bias,
+                                         (a.flags & GF_GELU) != 0 ? 1 : 0);
+  if (e != cudaSuccess) throw std::runtime_error(std::string("skinny_gemm launch failed: ") + cudaGetErrorString(e));
 }
 
 }  // namespace

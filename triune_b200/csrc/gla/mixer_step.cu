@@ -16,6 +16,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "../common/dependent_launch.cuh"
 #include "gla.cuh"
 
 namespace tb {
@@ -37,6 +38,8 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.y, b = blockIdx.z, HD = p.H * D, c = blockIdx.x * MS_COLS + lane, r0 = warp * RP;
   const __nv_bfloat16* row = p.qkvg + (long long)b * p.ld + h * D;
+  allow_dependents();
+  wait_predecessors();
 
   float S[RP];
   const long long at = ((long long)(b * p.H + h) * D + r0) * D + c;
@@ -124,12 +127,11 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
 void launch_mixer_step(const MixerStep& p, int B, int D, bool delta, cudaStream_t s) {
   if (B <= 0 || p.H <= 0) return;
   const dim3 grid(D / MS_COLS, p.H, B);
-  if (D == 64 && delta) mixer_step_kernel<64, true><<<grid, MS_THREADS, 0, s>>>(p);
-  else if (D == 64) mixer_step_kernel<64, false><<<grid, MS_THREADS, 0, s>>>(p);
-  else if (D == 128 && delta) mixer_step_kernel<128, true><<<grid, MS_THREADS, 0, s>>>(p);
-  else if (D == 128) mixer_step_kernel<128, false><<<grid, MS_THREADS, 0, s>>>(p);
+  void (*kernel)(const MixerStep) = nullptr;
+  if (D == 64) kernel = delta ? mixer_step_kernel<64, true> : mixer_step_kernel<64, false>;
+  else if (D == 128) kernel = delta ? mixer_step_kernel<128, true> : mixer_step_kernel<128, false>;
   else throw std::runtime_error("mixer_step: head dimension must be 64 or 128");
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_dependent(kernel, grid, dim3(MS_THREADS), s, p);
   if (e != cudaSuccess) throw std::runtime_error(std::string("mixer_step launch failed: ") + cudaGetErrorString(e));
 }
 
