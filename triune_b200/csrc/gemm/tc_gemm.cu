@@ -31,8 +31,8 @@ namespace tb {
 
 namespace {
 
-template <int BN, bool A_MN, bool B_MN, int EPI>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+template <int BN, bool A_MN, bool B_MN, int EPI, int EW>
+__global__ void __launch_bounds__(gemm_threads(EW), 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux, const KParams p) {
   using Cfg = GemmCfg<BN>;
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint8_t* smemA = smem;
   uint8_t* smemB = smem + STAGES * Cfg::A_BYTES;
-  uint8_t* smem_epi = smem + STAGES * Cfg::STAGE_BYTES;  // 8 warps x 1 staging tile
+  uint8_t* smem_epi = smem + STAGES * Cfg::STAGE_BYTES;  // 32 KB of staging: two buffers for each of 8 warps, or one for each of 16
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_epi + 8 * EPI_TILE);
   uint64_t* full = bars;                    // [STAGES] TMA -> MMA
   uint64_t* empty = bars + STAGES;          // [STAGES] MMA -> TMA
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 8);
+      mbar_init(&acc_empty[a], EW);
     }
     mbar_fence_init();
     prefetch_tmap(&tmA);
@@ -192,12 +192,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..9)
-    // Short reductions (K = 384) make the epilogue the longer phase of a tile; eight warps halve it, which is worth
-    // more than a deeper load ring.
+    // ------------------------------------------------------------ epilogue (warps 2..)
+    // Short reductions (K = 384) make the epilogue the longer phase of a tile; more warps are worth more there than a
+    // deeper load ring.
     const int lane_base = (warp & 3) * 32;
     const int col_half = (warp - 2) >> 2;
-    uint8_t* my_stage = smem_epi + (warp - 2) * EPI_TILE;  // one staging tile per warp (a second one costs a load stage and measured slower)
+    uint8_t* my_stage = smem_epi + (warp - 2) * (8 * EPI_TILE / EW);
     int acc = 0;
     uint32_t acc_phase = 0, buf = 0;
     for (int t = blockIdx.x; t < p.total_tiles; t += gridDim.x) {
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         break;
       }
       tc_fence_after_sync();
-      run_epilogue<EPI>(p, tl, &tmC, &tmAux, tmem_base + acc * BN, BN, tl.n0 * NOUT, tl.m0, lane_base, col_half, lane,
+      run_epilogue<EPI, EW>(p, tl, &tmC, &tmAux, tmem_base + acc * BN, BN, tl.n0 * NOUT, tl.m0, lane_base, col_half, lane,
                         my_stage, buf);
       tc_fence_before_sync();
       __syncwarp();
@@ -245,32 +245,48 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   }
 }
 
-template <int BN, bool A_MN, bool B_MN, int EPI>
+template <int BN, bool A_MN, bool B_MN, int EPI, int EW>
 void launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmAux,
                     const KParams& kp, int grid, cudaStream_t stream) {
-  auto kern = tc_gemm_kernel<BN, A_MN, B_MN, EPI>;
+  auto kern = tc_gemm_kernel<BN, A_MN, B_MN, EPI, EW>;
   static PerDeviceOnce configured;  // the attribute is per device
   if (configured.first_use()) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::SMEM_BYTES);
     if (e != cudaSuccess) throw std::runtime_error(std::string("tc_gemm: cannot set shared memory size: ") + cudaGetErrorString(e));
   }
-  kern<<<grid, GEMM_THREADS, GemmCfg<BN>::SMEM_BYTES, stream>>>(tmA, tmB, tmC, tmAux, kp);
+  kern<<<grid, gemm_threads(EW), GemmCfg<BN>::SMEM_BYTES, stream>>>(tmA, tmB, tmC, tmAux, kp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("tc_gemm launch failed: ") + cudaGetErrorString(e));
+}
+
+// Epilogue warps. The activation epilogues spend more on arithmetic (two tanh and twenty packed operations per pair of outputs
+// with the derivative) or on reads than a tile's products take, and with two warps per scheduler much of that was latency:
+// sixteen warps there, eight where the epilogue only converts or a tile has few chunks. Before -> after at 65536 x 1536 x 384:
+// GELU 109 -> 91 us, with its derivative 131 -> 119 (3.8 TB/s), times saved rows 150 -> 123; at 8192 x 4096 x 1024 and above the
+// products hide either. Multiplied rows want K below 1024 (8192 x 6144 x 1536: 131 with eight warps, 135 with sixteen); SwiGLU
+// backward gains 2 to 5 % at 2048 and 8192 x 5632 x 2048, its forward loses as much.
+template <int BN, bool A_MN, bool B_MN, int EPI>
+void launch_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmAux, const KParams& kp,
+                int grid, cudaStream_t s) {
+  constexpr bool more = BN >= 128 && (EPI == EPI_GELU || EPI == EPI_DSWIGLU || EPI == EPI_MULAUX);
+  if constexpr (more) {
+    if (EPI != EPI_MULAUX || kp.K < 1024) return launch_variant<BN, A_MN, B_MN, EPI, 16>(tmA, tmB, tmC, tmAux, kp, grid, s);
+  }
+  if constexpr (!more || EPI == EPI_MULAUX) launch_variant<BN, A_MN, B_MN, EPI, 8>(tmA, tmB, tmC, tmAux, kp, grid, s);
 }
 
 template <int BN, bool A_MN, bool B_MN>
 void dispatch_epi(int epi, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
                   const CUtensorMap& tmAux, const KParams& kp, int grid, cudaStream_t s) {
-  if (epi == EPI_PLAIN) return launch_variant<BN, A_MN, B_MN, EPI_PLAIN>(tmA, tmB, tmC, tmAux, kp, grid, s);
-  if (epi == EPI_PLAIN_F32) return launch_variant<BN, A_MN, B_MN, EPI_PLAIN_F32>(tmA, tmB, tmC, tmAux, kp, grid, s);
+  if (epi == EPI_PLAIN) return launch_epi<BN, A_MN, B_MN, EPI_PLAIN>(tmA, tmB, tmC, tmAux, kp, grid, s);
+  if (epi == EPI_PLAIN_F32) return launch_epi<BN, A_MN, B_MN, EPI_PLAIN_F32>(tmA, tmB, tmC, tmAux, kp, grid, s);
   if constexpr (!A_MN) {  // the activation epilogues follow row-major activations
-    if (epi == EPI_GELU) return launch_variant<BN, A_MN, B_MN, EPI_GELU>(tmA, tmB, tmC, tmAux, kp, grid, s);
-    if (epi == EPI_MULAUX) return launch_variant<BN, A_MN, B_MN, EPI_MULAUX>(tmA, tmB, tmC, tmAux, kp, grid, s);
-    if (epi == EPI_DSWIGLU) return launch_variant<BN, A_MN, B_MN, EPI_DSWIGLU>(tmA, tmB, tmC, tmAux, kp, grid, s);
-    if (epi == EPI_ADDAUX) return launch_variant<BN, A_MN, B_MN, EPI_ADDAUX>(tmA, tmB, tmC, tmAux, kp, grid, s);
+    if (epi == EPI_GELU) return launch_epi<BN, A_MN, B_MN, EPI_GELU>(tmA, tmB, tmC, tmAux, kp, grid, s);
+    if (epi == EPI_MULAUX) return launch_epi<BN, A_MN, B_MN, EPI_MULAUX>(tmA, tmB, tmC, tmAux, kp, grid, s);
+    if (epi == EPI_DSWIGLU) return launch_epi<BN, A_MN, B_MN, EPI_DSWIGLU>(tmA, tmB, tmC, tmAux, kp, grid, s);
+    if (epi == EPI_ADDAUX) return launch_epi<BN, A_MN, B_MN, EPI_ADDAUX>(tmA, tmB, tmC, tmAux, kp, grid, s);
     if constexpr (!B_MN) {
-      if (epi == EPI_SWIGLU) return launch_variant<BN, A_MN, B_MN, EPI_SWIGLU>(tmA, tmB, tmC, tmAux, kp, grid, s);
+      if (epi == EPI_SWIGLU) return launch_epi<BN, A_MN, B_MN, EPI_SWIGLU>(tmA, tmB, tmC, tmAux, kp, grid, s);
     }
   }
   throw std::runtime_error("tc_gemm: activation epilogues need a K-major A operand");

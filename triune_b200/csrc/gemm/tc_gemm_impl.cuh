@@ -13,6 +13,7 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int GEMM_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
+constexpr int gemm_threads(int epi_warps) { return 64 + 32 * epi_warps; }
 constexpr int EPI_TILE = 32 * 128;  // one staged output tile: 32 rows x 128 bytes
 
 template <int BN>
@@ -180,18 +181,25 @@ __device__ __forceinline__ void report(const KParams& p, int code) {
 enum { EPI_PLAIN = 0, EPI_PLAIN_F32 = 1, EPI_GELU = 2, EPI_MULAUX = 3, EPI_SWIGLU = 4, EPI_DSWIGLU = 5, EPI_ADDAUX = 6 };
 
 // One accumulator tile (128 rows x n_cols fp32 in TMEM at tmem_acc) through the epilogue EPI and out to global
-// memory. Called by the eight epilogue warps of a CTA: a warp can only read the TMEM lanes of its quarter
-// (warp % 4), so two warps share every quarter and take alternate column chunks (col_half 0 / 1). Per chunk (64 bytes
+// memory. Called by the EW epilogue warps of a CTA: a warp can only read the TMEM lanes of its quarter
+// (warp % 4), so EW / 4 warps share every quarter and take column chunks in turn (col_half 0 to EW / 4 - 1). Per chunk (64 bytes
 // of output per row: 32 bf16 or 16 fp32 columns) a warp reads the accumulator, applies the epilogue in packed f32x2
 // arithmetic, writes its 32 rows into one of its two 64B-swizzled staging buffers and one lane hands the buffer to TMA
 // (plain store, or reduce-add for accumulate / split-K). The buffers alternate, and a buffer is reused once the store
 // issued two chunks earlier has read it, so a warp never waits for the store it has just issued: with one buffer per
 // warp that wait (about a microsecond per chunk) made short reductions epilogue-bound. Ragged M/N edges are clipped
-// by the tensor map. m_base is the first output row of this CTA's 128 rows, n0 the first output column of the tile;
+// by the tensor map. With sixteen warps (the epilogues with arithmetic or reads of their own) there is one buffer per warp in the
+// same shared memory, and the other three warps of a scheduler cover the wait. m_base is the first output row of this CTA's 128 rows, n0 the first output column of the tile;
 // `buf` carries the buffer choice from tile to tile.
 constexpr int EPI_BUF = 32 * 64;  // one staging buffer: 32 rows x 64 bytes
 
+template <int EW>
 __device__ __forceinline__ uint8_t* epi_claim(uint8_t* my_stage, uint32_t& buf, int lane) {
+  if constexpr (EW == 16) {
+    if (lane == 0) tma_store_wait_read<0>();
+    __syncwarp();
+    return my_stage;
+  }
   if (lane == 0) tma_store_wait_read<1>();
   __syncwarp();
   uint8_t* st = my_stage + buf * EPI_BUF;
@@ -201,7 +209,7 @@ __device__ __forceinline__ uint8_t* epi_claim(uint8_t* my_stage, uint32_t& buf, 
 // 16-byte unit j of row `lane` in a 64B-swizzled buffer
 __device__ __forceinline__ uint32_t epi_off(int lane, int j) { return lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4); }
 
-template <int EPI>
+template <int EPI, int EW = 8>
 __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, const CUtensorMap* tmC,
                                               const CUtensorMap* tmAux, uint32_t tmem_acc, int n_cols, int n0,
                                               int m_base, int lane_base, int col_half, int lane, uint8_t* my_stage,
@@ -217,7 +225,7 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, 
   const long long c_off = (long long)out_batch * p.strideC + (long long)gm * p.ldc;
   const __nv_bfloat16* bias = p.bias ? p.bias + (long long)tl.g * p.bias_stride : nullptr;
 #pragma unroll 1
-  for (int c = col_half * CW; c < n_cols; c += 2 * CW) {
+  for (int c = col_half * CW; c < n_cols; c += EW / 4 * CW) {
     if (n0 + c >= p.N) break;
     const bool timed = p.dbg != nullptr && lane == 0 && lane_base == 0 && col_half == 0;
     long long tk0 = 0, tk1 = 0, tk2 = 0, tk3 = 0;
@@ -279,7 +287,7 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, 
 #pragma unroll
         for (int i = 0; i < NP; ++i) v[i] = mul2(v[i], rs2);
       }
-      st = epi_claim(my_stage, buf, lane);
+      st = epi_claim<EW>(my_stage, buf, lane);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float4 o;
@@ -313,7 +321,7 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, 
             const uint64_t ndu = fma2(x2, NC3, NC0);  // -k0 (1 + 3 k1 x^2)
             dq[i] = f2_to_bf16x2(fma2(mul2(h, nq), ndu, sgm));
           }
-          uint8_t* sd = epi_claim(my_stage, buf, lane);
+          uint8_t* sd = epi_claim<EW>(my_stage, buf, lane);
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             *reinterpret_cast<uint4*>(sd + epi_off(lane, j)) =
@@ -362,7 +370,7 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, 
         }
       }
       if (timed) tk2 = clock64();
-      st = epi_claim(my_stage, buf, lane);
+      st = epi_claim<EW>(my_stage, buf, lane);
       if (timed) tk3 = clock64();
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -391,9 +399,10 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, const Tile& tl, 
 }
 
 // Stage one 32-row x 32-column bf16 chunk (16 packed pairs per lane) and hand it to TMA.
+template <int EW>
 __device__ __forceinline__ void epi_store_chunk(const CUtensorMap* tm, const uint32_t (&q)[16], int col, int row,
                                                 int batch, int lane, uint8_t* my_stage, uint32_t& buf) {
-  uint8_t* st = epi_claim(my_stage, buf, lane);
+  uint8_t* st = epi_claim<EW>(my_stage, buf, lane);
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     *reinterpret_cast<uint4*>(st + epi_off(lane, j)) = make_uint4(q[j * 4 + 0], q[j * 4 + 1], q[j * 4 + 2], q[j * 4 + 3]);
@@ -409,13 +418,14 @@ __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.0f, 1.
 
 // SwiGLU forward epilogue: n_cols accumulator columns = [gate (n_cols/2) | up (n_cols/2)] of output columns
 // [n0, n0 + n_cols/2). Same warp roles and staging as epilogue_tile.
+template <int EW>
 __device__ __forceinline__ void epilogue_tile_swiglu(const KParams& p, const Tile& tl, const CUtensorMap* tmC,
                                                      const CUtensorMap* tmAux, uint32_t tmem_acc, int n_cols, int n0,
                                                      int m_base, int lane_base, int col_half, int lane,
                                                      uint8_t* my_stage, uint32_t& buf) {
   const int half = n_cols >> 1;
 #pragma unroll 1
-  for (int c = col_half * 32; c < half; c += 64) {
+  for (int c = col_half * 32; c < half; c += EW / 4 * 32) {
     if (n0 + c >= p.N) break;
     uint32_t rg[32], ru[32];
     if (tl.k_iters > 0) {
@@ -458,14 +468,14 @@ __device__ __forceinline__ void epilogue_tile_swiglu(const KParams& p, const Til
       q[i] = p.glu_act == 0 ? pack_bf16x2(g0 * sigmoid_f(g0) * u0, g1 * sigmoid_f(g1) * u1)
                             : pack_bf16x2(fmaxf(g0, 0.f) * u0, fmaxf(g1, 0.f) * u1);
     }
-    epi_store_chunk(tmC, q, n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
+    epi_store_chunk<EW>(tmC, q, n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
     if (p.aux_out) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) q[i] = pack_bf16x2(__uint_as_float(rg[2 * i]), __uint_as_float(rg[2 * i + 1]));
-      epi_store_chunk(tmAux, q, n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
+      epi_store_chunk<EW>(tmAux, q, n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
 #pragma unroll
       for (int i = 0; i < 16; ++i) q[i] = pack_bf16x2(__uint_as_float(ru[2 * i]), __uint_as_float(ru[2 * i + 1]));
-      epi_store_chunk(tmAux, q, p.n_split + n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
+      epi_store_chunk<EW>(tmAux, q, p.n_split + n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
     }
   }
 }
@@ -473,6 +483,7 @@ __device__ __forceinline__ void epilogue_tile_swiglu(const KParams& p, const Til
 // SwiGLU backward epilogue: acc = d(hidden) for output columns [n0, n0 + n_cols); with g, u read from aux_in
 // ([M, 2 * n_split], row pitch ldc) it writes d(gate) = dh * u * silu'(g) and d(up) = dh * silu(g) into C
 // ([M, 2 * n_split]) at columns n0.. and n_split + n0...
+template <int EW>
 __device__ __forceinline__ void epilogue_tile_dswiglu(const KParams& p, const Tile& tl, const CUtensorMap* tmC,
                                                       uint32_t tmem_acc, int n_cols, int n0, int m_base, int lane_base,
                                                       int col_half, int lane, uint8_t* my_stage, uint32_t& buf) {
@@ -480,7 +491,7 @@ __device__ __forceinline__ void epilogue_tile_dswiglu(const KParams& p, const Ti
   const bool row_ok = gm < p.M;
   const long long c_off = (long long)gm * p.ldc;
 #pragma unroll 1
-  for (int c = col_half * 32; c < n_cols; c += 64) {
+  for (int c = col_half * 32; c < n_cols; c += EW / 4 * 32) {
     if (n0 + c >= p.N) break;
     uint4 gv[4], uv[4];
 #pragma unroll
@@ -511,22 +522,22 @@ __device__ __forceinline__ void epilogue_tile_dswiglu(const KParams& p, const Ti
       qg[i] = pack_bf16x2(d0 * u0 * s0 * (1.0f + g0 * (1.0f - s0)), d1 * u1 * s1 * (1.0f + g1 * (1.0f - s1)));
       qu[i] = pack_bf16x2(d0 * g0 * s0, d1 * g1 * s1);
     }
-    epi_store_chunk(tmC, qg, n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
-    epi_store_chunk(tmC, qu, p.n_split + n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
+    epi_store_chunk<EW>(tmC, qg, n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
+    epi_store_chunk<EW>(tmC, qu, p.n_split + n0 + c, m_base + lane_base, 0, lane, my_stage, buf);
   }
 }
 
 // One call site for every epilogue kind.
-template <int EPI>
+template <int EPI, int EW = 8>
 __device__ __forceinline__ void run_epilogue(const KParams& p, const Tile& tl, const CUtensorMap* tmC,
                                              const CUtensorMap* tmAux, uint32_t tmem_acc, int n_cols, int n0, int m_base,
                                              int lane_base, int col_half, int lane, uint8_t* my_stage, uint32_t& buf) {
   if constexpr (EPI == EPI_SWIGLU)
-    epilogue_tile_swiglu(p, tl, tmC, tmAux, tmem_acc, n_cols, n0, m_base, lane_base, col_half, lane, my_stage, buf);
+    epilogue_tile_swiglu<EW>(p, tl, tmC, tmAux, tmem_acc, n_cols, n0, m_base, lane_base, col_half, lane, my_stage, buf);
   else if constexpr (EPI == EPI_DSWIGLU)
-    epilogue_tile_dswiglu(p, tl, tmC, tmem_acc, n_cols, n0, m_base, lane_base, col_half, lane, my_stage, buf);
+    epilogue_tile_dswiglu<EW>(p, tl, tmC, tmem_acc, n_cols, n0, m_base, lane_base, col_half, lane, my_stage, buf);
   else
-    epilogue_tile<EPI>(p, tl, tmC, tmAux, tmem_acc, n_cols, n0, m_base, lane_base, col_half, lane, my_stage, buf);
+    epilogue_tile<EPI, EW>(p, tl, tmC, tmAux, tmem_acc, n_cols, n0, m_base, lane_base, col_half, lane, my_stage, buf);
 }
 
 }  // namespace
