@@ -47,10 +47,10 @@ constexpr int BMAT_BYTES = C * BST * 4;
 // shared-memory reads, no round trip per token), publishes the part's total, and after ONE barrier adds the totals of
 // the earlier parts while writing its rows. (The previous form scanned in place in shared memory: 64/P dependent
 // load-add-store round trips twice, up to 2.5 K clocks in the 128-thread kernel.)
+// `totals`: NTHR floats of scratch.
 template <int NTHR>
-__device__ __forceinline__ void build_cumsum(const uint8_t* g_tile, float* bmat, bool logits) {
+__device__ __forceinline__ void build_cumsum(const uint8_t* g_tile, float* bmat, float* totals, bool logits) {
   constexpr int PARTS = NTHR / 64, LEN = C / PARTS;
-  __shared__ float totals[PARTS * 64];
   const int tid = threadIdx.x, d = tid & 63, part = tid >> 6;
   float c[LEN];
   float run = 0.f;
@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(GLA_THREADS) gla_chunk_outer_kernel(const __gr
                                                                       float* __restrict__ out_decay, int NT, int H,
                                                                       int logits, int* status) {
   extern __shared__ uint8_t smem_raw[];
+  __shared__ float totals[GLA_THREADS];
   constexpr int HD = NS * D;
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(GLA_THREADS) gla_chunk_outer_kernel(const __gr
   __syncthreads();
   ok = bars->failed == 0;
   if (ok) {
-    build_cumsum<GLA_THREADS>(sG, bmat, logits != 0);
+    build_cumsum<GLA_THREADS>(sG, bmat, totals, logits != 0);
     for (int idx = tid; idx < 512; idx += blockDim.x) {
       const int row = idx >> 3, ch = idx & 7;
       uint4* px = reinterpret_cast<uint4*>(sX + sw_off(row, ch));
@@ -218,6 +219,17 @@ __global__ void __launch_bounds__(256) gla_scan_kernel(const float* __restrict__
 // Every exponential of the form e^{b_t - r_j} then costs one multiply on top of e^{b_t - r_i} (i = sub-chunk of t),
 // which a thread computes once per element: the special-function unit was a quarter of the backward kernel's time.
 constexpr int FTAB_FLOATS = 4 * 4 * D;
+// The forward kernel only needs j < i (the diagonal is 1): row i (i - 1) / 2 + j.
+constexpr int FTAB_LOWER_FLOATS = 6 * D;
+
+__device__ __forceinline__ void build_factor_tables_lower(const float* bmat, float* ftab) {
+  for (int idx = threadIdx.x; idx < FTAB_LOWER_FLOATS; idx += blockDim.x) {
+    const int r = idx >> 6, d = idx & 63, i = r >= 3 ? 3 : (r >= 1 ? 2 : 1), j = r - i * (i - 1) / 2;
+    const float rj = j == 0 ? 0.f : bmat[(16 * j - 1) * BST + d];
+    ftab[idx] = __expf(bmat[(16 * i - 1) * BST + d] - rj);
+  }
+  __syncthreads();
+}
 constexpr int GL_FLOATS = 4 * D;
 
 __device__ __forceinline__ void build_factor_tables(const float* bmat, float* ftab, float* gl) {
@@ -241,12 +253,12 @@ __device__ __forceinline__ void build_factor_tables(const float* bmat, float* ft
   __syncthreads();
 }
 
-// The four Q~ tiles; with ZERO their rows before the sub-chunk are written as zeros. A thread reads and writes the same place
+// The four Q~ tiles; with ALL (and a whole factor table) their rows before the sub-chunk are written as zeros. A thread reads and writes the same place
 // of every tile, so an output tile may be the q or k tile itself.
 struct QTiles {
   uint8_t* t[4];
 };
-template <bool ZERO>
+template <bool ALL>
 __device__ __forceinline__ void build_score_operands(const uint8_t* sQ, const uint8_t* sK, const QTiles& sA, uint8_t* sKt,
                                                      uint8_t* sKe, const float* bmat, const float* ftab,
                                                      const float* gl) {
@@ -271,7 +283,7 @@ __device__ __forceinline__ void build_score_operands(const uint8_t* sQ, const ui
     for (int j = 0; j < 4; ++j) {
       if (j < jrow) {
         float f[8];
-        ld8(ftab + (jrow * 4 + j) * D + ch * 8, f);
+        ld8(ftab + (ALL ? jrow * 4 + j : jrow * (jrow - 1) / 2 + j) * D + ch * 8, f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = qe[i] * f[i];
       } else if (j == jrow) {
@@ -281,7 +293,7 @@ __device__ __forceinline__ void build_score_operands(const uint8_t* sQ, const ui
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = 0.f;
       }
-      if (ZERO || j <= jrow) *reinterpret_cast<uint4*>(sA.t[j] + off) = pack8(o);
+      if (ALL || j <= jrow) *reinterpret_cast<uint4*>(sA.t[j] + off) = pack8(o);
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) o[i] = k[i] * __expf(rj[i] - bt[i]);  // K~: k_s e^{r_j(s) - b_s}
@@ -311,20 +323,22 @@ __device__ __forceinline__ void issue_score_mmas(uint32_t tmem, uint32_t p_col, 
 // ------------------------------------------------------------------------------------------------
 // Phase 3 forward: o = Q~(0) S_c + mask(P) V
 // A CTA takes a chunk of a head and walks its key slices; the Q~ tiles replace the q and gate tiles, K~ the k tile, so that
-// two CTAs (NS = 2: 112 KB each) share an SM and one's loads hide behind the other's operand construction, which
-// bounds the kernel (98 us for 8192 tokens, 16 heads of 128: 2.1 TB/s). Rows of Q~(j) before sub-chunk j stay unwritten: they only reach scores that the mask discards.
+// three CTAs (NS = 1: 75 KB each) or two (NS = 2: 108 KB) share an SM and one's loads hide behind the others' operand
+// construction, which bounds the kernel (8192 tokens, 16 heads of 128: 96 us, 2.1 TB/s; a third CTA took 16 x 2048 tokens, 6 heads
+// of 64 from 83 to 65 us, 4 x 16384 from 160 to 125, 2.4 TB/s). Rows of Q~(j) before sub-chunk j stay unwritten: they only reach scores that the mask discards.
 // ------------------------------------------------------------------------------------------------
 template <int NS>
 struct FwdGeom {
   static constexpr int TILES = 5 + NS + NS * NS;  // Q K G | 2 more Q~ | V | S
-  static constexpr int SMEM = TILES * TILE + BMAT_BYTES + FTAB_FLOATS * 4 + 1024 + 256;
+  static constexpr int SMEM = TILES * TILE + BMAT_BYTES + FTAB_LOWER_FLOATS * 4 + 256;
   static constexpr int TMEM_COLS = NS == 1 ? 128 : 256;  // scores, outputs of each value slice
+  static constexpr int CTAS = NS == 1 ? 3 : 2;           // per SM
 };
 
 constexpr int FWD_THREADS = 256;
 
 template <int NS>
-__global__ void __launch_bounds__(FWD_THREADS) gla_fwd_out_kernel(const __grid_constant__ CUtensorMap tmQ,
+__global__ void __launch_bounds__(FWD_THREADS, FwdGeom<NS>::CTAS) gla_fwd_out_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                   const __grid_constant__ CUtensorMap tmK,
                                                                   const __grid_constant__ CUtensorMap tmV,
                                                                   const __grid_constant__ CUtensorMap tmG,
@@ -332,11 +346,9 @@ __global__ void __launch_bounds__(FWD_THREADS) gla_fwd_out_kernel(const __grid_c
                                                                   int kcol, int vcol, int gcol,
                                                                   __nv_bfloat16* __restrict__ out, long long out_ld,
                                                                   int ocol, int NT, int rows, int H, int logits, int* status) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem[];  // no static shared memory before it: the space is wanted whole
   constexpr int HD = NS * D;
   using G = FwdGeom<NS>;
-  const uint32_t raw = smem_u32(smem_raw);
-  uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint8_t* sQ = smem;
   uint8_t* sK = smem + TILE;
   uint8_t* sG = smem + 2 * TILE;
@@ -346,7 +358,7 @@ __global__ void __launch_bounds__(FWD_THREADS) gla_fwd_out_kernel(const __grid_c
   uint8_t* sP = smem + 4 * TILE;                  // once the score products have read Q~(3)
   float* bmat = reinterpret_cast<float*>(smem + G::TILES * TILE);
   float* ftab = bmat + C * BST;
-  Bars* bars = reinterpret_cast<Bars*>(smem + G::TILES * TILE + BMAT_BYTES + FTAB_FLOATS * 4);
+  Bars* bars = reinterpret_cast<Bars*>(smem + G::TILES * TILE + BMAT_BYTES + FTAB_LOWER_FLOATS * 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int chunk = blockIdx.x % NT, bh = blockIdx.x / NT, h = bh % H, b = bh / H;
 
@@ -394,8 +406,8 @@ __global__ void __launch_bounds__(FWD_THREADS) gla_fwd_out_kernel(const __grid_c
     __syncthreads();
     ok = bars->failed == 0;
     if (!ok) break;
-    build_cumsum<FWD_THREADS>(sG, bmat, logits != 0);
-    build_factor_tables(bmat, ftab, nullptr);
+    build_cumsum<FWD_THREADS>(sG, bmat, ftab, logits != 0);
+    build_factor_tables_lower(bmat, ftab);
     build_score_operands<false>(sQ, sK, sA, sK, nullptr, bmat, ftab, nullptr);
     fence_proxy_async_smem();
     __syncthreads();
@@ -513,6 +525,7 @@ __global__ void __launch_bounds__(BWD_THREADS) gla_bwd_main_kernel(
     int dkcol, __nv_bfloat16* __restrict__ dv, long long dv_ld, int dvcol, float* __restrict__ dgl_local,
     float* __restrict__ chunk_tot, int NT, int rows, int H, int logits, int nchunks, int* status, long long* dbg) {
   extern __shared__ uint8_t smem_raw[];
+  __shared__ float totals[BWD_THREADS];
   using G = BwdGeom<NS>;
   constexpr int HD = NS * D, NB = G::NB;
   const uint32_t raw = smem_u32(smem_raw);
@@ -647,7 +660,7 @@ __global__ void __launch_bounds__(BWD_THREADS) gla_bwd_main_kernel(
   const int quarter = warp & 3, c0 = (warp >> 2) * CPW;  // TMEM lane quarter / first column of this warp
   const int row = quarter * 16 + (lane & 15);        // accumulator row owned by this thread when lane < 16
   if (ok) {
-    build_cumsum<BWD_THREADS>(sG, bmat, logits != 0);
+    build_cumsum<BWD_THREADS>(sG, bmat, totals, logits != 0);
     build_factor_tables(bmat, ftab, gl);
     build_score_operands<true>(sQ, sK, sA, sKt, sKe, bmat, ftab, gl);  // also K_end[s] = k_s e^{b_C - b_s}
     if (!mbar_wait(&bars->v[vbuf], (uint32_t)((nth / NB) & 1)) || !mbar_wait(&bars->s[sbuf], (uint32_t)((it / NB) & 1)))
