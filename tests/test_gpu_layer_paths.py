@@ -282,3 +282,25 @@ def test_write_strengths_against_fp64(rows, dim, H):
     b64 = torch.sigmoid(x64 @ w64.t())
     dx64, dw64 = torch.autograd.grad(b64, (x64, w64), db.double())
     assert _rel(beta, b64) < 2e-6 and _rel(dx, dx64) < 2.0 ** -8 and _rel(dw, dw64) < 2.0 ** -8  # fp32 sums; bf16 gradients
+
+
+@pytest.mark.parametrize("rows,V,offset", [(1, 1, 0), (3, 7, 0), (2, 8191, 0), (4, 32000, 0), (2, 32001, 3)])
+def test_largest_of_rows_as_torch_orders_them(rows, V, offset):
+    from triune_b200 import ops
+
+    x = torch.randn(rows, V + offset, device="cuda").bfloat16()[:, offset:]
+    for change in ("none", "ties", "nan", "lowest", "zeros"):
+        y = x.clone() if offset == 0 else x
+        if change == "ties":
+            y[:, V // 3:] = 9.0
+        elif change == "nan":
+            y[:, V // 2] = float("nan")
+            y[:, V - 1] = float("nan")
+        elif change == "lowest":
+            y[:] = float("-inf")
+        elif change == "zeros":
+            y[:] = 0.0
+            y[:, 0] = -0.0
+        out = torch.full((rows, 1), -1, device="cuda")
+        ops.argmax_into(y, out)
+        assert torch.equal(out, y.float().cpu().argmax(-1, keepdim=True).cuda()), change

@@ -226,6 +226,16 @@ Tensor colsum(const Tensor& x, const c10::optional<Tensor>& out, bool bf16) {
   return res;
 }
 
+// out (int64, one value per row) = index of the largest value of each row of x [rows, V] bf16
+void argmax_rows(const Tensor& x, Tensor& out) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1 && x.size(1) > 0, "argmax_rows: [rows, V] bf16 rows");
+  TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kLong && out.is_contiguous() && out.numel() == x.size(0) &&
+                  out.get_device() == x.get_device(), "argmax_rows: int64 [rows]");
+  c10::cuda::CUDAGuard guard(x.device());
+  tb::launch_argmax_rows(bf(x), x.stride(0), (int)x.size(0), (int)x.size(1), reinterpret_cast<long long*>(out.data_ptr<int64_t>()),
+                         cur_stream());
+}
+
 Tensor gather_rows(const Tensor& src, const Tensor& row_src, const c10::optional<Tensor>& row_scale) {
   check_bf16_cuda(src, "src");
   TORCH_CHECK(src.dim() == 2 && src.is_contiguous() && src.size(1) % 8 == 0, "src must be [rows, width%8==0]");
@@ -453,6 +463,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("rope_apply", &rope_apply);
   m.def("embedding_bwd", &embedding_bwd);
+  m.def("argmax_rows", &argmax_rows);
   m.def("colsum", &colsum, pybind11::arg("x"), pybind11::arg("out"), pybind11::arg("bf16") = false);
   m.def("gather_rows", &gather_rows);
   m.def("combine_rows", &combine_rows);

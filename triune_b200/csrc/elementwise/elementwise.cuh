@@ -11,6 +11,8 @@ namespace tb {
 // y = rmsnorm(x [+ res]) * w ; if res != null also writes sum_out = x + res. d % 8 == 0, d <= 2048.
 void launch_rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
                         __nv_bfloat16* sum_out, float* rstd, int rows, int d, float eps, cudaStream_t s);
+// out[row] = index of the row's largest value (argmax.cu).
+void launch_argmax_rows(const __nv_bfloat16* x, long long ld, int rows, int V, long long* out, cudaStream_t s);
 // Where column sums go: fp32 (added to what is there with `add`), or bf16.
 struct ColumnSum {
   float* out;

@@ -21,6 +21,7 @@ from typing import Any, Callable, Dict, List, Optional, Tuple
 import torch
 import torch.nn.functional as F
 
+from . import ops
 from .config import ModelConfig
 from .models.layer_state import LayerState
 
@@ -394,7 +395,7 @@ class GraphedGreedyDecoder:
             if s is not None and isinstance(c, tuple) and c[0] is not None:
                 s.copy_(c[0])
         self.out.index_copy_(1, self.step_idx, self.token)
-        self.token.copy_(logits[:, -1].argmax(-1, keepdim=True))
+        ops.argmax_into(logits[:, -1], self.token)
         self.pos.add_(1)
         self.step_idx.add_(1)
 

@@ -342,6 +342,16 @@ def swiglu_mlp(x, w13, w2):
 # ----------------------------------------------------------------------------
 # RMSNorm
 # ----------------------------------------------------------------------------
+def argmax_into(logits: torch.Tensor, out: torch.Tensor) -> None:
+    """``out`` [rows, 1] = index of the largest value of each row of ``logits`` [rows, V] (as ``torch.argmax`` orders them)."""
+    if (_ext.use_kernels(logits, out) and _ext.ext_available() and logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.stride(1) == 1
+            and 0 < logits.shape[1] < 2 ** 31 and out.dtype == torch.long and out.is_contiguous()):
+        _ext.ext().argmax_rows(logits, out)
+        _tick(1)
+    else:
+        out.copy_(logits.argmax(-1, keepdim=True))
+
+
 def _rmsnorm_bwd(x, w, dy, rstd, dres):
     """(dx, dw); the weight's gradient goes into its ``main_grad`` where it has one (then None)."""
     mg = getattr(w, "main_grad", None)
