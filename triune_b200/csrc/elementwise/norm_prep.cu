@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(256) column_parts_kernel(const float* __restri
 // (token, head, q-or-k) row of D elements, handled by D/8 lanes with one 16-byte load each; the rotation
 // partner of element i (i + D/2) lives in lane ^ (D/16). out: [tokens, 2, H, D] contiguous. cos/sin: rows of
 // `tab_ld` floats of which D/2 are used, token t uses position (t % T) (tokens are laid out [B, T]); read in place and in 16-byte
-// vectors. Vectors are numbered in 32 bits: their division into token, head and side in 64 bits cost a seventh of the time (32768 tokens, 6 heads of 64, before ->
-// after: forward 35 -> 30 us, backward 50 -> 40; 8192 tokens, 8 heads of 128: 25 -> 22 and 36 -> 29).
+// vectors. Vectors are numbered in 32 bits: their division into token, head and side in 64 bits cost a seventh of
+// the time (32768 tokens, 6 heads of 64, before -> after: forward 35 -> 30 us, backward 50 -> 40; 8192 tokens, 8 heads of 128: 25 -> 22 and 36 -> 29).
 template <int D>
 struct PrepGeom {
   static constexpr int LPV = D / 8;        // lanes per vector

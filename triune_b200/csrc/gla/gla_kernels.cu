@@ -325,7 +325,8 @@ __device__ __forceinline__ void issue_score_mmas(uint32_t tmem, uint32_t p_col, 
 // A CTA takes a chunk of a head and walks its key slices; the Q~ tiles replace the q and gate tiles, K~ the k tile, so that
 // three CTAs (NS = 1: 75 KB each) or two (NS = 2: 108 KB) share an SM and one's loads hide behind the others' operand
 // construction, which bounds the kernel (8192 tokens, 16 heads of 128: 96 us, 2.1 TB/s; a third CTA took 16 x 2048 tokens, 6 heads
-// of 64 from 83 to 65 us, 4 x 16384 from 160 to 125, 2.4 TB/s). Rows of Q~(j) before sub-chunk j stay unwritten: they only reach scores that the mask discards.
+// of 64 from 83 to 65 us, 4 x 16384 from 160 to 125, 2.4 TB/s). Rows of Q~(j) before sub-chunk j stay unwritten: they only
+// reach scores that the mask discards.
 // ------------------------------------------------------------------------------------------------
 template <int NS>
 struct FwdGeom {
