@@ -92,6 +92,32 @@ def test_products_of_few_tiles_against_fp32(M, N, K, a_mn, b_mn, what):
     assert torch.isfinite(got.float()).all()
 
 
+@pytest.mark.parametrize("M,N", [(0, 1536), (0, 72), (40, 0), (0, 0)])
+@pytest.mark.parametrize("K", [1536, 8192])
+def test_empty_products_of_long_reductions_do_nothing(M, N, K):
+    from triune_b200 import ops
+
+    empty = lambda *s: torch.empty(*s, device="cuda", dtype=torch.bfloat16)
+    for b_mn in (False, True) if N else (False,):  # rows of no columns are no operand of the tensor maps
+        a, b = empty(M, K), empty(K, N) if b_mn else empty(N, K)
+        for dtype in (torch.bfloat16, torch.float32):
+            assert ops.gemm(a, b, b_mn=b_mn, out_dtype=dtype).shape == (M, N)
+        assert ops.gemm(a, b, b_mn=b_mn, gelu=True, aux_out=empty(M, N)).shape == (M, N)
+        assert ops.gemm(a, b, b_mn=b_mn, dgelu_aux=empty(M, N)).shape == (M, N)
+
+
+def test_layers_over_no_rows_train():
+    from triune_b200 import ops
+
+    w1, b1, w2, b2 = (torch.randn(*s, device="cuda").bfloat16().requires_grad_(True) for s in ((2048, 1536), (2048,), (1536, 2048), (1536,)))
+    x = torch.empty(0, 1536, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    y = ops.mlp_gelu(x, w1, b1, w2, b2)
+    assert y.shape == (0, 1536)
+    frozen = ops.linear(x, w1.detach())
+    (dx,) = torch.autograd.grad(frozen, x, torch.empty_like(frozen))
+    assert dx.shape == x.shape
+
+
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17])
 @pytest.mark.parametrize("N,K", [(8, 8), (24, 72), (200, 384), (4760, 264), (2048, 5632), (19008, 520)])
 def test_products_of_a_few_rows_against_fp32(M, N, K):

@@ -343,6 +343,7 @@ struct SplitPlan {
 };
 SplitPlan split_plan(const GemmArgs& a) {
   SplitPlan p{1, 0};
+  if (a.M <= 0 || a.N <= 0 || a.K <= 0) return p;  // asked for before the launch looks at the sizes: no tiles to divide by
   if (a.M <= SKINNY_MAX_M && !a.a_mn_major && !a.b_mn_major && !(a.flags & GF_OUT_F32) && a.aux_in == nullptr && a.aux_out == nullptr) return p;
   if (a.mode != GEMM_DENSE || a.batch > 1 || a.strideA != 0 || a.strideB != 0 || a.row_scale != nullptr ||
       (a.flags & (GF_ACCUMULATE | GF_SWIGLU | GF_DSWIGLU | GF_ADDAUX | GF_SPLIT_SLICES)))
