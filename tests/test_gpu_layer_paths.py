@@ -177,6 +177,58 @@ def test_mixer_step_against_a_64_bit_statement(B, H, D, delta, learn_beta, rope,
     assert _rel(y.reshape(B, dim), o @ m.out_proj.weight.double().t()) < 2.0 ** -7  # two bf16 roundings
 
 
+@pytest.mark.parametrize("position", [-1, 64, 10 ** 12])
+def test_mixer_step_outside_the_rotary_table_is_nan(position):
+    B, H, D = 2, 2, 64
+    qkvg, state = torch.randn(B, 4 * H * D, device="cuda").bfloat16(), torch.randn(B, H, D, D, device="cuda")
+    tables = tuple(torch.ones(64, D, device="cuda") for _ in range(2))
+    with torch.no_grad():
+        for where in (position, torch.tensor([position], device="cuda")):
+            out, after = gla_cuda.mixer_step(qkvg, tables, where, state.clone(), False)
+            assert torch.isnan(out).all() and torch.isnan(after).all()
+        out, after = gla_cuda.mixer_step(qkvg, tables, 63, state.clone(), False)
+        assert torch.isfinite(out).all() and torch.isfinite(after).all()
+
+
+@pytest.mark.parametrize("mixer", ["gla", "gated_deltanet"])
+def test_replayed_decoding_past_the_first_rotary_tables(mixer):
+    from triune_b200.config import ModelConfig
+    from triune_b200.inference import GraphedGreedyDecoder, GraphedSpeculativeDecoder, generate_tokens
+    from triune_b200.models import TriuneTransformer
+    from triune_b200.models.factory import build_model
+    from triune_b200.utils import place_model
+
+    V = 64
+    cfg = ModelConfig(family="universal", vocab_size=V, hidden_dim=128, num_layers=2, num_heads=2, head_dim=64, mixer=mixer, ffn="swiglu",
+                      dense_hidden=256, tie_embeddings=False, rope_max_seq_len=32).validate()
+    torch.manual_seed(0)
+    m = place_model(build_model(cfg), torch.device("cuda"), torch.bfloat16).eval()
+    with torch.no_grad():  # a model that is sure of its next token, so that bf16 ties decide nothing
+        emb = torch.randn(V, 128, device="cuda")
+        m.embed_tokens.weight.copy_(emb)
+        m.lm_head.weight.copy_(emb.roll(1, 0) * 0.25)
+    dec = GraphedGreedyDecoder(m)
+    for length, new in ((5, 40), (5, 20), (70, 100), (9, 3), (9, 1)):  # captures made before and after the tables grew
+        ids = torch.randint(0, V, (1, length), device="cuda")
+        want, cache, _ = generate_tokens(m, ids, new, temperature=0.0, repetition_penalty=1.0, count_penalty=0.0)
+        assert dec.generate(ids, new)[0, length:].tolist() == want
+        for a, b in zip(dec.states, cache):
+            assert _rel(a, b[0]) < 1e-5
+    tight = GraphedGreedyDecoder(m, max_positions=64)
+    rows = dec.rotary[0]._cos.shape[0]
+    with pytest.raises(ValueError, match="max_positions"):
+        tight.generate(ids, rows)
+    if mixer == "gla":
+        t = place_model(TriuneTransformer.from_config(ModelConfig(vocab_size=256, hidden_dim=128, num_layers=5, num_heads=2, head_dim=64, num_experts=4,
+                        top_k=1, router_prefix_layers=1, reflex_exit_layer=2, limbic_exit_layer=3, expert_hidden=128, dense_hidden=128)),
+                        torch.device("cuda"), torch.bfloat16).eval()
+        spec = GraphedSpeculativeDecoder(t, k_draft=3)
+        spec.prefill(ids)
+        for mod in spec.rotary:
+            mod.max_seq_len, mod._cos, mod._sin = 16, None, None
+        assert spec.generate(ids, 40).shape[1] == ids.shape[1] + 40
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("T", [2, 16, 17, 63, 64, 65, 191, 256])
 def test_gated_attention_of_any_length_against_fp64(T, D):

@@ -808,6 +808,38 @@ def test_graphed_speculative_decoder_equals_greedy_and_accepts_agreeing_drafts()
     assert int(spec2.rounds.item()) <= 8  # 23 tokens at 4 per round, checked every 8 rounds
 
 
+def test_decoders_size_the_rotary_tables_for_the_tokens_to_come():
+    """Requests that cross the end of the rotary tables decode like the eager loop, which grows them as it goes, in whatever
+    order short and long requests come; what is past ``max_positions`` and past the tables at hand is refused."""
+    from triune_b200.inference import GraphedGreedyDecoder, GraphedSpeculativeDecoder, generate_tokens
+    from triune_b200.models.rotary import RotaryEmbedding
+
+    def short_tables():
+        torch.manual_seed(3)
+        m = tiny().eval()
+        for mod in m.modules():
+            if isinstance(mod, RotaryEmbedding):
+                mod.max_seq_len = 16
+        return m
+
+    a, b = short_tables(), short_tables()
+    greedy, spec = GraphedGreedyDecoder(b), GraphedSpeculativeDecoder(b, k_draft=3)
+    for length, new in ((3, 13), (12, 10), (40, 30), (5, 60), (9, 1)):
+        prompt = torch.randint(0, 256, (1, length), generator=torch.Generator().manual_seed(length))
+        want, _, _ = generate_tokens(a, prompt, new, temperature=0.0, repetition_penalty=1.0, count_penalty=0.0)
+        assert greedy.generate(prompt, new)[0, length:].tolist() == want
+        assert spec.generate(prompt, new)[0, length:].tolist() == want
+    for kind in (GraphedGreedyDecoder, GraphedSpeculativeDecoder):
+        dec = kind(short_tables(), max_positions=20)
+        prompt = torch.arange(1, 13).unsqueeze(0)
+        assert dec.generate(prompt, 8).shape[1] == 20
+        rows = max(mod._cos.shape[0] for mod in dec.rotary)
+        assert dec.generate(prompt, rows - 12).shape[1] == rows  # rows that are there anyway
+        rows = max(mod._cos.shape[0] for mod in dec.rotary)      # (a speculative decoder's last rounds may have grown them)
+        with pytest.raises(ValueError, match="max_positions"):
+            dec.generate(prompt, rows - 11)
+
+
 def test_streaming_finds_the_layer_stack_of_foreign_models():
     """Layer streaming locates the block stack of models it did not build: Hugging Face style nesting, or any longest
     list of same-typed blocks; streamed layers of such a model still train."""

@@ -13,6 +13,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <stdexcept>
 #include <string>
 
@@ -80,9 +81,9 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
     for (int i = 0; i < QW; ++i) ss += norm[which * QW + i];
     const float inv = 1.f / fmaxf(sqrtf(ss), 1e-6f);
     if (p.cos != nullptr) {
-      long long pos = p.pos != nullptr ? *p.pos : p.pos_host;
-      pos = pos < 0 ? 0 : (pos < p.table_rows ? pos : p.table_rows - 1);  // never outside the table
-      const float cs = p.cos[pos * D + d], sn = p.sin[pos * D + d];
+      const long long pos = p.pos != nullptr ? *p.pos : p.pos_host;
+      const bool inside = pos >= 0 && pos < p.table_rows;  // past the table there is no rotation: NaN, never another row's
+      const float cs = inside ? p.cos[pos * D + d] : NAN, sn = inside ? p.sin[pos * D + d] : NAN;
       f = d < D / 2 ? f * cs - feat[which][d + D / 2] * sn : f * cs + feat[which][d - D / 2] * sn;
     }
     vec[which][d] = f * inv;

@@ -24,6 +24,7 @@ import torch.nn.functional as F
 from . import ops
 from .config import ModelConfig
 from .models.layer_state import LayerState
+from .models.rotary import RotaryEmbedding
 
 DEFAULT_STOPS = ("\nUser:", "\nSystem:", "User:", "Assistant:")
 
@@ -338,6 +339,17 @@ def _cut_at_stop(text: str, stop: Tuple[str, ...]) -> str:
     return text[:cut].strip()
 
 
+def _cover_positions(rotary: List[RotaryEmbedding], device, positions: int, limit: int, spare: int = 0) -> List[torch.Tensor]:
+    """The rotary tables, grown to the ``positions`` that a request reaches and ``spare`` ones that only discarded steps do. Tables
+    grow up to ``limit`` rows for a request; what is past that and past the rows already there is refused."""
+    for mod in rotary:
+        built = 0 if mod._cos is None or mod._cos.device != device else mod._cos.shape[0]
+        rows = max(limit, mod.max_seq_len, built)
+        if positions > rows:
+            raise ValueError(f"the request reaches position {positions - 1}, past the {rows} positions of this decoder (max_positions)")
+    return [t for mod in rotary for t in mod.tables(1, device, max(positions + spare, 1) - 1)]
+
+
 class GraphedGreedyDecoder:
     """Greedy decoding with the whole per-token step (all layers, exit head, arg-max, state update) captured in ONE
     CUDA graph and replayed once per token, with no host synchronisation until the requested tokens are done.
@@ -346,6 +358,9 @@ class GraphedGreedyDecoder:
     by launch latency and Python, not by the GPU. Everything that changes between steps lives in device memory: the
     current token, the position (RoPE rows are gathered by a device index), the recurrent states (updated in place) and
     the output buffer. On a CPU device the same step function runs eagerly, which is what the tests compare against.
+
+    ``max_positions`` bounds the rotary tables that a request may ask for beyond those that the prompt itself needed; a request
+    that goes past it is refused before a token is decoded.
     """
 
     def __init__(self, model, batch_size: int = 1, decode_depth: Optional[int] = 2, max_positions: int = 32768):
@@ -359,6 +374,8 @@ class GraphedGreedyDecoder:
         self.token = torch.zeros(batch_size, 1, dtype=torch.long, device=self.device)
         self.out: Optional[torch.Tensor] = None
         self.host_pos = 0
+        self.rotary: List[RotaryEmbedding] = []
+        self.tables: List[torch.Tensor] = []  # the rotary tables that the captured step reads; held, so they outlive a replacement
 
     @torch.no_grad()
     def prefill(self, input_ids: torch.Tensor, prefill_chunk: int = 4096) -> torch.Tensor:
@@ -369,10 +386,7 @@ class GraphedGreedyDecoder:
         logits = None
         for s in range(0, input_ids.shape[1], prefill_chunk):
             logits, cache = advance(m, input_ids[:, s : s + prefill_chunk], cache, self.depth, last_token_only=True)
-        # make sure every rotary table covers the positions the graph will index
-        for mod in m.modules():
-            if hasattr(mod, "_build") and hasattr(mod, "head_dim") and hasattr(mod, "_cos"):
-                mod(1, self.device, offset=min(self.max_positions, max(mod.max_seq_len, input_ids.shape[1] + 1)) - 1)
+        self.rotary = [mod for mod in m.modules() if isinstance(mod, RotaryEmbedding)]
         new_states = [c[0] if isinstance(c, tuple) else None for c in cache]
         if len(self.states) == len(new_states) and all((a is None) == (b is None) for a, b in zip(self.states, new_states)):
             for a, b in zip(self.states, new_states):
@@ -402,6 +416,10 @@ class GraphedGreedyDecoder:
     @torch.no_grad()
     def decode(self, max_new_tokens: int) -> torch.Tensor:
         """-> [B, max_new_tokens] token ids (the first one is the token ``prefill`` returned)."""
+        tables = _cover_positions(self.rotary, self.device, self.host_pos + max_new_tokens, self.max_positions)
+        if len(tables) != len(self.tables) or any(a is not b for a, b in zip(tables, self.tables)):
+            self.graph = None  # the capture reads the tables that were there before
+            self.tables = tables
         if self.out is None or self.out.shape[1] < max_new_tokens:
             self.out = torch.zeros(self.B, max_new_tokens, dtype=torch.long, device=self.device)
             self.graph = None
@@ -414,13 +432,13 @@ class GraphedGreedyDecoder:
             for _ in range(max_new_tokens):
                 self._step()
             return self.out[:, :max_new_tokens].clone()
-        if self.graph is None:
+        if self.graph is None and max_new_tokens > 0:
             # snapshot, warm up on a side stream (allocator and autotune effects must not land in the capture), restore
             snap = ([None if s is None else s.clone() for s in self.states], self.pos.clone(), self.token.clone())
             side = torch.cuda.Stream()
             side.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(side):
-                for _ in range(2):
+                for _ in range(min(2, max_new_tokens)):  # not past the output buffer or the rotary tables
                     self._step()
             torch.cuda.current_stream().wait_stream(side)
             g = torch.cuda.CUDAGraph()
@@ -478,6 +496,8 @@ class GraphedSpeculativeDecoder:
         self.rounds = torch.zeros(1, dtype=torch.long, device=dev)
         self.out: Optional[torch.Tensor] = None
         self.graph = None
+        self.rotary: List[RotaryEmbedding] = []
+        self.tables: List[torch.Tensor] = []  # as in GraphedGreedyDecoder
         self._ar = torch.arange(self.k + 1, device=dev)
 
     @torch.no_grad()
@@ -489,9 +509,7 @@ class GraphedSpeculativeDecoder:
         logits = None
         for s in range(0, input_ids.shape[1], prefill_chunk):
             logits, cache = m(input_ids[:, s : s + prefill_chunk], force_depth=2, cache=cache, last_token_only=True)
-        for mod in m.modules():
-            if hasattr(mod, "_build") and hasattr(mod, "head_dim") and hasattr(mod, "_cos"):
-                mod(1, self.device, offset=min(self.max_positions, max(mod.max_seq_len, input_ids.shape[1] + 1)) - 1)
+        self.rotary = [mod for mod in m.modules() if isinstance(mod, RotaryEmbedding)]
         new_states = [c[0] for c in cache[: self.n_layers]]
         if len(self.states) == len(new_states):
             for a, b in zip(self.states, new_states):
@@ -560,6 +578,12 @@ class GraphedSpeculativeDecoder:
     def decode(self, max_new_tokens: int, rounds_per_check: int = 8) -> torch.Tensor:
         """-> [1, max_new_tokens]; the first token is the one ``prefill`` returned."""
         need = max_new_tokens + self.k + 2
+        # rounds are checked `rounds_per_check` at a time: the last ones may run past the end, and drafts past the last one
+        past = (max(rounds_per_check, 2) + 1) * (self.k + 1)
+        tables = _cover_positions(self.rotary, self.device, int(self.pos.item()) + max_new_tokens, self.max_positions, past)
+        if len(tables) != len(self.tables) or any(a is not b for a, b in zip(tables, self.tables)):
+            self.graph = None
+            self.tables = tables
         if self.out is None or self.out.shape[1] < need:
             self.out = torch.zeros(1, need, dtype=torch.long, device=self.device)
             self.graph = None

@@ -63,8 +63,9 @@ class RotaryEmbedding(nn.Module):
         self._cos, self._sin = cos, sin
 
     def tables(self, seq_len: int, device, offset=0):
-        """The whole tables [rows, head_dim], grown to cover ``offset + seq_len`` positions where ``offset`` is a number (a
-        position on the device relies on the caller having sized them)."""
+        """The whole tables [rows, head_dim], grown to cover ``offset + seq_len`` positions where ``offset`` is a number. A
+        position on the device relies on the caller having sized them: past the last row :meth:`forward` raises or asserts, and a
+        decoding step that reads the tables itself gives NaN."""
         device = torch.device(device)
         length = max(self.max_seq_len, 1)
         if not torch.is_tensor(offset):
