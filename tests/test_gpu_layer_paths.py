@@ -177,6 +177,21 @@ def test_mixer_step_against_a_64_bit_statement(B, H, D, delta, learn_beta, rope,
     assert _rel(y.reshape(B, dim), o @ m.out_proj.weight.double().t()) < 2.0 ** -7  # two bf16 roundings
 
 
+@pytest.mark.parametrize("use_rope", [False, True])
+@pytest.mark.parametrize("dtype,device", [(torch.int32, "cuda"), (torch.int16, "cuda"), (torch.float32, "cuda"), (torch.int64, "cuda"), (torch.int64, "cpu")])
+def test_decoding_step_takes_positions_of_any_number_type(use_rope, dtype, device):
+    from triune_b200.models.attention import VectorisedGLA
+
+    if use_rope and device == "cpu":
+        pytest.skip("rotary rows are gathered on the device")
+    m = VectorisedGLA(128, 2, 64, use_rope=use_rope).cuda().bfloat16().eval()
+    x, s0 = torch.randn(2, 1, 128, device="cuda").bfloat16(), torch.randn(2, 2, 64, 64, device="cuda")
+    with torch.no_grad():
+        want, (state, _) = m(x, cache=(s0.clone(), 9))
+        got, (after, at) = m(x, cache=(s0.clone(), torch.tensor([9], dtype=dtype, device=device)))
+    assert torch.equal(got, want) and torch.equal(after, state) and float(at) == 10
+
+
 @pytest.mark.parametrize("position", [-1, 64, 10 ** 12])
 def test_mixer_step_outside_the_rotary_table_is_nan(position):
     B, H, D = 2, 2, 64

@@ -169,10 +169,16 @@ def mixer_step(qkvg, rope, offset, state, delta: bool, x=None, beta_w=None):
     """One decoding step from the fused projection rows in one launch -> (out [B, H*D] bf16, state after the step).
     ``rope``: (cos, sin) tables [rows, D] or None; ``offset``: position, an int or a device tensor. The 64-wide GLA state is
     updated in place, as :func:`decode_step` does; the others come back as a new tensor."""
-    cos, sin = rope if rope is not None else (None, None)
-    dev_pos = offset if torch.is_tensor(offset) else None
+    cos = sin = dev_pos = None
+    pos = 0
+    if rope is not None:
+        cos, sin = rope
+        if not torch.is_tensor(offset):
+            pos = int(offset)
+        else:
+            dev_pos = offset if offset.dtype == torch.long else offset.reshape(-1)[:1].long()
     inplace = not delta and state.shape[-1] == 64
-    out, new = _ext.ext().mixer_step(qkvg, cos, sin, dev_pos, 0 if dev_pos is not None else int(offset), state, inplace, delta, x, beta_w)
+    out, new = _ext.ext().mixer_step(qkvg, cos, sin, dev_pos, pos, state, inplace, delta, x, beta_w)
     _tick(1)
     return out, new
 
