@@ -177,6 +177,44 @@ def test_mixer_step_against_a_64_bit_statement(B, H, D, delta, learn_beta, rope,
     assert _rel(y.reshape(B, dim), o @ m.out_proj.weight.double().t()) < 2.0 ** -7  # two bf16 roundings
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("delta,learn_beta,on_device", [(False, False, True), (False, False, False), (True, False, True), (True, True, True)])
+def test_verified_tokens_are_the_decoded_ones(D, delta, learn_beta, on_device):
+    from triune_b200.models.attention import VectorisedGLA
+
+    torch.manual_seed(D)
+    B, T, H = 1, 4, 3
+    m = VectorisedGLA(H * D, H, D, use_delta_rule=delta, learn_beta=learn_beta).cuda().bfloat16().eval()
+    x, s0 = torch.randn(B, T, H * D, device="cuda").bfloat16(), torch.randn(B, H, D, D, device="cuda")
+    at = lambda i: torch.tensor([i], device="cuda") if on_device else i
+    with torch.no_grad():
+        kept = s0.clone()
+        y, states = m.forward_token_states(x, kept, at(11))
+        assert torch.equal(kept, s0)
+        state = s0.clone()
+        for j in range(T):
+            one, (state, _) = m(x[:, j : j + 1], cache=(state.clone(), at(11 + j)))
+            # products of up to 16 rows add a row's terms in one order, whatever the number of rows
+            assert torch.equal(states[j], state) and torch.equal(y[:, j : j + 1], one), j
+
+
+@pytest.mark.parametrize("mixer", ["gla", "gated_deltanet"])
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_replayed_speculation_gives_the_tokens_of_plain_greedy_decoding(mixer, head_dim):
+    from triune_b200.config import ModelConfig
+    from triune_b200.inference import GraphedGreedyDecoder, GraphedSpeculativeDecoder
+    from triune_b200.models import TriuneTransformer
+    from triune_b200.utils import place_model
+
+    torch.manual_seed(1)
+    cfg = ModelConfig(vocab_size=256, hidden_dim=2 * head_dim, num_layers=5, num_heads=2, head_dim=head_dim, num_experts=4, top_k=1,
+                      router_prefix_layers=1, reflex_exit_layer=2, limbic_exit_layer=3, expert_hidden=128, dense_hidden=128, mixer=mixer)
+    m = place_model(TriuneTransformer.from_config(cfg), torch.device("cuda"), torch.bfloat16).eval()
+    ids = torch.randint(0, 256, (1, 21), device="cuda")
+    want = GraphedGreedyDecoder(m).generate(ids, 48)
+    assert torch.equal(GraphedSpeculativeDecoder(m, k_draft=3).generate(ids, 48), want)
+
+
 @pytest.mark.parametrize("use_rope", [False, True])
 @pytest.mark.parametrize("dtype,device", [(torch.int32, "cuda"), (torch.int16, "cuda"), (torch.float32, "cuda"), (torch.int64, "cuda"), (torch.int64, "cpu")])
 def test_decoding_step_takes_positions_of_any_number_type(use_rope, dtype, device):

@@ -145,6 +145,21 @@ class VectorisedGLA(nn.Module):
     def g_proj(self):
         return _ProjView(self, 3)
 
+    def _plain_beta(self):
+        """(whether kernels may form the write strengths from the weight, that weight or None); a wrapped projection runs its own
+        forward."""
+        plain = self.beta_proj is None or type(self.beta_proj) is nn.Linear
+        return plain, self.beta_proj.weight if plain and self.beta_proj is not None else None
+
+    def _strengths(self, x: torch.Tensor, x2: torch.Tensor) -> Optional[torch.Tensor]:
+        """Write strengths [rows, heads] of the delta rule, or None (1)."""
+        if not self.use_delta_rule or self.beta_proj is None:
+            return None
+        plain, w = self._plain_beta()
+        if plain and gla_cuda.strength_supported(x2, w):
+            return gla_cuda.write_strength(x2, w)
+        return torch.sigmoid(self.beta_proj(x)).view(x2.shape[0], self.heads)
+
     def forward(self, x: torch.Tensor, cache=None):
         B, T, _ = x.shape
         H, D = self.heads, self.head_dim
@@ -152,8 +167,7 @@ class VectorisedGLA(nn.Module):
         lora = getattr(self, "qkvg_lora", None)  # set by the fine-tuner (FusedProjectionLoRA)
         x2 = x.reshape(B * T, self.dim)
         qkvg = lora(x2) if lora is not None else ops.linear(x2, self.qkvg_weight)
-        plain_beta = self.beta_proj is None or type(self.beta_proj) is nn.Linear  # wrapped ones run their own forward below
-        beta_w = self.beta_proj.weight if plain_beta and self.beta_proj is not None else None
+        plain_beta, beta_w = self._plain_beta()
         if T == 1 and plain_beta and gla_cuda.step_supported(qkvg, state, H, D, x2, beta_w):
             rope = self.rope.tables(1, x.device, offset) if self.use_rope else None
             out, new_state = gla_cuda.mixer_step(qkvg, rope, offset, state, self.use_delta_rule, x2, beta_w)
@@ -166,12 +180,7 @@ class VectorisedGLA(nn.Module):
             out, new_state = gla_cuda.gla_attention_core(qkvg, cos, sin, state, B, T, H)
             y = _project(self.out_proj, out.view(B, T, self.hidden_dim), self.out_scale)
             return y, format_cache(new_state if cache is not None else None, cache, fmt, offset, T)
-        beta = None
-        if self.use_delta_rule and self.beta_proj is not None:
-            if plain_beta and gla_cuda.strength_supported(x2, beta_w):
-                beta = gla_cuda.write_strength(x2, beta_w)
-            else:
-                beta = torch.sigmoid(self.beta_proj(x)).view(B * T, H)
+        beta = self._strengths(x, x2)
         if self.use_delta_rule and (beta is None or beta.dtype == torch.float32) and gla_cuda.gdn_core_supported(qkvg, T, D, beta):
             out, new_state = gla_cuda.gdn_attention_core(qkvg, cos, sin, beta, state, B, T, H)
             y = _project(self.out_proj, out.view(B, T, self.hidden_dim))
@@ -196,23 +205,34 @@ class VectorisedGLA(nn.Module):
         H, D = self.heads, self.head_dim
         x2 = x.reshape(B * T, self.dim)
         qkvg = ops.linear(x2, self.qkvg_weight)
-        cos = sin = None
-        if self.use_rope:
-            cos, sin = self.rope(T, x.device, offset=offset)
-        q, k, v, g = ops.qk_feature_map(qkvg, cos, sin, B, T, H, D)
-        beta = None
-        if self.use_delta_rule and self.beta_proj is not None:
-            beta = torch.sigmoid(self.beta_proj(x)).view(B, T, H)
         outs, states, s = [], [], state
-        for j in range(T):
-            sl = slice(j, j + 1)
-            if self.use_delta_rule:
-                o, s = ops.gated_deltanet(q[:, sl], k[:, sl], v[:, sl], g[:, sl], beta=None if beta is None else beta[:, sl],
-                                          initial_state=s, gate_logits=True)
-            else:
-                o, s = ops.gla(q[:, sl], k[:, sl], v[:, sl], g[:, sl], initial_state=s, gate_logits=True)
-            outs.append(o)
-            states.append(s)
+        plain_beta, beta_w = self._plain_beta()
+        rows = qkvg.view(B, T, 4 * self.hidden_dim)
+        if plain_beta and gla_cuda.step_supported(rows[:, 0], state, H, D, x[:, 0], beta_w):
+            # the kernel of single tokens, so that a verified token and a decoded one are the same numbers
+            rope = self.rope.tables(T, x.device, offset) if self.use_rope else None
+            at = offset.reshape(-1)[:1].long() + torch.arange(T, device=offset.device) if torch.is_tensor(offset) else range(offset, offset + T)
+            for j in range(T):
+                o, s = gla_cuda.mixer_step(rows[:, j], rope, at[j : j + 1] if torch.is_tensor(at) else at[j], s, self.use_delta_rule,
+                                           x[:, j], beta_w, keep_state=True)
+                outs.append(o.unsqueeze(1))
+                states.append(s)
+        else:
+            cos = sin = None
+            if self.use_rope:
+                cos, sin = self.rope(T, x.device, offset=offset)
+            q, k, v, g = ops.qk_feature_map(qkvg, cos, sin, B, T, H, D)
+            beta = self._strengths(x, x2)
+            beta = None if beta is None else beta.view(B, T, H)
+            for j in range(T):
+                sl = slice(j, j + 1)
+                if self.use_delta_rule:
+                    o, s = ops.gated_deltanet(q[:, sl], k[:, sl], v[:, sl], g[:, sl], beta=None if beta is None else beta[:, sl],
+                                              initial_state=s, gate_logits=True)
+                else:  # a 64-wide state is advanced in place on the GPU
+                    o, s = ops.gla(q[:, sl], k[:, sl], v[:, sl], g[:, sl], initial_state=None if s is None else s.clone(), gate_logits=True)
+                outs.append(o)
+                states.append(s)
         out = torch.cat(outs, dim=1).reshape(B, T, self.hidden_dim).to(x.dtype)
         y = _project(self.out_proj, out, 1.0 if self.use_delta_rule else self.out_scale)
         return y, torch.stack(states)

@@ -165,10 +165,10 @@ def step_supported(qkvg, state, H: int, D: int, x=None, beta_w=None) -> bool:
             and state.shape == (qkvg.shape[0], H, D, D))
 
 
-def mixer_step(qkvg, rope, offset, state, delta: bool, x=None, beta_w=None):
+def mixer_step(qkvg, rope, offset, state, delta: bool, x=None, beta_w=None, keep_state: bool = False):
     """One decoding step from the fused projection rows in one launch -> (out [B, H*D] bf16, state after the step).
     ``rope``: (cos, sin) tables [rows, D] or None; ``offset``: position, an int or a device tensor. The 64-wide GLA state is
-    updated in place, as :func:`decode_step` does; the others come back as a new tensor."""
+    updated in place, as :func:`decode_step` does, unless ``keep_state``; the others come back as a new tensor."""
     cos = sin = dev_pos = None
     pos = 0
     if rope is not None:
@@ -177,7 +177,7 @@ def mixer_step(qkvg, rope, offset, state, delta: bool, x=None, beta_w=None):
             pos = int(offset)
         else:
             dev_pos = offset if offset.dtype == torch.long else offset.reshape(-1)[:1].long()
-    inplace = not delta and state.shape[-1] == 64
+    inplace = not delta and state.shape[-1] == 64 and not keep_state
     out, new = _ext.ext().mixer_step(qkvg, cos, sin, dev_pos, pos, state, inplace, delta, x, beta_w)
     _tick(1)
     return out, new
