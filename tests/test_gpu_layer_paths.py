@@ -215,6 +215,36 @@ def test_replayed_speculation_gives_the_tokens_of_plain_greedy_decoding(mixer, h
     assert torch.equal(GraphedSpeculativeDecoder(m, k_draft=3).generate(ids, 48), want)
 
 
+@pytest.mark.parametrize("T,grad", [(1, False), (5, False), (70, True)])
+def test_a_write_strength_projection_with_hooks_or_a_bias_is_called(T, grad):
+    from triune_b200.models.attention import VectorisedGLA
+
+    torch.manual_seed(2)
+    m = VectorisedGLA(256, 2, 128, use_delta_rule=True, learn_beta=True).cuda().bfloat16()
+    x, cache = torch.randn(2, T, 256, device="cuda").bfloat16(), (torch.randn(2, 2, 128, 128, device="cuda"), 3)
+
+    def run():
+        with torch.set_grad_enabled(grad):
+            return m(x, cache=(cache[0].clone(), 3))[0].detach()
+
+    plain, seen = run(), []
+    for register in (m.beta_proj.register_forward_hook, m.beta_proj.register_forward_pre_hook,
+                     torch.nn.modules.module.register_module_forward_hook):
+        handle = register(lambda mod, *a: seen.append(mod is m.beta_proj) and None)
+        hooked = run()
+        handle.remove()
+        assert any(seen) and _rel(hooked, plain) < 0.01, register  # its own forward rounds the strength to bf16
+        seen.clear()
+    shut = m.beta_proj.register_forward_hook(lambda mod, a, out: out - 1e4)  # a strength of zero writes nothing
+    nothing = run()
+    shut.remove()
+    m.beta_proj.bias = torch.nn.Parameter(torch.full((2,), -1e4, device="cuda", dtype=torch.bfloat16))
+    assert torch.equal(run(), nothing) and _rel(nothing, plain) > 0.05
+    m.beta_proj.bias = None
+    m.beta_proj.forward = lambda a: torch.nn.functional.linear(a, m.beta_proj.weight) - 1e4
+    assert torch.equal(run(), nothing)
+
+
 @pytest.mark.parametrize("use_rope", [False, True])
 @pytest.mark.parametrize("dtype,device", [(torch.int32, "cuda"), (torch.int16, "cuda"), (torch.float32, "cuda"), (torch.int64, "cuda"), (torch.int64, "cpu")])
 def test_decoding_step_takes_positions_of_any_number_type(use_rope, dtype, device):

@@ -146,10 +146,15 @@ class VectorisedGLA(nn.Module):
         return _ProjView(self, 3)
 
     def _plain_beta(self):
-        """(whether kernels may form the write strengths from the weight, that weight or None); a wrapped projection runs its own
-        forward."""
-        plain = self.beta_proj is None or type(self.beta_proj) is nn.Linear
-        return plain, self.beta_proj.weight if plain and self.beta_proj is not None else None
+        """(whether kernels may form the write strengths from the weight, that weight or None). A projection with a bias, hooks or a
+        forward of its own is called as a module."""
+        m = self.beta_proj
+        if m is None:
+            return True, None
+        plain = (type(m) is nn.Linear and m.bias is None and "forward" not in vars(m)
+                 and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+                 and not nn.modules.module._has_any_global_hook())
+        return plain, m.weight if plain else None
 
     def _strengths(self, x: torch.Tensor, x2: torch.Tensor) -> Optional[torch.Tensor]:
         """Write strengths [rows, heads] of the delta rule, or None (1)."""
