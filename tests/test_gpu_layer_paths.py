@@ -431,6 +431,32 @@ def test_fused_delta_rule_rows_match_separate_tensors(T, D):
     assert torch.equal(got[0], want[0]) and _rel(got[1], want[1]) < 1e-6 and torch.equal(got[2], want[2])
 
 
+@pytest.mark.parametrize("H", [16, 17, 24])
+def test_training_pass_of_any_number_of_heads(H, monkeypatch):
+    from triune_b200 import ops
+    from triune_b200.models.attention import VectorisedGLA
+
+    torch.manual_seed(H)
+    B, T, D, dim = 2, 70, 64, 256
+    m = VectorisedGLA(dim, H, D, use_delta_rule=True, learn_beta=True, use_rope=False).cuda().bfloat16()
+    x, w = torch.randn(B, T, dim, device="cuda").bfloat16().requires_grad_(True), torch.randn(B, T, dim, device="cuda").bfloat16()
+    params = (x, m.qkvg_weight, m.beta_proj.weight, m.out_proj.weight)
+    core, taken = gla_cuda.gdn_attention_core, []
+    monkeypatch.setattr(gla_cuda, "gdn_attention_core", lambda *a: taken.append(1) or core(*a))
+    y = m(x)[0]
+    got = (y, *torch.autograd.grad(y, params, w))
+    assert taken
+    x2 = x.reshape(B * T, dim)
+    q, k, v, g = ops.qk_feature_map(ops.linear(x2, m.qkvg_weight), None, None, B, T, H, D)
+    beta = m._strengths(x, x2).view(B, T, H)
+    o = ops.gated_deltanet(q, k, v, g, beta=beta, gate_logits=True)[0]
+    y2 = ops.linear(o.reshape(B, T, H * D), m.out_proj.weight)
+    want = (y2, *torch.autograd.grad(y2, params, w))
+    # the same kernels on separate tensors; the strengths' gradients come from shared-memory atomics, whose order differs
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b) if i in (0, 2, 4) else _rel(a, b) < 2.0 ** -8, i
+
+
 @pytest.mark.parametrize("rows,dim,H", [(1, 8, 1), (15, 264, 6), (16, 384, 8), (33, 520, 9), (600, 2048, 16), (9000, 1024, 8)])
 def test_write_strengths_against_fp64(rows, dim, H):
     gen = torch.Generator(device="cuda").manual_seed(rows)

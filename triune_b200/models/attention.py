@@ -186,7 +186,8 @@ class VectorisedGLA(nn.Module):
             y = _project(self.out_proj, out.view(B, T, self.hidden_dim), self.out_scale)
             return y, format_cache(new_state if cache is not None else None, cache, fmt, offset, T)
         beta = self._strengths(x, x2)
-        if self.use_delta_rule and (beta is None or beta.dtype == torch.float32) and gla_cuda.gdn_core_supported(qkvg, T, D, beta):
+        if self.use_delta_rule and gla_cuda.gdn_core_supported(qkvg, T, D, beta):
+            beta = None if beta is None else beta.float().contiguous()  # whoever formed them: more heads than the kernel's, a wrapped projection
             out, new_state = gla_cuda.gdn_attention_core(qkvg, cos, sin, beta, state, B, T, H)
             y = _project(self.out_proj, out.view(B, T, self.hidden_dim))
             return y, format_cache(new_state if cache is not None else None, cache, fmt, offset, T)
