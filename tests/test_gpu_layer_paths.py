@@ -335,6 +335,29 @@ def test_gated_attention_of_any_length_against_fp64(T, D):
         assert _rel(a, b) < limit, (n, _rel(a, b))
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("T,at", [(21, 7), (63, 40), (70, 66), (127, 64)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+def test_gates_that_are_no_numbers_reach_what_depends_on_them(T, at, D, value):
+    B, H = 2, 2
+    q, k, v, g, s0 = _mixer_inputs(B, T, H, D, seed=T)
+    g[0, at, 1, 5] = value
+    ins = [t.requires_grad_(True) for t in (q, k, v, g, s0)]
+    o, s = gla_cuda._GLAFn.apply(*ins, True)
+    wo, ws = torch.randn_like(o), torch.randn_like(s)
+    got = (o, s, *torch.autograd.grad((o.float() * wo).sum() + (s * ws).sum(), ins))
+    x = [t.detach().double().requires_grad_(True) for t in ins]
+    gl = F.logsigmoid(x[3])
+    oo, ss = ref.gla_recurrent(*x[:3], gl if T < 64 else gl.clamp(min=gla_cuda.GLA_MIN_LOG_DECAY), x[4])
+    want = (oo, ss, *torch.autograd.grad((oo * wo.double()).sum() + (ss * ws.double()).sum(), x))
+    for n, a, b in zip(("o", "s", "dq", "dk", "dv", "dg", "ds0"), got, want):
+        if T >= 64 and n not in ("o", "s", "dq"):  # whole chunks spread the state's gradient over all that its products touch
+            a, b = a[:, 64:], b[:, 64:]
+            if n == "ds0":
+                continue
+        assert torch.equal(torch.isnan(a), torch.isnan(b)), n
+
+
 @pytest.mark.parametrize("T,D", [(21, 128), (150, 64), (150, 128)])
 def test_fused_projection_rows_match_separate_tensors(T, D):
     B, H = 2, 2

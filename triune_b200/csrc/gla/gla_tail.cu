@@ -48,8 +48,10 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 __device__ __forceinline__ float raw_decay(float x, int logits) {
-  return logits ? fminf(x, 0.f) - log1pf(__expf(-fabsf(x))) : fminf(x, 0.f);
+  return logits ? fminf(x, 0.f) - log1pf(__expf(-fabsf(x))) : (x > 0.f ? 0.f : x);
 }
+// Selections, not fmaxf: a gate that is not a number stays one, as in the PyTorch statements of these tokens.
+__device__ __forceinline__ float at_least(float decay, float floor) { return decay < floor ? floor : decay; }
 
 // Tokens [t, t + m) of `width` columns into dst[token][width] as fp32, optionally as decays e^{max(g, floor)}.
 __device__ __forceinline__ void stage(const __nv_bfloat16* src, long long ld, int m, int width, float* dst) {
@@ -67,7 +69,7 @@ __device__ __forceinline__ void stage_decay(const __nv_bfloat16* src, long long 
     float f[8];
     unpack8(*reinterpret_cast<const uint4*>(src + t * ld + c), f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = __expf(fmaxf(raw_decay(f[j], logits), floor));
+    for (int j = 0; j < 8; ++j) f[j] = __expf(at_least(raw_decay(f[j], logits), floor));
     st8(dst + t * width + c, f);
   }
 }
@@ -204,7 +206,7 @@ __global__ void __launch_bounds__(THREADS) gla_tail_keys_bwd_kernel(const TailAr
     __syncthreads();
     for (int t = m - 1; t >= 0; --t) {
       const float q = sq[t * WIDE + kr], k = sk[t * WIDE + kr], x = se[t * WIDE + kr];
-      const float decay = raw_decay(x, p.logits), e = __expf(fmaxf(decay, p.floor));
+      const float decay = raw_decay(x, p.logits), e = __expf(at_least(decay, p.floor));
       float v[RP], d[RP], acc = 0.f;
       read_run<RP>(sv + t * D, s, v);
       read_run<RP>(sd + t * D, s, d);
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(THREADS) gla_tail_keys_bwd_kernel(const TailAr
       if (s == 0) {
         suffix += qdq[(ta + t) * WIDE + kr] - k * acc;
         float slope = 0.f;
-        if (p.logits) slope = decay >= p.floor ? 1.f / (1.f + __expf(x)) : 0.f;
+        if (p.logits) slope = decay < p.floor ? 0.f : 1.f / (1.f + __expf(x));
         else slope = (x <= 0.f && x >= p.floor) ? 1.f : 0.f;
         sx[t * WIDE + kr] = acc;
         sy[t * WIDE + kr] = suffix * slope;
