@@ -35,6 +35,22 @@ def test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims):
     assert _rel(s, ss) < 1e-6        # the state is fp32 throughout
 
 
+@pytest.mark.parametrize("T,at,D", [(8, 5, 64), (19, 9, 128), (70, 33, 64)])
+@pytest.mark.parametrize("where", ["v", "k", "q", "beta"])
+def test_delta_rule_prompts_keep_what_is_no_number_from_earlier_tokens(T, at, D, where):
+    q, k, v, g, s0 = _mixer_inputs(2, T, 2, D)
+    beta = torch.rand(2, T, 2, device="cuda")
+    clean, _ = gla_cuda.gdn_recurrent(q, k, v, g, beta, s0, 1.0, True)
+    for value in (float("nan"), float("inf")):
+        x = {"q": q.clone(), "k": k.clone(), "v": v.clone(), "beta": beta.clone()}
+        x[where][(0, at, 1) if where == "beta" else (0, at, 1, 3)] = value
+        o, s = gla_cuda.gdn_recurrent(x["q"], x["k"], x["v"], g, x["beta"], s0, 1.0, True)
+        oo, ss = ref.gated_deltanet_recurrent(*(x[n].double() for n in "qkv"), F.logsigmoid(g.double()).clamp(min=gla_cuda.GLA_MIN_LOG_DECAY),
+                                              x["beta"].double(), s0.double(), 1.0)
+        assert torch.equal(o[:, :at], clean[:, :at])
+        assert torch.equal(torch.isfinite(o), torch.isfinite(oo)) and torch.equal(torch.isfinite(s), torch.isfinite(ss))
+
+
 def test_a_thread_without_a_context_of_its_own_runs_tensor_map_kernels():
     import threading
 

@@ -408,7 +408,8 @@ __global__ void __launch_bounds__(128) gdn_block_walk_kernel(const float* __rest
           const float* a = tri + GB * GB + (j + e) * GB;
           float o = val[e];
 #pragma unroll
-          for (int m = 0; m < GB; ++m) o += a[m] * (col ? u[1][m] : u[0][m]);
+          for (int m = 0; m < GB; ++m)
+            if (m <= j + e) o += a[m] * (col ? u[1][m] : u[0][m]);  // later tokens are left out, not multiplied by zero: they may be infinite
           out[(row0 + t) * o_ld + ocol + h * D + c0 + col] = __float2bfloat16(o * scale);
         }
       }
