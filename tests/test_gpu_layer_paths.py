@@ -448,6 +448,35 @@ def test_delta_rule_training_of_any_length_against_fp64(T, D, with_beta):
         assert _rel(a, b) < limit, (n, _rel(a, b))
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38])
+def test_state_pass_of_the_delta_rule_keeps_infinite_states_infinite(D, value):
+    """As fp32 arithmetic has it: in the column of an infinite element of the initial state the effective values are infinite with the
+    other sign (equal keys, small strengths and open gates, so that every token reads it with one sign), and so are the rows that
+    keys add them to; the element itself is no number then."""
+    from triune_b200 import ops
+
+    B, T, H = 1, 64, 2
+    q, k, v, g, s0 = _mixer_inputs(B, T, H, D, seed=D)
+    s0[0, 1, 7, 9] = value
+    g.fill_(20.0)
+    k.fill_(D ** -0.5)
+    beta = torch.full((B, T, H), 0.01, device="cuda")
+    o, s = ops.gated_deltanet(q.requires_grad_(True), k, v, g, beta=beta, initial_state=s0, gate_logits=True)
+    clean = ops.gated_deltanet(q, k, v, g, beta=beta, initial_state=torch.where(torch.isfinite(s0) & (s0.abs() < 1e38), s0, 0.0), gate_logits=True)[1]
+    touched = torch.zeros_like(s, dtype=torch.bool)
+    touched[0, 1, :, 9] = True
+    assert torch.equal(s[~touched], clean[~touched])
+    column = s[0, 1, :, 9]
+    others = torch.arange(D, device="cuda") != 7
+    if value != value:
+        assert torch.isnan(column).all()
+    elif value == 3.0e38:
+        assert not torch.isnan(column).any()
+    else:
+        assert torch.isinf(column[others]).all() and (torch.sign(column[others]) == -torch.sign(torch.tensor(value))).all()
+
+
 @pytest.mark.parametrize("T,D", [(21, 128), (150, 64), (128, 128)])
 def test_fused_delta_rule_rows_match_separate_tensors(T, D):
     from triune_b200 import ops

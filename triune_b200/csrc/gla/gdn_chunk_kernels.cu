@@ -25,6 +25,7 @@
 // Replaces the reference's Python chunk loop and Triton forward (triune/kernels/fast_gla.py:382-550, 781-836).
 #include <cuda.h>
 
+#include <cmath>
 #include <stdexcept>
 #include <string>
 
@@ -472,14 +473,18 @@ __device__ __forceinline__ void mma_step(float (&c)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 // x = hi + mid + lo in bf16 with an error below 2^-26 |x| (each part takes eight bits of the rest, which is exact in fp32);
-// two neighbours at once, stored `part` elements apart.
+// two neighbours at once, stored `part` elements apart. What rounds to an infinite first part has no rest (inf - inf is no number).
+__device__ __forceinline__ float rest_of(float x, uint32_t part_bits) {
+  const float part = __uint_as_float(part_bits);
+  return fabsf(part) == INFINITY ? 0.f : x - part;
+}
 __device__ __forceinline__ void store_parts(__nv_bfloat16* dst, int part, float x0, float x1) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const uint32_t u = pack_bf16x2(x0, x1);
     *reinterpret_cast<uint32_t*>(dst + i * part) = u;
-    x0 -= __uint_as_float(u << 16);
-    x1 -= __uint_as_float(u & 0xffff0000u);
+    x0 = rest_of(x0, u << 16);
+    x1 = rest_of(x1, u & 0xffff0000u);
   }
 }
 
