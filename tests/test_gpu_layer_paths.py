@@ -374,6 +374,30 @@ def test_gates_that_are_no_numbers_reach_what_depends_on_them(T, at, D, value):
         assert torch.equal(torch.isnan(a), torch.isnan(b)), n
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_wider_operands_are_not_rounded_after_the_last_chunk(D):
+    from triune_b200 import ops
+
+    B, T, H = 2, 100, 2
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    q, k, v = F.normalize(rnd(B, T, H, D), dim=-1).bfloat16(), F.normalize(rnd(B, T, H, D), dim=-1), rnd(B, T, H, D)
+    g = -0.05 * torch.rand(B, T, H, D, device="cuda", generator=gen)  # fp32 log decays, keys and values beside bf16 queries
+    k, v, g = (t.requires_grad_(True) for t in (k, v, g))
+    o, s = ops.gla(q, k, v, g)
+    ds = torch.randn_like(s)
+    got = (s, *(t[:, 64:] for t in torch.autograd.grad(s, (k, v, g), ds)))
+    x = [t.detach().double() for t in (q, k, v, g)]
+    with torch.no_grad():
+        _, s64 = ops.gla(*(t[:, :64] for t in (q, k, v, g)))
+    tail = [t[:, 64:].clone().requires_grad_(True) for t in x[1:]]
+    oo, ss = ref.gla_recurrent(x[0][:, 64:], *tail, s64.double())
+    want = (ss, *torch.autograd.grad(ss, tail, ds.double()))
+    for n, a, b in zip(("s", "dk", "dv", "dg"), got, want):
+        assert _rel(a, b) < 1e-5, (n, _rel(a, b))  # fp32 throughout: rounded operands are 2^-9 off
+    assert _rel(o[:, 64:], oo) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("T,D", [(21, 128), (150, 64), (150, 128)])
 def test_fused_projection_rows_match_separate_tensors(T, D):
     B, H = 2, 2

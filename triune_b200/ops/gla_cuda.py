@@ -98,13 +98,23 @@ class _GLAFn(torch.autograd.Function):
 
 def gla_chunk(q, k, v, g, initial_state, scale, gate_logits):
     """Kernel path of ``ops.gla`` for T >= 64, or one token with a state. The last T % 64 tokens are walked in fp32."""
+    from . import reference as ref
+
     B, T, H, D = q.shape
     square = D == v.shape[-1]
     if not (square and (D == 64 or (D == 128 and T > 1))):
         return _gla_wide_heads(q, k, v, g, initial_state, scale, gate_logits)
     if T == 1:
         return decode_step(q, k, v, g, initial_state, gate_logits)
-    out, state = _GLAFn.apply(q, k, v, g, initial_state, gate_logits)
+    Tm = T // 64 * 64
+    if Tm == T or all(t.dtype == torch.bfloat16 for t in (k, v, g)):
+        out, state = _GLAFn.apply(q, k, v, g, initial_state, gate_logits)
+    else:  # whole chunks round their operands to bf16, the tokens after them do not: the reference op finishes wider ones
+        out, state = _GLAFn.apply(q[:, :Tm], k[:, :Tm], v[:, :Tm], g[:, :Tm], initial_state, gate_logits)
+        gl = torch.nn.functional.logsigmoid(g[:, Tm:].float()) if gate_logits else g[:, Tm:].float()
+        gl = gl.clamp(min=GLA_MIN_LOG_DECAY, max=0.0)
+        o2, state = ref.gla_chunk(q[:, Tm:], k[:, Tm:], v[:, Tm:], gl, state, 1.0)
+        out = torch.cat((out, o2.to(out.dtype)), dim=1)
     if scale != 1.0:
         out = out * scale
     return out, state
