@@ -154,6 +154,31 @@ def test_products_of_a_few_rows_against_fp32(M, N, K):
         assert _rel(h, F.silu(gate) * up) < 2.0 ** -8
 
 
+def test_kernels_without_an_autograd_function_refuse_tangents_and_survive_a_trace():
+    import torch.autograd.forward_ad as fw
+
+    from triune_b200 import ops
+    from triune_b200.models.attention import VectorisedGLA
+
+    rnd = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    x, w13, w2, wide, b1, b2 = rnd(5, 128), rnd(512, 128), rnd(128, 256), rnd(128, 512), rnd(512), rnd(128)
+    m = VectorisedGLA(128, 2, 64).cuda().bfloat16().eval()
+    state = torch.randn(5, 2, 64, 64, device="cuda")
+    calls = (lambda a: ops.swiglu_mlp(a, w13, w2), lambda a: ops.mlp_gelu(a, w13, b1, wide, b2),
+             lambda a: m(a.unsqueeze(1), cache=(state.clone(), 3))[0])
+    with torch.no_grad():
+        for call in calls:
+            want = call(x)
+            with fw.dual_level():
+                assert _rel(call(x), want) < 2.0 ** -7  # a single token takes its general path here
+                with pytest.raises(NotImplementedError):
+                    call(fw.make_dual(x, torch.ones_like(x)))
+        for call in calls[:2]:
+            traced = torch.jit.trace(call, (x,), check_trace=False)
+            y = rnd(5, 128)
+            assert torch.equal(traced(y), call(y))
+
+
 @pytest.mark.parametrize("B,H,D,delta,learn_beta,rope,on_device", [
     (1, 1, 64, False, False, True, False), (3, 2, 64, False, False, False, True), (2, 3, 128, False, False, True, True),
     (1, 2, 128, True, True, True, False), (5, 1, 64, True, False, True, True), (2, 4, 64, True, True, False, False),

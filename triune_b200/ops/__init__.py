@@ -17,6 +17,7 @@ from typing import Optional, Tuple
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from .. import _ext
 from . import reference as ref
@@ -223,10 +224,16 @@ def _wants_grad(*tensors) -> bool:
     return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
 
 
+def inference_call(*tensors) -> bool:
+    """True where kernels may run outside an autograd function: no gradient is wanted, no forward-mode level is open (the function
+    refuses tangents, a bare kernel would drop them) and nothing is traced (a trace records the function, not the kernels)."""
+    return not (_wants_grad(*tensors) or forward_ad._current_level >= 0 or torch.jit.is_tracing())
+
+
 def mlp_gelu(x, w1, b1, w2, b2):
     """Dense FFN: gelu_tanh(x w1^T + b1) w2^T + b2."""
     if _ext.use_kernels(x, w1, w2) and x.dtype == torch.bfloat16 and b1 is not None and b2 is not None:
-        if not _wants_grad(x, w1, b1, w2, b2):
+        if inference_call(x, w1, b1, w2, b2):
             # inference: the GELU epilogue skips the derivative tile (half the bytes written by the first GEMM)
             K = x.shape[-1]
             x2 = x.reshape(-1, K)
@@ -325,7 +332,7 @@ def swiglu_mlp(x, w13, w2):
     H = w13.shape[0] // 2
     if (_ext.use_kernels(x, w13, w2) and x.dtype == torch.bfloat16 and H % 32 == 0 and w13.shape[1] % 8 == 0
             and w2.shape[0] % 8 == 0 and w13.is_contiguous() and w2.is_contiguous()):
-        if not _wants_grad(x, w13, w2):
+        if inference_call(x, w13, w2):
             # inference: the pre-activations of the backward pass are not written, and few rows take the streaming product
             x2 = x.reshape(-1, x.shape[-1])
             if not _tma_ok(x2):

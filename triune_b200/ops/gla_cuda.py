@@ -15,6 +15,7 @@ import os
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad
 
 from .. import _ext
 
@@ -170,7 +171,8 @@ def step_supported(qkvg, state, H: int, D: int, x=None, beta_w=None) -> bool:
     """True when :func:`mixer_step` covers a single token: bf16 projection rows, head dim 64 or 128, fp32 state, no gradient."""
     if beta_w is not None and not (beta_w.is_cuda and beta_w.is_contiguous() and _aligned_rows(beta_w) and _aligned_rows(x)):
         return False
-    return (_ext.use_kernels(qkvg, state) and not torch.is_grad_enabled() and torch.is_tensor(state) and D in (64, 128)
+    return (_ext.use_kernels(qkvg, state) and not torch.is_grad_enabled() and forward_ad._current_level < 0 and torch.is_tensor(state)
+            and D in (64, 128)
             and _aligned_rows(qkvg) and state.dtype == torch.float32 and state.is_contiguous()
             and state.shape == (qkvg.shape[0], H, D, D))
 
