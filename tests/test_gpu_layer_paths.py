@@ -441,6 +441,30 @@ def test_fused_projection_rows_match_separate_tensors(T, D):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
+def _off_by_one(t):  # the same values, contiguous, four or two bytes past a 16-byte boundary
+    flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    return flat[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("T,D", [(1, 64), (9, 64), (9, 128)])
+def test_rotary_tables_and_gradients_of_any_alignment(T, D):
+    from triune_b200 import ops
+
+    B, H = 2, 2
+    x = torch.randn(B * T, 4 * H * D, device="cuda").bfloat16().requires_grad_(True)
+    cos, sin = ops.rope_tables(T, D, 10000.0, 0, x.device)
+    odd = torch.randn(T, D + 3, device="cuda")[:, :D].copy_(cos)  # rows of an odd pitch
+    want = ops.qk_feature_map(x, cos, sin, B, T, H, D)
+    for c, s in ((_off_by_one(cos), _off_by_one(sin)), (odd, sin), (cos[:, : D // 2].clone(), sin[:, : D // 2].clone())):
+        assert all(torch.equal(a, b) for a, b in zip(ops.qk_feature_map(x, c, s, B, T, H, D), want))
+    if T > 1:
+        beta, d = torch.rand(B * T, H, device="cuda"), torch.randn(B * T, H * D, device="cuda").bfloat16()
+        for core in (lambda: gla_cuda.gla_attention_core(x, cos, sin, None, B, T, H)[0],
+                     lambda: gla_cuda.gdn_attention_core(x, cos, sin, beta, None, B, T, H)[0]):
+            a, b = (torch.autograd.grad(core(), x, g)[0] for g in (d, _off_by_one(d)))
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("rows,d", [(1, 8), (1, 2048), (7, 264), (37, 1536), (1185, 384), (1184, 776), (2375, 2040), (9480, 512), (5000, 1032)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_norm_rows_against_fp64(rows, d, residual):

@@ -520,7 +520,7 @@ def half_tables(cos, sin, D: int):
         return None, None
     cs, sn = (t[:, : D // 2].float() for t in (cos, sin))
     if any(t.stride(1) != 1 or t.stride(0) % 4 != 0 or t.stride(0) != cs.stride(0) or t.data_ptr() % 16 != 0 for t in (cs, sn)):
-        cs, sn = cs.contiguous(), sn.contiguous()
+        cs, sn = (t.clone(memory_format=torch.contiguous_format) for t in (cs, sn))  # also where they are contiguous, but not aligned
     return cs, sn
 
 

@@ -163,6 +163,11 @@ def decode_step(q, k, v, g, state, gate_logits):
     return out.view(B, 1, H, D), st
 
 
+def _aligned_copy(t):
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _aligned_rows(t) -> bool:
     return t.dtype == torch.bfloat16 and t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
 
@@ -285,7 +290,7 @@ class _GDNCoreFn(torch.autograd.Function):
         B, T, H, D, has_init = ctx.dims
         HD = H * D
         e = _ext.ext()
-        dout = qkvg.new_zeros(B * T, HD) if dout is None else dout.contiguous()
+        dout = qkvg.new_zeros(B * T, HD) if dout is None else _aligned_copy(dout)
         dqk, dqkvg = torch.empty_like(qk), torch.empty_like(qkvg)
         dfl = dfin.float().reshape(B * H, D, D).contiguous() if dfin is not None else None
         dbeta, ds0, status = e.gdn_chunk_bwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, dout, 0, beta, dfl, list(saved), dqk, 0, dqk, HD,
@@ -394,7 +399,7 @@ class _GLACoreFn(torch.autograd.Function):
         B, T, H, D, grad_init = ctx.dims
         HD = H * D
         e = _ext.ext()
-        dout = qkvg.new_zeros(B * T, HD) if dout is None else dout.contiguous()
+        dout = qkvg.new_zeros(B * T, HD) if dout is None else _aligned_copy(dout)
         dqk = torch.empty_like(qk)
         dqkvg = torch.empty_like(qkvg)
         status, dinit = e.gla_bwd(qk, 0, qk, HD, qkvg, 2 * HD, qkvg, 3 * HD, dout, 0, states, decay, dqk, 0, dqk, HD, dqkvg,
