@@ -423,6 +423,32 @@ def test_wider_operands_are_not_rounded_after_the_last_chunk(D):
     assert _rel(o[:, 64:], oo) < 2.0 ** -8
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_many_sequences_and_none(D):
+    from triune_b200.models.attention import VectorisedGLA
+
+    B, T, H = 65539, 2, 1
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    x = torch.randn(B * T, 4 * H * D, device="cuda", generator=gen).bfloat16().requires_grad_(True)
+    ends = torch.tensor([0, 1, 65534, 65535, 65536, 65538], device="cuda")  # past the largest grid dimension that is not x
+    few = x.detach().view(B, T, -1)[ends].reshape(-1, 4 * H * D).requires_grad_(True)
+    w = torch.randn(B * T, H * D, device="cuda", generator=gen).bfloat16()
+    o, s = gla_cuda.gla_attention_core(x, None, None, None, B, T, H)
+    (dx,) = torch.autograd.grad(o, x, w)
+    oo, ss = gla_cuda.gla_attention_core(few, None, None, None, len(ends), T, H)
+    (want,) = torch.autograd.grad(oo, few, w.view(B, T, -1)[ends].reshape(-1, H * D))
+    pick = lambda t: t.view(B, T, -1)[ends].reshape(len(ends) * T, -1)
+    assert torch.equal(pick(o), oo) and torch.equal(s[ends], ss) and torch.equal(pick(dx), want)
+    with torch.no_grad():
+        rows = x.detach()[:B]
+        o, s = gla_cuda.mixer_step(rows, None, 0, s, False, keep_state=True)
+        oo, ss = gla_cuda.mixer_step(rows[ends], None, 0, ss, False, keep_state=True)
+        assert torch.equal(o[ends], oo) and torch.equal(s[ends], ss)
+        m = VectorisedGLA(D, 1, D).cuda().bfloat16().eval()
+        y, (state, at) = m(torch.empty(0, 5, D, device="cuda", dtype=torch.bfloat16), cache=(None, 0))
+        assert y.shape == (0, 5, D) and state.shape == (0, 1, D, D) and at == 5
+
+
 @pytest.mark.parametrize("T,D", [(21, 128), (150, 64), (150, 128)])
 def test_fused_projection_rows_match_separate_tensors(T, D):
     B, H = 2, 2

@@ -100,9 +100,9 @@ template <int D, bool REV>
 __global__ void __launch_bounds__(THREADS) gla_tail_values_kernel(const TailArgs p) {
   constexpr int RP = D / 8;
   __shared__ __align__(16) float sk[TT * D], sq[TT * D], se[TT * D], sv[TT * WIDE], so[TT * WIDE];
-  const int c0 = blockIdx.x * WIDE, h = blockIdx.y, b = blockIdx.z;
+  const int c0 = (blockIdx.x % (D / WIDE)) * WIDE, h = blockIdx.y, b = blockIdx.x / (D / WIDE);
   const int col = threadIdx.x >> 3, s = threadIdx.x & 7;
-  const long long row0 = (long long)b * p.rows + p.t0, sat = (long long)(b * p.H + h) * D * D + c0 + col;
+  const long long row0 = (long long)b * p.rows + p.t0, sat = ((long long)b * p.H + h) * D * D + c0 + col;
   const float* init = REV ? p.dstate1 : p.state0;
   float S[RP];
 #pragma unroll
@@ -155,9 +155,9 @@ __global__ void __launch_bounds__(THREADS) gla_tail_keys_bwd_kernel(const TailAr
   constexpr int RP = D / 8;
   __shared__ __align__(16) float sv[TT * D], sd[TT * D], sk[TT * WIDE], sq[TT * WIDE], se[TT * WIDE], sx[TT * WIDE], sy[TT * WIDE];
   __shared__ float qdq[64 * WIDE];
-  const int r0 = blockIdx.x * WIDE, h = blockIdx.y, b = blockIdx.z;
+  const int r0 = (blockIdx.x % (D / WIDE)) * WIDE, h = blockIdx.y, b = blockIdx.x / (D / WIDE);
   const int kr = threadIdx.x >> 3, s = threadIdx.x & 7;
-  const long long row0 = (long long)b * p.rows + p.t0, hat = (long long)(b * p.H + h) * D + r0 + kr, sat = hat * D;
+  const long long row0 = (long long)b * p.rows + p.t0, hat = ((long long)b * p.H + h) * D + r0 + kr, sat = hat * D;
   const int tiles = (p.n + TT - 1) / TT, hc = h * D + r0;
   float S[RP];
 #pragma unroll
@@ -259,10 +259,11 @@ void launched(const char* what) {
 
 void launch_gla_tail_fwd(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const GlaMat& O, const float* state0,
                          float* state1, const GlaTail& t, cudaStream_t s) {
+  if (t.B <= 0 || t.H <= 0) return;
   TailArgs a = tail_args(Q, K, V, G, t);
   a.out = at_out(O), a.out_ld = O.ld;
   a.state0 = state0, a.state1 = state1;
-  const dim3 grid(t.D / WIDE, t.H, t.B);
+  const dim3 grid((unsigned)t.B * (t.D / WIDE), t.H);  // sequences along x: the other two dimensions end at 65535
   if (t.D == 64) gla_tail_values_kernel<64, false><<<grid, THREADS, 0, s>>>(a);
   else gla_tail_values_kernel<128, false><<<grid, THREADS, 0, s>>>(a);
   launched("gla_tail_fwd");
@@ -271,12 +272,13 @@ void launch_gla_tail_fwd(const GlaMat& Q, const GlaMat& K, const GlaMat& V, cons
 void launch_gla_tail_bwd(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const GlaMat& dO, const GlaMat& dQ,
                          const GlaMat& dK, const GlaMat& dV, const GlaMat& dG, const float* state0, const float* dstate1,
                          const float* end1, float* dstate0, float* end0, const GlaTail& t, cudaStream_t s) {
+  if (t.B <= 0 || t.H <= 0) return;
   TailArgs a = tail_args(Q, K, V, G, t);
   a.dout = at(dO), a.do_ld = dO.ld;
   a.dq = at_out(dQ), a.dk = at_out(dK), a.dv = at_out(dV), a.dg = at_out(dG);
   a.dq_ld = dQ.ld, a.dk_ld = dK.ld, a.dv_ld = dV.ld, a.dg_ld = dG.ld;
   a.state0 = state0, a.dstate1 = dstate1, a.end1 = end1, a.dstate0 = dstate0, a.end0 = end0;
-  const dim3 grid(t.D / WIDE, t.H, t.B);
+  const dim3 grid((unsigned)t.B * (t.D / WIDE), t.H);  // sequences along x: the other two dimensions end at 65535
   if (t.D == 64) {
     gla_tail_keys_bwd_kernel<64><<<grid, THREADS, 0, s>>>(a);
     gla_tail_values_kernel<64, true><<<grid, THREADS, 0, s>>>(a);

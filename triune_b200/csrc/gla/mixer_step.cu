@@ -37,13 +37,14 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
   constexpr int RP = D / MS_PARTS, QW = D / 32;  // state rows per thread; warps per q or k vector
   __shared__ float feat[2][D], vec[2][D], dec[D], norm[MS_THREADS / 32], bsum[MS_THREADS / 32], part[2][MS_PARTS][MS_COLS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = blockIdx.y, b = blockIdx.z, HD = p.H * D, c = blockIdx.x * MS_COLS + lane, r0 = warp * RP;
+  constexpr int GROUPS = D / MS_COLS;
+  const int h = blockIdx.y, b = blockIdx.x / GROUPS, HD = p.H * D, c = (blockIdx.x % GROUPS) * MS_COLS + lane, r0 = warp * RP;
   const __nv_bfloat16* row = p.qkvg + (long long)b * p.ld + h * D;
   allow_dependents();
   wait_predecessors();
 
   float S[RP];
-  const long long at = ((long long)(b * p.H + h) * D + r0) * D + c;
+  const long long at = (((long long)b * p.H + h) * D + r0) * D + c;
 #pragma unroll
   for (int r = 0; r < RP; ++r) S[r] = p.state_in[at + (long long)r * D];
   const float v = __bfloat162float(row[2 * HD + c]);
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
 
 void launch_mixer_step(const MixerStep& p, int B, int D, bool delta, cudaStream_t s) {
   if (B <= 0 || p.H <= 0) return;
-  const dim3 grid(D / MS_COLS, p.H, B);
+  const dim3 grid((unsigned)B * (D / MS_COLS), p.H);  // sequences along x: the other two dimensions end at 65535
   void (*kernel)(const MixerStep) = nullptr;
   if (D == 64) kernel = delta ? mixer_step_kernel<64, true> : mixer_step_kernel<64, false>;
   else if (D == 128) kernel = delta ? mixer_step_kernel<128, true> : mixer_step_kernel<128, false>;
