@@ -449,6 +449,19 @@ def test_many_sequences_and_none(D):
         assert y.shape == (0, 5, D) and state.shape == (0, 1, D, D) and at == 5
 
 
+@pytest.mark.parametrize("T", [5, 64, 70])
+@pytest.mark.parametrize("delta", [False, True])
+def test_a_state_on_the_host_is_refused(T, delta):
+    from triune_b200.models.attention import VectorisedGLA
+
+    m = VectorisedGLA(128, 1, 128, use_delta_rule=delta, learn_beta=delta).cuda().bfloat16()
+    x = torch.randn(2, T, 128, device="cuda").bfloat16()
+    with pytest.raises(RuntimeError):  # before a kernel sees the pointer
+        m(x, cache=(torch.zeros(2, 1, 128, 128), 0))
+    y, (state, _) = m(x, cache=(torch.zeros(2, 1, 128, 128, device="cuda"), 0))
+    assert torch.isfinite(y).all() and torch.isfinite(state).all()
+
+
 @pytest.mark.parametrize("T,D", [(21, 128), (150, 64), (150, 128)])
 def test_fused_projection_rows_match_separate_tensors(T, D):
     B, H = 2, 2

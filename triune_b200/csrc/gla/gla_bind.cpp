@@ -21,6 +21,12 @@ tb::GlaMat mat(const Tensor& t, int64_t col0) {
   return tb::GlaMat{t.data_ptr(), t.stride(0), (int)col0};
 }
 
+// A state or its gradient as the kernels read it: fp32 [.., D, D], contiguous, on the device of the rows `q`.
+Tensor state_of(const Tensor& t, const Tensor& q, int64_t numel, const char* what) {
+  TORCH_CHECK(t.is_cuda() && t.get_device() == q.get_device() && t.numel() == numel, what, ": [B, H, D, D] on the device of the rows");
+  return t.to(at::kFloat).contiguous();
+}
+
 // Forward over [B*T] rows: whole chunks of 64 tokens on the chunk kernels, the T % 64 tokens after them one by one in fp32
 // (all of them where T < 64, and then without the chunk kernels' clamp of the log decay, which that case never had).
 // Returns (states bf16 [BH*NT,D,D], decay fp32 [BH*NT,D], final_state fp32 [BH,D,D], status) and, where there are both
@@ -40,8 +46,7 @@ std::vector<Tensor> gla_fwd(const Tensor& q, int64_t qcol, const Tensor& k, int6
   const float* ip = nullptr;
   Tensor initc, mid;
   if (init.has_value() && init->defined()) {
-    initc = init->to(at::kFloat).contiguous();
-    TORCH_CHECK(initc.numel() == BH * D * D, "gla_fwd: initial state [B, H, D, D]");
+    initc = state_of(*init, q, BH * D * D, "gla_fwd: initial state");
     ip = initc.data_ptr<float>();
   }
   if (NT > 0) {
@@ -83,8 +88,8 @@ std::vector<Tensor> gla_bwd(const Tensor& q, int64_t qcol, const Tensor& k, int6
   Tensor dinit = torch::empty({BH, D, D}, f32);
   if (dfin.has_value() && dfin->defined()) {
     TORCH_CHECK(fin.has_value() && fin->defined(), "the final state is needed with its gradient");
-    dnext = dfin->to(at::kFloat).reshape({BH, D, D}).contiguous();
-    end_term = (dnext * fin->to(at::kFloat).reshape({BH, D, D})).sum(-1).contiguous();
+    dnext = state_of(*dfin, q, BH * D * D, "gla_bwd: gradient of the final state").reshape({BH, D, D});
+    end_term = (dnext * state_of(*fin, q, BH * D * D, "gla_bwd: final state").reshape({BH, D, D})).sum(-1).contiguous();
   }
   auto fp = [](const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; };
   auto s = cur_stream();
@@ -92,8 +97,7 @@ std::vector<Tensor> gla_bwd(const Tensor& q, int64_t qcol, const Tensor& k, int6
     const tb::GlaTail t{(int)B, (int)H, (int)D, (int)T, (int)(NT * 64), (int)rest, gate_logits, NT > 0 ? tb::GLA_MIN_LOG_DECAY : -INFINITY};
     Tensor from, dmid = NT > 0 ? torch::empty({BH, D, D}, f32) : dinit, emid = torch::empty({BH, D}, f32);
     if (before_rest.has_value() && before_rest->defined()) {
-      from = before_rest->to(at::kFloat).contiguous();
-      TORCH_CHECK(from.numel() == BH * D * D, "gla_bwd: state [B, H, D, D] before the last tokens");
+      from = state_of(*before_rest, q, BH * D * D, "gla_bwd: state before the last tokens");
     }
     TORCH_CHECK(NT == 0 || from.defined(), "gla_bwd: the state after the whole chunks is needed");
     tb::launch_gla_tail_bwd(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), mat(dout, docol), mat(dq, dqcol), mat(dk, dkcol),
@@ -227,13 +231,12 @@ std::vector<Tensor> gdn_chunk_fwd(const Tensor& q, int64_t qcol, const Tensor& k
   Tensor betac, initc;
   if (beta.has_value() && beta->defined()) {
     betac = beta->to(at::kFloat).contiguous();
-    TORCH_CHECK(betac.numel() == B * T * H, "beta must be [B*T, H]");
+    TORCH_CHECK(betac.is_cuda() && betac.get_device() == q.get_device() && betac.numel() == B * T * H, "beta must be [B*T, H] on the device of the rows");
     bp = betac.data_ptr<float>();
   }
   const float* ip = nullptr;
   if (init.has_value() && init->defined()) {
-    initc = init->to(at::kFloat).contiguous();
-    TORCH_CHECK(initc.numel() == BH * D * D, "init must be [B*H, D, D]");
+    initc = state_of(*init, q, BH * D * D, "gdn_chunk_fwd: initial state");
     ip = initc.data_ptr<float>();
   }
   tb::GdnScratch w{bfp(U0), bfp(W), bfp(Tm), bfp(Kend), decay.data_ptr<float>(),
