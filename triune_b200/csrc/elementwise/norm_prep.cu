@@ -1,7 +1,7 @@
 // Bandwidth-bound row kernels: RMSNorm (+ residual add) forward/backward and the GLA q/k feature
-// map (ELU+1 -> L2 normalise -> half-split RoPE) forward/backward. One warp owns one row (RMSNorm) or
-// one (token, head) vector (feature map); all global traffic is 16-byte (RMSNorm) or 4-byte-pair
-// coalesced (feature map) and every tensor is touched exactly once per pass.
+// map (ELU+1 -> L2 normalise -> half-split RoPE) forward/backward. A row of RMSNorm belongs to one warp (forward, many narrow
+// rows) or to the warps of a block (other forwards, every backward), a (token, head) vector of the feature map to D / 8 lanes; all
+// global traffic is in 16-byte accesses and every tensor is touched exactly once per pass.
 //
 // Reference semantics: triune/kernels/fast_rmsnorm.py:181-335 (norm, fused add-norm),
 // triune/model/attention.py:14-80 and :509-531 (feature map + RoPE).

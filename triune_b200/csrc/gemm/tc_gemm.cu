@@ -1,12 +1,12 @@
 // bf16 GEMM on the 5th-generation tensor cores: C = alpha * A * B^T (+ epilogue).
 //
-// One persistent CTA per SM, 320 threads, three roles:
+// One persistent CTA per SM, 320 threads (576 where the epilogue has arithmetic or reads of its own, see launch_epi), three roles:
 //   warp 0    TMA producer: cp.async.bulk.tensor tiles of A (128 x 64) and B (BN x 64) into a ring of
 //             128B-swizzled shared-memory stages, completion signalled on mbarriers;
 //   warp 1    MMA issuer: one thread issues tcgen05.mma (M=128, N=BN, K=16) reading the stages through
 //             shared-memory descriptors and accumulating into TMEM; tcgen05.commit releases a stage
 //             back to the producer and, after the last K step, publishes the accumulator;
-//   warps 2-9 epilogue: tcgen05.ld the fp32 accumulator (lane == output row), apply the epilogue in packed
+//   warps 2.. (eight or sixteen) epilogue: tcgen05.ld the fp32 accumulator (lane == output row), apply the epilogue in packed
 //             f32x2 arithmetic (bias, GELU plus its derivative, multiply by saved rows, row scale), stage the
 //             converted rows in shared memory and hand them to TMA (store or reduce-add).
 // The accumulator is double-buffered in TMEM (2 x BN columns) so the epilogue of tile i overlaps the

@@ -7,7 +7,7 @@
 //   Lraw[t,s] = sum_d k_td k_sd e^{bp_td - b_sd} (s < t)    L = diag(beta) Lraw    T = (I + L)^-1
 //   A[t,s]    = sum_d q_td k_sd e^{b_td - b_sd}  (s <= t)
 //   F1  U0 = T (beta V), W = T (beta Kbar)                     per chunk, tcgen05
-//   F2  U = U0 - W S,  S' = diag(e^{b_C}) S + Kend^T U         sequential over chunks, fp32 CUDA cores, dv-sliced
+//   F2  U = U0 - W S,  S' = diag(e^{b_C}) S + Kend^T U         sequential over chunks, mma.sync, dv-sliced
 //   F3  O = A U + Qbar S                                        per chunk, tcgen05
 //   B1  G1 = A^T dO, H1 = Qbar^T dO                             per chunk, tcgen05
 //   B2  dU = G1 + Kend dS',  dS = H1 + e^{b_C} dS' - W^T dU     reverse sequential (same kernel as F2)
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(GDN_THREADS) gdn_wy_kernel(
 // F2 / B2: the sequential pass over the chunks of one (batch, head), split over slices of 32 state columns.
 //   forward:  U  = U0 - W S,        S <- e^{b_C} S + Kend^T U          (X1 = W,    X2 = Kend)
 //   reverse:  dU = G1 + Kend dS,    dS <- H1 + e^{b_C} dS - W^T dU     (X1 = Kend, X2 = W)
-// fp32 arithmetic (the products are 64 x D x 32 per chunk and strictly sequential); the operand tiles of the next chunk are
+// fp32 state and sums (the products are 64 x D x 32 per chunk and strictly sequential); the operand tiles of the next chunk are
 // fetched with cp.async while the current one is processed.
 // ------------------------------------------------------------------------------------------------
 constexpr int DVS = 32;  // state columns per CTA
@@ -488,8 +488,9 @@ __device__ __forceinline__ void store_parts(__nv_bfloat16* dst, int part, float 
   }
 }
 
-// Both products on warp-level matrix instructions with nothing lost: X1 and X2 are bf16 to begin with, and the fp32 side (state,
-// product 1) enters as three bf16 parts, whose products are exact in the fp32 accumulators. The state slice never leaves the
+// Both products on warp-level matrix instructions with no operand rounded: X1 and X2 are bf16 to begin with, and the fp32 side
+// (state, product 1) enters as three bf16 parts, which carry all 24 bits and whose products with bf16 are exact; the sums are the
+// matrix unit's fp32 accumulation, in another order than the fp32 pipes'. The state slice never leaves the
 // accumulator registers of product 2 (a warp owns 16 key rows); a chunk costs two barriers. On the fp32 pipes, bound by shared-memory
 // reads and three barriers, a chunk took 6.4 us (D = 128), now 2.7 forward and 3.3 in reverse: 4 x 2048 tokens, 8 heads 204 -> 86
 // and 205 -> 105 us. Errors against 64 bits of outputs, states and gradients are the same to four digits.
