@@ -334,9 +334,11 @@ int dense_tiles(const GemmArgs& a, int BN) {
   return ((a.M + BM - 1) / BM) * ((a.N + BN - 1) / BN) * (a.batch < 1 ? 1 : a.batch);
 }
 
-// A reduction is split over idle SMs where the tiles fill at most half of them and the time saved (0.4 us an iteration of
-// 64, measured with operands in L2) outweighs the second kernel (about 5 us with the write and read of the parts). Weight
-// gradients of narrow layers are the case: 1536 x 384 over 32768 rows 224 -> 44 us, 384 x 384 146 -> 22 us.
+// A reduction is split over idle SMs where the tiles fill at most half of them and the iterations saved outweigh the parts: an
+// iteration of 64 takes 0.28 us (0.42 in the 384-wide pair configuration) with operands in L2, the second kernel 3 us and
+// 0.15 us per MB of parts written and read, and a product whose epilogue keeps it off the 384-wide pairs loses 2 us more to them.
+// That line separates 142 measured products; without it 8192 x 384 x 1536 lost 2 us plain and 6 us with GELU (15.0 -> 21.4).
+// Weight gradients of narrow layers gain most: 1536 x 384 over 32768 rows 224 -> 44 us, 384 x 384 146 -> 22 us.
 constexpr int SPLIT_MIN_ITERS = 24;  // shorter: narrower tiles instead
 struct SplitPlan {
   int splits, pair;
@@ -358,14 +360,22 @@ SplitPlan split_plan(const GemmArgs& a) {
   if (tiles * 2 > slots) return p;
   int splits = slots / tiles;
   if (splits > iters / 8) splits = iters / 8;
-  if (splits > 1) p.splits = splits;
+  if (splits < 2) return p;
+  const int whole_pair = pairs_enabled() ? tc_gemm_pair_config(a) : 0;  // what the product runs on in one piece
+  const double saved = (iters - (iters + splits - 1) / splits) * (whole_pair == 384 ? 0.42 : 0.28);
+  const double cost = 3.0 + 0.15e-6 * 4.0 * splits * a.M * a.N + (p.pair == 384 && whole_pair != 384 ? 2.0 : 0.0);
+  if (saved > cost) p.splits = splits;
   return p;
 }
 
 // Few tiles and a short reduction (or one split as far as it goes): narrower tiles put more SMs to work.
 int narrowed_width(const GemmArgs& a, int BN, int splits) {
   if (splits == 1 && (a.flags & GF_ACCUMULATE) && (a.K + BK - 1) / BK >= 16) return BN;  // splits by itself, into the accumulator
-  while (BN > 64 && dense_tiles(a, BN) * splits * 2 <= sm_count()) BN = BN == 256 ? 128 : 64;
+  while (BN > 64 && dense_tiles(a, BN) * splits * 2 <= sm_count()) {
+    const int next = BN == 192 && a.N % 128 != 0 ? 64 : BN > 128 ? 128 : 64;
+    if (dense_tiles(a, next) * splits > sm_count()) break;  // a second wave costs more than wider tiles (4096 x 384 x 384: 7.2 -> 8.1 us)
+    BN = next;
+  }
   return BN;
 }
 
