@@ -651,7 +651,8 @@ def test_write_strengths_against_fp64(rows, dim, H):
     assert _rel(beta, b64) < 2e-6 and _rel(dx, dx64) < 2.0 ** -8 and _rel(dw, dw64) < 2.0 ** -8  # fp32 sums; bf16 gradients
 
 
-@pytest.mark.parametrize("rows,V,offset", [(1, 1, 0), (3, 7, 0), (2, 8191, 0), (4, 32000, 0), (2, 32001, 3)])
+@pytest.mark.parametrize("rows,V,offset", [(1, 1, 0), (3, 7, 0), (5, 256, 0), (5, 257, 0), (3, 263, 1), (2, 2048, 0), (2, 2049, 0), (2, 8191, 0),
+                                         (4, 32000, 0), (2, 32001, 3)])
 def test_largest_of_rows_as_torch_orders_them(rows, V, offset):
     from triune_b200 import ops
 
