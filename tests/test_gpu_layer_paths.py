@@ -504,7 +504,8 @@ def test_rotary_tables_and_gradients_of_any_alignment(T, D):
             assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("rows,d", [(1, 8), (1, 2048), (7, 264), (37, 1536), (1185, 384), (1184, 776), (2375, 2040), (9480, 512), (5000, 1032)])
+@pytest.mark.parametrize("rows,d", [(1, 8), (1, 2048), (7, 264), (37, 1536), (1185, 384), (1184, 776), (2375, 2040), (9480, 512), (5000, 1032),
+                                    (2368, 776), (2369, 520), (2369, 768), (2400, 1024), (9473, 1024)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_norm_rows_against_fp64(rows, d, residual):
     from triune_b200 import ops

@@ -113,9 +113,12 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
   }
 }
 
-// The same with a row spread over the warps of a block, eight columns a thread and R rows in flight, for rows wider than 512
-// (a warp that holds 1536 columns has little else in flight) and for few rows (decoding: one row is a chain of latencies, and a
-// warp alone walks eight loads before it can sum). Measured against the kernel above, with the residual: NUMBERS_FWD
+// The same with a row spread over the warps of a block, eight columns a thread and R rows in flight, for wide rows (a warp that
+// holds 1536 columns has little else in flight) and for few (decoding: one row is a chain of latencies, and a warp alone walks
+// eight loads before it can sum). In a replayed graph, kernel above -> this one: 1 x 2048 4.5 -> 1.8 us, 1184 x 1024 3.3 -> 2.6,
+// 8192 x 1536 12.3 -> 9.6 (with the residual 25.3 -> 18.2), 32768 x 2048 94 -> 46. Many rows of up to 1024 columns stay above
+// (above, here): 8192 x 384 4.0, 4.2 us; 32768 x 512 8.2, 10.4; 8192 x 1024 5.3, 6.4; with the residual 4000 x 768 4.2, 5.8, 8192 x
+// 1024 8.3, 9.3, but 2331 x 768 3.8, 3.3 and, out of L2, 16384 x 1024 25.4, 23.4: see rows_per_warp.
 // `wpr` warps per row; the block's warps / wpr rows side by side.
 template <bool HAS_RES, int R>
 __global__ void __launch_bounds__(256) rmsnorm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
@@ -468,13 +471,20 @@ WideGeom wide_geom(int rows, int d, int cap) {
   return g;
 }
 
+// Where a warp per row is the better forward kernel (figures above).
+bool rows_per_warp(int rows, int d, bool residual) {
+  if (d > 1024 || rows <= 148 * 8) return false;
+  if (!residual || d <= 512) return true;
+  return rows > 148 * 16 && (d <= 768 || rows <= 148 * 64);
+}
+
 template <bool HAS_RES>
 void rmsnorm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y, __nv_bfloat16* sum_out,
                  float* rstd, int rows, int d, float eps, cudaStream_t s) {
-  if (rows > 148 * 8 && d <= (HAS_RES ? 512 : 1024)) {
+  if (rows_per_warp(rows, d, HAS_RES)) {
     const int grid = row_grid(rows, 8);
     if (d <= 512) rmsnorm_fwd_kernel<HAS_RES, 2><<<grid, 256, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps);
-    else if constexpr (!HAS_RES) rmsnorm_fwd_kernel<false, 4><<<grid, 256, 0, s>>>(x, nullptr, w, y, nullptr, rstd, rows, d, eps);
+    else rmsnorm_fwd_kernel<HAS_RES, 4><<<grid, 256, 0, s>>>(x, res, w, y, sum_out, rstd, rows, d, eps);
     return;
   }
   const WideGeom g = wide_geom(rows, d, 148 * 8);
