@@ -24,6 +24,8 @@ def _mixer_inputs(B, T, H, D, seed=0):
 @pytest.mark.parametrize("B,T,H,D,beta_dims", [
     (1, 7, 2, 64, 1), (1, 8, 1, 64, 0), (2, 9, 3, 64, 1), (1, 15, 1, 128, 0), (2, 16, 2, 128, 2), (3, 65, 2, 64, 2), (1, 131, 2, 128, 1),
     (8, 500, 8, 128, 1),  # 64 heads: more tokens than one segment of records
+    (1, 11, 2, 64, 1), (1, 12, 2, 64, 1), (2, 8, 8, 128, 1), (2, 8, 9, 128, 1), (4, 47, 96, 64, 1), (4, 48, 96, 64, 1),  # ends of the rule
+    (7, 64, 64, 64, 0), (7, 64, 65, 64, 0), (2, 512, 256, 64, 1), (3, 512, 171, 64, 1),
 ])
 def test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims):
     q, k, v, g, s0 = _mixer_inputs(B, T, H, D)
@@ -35,7 +37,7 @@ def test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims):
     assert _rel(s, ss) < 1e-6        # the state is fp32 throughout
 
 
-@pytest.mark.parametrize("T,at,D", [(8, 5, 64), (19, 9, 128), (70, 33, 64)])
+@pytest.mark.parametrize("T,at,D", [(8, 5, 64), (12, 5, 64), (19, 9, 128), (70, 33, 64)])
 @pytest.mark.parametrize("where", ["v", "k", "q", "beta"])
 def test_delta_rule_prompts_keep_what_is_no_number_from_earlier_tokens(T, at, D, where):
     q, k, v, g, s0 = _mixer_inputs(2, T, 2, D)

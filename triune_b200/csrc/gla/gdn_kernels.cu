@@ -162,8 +162,8 @@ __global__ void __launch_bounds__(D* NPART) gdn_recurrent_kernel(
 // partial results of a block (2 columns x 8 tokens x {k, q}) with one 30-exchange reduce-scatter that leaves two of them
 // in each lane. Products run in packed f32x2 over row pairs. Bound by the latency of that chain (issue slots 37 % used at
 // one warp per scheduler), not by memory (DRAM 3 %). Measured, 16 heads of 128, 8192 tokens: one sequence 9010 -> 1155 us
-// (four tokens a round: 1853 us), four sequences 9056 -> 3460 us; 6 heads of 64: 5007 -> 896 us. The token kernel keeps
-// prompts of fewer than GDN_BLOCK_MIN_T tokens, where one launch beats two.
+// (four tokens a round: 1853 us), four sequences 9056 -> 3460 us; 6 heads of 64: 5007 -> 896 us. Short prompts and many heads stay
+// with the token kernel, see gdn_in_blocks.
 // ------------------------------------------------------------------------------------------------
 constexpr int GB = 8;  // tokens per block
 constexpr int GDN_TRI = 2 * GB * GB;
@@ -449,8 +449,20 @@ int segment_tokens(int BH, int D) {
 
 }  // namespace
 
+// Eight tokens a round win where the recurrence is a chain that the chip waits for: the walk's work grows with the heads, the token
+// kernel's time hardly does until its CTAs fill the SMs. Token kernel -> blocks, us: 16 heads of 64, 8 tokens 10 -> 10.5, 16 tokens 14 ->
+// 12, 512 tokens 318 -> 71; 256 of 64, 16 tokens 17 -> 20, 32 tokens 30 -> 28; 512 of 64, 130 tokens 142 -> 157, 512 tokens 539 -> 530; 16 of
+// 128, 8 tokens 14 -> 13; 128 of 128, 16 tokens 24 -> 32, 32 tokens 42 -> 41; 256 of 128, 130 tokens 223 -> 240, 512 tokens 849 -> 796;
+// 1024 of 64, 512 tokens 963 -> 1019.
+static bool gdn_in_blocks(long long heads, int T, int D) {
+  if (D != 64 && D != 128) return false;
+  if (T >= 512) return heads <= 512;
+  const long long halves = heads * (D / 64);
+  return T >= (D == 128 && heads <= 16 ? 8 : 12) && halves <= 448 && T * 8 >= halves;
+}
+
 long long gdn_block_workspace_floats(int B, int T, int H, int D) {
-  if (T < GDN_BLOCK_MIN_T || (D != 64 && D != 128)) return 0;
+  if (!gdn_in_blocks((long long)B * H, T, D)) return 0;
   const int seg = segment_tokens(B * H, D), nt = T < seg ? T : seg;
   return (long long)B * H * ((nt + GB - 1) / GB) * ((1 + 3 * GB) * D + GDN_TRI);
 }
