@@ -445,6 +445,7 @@ Tensor tier_render(const Tensor& act, const Tensor& tiers) {
 }  // namespace
 
 void register_gemm(pybind11::module& m);
+void register_decode(pybind11::module& m);
 void register_hybrid(pybind11::module& m);
 void register_gla(pybind11::module& m);
 void register_quant(pybind11::module& m);
@@ -452,6 +453,7 @@ void register_comm(pybind11::module& m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   register_gemm(m);
+  register_decode(m);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("dy"), pybind11::arg("rstd"),
         pybind11::arg("dres"), pybind11::arg("dw_into") = pybind11::none(), pybind11::arg("dw_bf16") = false);

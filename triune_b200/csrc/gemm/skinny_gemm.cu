@@ -138,14 +138,14 @@ bool launch_skinny_gemm(const GemmArgs& a, cudaStream_t s) {
   // rows are read in 16-byte vectors
   if (a.K % 8 != 0 || ((reinterpret_cast<uintptr_t>(a.A) | reinterpret_cast<uintptr_t>(a.B)) & 15) != 0) return false;
   const int blocks = (a.N + SK_ROWS - 1) / SK_ROWS;
-  // about 16 streaming warps per SM of 148, at least one 64-wide step of K for each
+  const int warps = skinny_warps(a.N, a.K);
   if (a.M <= 8) {
-    if (blocks <= 296 && a.K > 512) run<16, 1>(a, blocks, s);
-    else if (blocks <= 1184 && a.K > 256) run<8, 1>(a, blocks, s);
+    if (warps == 16) run<16, 1>(a, blocks, s);
+    else if (warps == 8) run<8, 1>(a, blocks, s);
     else run<4, 1>(a, blocks, s);
   } else {
-    if (blocks <= 296 && a.K > 512) run<16, 2>(a, blocks, s);
-    else if (blocks <= 1184 && a.K > 256) run<8, 2>(a, blocks, s);
+    if (warps == 16) run<16, 2>(a, blocks, s);
+    else if (warps == 8) run<8, 2>(a, blocks, s);
     else run<4, 2>(a, blocks, s);
   }
   cudaError_t e = cudaGetLastError();

@@ -72,6 +72,12 @@ void launch_tc_gemm(const GemmArgs& args, cudaStream_t stream);
 // Products of at most SKINNY_MAX_M rows with a K-major weight (plain, bias, GELU or SwiGLU, bf16 output): streams the weight
 // through warp-level matrix instructions (skinny_gemm.cu). Returns false, launching nothing, for every other call.
 constexpr int SKINNY_MAX_M = 16;
+// Slices of its reduction whose sums are added in order: the W warps of a CTA. About 16 streaming warps per SM of 148, at least one
+// 64-wide step of K for each. Slice w of W takes the steps [w * steps / W, (w + 1) * steps / W).
+inline int skinny_warps(int N, int K) {
+  const int blocks = (N + 15) / 16;
+  return blocks <= 296 && K > 512 ? 16 : blocks <= 1184 && K > 256 ? 8 : 4;
+}
 bool launch_skinny_gemm(const GemmArgs& args, cudaStream_t stream);
 
 // CTA-pair (tcgen05 cta_group::2) variant for dense products with long reductions; returns false, launching

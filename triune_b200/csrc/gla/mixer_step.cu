@@ -18,7 +18,7 @@
 #include <string>
 
 #include "../common/dependent_launch.cuh"
-#include "gla.cuh"
+#include "mixer_math.cuh"
 
 namespace tb {
 
@@ -51,14 +51,8 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
   float bdot = 0.f;
   if (DELTA && p.beta_w != nullptr) {
     const __nv_bfloat16 *x = p.x + (long long)b * p.ldx, *w = p.beta_w + (long long)h * p.dim;
-    for (int i = tid * 8; i < p.dim; i += MS_THREADS * 8) {
-      const uint4 xv = *reinterpret_cast<const uint4*>(x + i), wv = *reinterpret_cast<const uint4*>(w + i);
-      const uint32_t xa[4] = {xv.x, xv.y, xv.z, xv.w}, wa[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        bdot += __uint_as_float(xa[j] << 16) * __uint_as_float(wa[j] << 16) +
-                __uint_as_float(xa[j] & 0xffff0000u) * __uint_as_float(wa[j] & 0xffff0000u);
-    }
+    for (int i = tid * 8; i < p.dim; i += MS_THREADS * 8)
+      bdot = mix_dot8(*reinterpret_cast<const uint4*>(x + i), *reinterpret_cast<const uint4*>(w + i), bdot);
     bdot = ms_warp_sum(bdot);
     if (lane == 0) bsum[warp] = bdot;
   }
@@ -66,26 +60,25 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
   float f = 0.f;
   if (which < 2) {
     const float raw = __bfloat162float(row[which * HD + d]);
-    f = raw > 0.f ? raw + 1.f : __expf(raw);
+    f = mix_feature(raw);
     const float ss = ms_warp_sum(f * f);
     if (lane == 0) norm[warp] = ss;
     feat[which][d] = f;
   }
   for (int i = tid; i < D; i += MS_THREADS) {
-    const float g = __bfloat162float(row[3 * HD + i]);
-    dec[i] = __expf(fmaxf(fminf(g, 0.f) - log1pf(__expf(-fabsf(g))), GLA_MIN_LOG_DECAY));
+    dec[i] = mix_decay(__bfloat162float(row[3 * HD + i]));
   }
   __syncthreads();
   if (which < 2) {
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < QW; ++i) ss += norm[which * QW + i];
-    const float inv = 1.f / fmaxf(sqrtf(ss), 1e-6f);
+    const float inv = mix_inverse_norm(ss);
     if (p.cos != nullptr) {
       const long long pos = p.pos != nullptr ? *p.pos : p.pos_host;
       const bool inside = pos >= 0 && pos < p.table_rows;  // past the table there is no rotation: NaN, never another row's
       const float cs = inside ? p.cos[pos * D + d] : NAN, sn = inside ? p.sin[pos * D + d] : NAN;
-      f = d < D / 2 ? f * cs - feat[which][d + D / 2] * sn : f * cs + feat[which][d - D / 2] * sn;
+      f = mix_rotate(f, feat[which][d < D / 2 ? d + D / 2 : d - D / 2], cs, sn, d < D / 2);
     }
     vec[which][d] = f * inv;
   }
@@ -94,13 +87,13 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
   if constexpr (DELTA) {
     float acc = 0.f;
 #pragma unroll
-    for (int r = 0; r < RP; ++r) acc += vec[1][r0 + r] * S[r];
+    for (int r = 0; r < RP; ++r) acc = __fmaf_rn(vec[1][r0 + r], S[r], acc);
     part[0][warp][lane] = acc;
     if (p.beta_w != nullptr) {
       float z = 0.f;
 #pragma unroll
       for (int i = 0; i < MS_THREADS / 32; ++i) z += bsum[i];
-      beta = 1.f / (1.f + __expf(-z));
+      beta = mix_strength(z);
     }
     __syncthreads();
 #pragma unroll
@@ -110,8 +103,8 @@ __global__ void __launch_bounds__(MS_THREADS) mixer_step_kernel(const MixerStep 
   float acc = 0.f;
 #pragma unroll
   for (int r = 0; r < RP; ++r) {
-    S[r] = dec[r0 + r] * S[r] + vec[1][r0 + r] * u;
-    acc += vec[0][r0 + r] * S[r];
+    S[r] = mix_state(S[r], dec[r0 + r], vec[1][r0 + r], u);
+    acc = __fmaf_rn(vec[0][r0 + r], S[r], acc);
     p.state_out[at + (long long)r * D] = S[r];
   }
   part[1][warp][lane] = acc;

@@ -25,6 +25,7 @@ from . import ops
 from .config import ModelConfig
 from .models.layer_state import LayerState
 from .models.rotary import RotaryEmbedding
+from .runtime import dense_step
 
 DEFAULT_STOPS = ("\nUser:", "\nSystem:", "User:", "Assistant:")
 
@@ -357,7 +358,8 @@ class GraphedGreedyDecoder:
     A decode step of a small model is a few hundred kernel launches of a few microseconds each: run eagerly it is bound
     by launch latency and Python, not by the GPU. Everything that changes between steps lives in device memory: the
     current token, the position (RoPE rows are gathered by a device index), the recurrent states (updated in place) and
-    the output buffer. On a CPU device the same step function runs eagerly, which is what the tests compare against.
+    the output buffer. On a CPU device the same step function runs eagerly, which is what the tests compare against. Where one
+    kernel covers the model (``runtime/dense_step.py``), a step is that kernel, launched once per token, instead of a capture.
 
     ``max_positions`` bounds the rotary tables that a request may ask for beyond those that the prompt itself needed; a request
     that goes past it is refused before a token is decoded.
@@ -432,6 +434,8 @@ class GraphedGreedyDecoder:
             for _ in range(max_new_tokens):
                 self._step()
             return self.out[:, :max_new_tokens].clone()
+        if self.graph is None and max_new_tokens > 0:
+            self.graph = dense_step.plan(self.model, self.states, self.token, self.out, self.pos, self.step_idx)
         if self.graph is None and max_new_tokens > 0:
             # snapshot, warm up on a side stream (allocator and autotune effects must not land in the capture), restore
             snap = ([None if s is None else s.clone() for s in self.states], self.pos.clone(), self.token.clone())
