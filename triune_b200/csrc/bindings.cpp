@@ -4,6 +4,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include "block/launch.h"
 #include "elementwise/elementwise.cuh"
 #include "gemm/tc_gemm.cuh"
 #include "gla/gla.cuh"
@@ -27,6 +28,8 @@ void check_bf16_cuda(const Tensor& t, const char* name) {
   TORCH_CHECK((reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, name, " must start on a 16-byte boundary");
 }
 
+}  // namespace
+namespace tb_launch {
 std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
   check_bf16_cuda(x, "x");
   TORCH_CHECK(x.is_contiguous() && w.is_contiguous(), "rmsnorm: contiguous inputs required");
@@ -48,6 +51,8 @@ std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& re
                          rstd.data_ptr<float>(), rows, d, (float)eps, cur_stream());
   return {y, rstd, has_res ? sum_out : Tensor()};
 }
+}  // namespace tb_launch
+namespace {
 
 // Where a gradient's column sums go: into `into` (fp32, added), or a new tensor, bf16 on request and else fp32.
 tb::ColumnSum column_sum(const c10::optional<Tensor>& into, bool bf16, int64_t n, const Tensor& like, Tensor& res) {
@@ -60,6 +65,8 @@ tb::ColumnSum column_sum(const c10::optional<Tensor>& into, bool bf16, int64_t n
 }
 
 // Returns (dx, dw): dw as column_sum says.
+}  // namespace
+namespace tb_launch {
 std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& dy, const Tensor& rstd,
                                 const c10::optional<Tensor>& dres, const c10::optional<Tensor>& dw_into, bool dw_bf16) {
   check_bf16_cuda(x, "x");
@@ -77,6 +84,8 @@ std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& 
                          partial.data_ptr<float>(), to, rows, d, cur_stream());
   return {dx, dw};
 }
+}  // namespace tb_launch
+namespace {
 
 // Row pitch of rotary tables: fp32 rows that the kernels read in 16-byte vectors.
 int table_pitch(const Tensor& cs, const Tensor& sn, int64_t T, int64_t D) {
@@ -89,6 +98,8 @@ int table_pitch(const Tensor& cs, const Tensor& sn, int64_t T, int64_t D) {
 }
 
 // in: [tokens, ld] with q at col 0 and k at col k_off; returns [tokens, 2, H, D].
+}  // namespace
+namespace tb_launch {
 Tensor qk_prep_fwd(const Tensor& in, int64_t k_off, const c10::optional<Tensor>& cs, const c10::optional<Tensor>& sn,
                    int64_t T, int64_t H, int64_t D) {
   check_bf16_cuda(in, "in");
@@ -114,6 +125,8 @@ void qk_prep_bwd(const Tensor& in, int64_t k_off, const Tensor& dout, Tensor& d_
                          rope ? cs->data_ptr<float>() : nullptr, rope ? sn->data_ptr<float>() : nullptr, rope ? table_pitch(*cs, *sn, T, D) : 0, in.size(0),
                          (int)T, (int)H, (int)D, cur_stream());
 }
+}  // namespace tb_launch
+namespace {
 
 // Cross entropy that leaves the logits intact: returns (per-row loss, grad_scale * (softmax - onehot) as a new tensor).
 std::vector<Tensor> ce_loss_grad(const Tensor& logits, const Tensor& targets, int64_t ignore_index, double grad_scale) {
@@ -211,6 +224,8 @@ Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, int64_t ignore_index, d
 }
 
 // Column sums of a bf16 [M, N] matrix in fp32: returns a new [N] tensor (rounded to bf16 on request), or adds into `out`.
+}  // namespace
+namespace tb_launch {
 Tensor colsum(const Tensor& x, const c10::optional<Tensor>& out, bool bf16) {
   check_bf16_cuda(x, "x");
   TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && x.size(1) % 8 == 0 && x.stride(0) % 8 == 0,
@@ -225,6 +240,8 @@ Tensor colsum(const Tensor& x, const c10::optional<Tensor>& out, bool bf16) {
   tb::launch_colsum(bf(x), x.stride(0), M, N, partial.data_ptr<float>(), parts, to, cur_stream());
   return res;
 }
+}  // namespace tb_launch
+namespace {
 
 // out (int64, one value per row) = index of the largest value of each row of x [rows, V] bf16
 void argmax_rows(const Tensor& x, Tensor& out) {
@@ -446,14 +463,17 @@ Tensor tier_render(const Tensor& act, const Tensor& tiers) {
 
 void register_gemm(pybind11::module& m);
 void register_decode(pybind11::module& m);
+void register_block(pybind11::module& m);
 void register_hybrid(pybind11::module& m);
 void register_gla(pybind11::module& m);
 void register_quant(pybind11::module& m);
 void register_comm(pybind11::module& m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  using namespace tb_launch;
   register_gemm(m);
   register_decode(m);
+  register_block(m);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("dy"), pybind11::arg("rstd"),
         pybind11::arg("dres"), pybind11::arg("dw_into") = pybind11::none(), pybind11::arg("dw_bf16") = false);

@@ -16,6 +16,7 @@ import torch.utils.checkpoint
 
 from .. import ops
 from ..config import NUM_EXPERTS, TOP_K_EXPERTS, checkpoint_bwd_ctx
+from . import native_block
 from .attention import HybridAttention
 from .moe import MoE_FFN
 from .norms import RMSNorm
@@ -67,6 +68,9 @@ class TransformerBlock(nn.Module):
         return self.ffn(n, update_stats=update_stats) if isinstance(self.ffn, MoE_FFN) else self.ffn(n)
 
     def _body(self, x, cache, update_stats):
+        whole = native_block.run(self.norm1, self.attn, self.norm2, self.ffn, x, cache)
+        if whole is not None:
+            return whole
         attn_out, new_cache = self.attn(self.norm1(x), cache=cache)
         n2, x = self.norm2.forward_add(attn_out, x)
         return x + self._ffn(n2, update_stats), new_cache

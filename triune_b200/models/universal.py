@@ -17,6 +17,7 @@ import torch.nn.functional as F
 
 from .. import ops
 from ..config import ModelConfig
+from . import native_block
 from .attention import SoftmaxAttention, VectorisedGLA
 from .block import DenseFFN
 from .norms import RMSNorm
@@ -120,6 +121,9 @@ class UniversalBlock(nn.Module):
         self._use_gradient_checkpointing = False
 
     def _body(self, x, cache):
+        whole = native_block.run(self.input_norm, self.attn, self.post_attn_norm, self.mlp, x, cache)
+        if whole is not None:
+            return whole
         a, new_cache = self.attn(self.input_norm(x), cache=cache)
         n, x = self.post_attn_norm.forward_add(a, x)
         return x + self.mlp(n), new_cache
