@@ -44,6 +44,34 @@ def test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims):
     assert _rel(s, ss) < 1e-6        # the state is fp32 throughout
 
 
+@pytest.mark.parametrize("B,T,H,D,beta_dims", [
+    (1, 8, 16, 128, 1), (1, 17, 5, 128, 2), (1, 31, 3, 64, 0), (2, 33, 7, 64, 1),          # blocks of sixteen and their remainders
+    (4, 12, 16, 64, 1), (4, 11, 16, 128, 1), (4, 12, 16, 128, 0), (8, 24, 16, 64, 1), (8, 23, 16, 128, 1), (8, 24, 16, 128, 2),
+    (17, 31, 8, 64, 1), (17, 32, 8, 64, 1), (32, 32, 16, 128, 1), (27, 140, 19, 128, 1), (19, 140, 27, 64, 1),  # ends of the rule, segments
+])
+def test_rounds_of_sixteen_tokens_against_the_token_recurrence(B, T, H, D, beta_dims):
+    test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38])
+@pytest.mark.parametrize("where", ["k", "q", "state"])
+def test_rounds_of_sixteen_tokens_with_infinities_and_overflow(where, value):
+    q, k, v, g, s0 = _mixer_inputs(1, 45, 2, 64)
+    x = {"k": k.clone(), "q": q.clone(), "state": s0.clone()}
+    x[where][(0, 1, 3, 5) if where == "state" else (0, 20, 1, 3)] = value
+    o, s = gla_cuda.gdn_recurrent(x["q"], x["k"], v, g, None, x["state"], 1.0, True)
+    # token by token: one call a token is the token kernel's
+    rows, state = [], x["state"]
+    for t in range(45):
+        a, state = gla_cuda.gdn_recurrent(x["q"][:, t : t + 1], x["k"][:, t : t + 1], v[:, t : t + 1], g[:, t : t + 1], None, state, 1.0, True)
+        rows.append(a)
+    want = torch.cat(rows, 1)
+    for a, b in ((o, want), (s, state)):
+        assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isinf(a), torch.isinf(b))
+        ok = torch.isfinite(b)
+        assert torch.equal(a[torch.isinf(a)], b[torch.isinf(b)]) and _rel(a[ok], b[ok]) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("T,at,D", [(8, 5, 64), (12, 5, 64), (19, 9, 128), (70, 33, 64)])
 @pytest.mark.parametrize("where", ["v", "k", "q", "beta"])
 def test_delta_rule_prompts_keep_what_is_no_number_from_earlier_tokens(T, at, D, where):

@@ -20,6 +20,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "../common/per_device.h"
 #include "../common/ptx.cuh"
 #include "gla.cuh"
 
@@ -147,36 +148,50 @@ __global__ void __launch_bounds__(D* NPART) gdn_recurrent_kernel(
 }
 
 // ------------------------------------------------------------------------------------------------
-// The same recurrence, eight tokens at a time, for prompts.
+// The same recurrence, sixteen tokens at a time, for prompts.
 //
 // One token at a time the recurrence is a chain: a contraction over all key rows, its sum across threads, then the update
-// that the next token's contraction waits for (2100 clocks a token in the kernel above). Eight tokens share ONE such round:
-// with P_j = product of the decays up to and including token j of the block and S the state before it,
-//   x_j  = v_j - (k_j P_{j-1})^T S                                     eight contractions with the same S
-//   u_j  = x_j - sum_{i<j} L_ji u_i      L_ji = sum_d k_j (beta k)_i dec_{i+1..j-1}
-//   o_j  = (q_j P_j)^T S + sum_{i<=j} A_ji u_i    A_ji = sum_d q_j (beta k)_i dec_{i+1..j}
-//   S   <- P_7 S + sum_j (beta k_j dec_{j+1..7}) u_j^T
-// Everything is fp32 with exponents <= 0, as in the token form. What does not depend on the state (the scaled vectors and
-// the small triangles) is formed once per head by gdn_block_prep_kernel, one warp per block of tokens, instead of by every
-// group of value columns; it leaves records of 25 D + 128 floats. Value columns never mix, so the walk runs on
-// B * H * D / 16 CTAs of 16 columns: a half warp holds two columns, 16 lanes x D / 16 rows each, and sums the 32
-// partial results of a block (2 columns x 8 tokens x {k, q}) with one 30-exchange reduce-scatter that leaves two of them
-// in each lane. Products run in packed f32x2 over row pairs. Bound by the latency of that chain (issue slots 37 % used at
-// one warp per scheduler), not by memory (DRAM 3 %). Measured, 16 heads of 128, 8192 tokens: one sequence 9010 -> 1155 us
-// (four tokens a round: 1853 us), four sequences 9056 -> 3460 us; 6 heads of 64: 5007 -> 896 us. Short prompts and many heads stay
-// with the token kernel, see gdn_in_blocks.
+// that the next token's contraction waits for (2100 clocks a token in the kernel above). Sixteen tokens share ONE such round:
+// with P_j = product of the decays up to and including token j of the block, S the state before it and L strictly lower,
+//   x_j  = v_j - (k_j P_{j-1})^T S            L_ji = sum_d k_j (beta k)_i dec_{i+1..j-1}
+//   u    = T x, T = (1 + L)^-1                A_ji = sum_d q_j (beta k)_i dec_{i+1..j}
+//   o_j  = (q_j P_j)^T S + sum_{i<=j} A_ji u_i
+//   S   <- P_15 S + sum_j (beta k_j dec_{j+1..15}) u_j^T
+// Exponents are <= 0 as in the token form. What does not depend on the state (the scaled vectors, T and A) is formed once per
+// head by gdn_block_prep in fp32, four warps per block of tokens, and left as a record. Value columns never mix, so the
+// walk runs on B * H * D / 16 CTAs of 16 columns whose four warps share the key rows.
+//
+// The products of the walk are warp-level matrix instructions on tf32 numbers with fp32 sums, each operand as the sum of two:
+// x = hi + lo keeps 22 to 24 bits, hi hi + hi lo + lo hi leaves 2^-23 of a product, and the state stays fp32 (relative error of the
+// state after 8192 tokens 4e-7, as with fp32 multiply-adds). The state is held transposed: the fragment that
+// the update leaves it in is the operand that the next round's contraction takes it from, the order of key rows within an
+// instruction being free. Rows of a record are padded so that its fragments are read without bank conflicts.
+//
+// The launch that walks a segment of tokens also forms the next one's records, in CTAs behind its own. A block's outputs wait for the next
+// round's barrier, so that there is one barrier a round. Bound by the issue slots of one warp per scheduler (81 matrix
+// instructions of 12 clocks and 700 others in the 2500 clocks of a round of 128-wide heads; eight warps a CTA repeat more than they hide:
+// 1030 against 930 us). Measured, token by token -> eight tokens a round in fp32 multiply-adds -> here: one sequence of 8192 tokens, 16 heads of
+// 128, 9010 -> 1164 -> 865 us; 6 heads of 64 5007 -> 960 -> 490; four sequences of 16384, 6 heads of 64 2080 -> 1100; 4 x 512, 16 heads of
+// 128 224 -> 169; see gdn_in_blocks for the sizes that take it.
 // ------------------------------------------------------------------------------------------------
-constexpr int GB = 8;  // tokens per block
-constexpr int GDN_TRI = 2 * GB * GB;
+constexpr int GB = 16;  // tokens per block
 template <int D>
-constexpr int gdn_rec_floats() { return (1 + 3 * GB) * D + GDN_TRI; }  // P_7 | k P | q P | (beta k) dec | L | A
+struct GdnRec {  // floats of a record: k P and q P [32][PK] | (beta k) dec [16][PE] | T [16][PT] | A [16][PT] | P_15 [D] | v bf16 [D][24]
+  static constexpr int PK = D + 8, PE = D + 4, PT = 24, PV = 12;
+  static constexpr int E = 2 * GB * PK, TRI = E + GB * PE, A = TRI + GB * PT, P = A + GB * PT, COMMON = P + D, FLOATS = COMMON + D * PV;
+  static_assert(COMMON % 4 == 0 && PV % 4 == 0, "records are copied in 16-byte words");
+};
 
-// Reduce-scatter of N values over the sixteen lanes of a half warp: lane l gets the sums of values l * N / 16 + [0, N / 16).
-template <int N>
-__device__ __forceinline__ void reduce_scatter16(float (&v)[N], int lane) {
-  int n = N / 2;
+// e^gdn_log_decay: a sigmoid where the gates are logits.
+__device__ __forceinline__ float gdn_decay(float x, bool logits) {
+  return logits ? fmaxf(__fdividef(1.f, 1.f + __expf(-x)), 6.7379469990854671e-3f) : __expf(gdn_log_decay(x, false));
+}
+
+// Sum of v[l] over the lanes, in lane l.
+__device__ __forceinline__ float reduce_scatter32(float (&v)[32], int lane) {
+  int n = 16;
 #pragma unroll
-  for (int s = 8; s >= 1; s >>= 1, n >>= 1) {
+  for (int s = 16; s >= 1; s >>= 1, n >>= 1) {
     const bool up = (lane & s) != 0;
 #pragma unroll
     for (int i = 0; i < n; ++i) {
@@ -184,11 +199,11 @@ __device__ __forceinline__ void reduce_scatter16(float (&v)[N], int lane) {
       v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
     }
   }
+  return v[0];
 }
 
 template <int N>
-__device__ __forceinline__ void load_bf16_row(const __nv_bfloat16* p, bool ok, float (&f)[N]) {
-  uint32_t w[N / 2];
+__device__ __forceinline__ void load_bf16_row(const __nv_bfloat16* p, bool ok, uint32_t (&w)[N / 2]) {
   if constexpr (N == 4) {
     const uint2 x = ok ? *reinterpret_cast<const uint2*>(p) : make_uint2(0u, 0u);
     w[0] = x.x;
@@ -196,6 +211,9 @@ __device__ __forceinline__ void load_bf16_row(const __nv_bfloat16* p, bool ok, f
   } else {
     w[0] = ok ? *reinterpret_cast<const uint32_t*>(p) : 0u;
   }
+}
+template <int N>
+__device__ __forceinline__ void unpack_bf16(const uint32_t (&w)[N / 2], float (&f)[N]) {
 #pragma unroll
   for (int i = 0; i < N / 2; ++i) {
     f[2 * i] = __uint_as_float(w[i] << 16);
@@ -210,295 +228,658 @@ __device__ __forceinline__ void store_rec(float* p, const float (&f)[N]) {
   else
     *reinterpret_cast<float2*>(p) = make_float2(f[0], f[1]);
 }
+template <int N>
+__device__ __forceinline__ void load_rec(const float* p, float (&f)[N]) {
+  if constexpr (N == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
+  } else {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    f[0] = v.x, f[1] = v.y;
+  }
+}
 
-// Tokens [t0, t0 + nt) of every sequence -> records [B * H, ceil(nt / GB)]. One warp per record; D / 32 dims per lane.
 template <int D>
-__global__ void __launch_bounds__(128) gdn_block_prep_kernel(
-    const __nv_bfloat16* __restrict__ q, long long q_ld, int qcol, const __nv_bfloat16* __restrict__ k, long long k_ld,
-    int kcol, const __nv_bfloat16* __restrict__ g, long long g_ld, int gcol, const float* __restrict__ beta, int beta_mode,
-    float* __restrict__ rec, int T, int t0, int nt, int H, int logits, int nrec) {
-  constexpr int N = D / 32, REC = gdn_rec_floats<D>();
-  const int lane = threadIdx.x & 31, id = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (id >= nrec) return;
-  const int nb = (nt + GB - 1) / GB, bh = id / nb, blk = id % nb, h = bh % H;
+struct GdnPrepShared {
+  float dec[GB][D];
+  __nv_bfloat16 k[GB][D], q[GB][D];
+  uint32_t v[D][GdnRec<D>::PV];  // pairs of tokens
+  float L[GB][GB + 1], beta[GB];
+};
+
+struct GdnBlockArgs {
+  const __nv_bfloat16 *q, *k, *v, *g;
+  long long q_ld, k_ld, v_ld, g_ld, o_ld;
+  int qcol, kcol, vcol, gcol, ocol;
+  const float* beta;
+  int beta_mode;
+  float* state;
+  __nv_bfloat16* out;
+  int T, H, logits;
+  float scale;
+};
+
+// Record `index` of [B * H, ceil(nt / GB)] for tokens [t0, t0 + nt) of every sequence, by a CTA of four warps. A warp carries the vectors
+// of two tokens forward at a time, so that the later tokens' rows are read and unpacked half as often, and takes an early and a late pair.
+template <int D>
+__device__ __forceinline__ void gdn_block_prep(const GdnBlockArgs& a, GdnPrepShared<D>& sh, float* rec, int t0, int nt, int index) {
+  const __nv_bfloat16 *q = a.q, *k = a.k, *v = a.v, *g = a.g;
+  const long long q_ld = a.q_ld, k_ld = a.k_ld, v_ld = a.v_ld, g_ld = a.g_ld;
+  const int qcol = a.qcol, kcol = a.kcol, vcol = a.vcol, gcol = a.gcol, beta_mode = a.beta_mode, T = a.T, H = a.H, logits = a.logits;
+  const float* beta = a.beta;
+  constexpr int N = D / 32;
+  using R = GdnRec<D>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nb = (nt + GB - 1) / GB, bh = index / nb, blk = index % nb, h = bh % H;
   const long long row0 = (long long)(bh / H) * T + t0 + blk * GB;
-  const int left = nt - blk * GB, d0 = h * D + lane * N;
-  float qv[GB][N], kv[GB][N], dec[GB][N], bt[GB][N];
+  const int left = nt - blk * GB;
+  float* out = rec + (long long)index * R::FLOATS;
 #pragma unroll
-  for (int j = 0; j < GB; ++j) {
+  for (int i = tid; i < GB * (D / 4); i += 128) {  // eight bytes at a time: rows start on 8-byte boundaries
+    const int j = i / (D / 4), c = (i % (D / 4)) * 4;
     const bool ok = j < left;
     const long long r = row0 + j;
-    load_bf16_row<N>(q + r * q_ld + qcol + d0, ok, qv[j]);
-    load_bf16_row<N>(k + r * k_ld + kcol + d0, ok, kv[j]);
-    load_bf16_row<N>(g + r * g_ld + gcol + d0, ok, dec[j]);
-    const float b1 = (ok && beta_mode == 1) ? beta[r * H + h] : 1.f;
+    const uint2 zero = make_uint2(0u, 0u);
+    *reinterpret_cast<uint2*>(&sh.k[j][c]) = ok ? *reinterpret_cast<const uint2*>(k + r * k_ld + kcol + h * D + c) : zero;
+    *reinterpret_cast<uint2*>(&sh.q[j][c]) = ok ? *reinterpret_cast<const uint2*>(q + r * q_ld + qcol + h * D + c) : zero;
+    const uint2 gw = ok ? *reinterpret_cast<const uint2*>(g + r * g_ld + gcol + h * D + c) : zero;
+    const float x[4] = {__uint_as_float(gw.x << 16), __uint_as_float(gw.x & 0xffff0000u), __uint_as_float(gw.y << 16), __uint_as_float(gw.y & 0xffff0000u)};
+    float f[4];
 #pragma unroll
-    for (int i = 0; i < N; ++i) bt[j][i] = (ok && beta_mode == 2) ? beta[r * H * D + d0 + i] : b1;
+    for (int n = 0; n < 4; ++n) f[n] = ok ? gdn_decay(x[n], logits != 0) : 1.f;
+    *reinterpret_cast<float4*>(&sh.dec[j][c]) = make_float4(f[0], f[1], f[2], f[3]);
+    const uint2 vw = ok ? *reinterpret_cast<const uint2*>(v + r * v_ld + vcol + h * D + c) : zero;
+    unsigned short* vt = reinterpret_cast<unsigned short*>(sh.v[c]) + j;
+    vt[0] = (unsigned short)vw.x, vt[2 * R::PV] = (unsigned short)(vw.x >> 16);
+    vt[4 * R::PV] = (unsigned short)vw.y, vt[6 * R::PV] = (unsigned short)(vw.y >> 16);
   }
-  float* out = rec + (long long)id * REC + lane * N;
-  float p[N], f[N];
+  if (tid < GB) sh.beta[tid] = (tid < left && beta_mode == 1) ? beta[(row0 + tid) * H + h] : 1.f;
+  __syncthreads();
+  for (int i = tid; i < D * 2; i += 128)  // sixteen values of a column: two 16-byte words
+    *reinterpret_cast<uint4*>(out + R::COMMON + (i >> 1) * R::PV + (i & 1) * 4) = *reinterpret_cast<const uint4*>(&sh.v[i >> 1][(i & 1) * 4]);
+  if (tid < D) {  // k_j P_{j-1}, q_j P_j; tokens past the end write nothing and leave the state as it is
+    float p = 1.f;
 #pragma unroll
-  for (int i = 0; i < N; ++i) p[i] = 1.f;
-#pragma unroll
-  for (int j = 0; j < GB; ++j) {  // k_j P_{j-1}, q_j P_j; tokens past the end write nothing and leave the state as it is
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      dec[j][i] = j < left ? __expf(gdn_log_decay(dec[j][i], logits != 0)) : 1.f;
-      f[i] = kv[j][i] * p[i];
+    for (int j = 0; j < GB; ++j) {
+      out[j * R::PK + tid] = __bfloat162float(sh.k[j][tid]) * p;
+      p *= sh.dec[j][tid];
+      out[(GB + j) * R::PK + tid] = __bfloat162float(sh.q[j][tid]) * p;
     }
-    store_rec<N>(out + (1 + j) * D, f);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      p[i] *= dec[j][i];
-      f[i] = qv[j][i] * p[i];
-    }
-    store_rec<N>(out + (1 + GB + j) * D, f);
+    out[R::P + tid] = p;
   }
-  store_rec<N>(out, p);
-  float* tri = rec + (long long)id * REC + (1 + 3 * GB) * D;
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    const int i = half == 0 ? 2 * warp : GB - 2 - 2 * warp;  // w: (beta k)_i and (beta k)_{i+1} carried forward through the later decays
+    float w[2][N], sums[2][2 * GB];
 #pragma unroll
-  for (int i = 0; i < GB; ++i) {  // w = (beta k)_i carried forward through the decays of the later tokens
-    float w[N], sums[2 * GB];
+    for (int e = 0; e < 2; ++e) {
 #pragma unroll
-    for (int j = 0; j < 2 * GB; ++j) sums[j] = 0.f;
+      for (int n = 0; n < N; ++n)
+        w[e][n] = __bfloat162float(sh.k[i + e][lane * N + n]) *
+                  ((beta_mode == 2 && i + e < left) ? beta[(row0 + i + e) * H * D + h * D + lane * N + n] : sh.beta[i + e]);
 #pragma unroll
-    for (int n = 0; n < N; ++n) w[n] = bt[i][n] * kv[i][n];
+      for (int j = 0; j < 2 * GB; ++j) sums[e][j] = 0.f;
+    }
 #pragma unroll
-    for (int j = i; j < GB; ++j) {
-      if (j > i) {
+    for (int j = 0; j < GB; ++j) {
+      if (j >= i) {  // the same for all lanes
+        uint32_t kw[N / 2], qw[N / 2];
+        float kf[N], qf[N], dec[N];
+        load_bf16_row<N>(&sh.k[j][lane * N], true, kw);
+        load_bf16_row<N>(&sh.q[j][lane * N], true, qw);
+        unpack_bf16<N>(kw, kf);
+        unpack_bf16<N>(qw, qf);
+        load_rec<N>(&sh.dec[j][lane * N], dec);
 #pragma unroll
-        for (int n = 0; n < N; ++n) {
-          sums[j] += kv[j][n] * w[n];
-          w[n] *= dec[j][n];
+        for (int e = 0; e < 2; ++e) {
+          if (j > i + e) {
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+              sums[e][j] += kf[n] * w[e][n];
+              w[e][n] *= dec[n];
+            }
+          }
+          if (j >= i + e) {
+#pragma unroll
+            for (int n = 0; n < N; ++n) sums[e][GB + j] += qf[n] * w[e][n];
+          }
         }
       }
-#pragma unroll
-      for (int n = 0; n < N; ++n) sums[GB + j] += qv[j][n] * w[n];
     }
-    store_rec<N>(out + (1 + 2 * GB + i) * D, w);
-    reduce_scatter16(sums, lane);
-    const float s = sums[0] + __shfl_xor_sync(0xffffffffu, sums[0], 16);
-    if (lane < 16) tri[lane * GB + i] = s;  // lanes 0..7: L[j = lane][i] (zero for i >= j); lanes 8..15: A[j = lane - 8][i]
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      store_rec<N>(out + R::E + (i + e) * R::PE + lane * N, w[e]);
+      const float v = reduce_scatter32(sums[e], lane);  // lanes 0..15: L[j = lane][i + e] (zero for i + e >= j), 16..31: A[j][i + e]
+      if (lane < GB) sh.L[lane][i + e] = v;
+      else out[R::A + (lane - GB) * R::PT + i + e] = v;
+    }
+  }
+  __syncthreads();
+  if (tid < GB) {  // column `tid` of (1 + L)^-1
+    float t[GB];
+#pragma unroll
+    for (int i = 0; i < GB; ++i) {
+      t[i] = i == tid ? 1.f : 0.f;
+#pragma unroll
+      for (int m = 0; m < i; ++m) t[i] -= sh.L[i][m] * t[m];
+      out[R::TRI + i * R::PT + tid] = t[i];
+    }
   }
 }
 
 constexpr int GDN_COLS = 16;  // value columns per CTA
 constexpr int GDN_STAGES = 3;
 
-// A later token of a block enters the sum of an earlier one's output times a zero of the triangle, which is nothing unless its value
-// is infinite or no number. MASK leaves it out instead. Such a value stays in the state, whatever follows: without MASK, true is
-// returned (to all threads) where the state ends up so, and the state in memory is as it was.
-template <int D, bool MASK>
-__device__ __forceinline__ bool gdn_walk(float (*stage)[gdn_rec_floats<D>()], const float* __restrict__ rec,
-                                         const __nv_bfloat16* __restrict__ v, long long v_ld, int vcol, float* __restrict__ state,
-                                         __nv_bfloat16* __restrict__ out, long long o_ld, int ocol, int T, int t0, int nt, int H,
-                                         float scale) {
-  constexpr int REC = gdn_rec_floats<D>(), NP = D / 32, NV = REC / 4;  // NP row pairs per lane
-  const int tid = threadIdx.x, lane = tid & 31, l16 = lane & 15;
-  const int bh = blockIdx.x / (D / GDN_COLS), h = bh % H;
-  const int c0 = (blockIdx.x % (D / GDN_COLS)) * GDN_COLS + (tid >> 4) * 2;  // two columns per half warp
-  const int nb = (nt + GB - 1) / GB;
-  const long long row0 = (long long)(bh / H) * T + t0;
-  const float* src = rec + (long long)bh * nb * REC;
-  auto row = [&](int pr) { return (pr >> 1) * 64 + l16 * 4 + (pr & 1) * 2; };  // 16 lanes read 256 consecutive bytes
+struct Split {
+  uint32_t hi, lo;
+};
+__device__ __forceinline__ Split split_tf32(float x) {
+  Split s;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(s.hi) : "f"(x));
+  s.lo = __float_as_uint(x - __uint_as_float(s.hi));
+  return s;
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// An accumulator tile (16 value columns x 8) as the operand of the next product: its columns 2 t and 2 t + 1 are k = t and t + 4.
+__device__ __forceinline__ void operand(const float (&c)[4], Split (&v)[4]) {
+  v[0] = split_tf32(c[0]), v[1] = split_tf32(c[2]), v[2] = split_tf32(c[1]), v[3] = split_tf32(c[3]);
+}
+__device__ __forceinline__ void multiply(float (&c)[4], const Split (&a)[4], float b0, float b1) {
+  const Split x = split_tf32(b0), y = split_tf32(b1);
+  mma_tf32(c, a[0].lo, a[1].lo, a[2].lo, a[3].lo, x.hi, y.hi);
+  mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, x.lo, y.lo);
+  mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, x.hi, y.hi);
+}
 
-  uint64_t S[2][NP];
-  float* sp = state + (long long)bh * D * D + c0;
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    const float2 x = *reinterpret_cast<const float2*>(sp + (long long)row(i) * D);
-    const float2 y = *reinterpret_cast<const float2*>(sp + (long long)(row(i) + 1) * D);
-    S[0][i] = pack_f2(x.x, y.x);
-    S[1][i] = pack_f2(x.y, y.y);
+template <int D>
+struct GdnWalkShared {
+  float stage[GDN_STAGES][GdnRec<D>::COMMON + GDN_COLS * GdnRec<D>::PV];
+  float4 red[2][2][4][2][32];  // partial sums of the four warps, of alternating blocks: k P rows, q P rows
+  uint64_t full[GDN_STAGES];
+  int odd;                  // first token of a block at which something is no number
+};
+
+// One CTA's columns. A lane (g, t) = (lane / 4, lane % 4) of warp w holds the state of columns g, g + 8 and key rows w D / 4 + 8 n + 2 t + {0, 1}.
+template <int D>
+struct GdnWalk {
+  static constexpr int NT = D / 32;  // tiles of eight key rows of a warp
+  using R = GdnRec<D>;
+  const GdnBlockArgs& a;
+  GdnWalkShared<D>& sh;
+  const float* const rec;
+  const int nt, tid, lane, warp, g, t, bh, h, c0, nb;
+  const long long row0;
+  float S[NT][4];
+
+  __device__ __forceinline__ GdnWalk(const GdnBlockArgs& a_, GdnWalkShared<D>& sh_, const float* rec_, int t0, int nt_)
+      : a(a_), sh(sh_), rec(rec_), nt(nt_), tid(threadIdx.x), lane(threadIdx.x & 31), warp(threadIdx.x >> 5), g(lane >> 2), t(lane & 3), bh(blockIdx.x / (D / GDN_COLS)),
+        h(bh % a_.H), c0((blockIdx.x % (D / GDN_COLS)) * GDN_COLS), nb((nt_ + GB - 1) / GB), row0((long long)(bh / a_.H) * a_.T + t0) {}
+
+  __device__ __forceinline__ float* state_at(int n, int i) const {  // of S[n][i]
+    return a.state + ((long long)bh * D + warp * (D / 4) + n * 8 + 2 * t + (i & 1)) * D + c0 + g + (i >> 1) * 8;
   }
-  auto fetch = [&](int blk) {
-    if (blk < nb) {
-      const float4* from = reinterpret_cast<const float4*>(src + (long long)blk * REC);
-      float4* to = reinterpret_cast<float4*>(&stage[blk % GDN_STAGES][0]);
-      for (int i = tid; i < NV; i += 128)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + i)), "l"(from + i)
-                     : "memory");
+  __device__ __forceinline__ void load_state() {
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) S[n][i] = *state_at(n, i);
+  }
+  __device__ __forceinline__ void store_state() const {
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *state_at(n, i) = S[n][i];
+  }
+  __device__ __forceinline__ void start() {
+    if (tid == 0) {
+      for (int i = 0; i < GDN_STAGES; ++i) mbar_init(&sh.full[i], 1);
+      mbar_fence_init();
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // lane l of a half warp ends up with the results of tokens j, j + 1 for {k, q}[l >> 3] and column (l >> 2) & 1
-  const int j = (l16 & 3) * 2, col = (l16 >> 2) & 1;
-  const bool reads = l16 >= 8;
-  const unsigned short* vp = reinterpret_cast<const unsigned short*>(v) + vcol + h * D + c0 + col;
-  uint32_t vraw[2], vnext[2];
-  auto values = [&](int blk) {  // raw bits: converting here would wait for the load
+    __syncthreads();
+  }
+  // A block's record without the other CTAs' columns, by thread 0.
+  __device__ __forceinline__ void fetch(int blk) {
+    if (tid == 0 && blk < nb) {
+      const float* from = rec + ((long long)bh * nb + blk) * R::FLOATS;
+      float* to = sh.stage[blk % GDN_STAGES];
+      uint64_t* bar = &sh.full[blk % GDN_STAGES];
+      constexpr uint32_t common = R::COMMON * 4, columns = GDN_COLS * R::PV * 4;
+      mbar_expect_tx(bar, common + columns);
+      copy(to, from, common, bar);
+      copy(to + R::COMMON, from + R::COMMON + c0 * R::PV, columns, bar);
+    }
+  }
+  __device__ __forceinline__ static void copy(float* to, const float* from, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(to)), "l"(from), "r"(bytes),
+                 "r"(smem_u32(bar))
+                 : "memory");
+  }
+  // False where it never arrived. `nth`: how many records this stage held before this one.
+  __device__ __forceinline__ bool landed(int blk, int nth) { return mbar_wait(&sh.full[blk % GDN_STAGES], nth & 1); }
+  // x = v - s for tokens 8 e + 2 t, 8 e + 2 t + 1 of columns g, then of g + 8.
+  __device__ __forceinline__ void values(const float* r, int e, float (&f)[4]) const {
+    const uint32_t lo = __float_as_uint(r[R::COMMON + g * R::PV + 4 * e + t]), hi = __float_as_uint(r[R::COMMON + (g + 8) * R::PV + 4 * e + t]);
+    f[0] = __uint_as_float(lo << 16), f[1] = __uint_as_float(lo & 0xffff0000u);
+    f[2] = __uint_as_float(hi << 16), f[3] = __uint_as_float(hi & 0xffff0000u);
+  }
+
+  __device__ __forceinline__ void leave(int buf, int part, const float (&f)[4], const float (&s)[4]) const {
+    sh.red[buf][part][warp][0][lane] = make_float4(f[0], f[1], f[2], f[3]);
+    sh.red[buf][part][warp][1][lane] = make_float4(s[0], s[1], s[2], s[3]);
+  }
+  __device__ __forceinline__ void total(int buf, int part, int e, float (&s)[4]) const {
+    s[0] = s[1] = s[2] = s[3] = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float4 f = sh.red[buf][part][w][e][lane];
+      s[0] += f.x, s[1] += f.y, s[2] += f.z, s[3] += f.w;
+    }
+  }
+  __device__ __forceinline__ bool put(const float (&o)[4], int blk, int e, int limit) const {  // outputs of tokens 8 e + 2 t + {0, 1}
+    const int tok = 8 * e + 2 * t, left = min(limit, nt - blk * GB);
+    __nv_bfloat16* to = a.out + (row0 + blk * GB + tok) * a.o_ld + (a.ocol + h * D + c0 + g);
+    if (tok < left) to[0] = __float2bfloat16(o[0] * a.scale), to[8] = __float2bfloat16(o[2] * a.scale);
+    if (tok + 1 < left) to[a.o_ld] = __float2bfloat16(o[1] * a.scale), to[a.o_ld + 8] = __float2bfloat16(o[3] * a.scale);
+    return (tok < left && !(fmaxf(fabsf(o[0]), fabsf(o[2])) < INFINITY && o[0] == o[0] && o[2] == o[2])) ||
+           (tok + 1 < left && !(fmaxf(fabsf(o[1]), fabsf(o[3])) < INFINITY && o[1] == o[1] && o[3] == o[3]));
+  }
+
+  // A block's round, its record in `r`: outputs of its tokens before `limit`, and the state after all of them. Tokens from
+  // `limit` on count as nothing (LIMIT), as they are behind a token that is no number. True where an output is no number.
+  template <bool LIMIT>
+  __device__ __forceinline__ bool round(const float* r, int blk, int limit) {
+    float acc[4][4];  // [16 columns] x [k P of tokens 0-7, 8-15 | q P of tokens 0-7, 8-15], of this warp's key rows
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      Split s[4];
+      operand(S[n], s);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 b = *reinterpret_cast<const float2*>(r + (8 * j + g) * R::PK + warp * (D / 4) + 8 * n + 2 * t);
+        multiply(acc[j], s, b.x, b.y);
+      }
+    }
+    const int buf = blk & 1;
+    leave(buf, 0, acc[0], acc[1]);
+    leave(buf, 1, acc[2], acc[3]);
+    __syncthreads();  // and every warp is done with the block before
+    float x[2][4];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int t = blk * GB + j + e;
-      vnext[e] = (!reads && t < nt) ? (uint32_t)vp[(row0 + t) * v_ld] : 0u;
-    }
-  };
-  values(0);
-  fetch(0);
-  fetch(1);
-  for (int blk = 0; blk < nb; ++blk) {
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();  // this block's record has landed for every thread, and the one before it has been read by every thread
-    fetch(blk + 2);
-    vraw[0] = vnext[0];
-    vraw[1] = vnext[1];
-    values(blk + 1);
-    const float* r = &stage[blk % GDN_STAGES][0];
-    float val[4 * GB];
+      float f[4];
+      values(r, e, f);
+      total(buf, 0, e, x[e]);
 #pragma unroll
-    for (int w = 0; w < 2 * GB; ++w) {
-      uint64_t a0, a1;
-#pragma unroll
-      for (int i = 0; i < NP; i += 2) {
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(r + (1 + w) * D + row(i));
-        a0 = i == 0 ? mul2(x.x, S[0][0]) : fma2(x.x, S[0][i], a0);
-        a1 = i == 0 ? mul2(x.x, S[1][0]) : fma2(x.x, S[1][i], a1);
-        a0 = fma2(x.y, S[0][i + 1], a0);
-        a1 = fma2(x.y, S[1][i + 1], a1);
-      }
-      float lo, hi;
-      unpack_f2(a0, lo, hi);
-      val[(w / GB) * 2 * GB + w % GB] = lo + hi;
-      unpack_f2(a1, lo, hi);
-      val[(w / GB) * 2 * GB + GB + w % GB] = lo + hi;
-    }
-    reduce_scatter16(val, lane);
-    const float x0 = __uint_as_float(vraw[0] << 16) - val[0], x1 = __uint_as_float(vraw[1] << 16) - val[1];
-    const float* tri = r + (1 + 3 * GB) * D;
-    float u[2][GB];
-#pragma unroll
-    for (int i = 0; i < GB; ++i) {
-#pragma unroll
-      for (int c = 0; c < 2; ++c) u[c][i] = __shfl_sync(0xffffffffu, (i & 1) ? x1 : x0, (lane & 16) + c * 4 + i / 2);
-    }
-#pragma unroll
-    for (int i = 1; i < GB; ++i) {
-      float l[GB];
-      *reinterpret_cast<float4*>(l) = *reinterpret_cast<const float4*>(tri + i * GB);
-      if (i > 4) *reinterpret_cast<float4*>(l + 4) = *reinterpret_cast<const float4*>(tri + i * GB + 4);
-#pragma unroll
-      for (int m = 0; m < i; ++m) {
-        u[0][i] -= l[m] * u[0][m];
-        u[1][i] -= l[m] * u[1][m];
+      for (int i = 0; i < 4; ++i) {
+        x[e][i] = f[i] - x[e][i];
+        if (LIMIT && 8 * e + 2 * t + (i & 1) >= limit) x[e][i] = 0.f;
       }
     }
-#pragma unroll
-    for (int i = 0; i < NP; i += 2) {
-      const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(r + row(i));
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        S[c][i] = mul2(S[c][i], p.x);
-        S[c][i + 1] = mul2(S[c][i + 1], p.y);
-      }
-    }
-#pragma unroll
-    for (int w = 0; w < GB; ++w) {
-      const uint64_t u0 = pack_f2(u[0][w], u[0][w]), u1 = pack_f2(u[1][w], u[1][w]);
-#pragma unroll
-      for (int i = 0; i < NP; i += 2) {
-        const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(r + (1 + 2 * GB + w) * D + row(i));
-        S[0][i] = fma2(e.x, u0, S[0][i]);
-        S[0][i + 1] = fma2(e.y, u0, S[0][i + 1]);
-        S[1][i] = fma2(e.x, u1, S[1][i]);
-        S[1][i + 1] = fma2(e.y, u1, S[1][i + 1]);
-      }
-    }
-    if (reads) {
+    float u[2][4];
+    {
+      Split x0[4], x1[4];
+      operand(x[0], x0);
+      operand(x[1], x1);
+      const float* tri = r + R::TRI + 2 * t;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int t = blk * GB + j + e;
-        if (t < nt) {
-          const float* a = tri + GB * GB + (j + e) * GB;
-          float o = val[e];
-#pragma unroll
-          for (int m = 0; m < GB; ++m)
-            if (!MASK || m <= j + e) o += a[m] * (col ? u[1][m] : u[0][m]);
-          out[(row0 + t) * o_ld + ocol + h * D + c0 + col] = __float2bfloat16(o * scale);
+        u[e][0] = u[e][1] = u[e][2] = u[e][3] = 0.f;
+        const float2 b0 = *reinterpret_cast<const float2*>(tri + (8 * e + g) * R::PT);
+        multiply(u[e], x0, b0.x, b0.y);
+        if (e == 1) {
+          const float2 b1 = *reinterpret_cast<const float2*>(tri + (8 + g) * R::PT + 8);
+          multiply(u[e], x1, b1.x, b1.y);
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (LIMIT && 8 * e + 2 * t + (i & 1) >= limit) u[e][i] = 0.f;
       }
     }
+    Split u0[4], u1[4];
+    operand(u[0], u0);
+    operand(u[1], u1);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      const int d = warp * (D / 4) + 8 * n;
+      const float2 p = *reinterpret_cast<const float2*>(r + R::P + d + 2 * t);
+      S[n][0] *= p.x, S[n][1] *= p.y, S[n][2] *= p.x, S[n][3] *= p.y;
+      const float* e = r + R::E + 2 * t * R::PE + d + g;
+      multiply(S[n], u0, e[0], e[R::PE]);
+      multiply(S[n], u1, e[8 * R::PE], e[9 * R::PE]);
+    }
+    bool odd = false;
+    if (warp < 2) {  // outputs of tokens 8 warp + ...
+      float o[4];
+      total(buf, 1, warp, o);
+      const float* tri = r + R::A + (8 * warp + g) * R::PT + 2 * t;
+      const float2 b0 = *reinterpret_cast<const float2*>(tri);
+      multiply(o, u0, b0.x, b0.y);
+      if (warp == 1) {
+        const float2 b1 = *reinterpret_cast<const float2*>(tri + 8);
+        multiply(o, u1, b1.x, b1.y);
+      }
+      odd = put(o, blk, warp, limit);
+    }
+    return odd;
   }
-  if (!MASK) {
+
+  __device__ __forceinline__ bool state_odd() const {
     bool odd = false;
 #pragma unroll
-    for (int i = 0; i < 2 * NP; ++i) {
-      float a, b;
-      unpack_f2(S[i & 1][i >> 1], a, b);
-      odd |= !(fabsf(a) < INFINITY) || !(fabsf(b) < INFINITY);
-    }
-    if (__syncthreads_or(odd)) return true;
-  }
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    float a, b, c, d;
-    unpack_f2(S[0][i], a, b);
-    unpack_f2(S[1][i], c, d);
-    *reinterpret_cast<float2*>(sp + (long long)row(i) * D) = make_float2(a, c);
-    *reinterpret_cast<float2*>(sp + (long long)(row(i) + 1) * D) = make_float2(b, d);
+      for (int i = 0; i < 4; ++i) odd |= !(fabsf(S[n][i]) < INFINITY);
+    return odd;
   }
-  return false;
+
+  // The whole segment; true (to all threads) where an output or the state after it is no number. The state in memory is as it was. The rounds
+  // are those of round(), in another order: a block's outputs wait for the next round's barrier, so that there is one barrier a
+  // round, and what they need from the state is multiplied while the triangle's short chain runs.
+  __device__ __forceinline__ bool walk() {
+    start();
+    fetch(0);
+    fetch(1);
+    load_state();
+    bool odd = false, late = !landed(0, 0);
+    int at = 0, lap = 0;      // stage of the block, records that it held before
+    Split u0[4], u1[4];       // of the block before
+    float2 a0, a1;            // its row of A
+    a0 = a1 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u0[i] = u1[i] = Split{0u, 0u};
+    auto outputs = [&](int blk) {  // of a block whose sums all warps have left
+      const int e = warp & 1;
+      if ((warp >> 1) == (blk & 1)) {
+        float o[4];
+        total(blk & 1, 1, e, o);
+        multiply(o, u0, a0.x, a0.y);
+        if (e == 1) multiply(o, u1, a1.x, a1.y);
+        odd |= put(o, blk, e, GB);
+      }
+    };
+    for (int blk = 0; blk < nb; ++blk) {
+      const float* r = sh.stage[at];
+      const int buf = blk & 1;
+      Split s[NT][4];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) operand(S[n], s[n]);
+      float kp[2][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kp[j][i] = 0.f;
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float2 b = *reinterpret_cast<const float2*>(r + (8 * j + g) * R::PK + warp * (D / 4) + 8 * n + 2 * t);
+          multiply(kp[j], s[n], b.x, b.y);
+        }
+      leave(buf, 0, kp[0], kp[1]);
+      __syncthreads();  // all warps' sums; the record of the block before has been read
+      fetch(blk + 2);   // in its place
+      if (blk > 0) outputs(blk - 1);
+      float x[2][4];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float f[4];
+        values(r, e, f);
+        total(buf, 0, e, x[e]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[e][i] = f[i] - x[e][i];
+      }
+      float u[2][4], qp[2][4];
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) u[e][i] = qp[e][i] = 0.f;
+      {
+        Split x0[4], x1[4];
+        operand(x[0], x0);
+        operand(x[1], x1);
+        const float* tri = r + R::TRI + g * R::PT + 2 * t;
+        const float2 b0 = *reinterpret_cast<const float2*>(tri), b1 = *reinterpret_cast<const float2*>(tri + 8 * R::PT),
+                     b2 = *reinterpret_cast<const float2*>(tri + 8 * R::PT + 8);
+        multiply(u[0], x0, b0.x, b0.y);
+        multiply(u[1], x0, b1.x, b1.y);
+        multiply(u[1], x1, b2.x, b2.y);
+      }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float2 b = *reinterpret_cast<const float2*>(r + (GB + 8 * j + g) * R::PK + warp * (D / 4) + 8 * n + 2 * t);
+          multiply(qp[j], s[n], b.x, b.y);
+        }
+      leave(buf, 1, qp[0], qp[1]);
+      operand(u[0], u0);
+      operand(u[1], u1);
+      a0 = *reinterpret_cast<const float2*>(r + R::A + (8 * (warp & 1) + g) * R::PT + 2 * t);
+      a1 = *reinterpret_cast<const float2*>(r + R::A + (8 * (warp & 1) + g) * R::PT + 2 * t + 8);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const int d = warp * (D / 4) + 8 * n;
+        const float2 p = *reinterpret_cast<const float2*>(r + R::P + d + 2 * t);
+        S[n][0] *= p.x, S[n][1] *= p.y, S[n][2] *= p.x, S[n][3] *= p.y;
+        const float* e = r + R::E + 2 * t * R::PE + d + g;
+        multiply(S[n], u0, e[0], e[R::PE]);
+        multiply(S[n], u1, e[8 * R::PE], e[9 * R::PE]);
+      }
+      if (++at == GDN_STAGES) at = 0, ++lap;
+      if (blk + 1 < nb && !late) late = !landed(blk + 1, lap);  // what did not arrive is read as it is, and walked again
+    }
+    __syncthreads();
+    if (nb > 0) outputs(nb - 1);
+    return __syncthreads_or(odd || late || state_odd());
+  }
+
+  // The same where something is no number. A later token of a block enters an earlier one's sums times a zero of a triangle, which
+  // is nothing unless it is infinite or no number, and an operand of two parts does not carry an infinity. So: rounds up to the block at
+  // which something turns up, of that block the tokens before it, and then token by token as the recurrence says.
+  __device__ void walk_again() {
+    load_state();
+    for (int blk = 0; blk < nb; ++blk) {
+      __syncthreads();
+      if (tid == 0) sh.odd = GB;
+      float* r = sh.stage[0];
+      const float* src = rec + ((long long)bh * nb + blk) * R::FLOATS;
+      for (int i = tid; i < R::COMMON + GDN_COLS * R::PV; i += 128) r[i] = src[i < R::COMMON ? i : i + c0 * R::PV];
+      __syncthreads();
+      // the first token with a part that is no number
+      int first = GB;
+      for (int i = tid; i < GB * D; i += 128) {
+        const int tok = i / D, d = i % D;
+        const bool bad = !(fabsf(r[tok * R::PK + d]) < INFINITY) || !(fabsf(r[(GB + tok) * R::PK + d]) < INFINITY) ||
+                         !(fabsf(r[R::E + tok * R::PE + d]) < INFINITY);
+        if (bad) first = min(first, tok);
+      }
+      for (int i = tid; i < GB * GB; i += 128) {
+        const int tok = i / GB, m = i % GB;
+        if (!(fabsf(r[R::TRI + tok * R::PT + m]) < INFINITY) || !(fabsf(r[R::A + tok * R::PT + m]) < INFINITY)) first = min(first, tok);
+      }
+      for (int i = tid; i < D; i += 128)
+        if (!(fabsf(r[R::P + i]) < INFINITY)) first = min(first, GB - 1);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float f[4];
+        values(r, e, f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (!(fabsf(f[i]) < INFINITY)) first = min(first, 8 * e + 2 * t + (i & 1));
+      }
+      if (first < GB) atomicMin(&sh.odd, first);
+      __syncthreads();
+      int limit = sh.odd;
+      float kept[NT][4];
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kept[n][i] = S[n][i];
+      bool stop = limit < GB;
+      if (stop) {
+        // vectors of the tokens from `limit` on must not meet the zeros either
+        for (int i = tid; i < GB * D; i += 128) {
+          const int tok = i / D, d = i % D;
+          if (tok >= limit) r[tok * R::PK + d] = r[(GB + tok) * R::PK + d] = r[R::E + tok * R::PE + d] = 0.f;
+        }
+        for (int i = tid; i < GB * GB; i += 128) {
+          const int tok = i / GB, m = i % GB;
+          if (tok >= limit || m >= limit) r[R::TRI + tok * R::PT + m] = r[R::A + tok * R::PT + m] = 0.f;
+        }
+        __syncthreads();
+        if (__syncthreads_or(round<true>(r, blk, limit))) limit = 0;  // too large for a sum already
+      } else {
+        stop = __syncthreads_or(round<false>(r, blk, GB) || state_odd());
+      }
+      if (stop) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) S[n][i] = kept[n][i];
+        tokens(blk * GB, blk * GB + (limit < GB ? limit : 0));  // what overflows is as the token kernel has it
+        return;
+      }
+    }
+    store_state();
+  }
+
+  // Token by token from `from` on; outputs from token `first` on. The state goes through shared memory: thread (p, c) has D / 8 rows of column c.
+  __device__ void tokens(int from, int first) {
+    constexpr int RP = D / 8;
+    __syncthreads();
+    float* Sm = sh.stage[0];                    // [D][16]
+    float *kr = Sm + D * GDN_COLS, *kb = kr + D, *qr = kb + D, *dec = qr + D;
+    float* part = dec + D;                      // [2][8][16]
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) Sm[(warp * (D / 4) + n * 8 + 2 * t + (i & 1)) * GDN_COLS + g + (i >> 1) * 8] = S[n][i];
+    __syncthreads();
+    const int c = tid % GDN_COLS, p = tid / GDN_COLS;
+    float st[RP];
+#pragma unroll
+    for (int i = 0; i < RP; ++i) st[i] = Sm[(p * RP + i) * GDN_COLS + c];
+    for (int tok = from; tok < nt; ++tok) {
+      const long long row = row0 + tok;
+      __syncthreads();
+      for (int d = tid; d < D; d += 128) {
+        const float kk = __bfloat162float(a.k[row * a.k_ld + a.kcol + h * D + d]);
+        const float b = a.beta_mode == 0 ? 1.f : a.beta_mode == 1 ? a.beta[row * a.H + h] : a.beta[(row * a.H + h) * D + d];
+        kr[d] = kk;
+        kb[d] = b * kk;
+        qr[d] = __bfloat162float(a.q[row * a.q_ld + a.qcol + h * D + d]);
+        dec[d] = __expf(gdn_log_decay(__bfloat162float(a.g[row * a.g_ld + a.gcol + h * D + d]), a.logits != 0));
+      }
+      __syncthreads();
+      float acc = 0.f;
+#pragma unroll
+      for (int i = 0; i < RP; ++i) acc += kr[p * RP + i] * st[i];
+      part[p * GDN_COLS + c] = acc;
+      __syncthreads();
+      float u = __bfloat162float(a.v[row * a.v_ld + a.vcol + h * D + c0 + c]), o = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) u -= part[i * GDN_COLS + c];
+#pragma unroll
+      for (int i = 0; i < RP; ++i) {
+        st[i] = dec[p * RP + i] * st[i] + kb[p * RP + i] * u;
+        o += qr[p * RP + i] * st[i];
+      }
+      part[(8 + p) * GDN_COLS + c] = o;
+      __syncthreads();
+      if (p == 0 && tok >= first) {
+        o = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o += part[(8 + i) * GDN_COLS + c];
+        a.out[row * a.o_ld + a.ocol + h * D + c0 + c] = __float2bfloat16(o * a.scale);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RP; ++i) a.state[((long long)bh * D + p * RP + i) * D + c0 + c] = st[i];
+  }
+};
+
+// In a function of its own, so that its registers are not the common walk's.
+template <int D>
+__device__ __noinline__ void gdn_walk_again(const GdnBlockArgs& a, GdnWalkShared<D>& sh, const float* rec, int t0, int nt) {
+  GdnWalk<D> w(a, sh, rec, t0, nt);
+  w.walk_again();
 }
 
-// The masked walk in a function of its own: 8192 tokens, 16 heads of 128 take 1031 us without it, 1064 with it, and 1107 with its
-// selections in the common loop.
+// The first `walks` CTAs walk tokens [t0, t0 + nt) by the records in `rec`; the others form those of the tokens after them, of which there
+// are `next_nt`, in `next_rec`, on the SMs and issue slots that the walk leaves free.
 template <int D>
-__device__ __noinline__ void gdn_walk_again(float (*stage)[gdn_rec_floats<D>()], const float* __restrict__ rec,
-                                            const __nv_bfloat16* __restrict__ v, long long v_ld, int vcol, float* __restrict__ state,
-                                            __nv_bfloat16* __restrict__ out, long long o_ld, int ocol, int T, int t0, int nt, int H,
-                                            float scale) {
-  gdn_walk<D, true>(stage, rec, v, v_ld, vcol, state, out, o_ld, ocol, T, t0, nt, H, scale);
-}
-
-template <int D>
-__global__ void __launch_bounds__(128) gdn_block_walk_kernel(const float* __restrict__ rec, const __nv_bfloat16* __restrict__ v,
-                                                             long long v_ld, int vcol, float* __restrict__ state,
-                                                             __nv_bfloat16* __restrict__ out, long long o_ld, int ocol, int T,
-                                                             int t0, int nt, int H, float scale) {
-  __shared__ __align__(16) float stage[GDN_STAGES][gdn_rec_floats<D>()];
-  if (gdn_walk<D, false>(stage, rec, v, v_ld, vcol, state, out, o_ld, ocol, T, t0, nt, H, scale))
-    gdn_walk_again<D>(stage, rec, v, v_ld, vcol, state, out, o_ld, ocol, T, t0, nt, H, scale);
+__global__ void __launch_bounds__(128) gdn_block_kernel(const __grid_constant__ GdnBlockArgs a, int walks, const float* rec, int t0, int nt,
+                                                        float* next_rec, int next_nt) {
+  extern __shared__ __align__(16) uint8_t block_smem[];
+  if ((int)blockIdx.x >= walks) {
+    gdn_block_prep<D>(a, *reinterpret_cast<GdnPrepShared<D>*>(block_smem), next_rec, t0 + nt, next_nt, (int)blockIdx.x - walks);
+    return;
+  }
+  GdnWalkShared<D>& sh = *reinterpret_cast<GdnWalkShared<D>*>(block_smem);
+  GdnWalk<D> w(a, sh, rec, t0, nt);
+  if (w.walk()) gdn_walk_again<D>(a, sh, rec, t0, nt);
+  else w.store_state();
 }
 
 template <int D>
 void run_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode, float* state,
                 const GlaMat& O, int B, int T, int H, bool logits, float scale, float* rec, int seg, cudaStream_t s) {
   auto p = [](const GlaMat& m) { return reinterpret_cast<const __nv_bfloat16*>(m.ptr); };
-  for (int t0 = 0; t0 < T; t0 += seg) {
-    const int nt = T - t0 < seg ? T - t0 : seg, nrec = B * H * ((nt + GB - 1) / GB);
-    gdn_block_prep_kernel<D><<<(nrec + 3) / 4, 128, 0, s>>>(p(Q), Q.ld, Q.col0, p(K), K.ld, K.col0, p(G), G.ld, G.col0, beta,
-                                                           beta_mode, rec, T, t0, nt, H, logits ? 1 : 0, nrec);
-    gdn_block_walk_kernel<D><<<B * H * (D / GDN_COLS), 128, 0, s>>>(rec, p(V), V.ld, V.col0, state,
-                                                                   reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(O.ptr)), O.ld,
-                                                                   O.col0, T, t0, nt, H, scale);
+  constexpr int walk_smem = (int)sizeof(GdnWalkShared<D>), prep_smem = (int)sizeof(GdnPrepShared<D>);
+  static PerDeviceOnce once;
+  if (once.first_use()) {
+    const cudaError_t e = cudaFuncSetAttribute(gdn_block_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_smem);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("gdn_blocks attribute: ") + cudaGetErrorString(e));
+  }
+  const GdnBlockArgs a{p(Q), p(K), p(V), p(G), Q.ld, K.ld, V.ld, G.ld, O.ld, Q.col0, K.col0, V.col0, G.col0, O.col0, beta, beta_mode, state,
+                       reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(O.ptr)), T, H, logits ? 1 : 0, scale};
+  auto tokens = [&](int t0) { return T - t0 < seg ? T - t0 : seg; };
+  auto records = [&](int nt) { return B * H * ((nt + GB - 1) / GB); };
+  float* half[2] = {rec, rec + (long long)records(tokens(0)) * GdnRec<D>::FLOATS};
+  gdn_block_kernel<D><<<records(tokens(0)), 128, prep_smem, s>>>(a, 0, nullptr, 0, 0, half[0], tokens(0));
+  for (int t0 = 0, i = 0; t0 < T; t0 += seg, ++i) {
+    const int nt = tokens(t0), after = t0 + nt < T ? tokens(t0 + nt) : 0, walks = B * H * (D / GDN_COLS);
+    gdn_block_kernel<D><<<walks + records(after), 128, walk_smem, s>>>(a, walks, half[i & 1], t0, nt, half[~i & 1], after);
   }
 }
 
-// Tokens per segment: whole blocks whose records fill at most 48 MB (they are read back from the 126 MB L2), at least 128
-// tokens so that the two launches of a segment stay small beside its walk.
+constexpr int rec_floats(int D) { return D == 64 ? GdnRec<64>::FLOATS : GdnRec<128>::FLOATS; }
+
+// Tokens per segment: whole blocks whose records fill at most 40 MB (with the next segment's they are read back from the 126 MB
+// L2), at least 128 tokens so that the launch of a segment stays small beside its walk (256 heads of 128, 512 tokens:
+// 702 us, and 806 with 64).
 int segment_tokens(int BH, int D) {
-  const long long per_block = (long long)BH * ((1 + 3 * GB) * D + GDN_TRI) * 4;
-  const long long blocks = (48ll << 20) / per_block;
-  return (int)(blocks < 16 ? 16 : blocks) * GB;
+  const long long blocks = (40ll << 20) / ((long long)BH * rec_floats(D) * 4);
+  return (int)(blocks < 8 ? 8 : blocks) * GB;
 }
 
 }  // namespace
 
-// Eight tokens a round win where the recurrence is a chain that the chip waits for: the walk's work grows with the heads, the token
-// kernel's time hardly does until its CTAs fill the SMs. Token kernel -> blocks, us: 16 heads of 64, 8 tokens 10 -> 10.5, 16 tokens 14 ->
-// 12, 512 tokens 318 -> 71; 256 of 64, 16 tokens 17 -> 20, 32 tokens 30 -> 28; 512 of 64, 130 tokens 142 -> 157, 512 tokens 539 -> 530; 16 of
-// 128, 8 tokens 14 -> 13; 128 of 128, 16 tokens 24 -> 32, 32 tokens 42 -> 41; 256 of 128, 130 tokens 223 -> 240, 512 tokens 849 -> 796;
-// 1024 of 64, 512 tokens 963 -> 1019.
+// Sixteen tokens a round win where the recurrence is a chain that the chip waits for: the walk's work grows with the heads, the token
+// kernel's time hardly does until its CTAs fill the SMs, and a round costs the same for one token as for sixteen. Token kernel -> blocks,
+// us: 16 heads of 64, 8 tokens 7.1 -> 8.0, 12 tokens 9.5 -> 8.4, 512 tokens 315 -> 40; 128 of 64, 17 tokens 13 -> 15, 24 tokens 17 -> 15; 256
+// of 64, 24 tokens 20 -> 21, 32 tokens 26 -> 21; 512 of 64, 32 tokens 36 -> 35, 130 tokens 137 -> 140, 512 tokens 533 -> 508; 1024 of 64, 130
+// tokens 247 -> 268; 16 of 128, 4 tokens 7.4 -> 9.8, 8 tokens 11.5 -> 10.3; 64 of 128, 8 tokens 11.7 -> 14.4, 12 tokens 16.1 -> 15.0; 128 of
+// 128, 17 tokens 22 -> 28, 24 tokens 28.7 -> 27.5; 512 of 128, 24 tokens 85 -> 93, 32 tokens 111 -> 97, 512 tokens 1676 -> 1353. More than
+// 512 heads would take hundreds of megabytes of records.
 static bool gdn_in_blocks(long long heads, int T, int D) {
   if (D != 64 && D != 128) return false;
-  if (T >= 512) return heads <= 512;
-  const long long halves = heads * (D / 64);
-  return T >= (D == 128 && heads <= 16 ? 8 : 12) && halves <= 448 && T * 8 >= halves;
+  const int least = D == 128 && heads <= 16 ? 8 : heads <= 64 ? 12 : heads <= 128 ? 24 : 32;
+  return heads <= 512 && T >= least;
 }
 
 long long gdn_block_workspace_floats(int B, int T, int H, int D) {
   if (!gdn_in_blocks((long long)B * H, T, D)) return 0;
   const int seg = segment_tokens(B * H, D), nt = T < seg ? T : seg;
-  return (long long)B * H * ((nt + GB - 1) / GB) * ((1 + 3 * GB) * D + GDN_TRI);
+  return (long long)B * H * ((nt + GB - 1) / GB) * rec_floats(D) * (T > seg ? 2 : 1);
 }
 
 void launch_gdn_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode,

@@ -96,8 +96,8 @@ void launch_gdn_recurrent(const GlaMat& Q, const GlaMat& K, const GlaMat& V, con
                           int beta_mode, float* state, const GlaMat& O, int B, int T, int H, int D, bool gate_logits,
                           float scale, cudaStream_t s);
 
-// The same, eight tokens per round; `workspace`: fp32 [gdn_block_workspace_floats(...)], 16-byte aligned, 0 floats where the token
-// recurrence is the faster one. q, k, g rows must start on 8-byte boundaries.
+// The same, sixteen tokens per round; `workspace`: fp32 [gdn_block_workspace_floats(...)], 16-byte aligned, 0 floats where the token
+// recurrence is the faster one. q, k, v, g rows must start on 8-byte boundaries.
 long long gdn_block_workspace_floats(int B, int T, int H, int D);
 void launch_gdn_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode,
                        float* state, const GlaMat& O, int B, int T, int H, int D, bool gate_logits, float scale, float* workspace,
