@@ -53,6 +53,49 @@ def test_rounds_of_sixteen_tokens_against_the_token_recurrence(B, T, H, D, beta_
     test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims)
 
 
+@pytest.mark.parametrize("chunks", [1, 2, 7, 8, 9, 15, 16, 17, 33])
+@pytest.mark.parametrize("D", [64, 128])
+def test_state_scan_over_batches_of_chunks(chunks, D):
+    from triune_b200 import ops
+
+    q, k, v, g, s0 = _mixer_inputs(1, 64 * chunks, 2, D)
+    odd = torch.empty(s0.numel() + 1, device="cuda")[1:].view_as(s0).copy_(s0)  # a state that starts on any number
+    x = [t.requires_grad_(True) for t in (q, k, v, g, odd)]
+    o, s = ops.gla(*x[:4], initial_state=x[4], gate_logits=True)
+    w, ws = torch.randn_like(o), torch.randn_like(s)
+    grads = torch.autograd.grad((o * w).sum() + (s * ws).sum(), x)
+    y = [t.detach().double().requires_grad_(True) for t in x]
+    gl = F.logsigmoid(y[3]).clamp(min=gla_cuda.GLA_MIN_LOG_DECAY)
+    S, rows = y[4], []
+    for c in range(64 * chunks):
+        S = S * gl[:, c].exp().unsqueeze(-1) + y[1][:, c].unsqueeze(-1) * y[2][:, c].unsqueeze(-2)
+        rows.append((y[0][:, c].unsqueeze(-2) @ S).squeeze(-2))
+    oo = torch.stack(rows, 1)
+    want = torch.autograd.grad((oo * w.double()).sum() + (S * ws.double()).sum(), y)
+    # states between chunks and chunk operands are bf16: a relative error of 2^-8 for each of a handful of roundings
+    assert _rel(o, oo) < 2.0 ** -6 and _rel(s, S) < 2.0 ** -6
+    # a gate's gradient is a sum of terms that nearly cancel: its bound follows from their sizes (_gate_error)
+    z = [t.detach() for t in y]
+    assert _gate_error(grads[3], want[3], z[0], z[1], want[0], want[1], (ws.double() * S.detach()).sum(-1), torch.sigmoid(-z[3])) < 1
+    for n in (0, 1, 2, 4):
+        assert _rel(grads[n], want[n]) < 2.0 ** -5, n
+
+
+@pytest.mark.parametrize("B,T,H,D", [(1, 1, 1, 64), (2, 37, 3, 64), (1, 4736, 1, 64), (1, 4737, 2, 64), (3, 17, 5, 128), (1, 1579, 3, 128), (5, 1000, 7, 128)])
+@pytest.mark.parametrize("rope", [False, True])
+def test_feature_map_of_few_and_many_tokens(B, T, H, D, rope):
+    from triune_b200 import ops
+
+    qkvg = torch.randn(B * T, 4 * H * D, device="cuda", generator=torch.Generator("cuda").manual_seed(T)).bfloat16()
+    cos, sin = ops.rope_tables(T, D, 10000.0, 0, "cuda") if rope else (None, None)
+    got = ops.qk_feature_map(qkvg, cos, sin, B, T, H, D)
+    for n, t in enumerate(got[:2]):
+        f = F.normalize(F.elu(qkvg[:, n * H * D : (n + 1) * H * D].reshape(B, T, H, D).double()) + 1.0, dim=-1, eps=1e-6)
+        if rope:
+            f = ref.apply_rope(f, cos.double(), sin.double())
+        assert (t.double() - f).abs().max() <= 2.0 ** -8 * f.abs().max()  # one rounding to bf16
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38])
 @pytest.mark.parametrize("where", ["k", "q", "state"])
 def test_rounds_of_sixteen_tokens_with_infinities_and_overflow(where, value):
