@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(256) column_parts_kernel(const float* __restri
 // (token, head, q-or-k) row of D elements, handled by D/8 lanes with one 16-byte load each; the rotation
 // partner of element i (i + D/2) lives in lane ^ (D/16). out: [tokens, 2, H, D] contiguous. cos/sin: rows of
 // `tab_ld` floats of which D/2 are used, token t uses position (t % T) (tokens are laid out [B, T]); read in place and in 16-byte
-// vectors. Vectors are numbered in 32 bits: their division into token, head and side in 64 bits cost a seventh of
-// the time (32768 tokens, 6 heads of 64, before -> after: forward 35 -> 30 us, backward 50 -> 40; 8192 tokens, 8 heads of 128: 25 -> 22 and 36 -> 29).
+// vectors. In the backward pass vectors are numbered in 32 bits: their division into token, head and side in 64 bits cost a seventh of
+// the time (32768 tokens, 6 heads of 64, before -> after: 50 -> 40 us; 8192 tokens, 8 heads of 128: 36 -> 29).
 template <int D>
 struct PrepGeom {
   static constexpr int LPV = D / 8;        // lanes per vector
@@ -349,47 +349,65 @@ __device__ __forceinline__ void table8(const float* t, long long at, float none,
   f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
 }
 
+// A warp takes one token: its lanes' rotary factors are read once for all heads, queries and keys, of which VPW vectors at a time pass
+// through it, PREP_AHEAD steps of loads in flight. Few tokens are cut into `parts` of their vectors. Bound by instructions, then by
+// memory; one vector after another with its token, head and factors looked up each time -> here: 32768 tokens, 6 heads of 64, 30 ->
+// 25 us (4.1 TB/s); 8192, 12 of 128, 31 -> 21; 8192, 16 of 128, 49 -> 31; 65536, 6 of 64, 59 -> 49. The backward pass, with
+// two rows and twice the registers a vector, is the slower for it (40 -> 51 us) and stays vector by vector.
+constexpr int PREP_AHEAD = 4;
+
 template <int D>
 __global__ void __launch_bounds__(256) qk_prep_fwd_kernel(const __nv_bfloat16* __restrict__ in, long long in_ld,
                                                           int k_col_offset, __nv_bfloat16* __restrict__ out,
                                                           const float* __restrict__ cs, const float* __restrict__ sn, int tab_ld,
-                                                          long long tokens, int T, int H) {
+                                                          long long tokens, int T, int H, int parts) {
   constexpr int LPV = PrepGeom<D>::LPV, VPW = PrepGeom<D>::VPW;
-  const int lane = threadIdx.x & 31, sub = lane % LPV, vin = lane / LPV;
-  const long long total = tokens * 2 * H;
+  const int lane = threadIdx.x & 31, sub = lane % LPV, vin = lane / LPV, steps = (2 * H + VPW - 1) / VPW;
+  const bool upper = sub >= LPV / 2;
+  const int ci = (sub % (LPV / 2)) * 8;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * VPW; base < total;
-       base += warps * VPW) {
-    const long long idx = base + vin;
-    const bool live = idx < total;
-    const unsigned cidx = (unsigned)(live ? idx : total - 1), pair = cidx / (unsigned)H, tok32 = pair >> 1;
-    const int h = (int)(cidx - pair * (unsigned)H), which = (int)(pair & 1u);
-    const long long tok = tok32;
-    float f[8];
-    load8(in + tok * in_ld + (which ? k_col_offset : 0) + h * D + sub * 8, f);
-    float ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      f[i] = f[i] > 0.f ? f[i] + 1.f : __expf(f[i]);
-      ss += f[i] * f[i];
-    }
-    ss = group_sum<LPV>(ss);
-    const float inv = 1.0f / fmaxf(sqrtf(ss), 1e-6f);
-    float o[8];
-    const bool upper = sub >= LPV / 2;
-    const long long pos = tok32 % (unsigned)T;
-    const int ci = (sub % (LPV / 2)) * 8;
+  for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < tokens * parts; item += warps) {
+    const long long tok = parts == 1 ? item : item / parts;
+    const int part = parts == 1 ? 0 : (int)(item - tok * parts);
+    const int s0 = part * steps / parts, s1 = (part + 1) * steps / parts;
+    const unsigned pos = (unsigned)tok % (unsigned)T;
+    const __nv_bfloat16* src = in + tok * in_ld + sub * 8;
+    __nv_bfloat16* dst = out + tok * 2 * H * D + sub * 8;
     float tc[8], ts[8];
-    table8(cs, pos * tab_ld + ci, 1.f, tc);
-    table8(sn, pos * tab_ld + ci, 0.f, ts);
+    table8(cs, (long long)pos * tab_ld + ci, 1.f, tc);
+    table8(sn, (long long)pos * tab_ld + ci, 0.f, ts);
+    for (int s = s0; s < s1; s += PREP_AHEAD) {
+      uint4 raw[PREP_AHEAD];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float mine = f[i] * inv;
-      const float other = __shfl_xor_sync(0xffffffffu, mine, LPV / 2);
-      const float c = tc[i], s = ts[i];
-      o[i] = upper ? (mine * c + other * s) : (mine * c - other * s);
+      for (int n = 0; n < PREP_AHEAD; ++n) {
+        const int v = min((s + n) * VPW + vin, 2 * H - 1);  // queries' heads, then keys'
+        if (s + n < s1) raw[n] = *reinterpret_cast<const uint4*>(src + (v < H ? v * D : k_col_offset + (v - H) * D));
+      }
+#pragma unroll
+      for (int n = 0; n < PREP_AHEAD; ++n) {
+        if (s + n >= s1) break;
+        const int v = (s + n) * VPW + vin;
+        float f[8];
+        unpack_row8(raw[n], f);
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          f[i] = f[i] > 0.f ? f[i] + 1.f : __expf(f[i]);
+          ss += f[i] * f[i];
+        }
+        ss = group_sum<LPV>(ss);
+        const float inv = 1.0f / fmaxf(sqrtf(ss), 1e-6f);
+        float o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float mine = f[i] * inv;
+          const float other = __shfl_xor_sync(0xffffffffu, mine, LPV / 2);
+          const float c = tc[i], t = ts[i];
+          o[i] = upper ? (mine * c + other * t) : (mine * c - other * t);
+        }
+        if (v < 2 * H) store8(dst + v * D, o);
+      }
     }
-    if (live) store8(out + ((tok * 2 + which) * H + h) * D + sub * 8, o);
   }
 }
 
@@ -446,6 +464,13 @@ __global__ void __launch_bounds__(256) qk_prep_bwd_kernel(const __nv_bfloat16* _
     }
     if (live) store8(d_in + tok * d_in_ld + (which ? k_col_offset : 0) + h * D + sub * 8, o);
   }
+}
+
+// Parts that a token's vectors are cut into: enough warps for the chip (eight on each of 592 schedulers), a step at least for each.
+inline int prep_parts(long long tokens, int H, int D) {
+  const int steps = (2 * H + 256 / D - 1) / (256 / D);
+  const long long want = (148ll * 32 + tokens - 1) / tokens;
+  return (int)(want < 1 ? 1 : want > steps ? steps : want);
 }
 
 inline int row_grid(long long work_items, int per_block) {
@@ -534,11 +559,11 @@ void launch_qk_prep_fwd(const __nv_bfloat16* in, long long in_ld, int k_col_offs
                         const float* sn, int tab_ld, long long tokens, int T, int H, int D, cudaStream_t s) {
   if (tokens == 0) return;
   check_vectors(tokens * 2 * H);
-  const int grid = row_grid(tokens * 2 * H, 8 * (256 / D));
+  const int parts = prep_parts(tokens, H, D), grid = row_grid(tokens * parts, 8);
   if (D == 64)
-    qk_prep_fwd_kernel<64><<<grid, 256, 0, s>>>(in, in_ld, k_col_offset, out, cs, sn, tab_ld, tokens, T, H);
+    qk_prep_fwd_kernel<64><<<grid, 256, 0, s>>>(in, in_ld, k_col_offset, out, cs, sn, tab_ld, tokens, T, H, parts);
   else
-    qk_prep_fwd_kernel<128><<<grid, 256, 0, s>>>(in, in_ld, k_col_offset, out, cs, sn, tab_ld, tokens, T, H);
+    qk_prep_fwd_kernel<128><<<grid, 256, 0, s>>>(in, in_ld, k_col_offset, out, cs, sn, tab_ld, tokens, T, H, parts);
 }
 
 void launch_qk_prep_bwd(const __nv_bfloat16* in, long long in_ld, int k_col_offset, const __nv_bfloat16* dout,
