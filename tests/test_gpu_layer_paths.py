@@ -53,6 +53,50 @@ def test_rounds_of_sixteen_tokens_against_the_token_recurrence(B, T, H, D, beta_
     test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims)
 
 
+@pytest.mark.parametrize("E,K,N,D,skew", [(8, 2, 1, 64, 0.0), (8, 1, 257, 72, 4.0), (16, 2, 1000, 384, 0.0), (64, 4, 300, 128, 6.0), (8, 2, 4096, 1536, 3.0)])
+def test_routing_statistics_in_one_kernel(E, K, N, D, skew, monkeypatch):
+    from triune_b200.models import MoE_FFN
+
+    def run(native):
+        torch.manual_seed(E + N)
+        m = MoE_FFN(D, num_experts=E, top_k=K, expert_hidden=64).cuda().bfloat16()
+        for name in ("expert_bias", "expert_load_ratio", "last_centroids"):
+            setattr(m, name, getattr(m, name).float())
+        m.expert_bias[0] += skew  # tokens beyond the capacity are dropped
+        m.train()
+        out = []
+        with monkeypatch.context() as mp:
+            if not native:
+                mp.setattr(MoE_FFN, "_stats_on_kernels", lambda *a: False)
+            for step in range(3):  # no centroids yet, then running ones
+                m._global_step.fill_(step * 700)
+                with torch.no_grad():
+                    m(torch.randn(1, N, D, device="cuda", generator=torch.Generator("cuda").manual_seed(step)).bfloat16())
+                out.append([t.clone() for t in (m.last_counts, m.last_accepted_counts, m.last_dropped_counts, m._overflow_counter, m._pending_bias_update,
+                                                m.expert_load_ratio, m.last_centroids)])
+                m.step_bias()
+        return out
+
+    got, want = run(True), run(False)
+    for g, w in zip(got, want):
+        for n in range(4):
+            assert g[n].dtype == w[n].dtype and g[n].shape == w[n].shape and torch.equal(g[n], w[n]), n
+        for n in (4, 5, 6):  # fp32, a few operations in another order
+            assert g[n].shape == w[n].shape and (g[n] - w[n]).abs().max() <= 2.0 ** -20 * max(1.0, float(w[n].abs().max())), n
+    assert skew == 0.0 or int(want[-1][3]) > 0
+
+
+@pytest.mark.parametrize("step", [0, 1, 12345, 10 ** 9])
+def test_router_temperature_at_a_step(step):
+    from triune_b200.models.moe import MOE_TEMPERATURE_STEPS
+    from triune_b200 import _ext
+
+    s = torch.tensor(step, device="cuda")
+    want = (1.0 - s.float() / MOE_TEMPERATURE_STEPS).clamp(min=0.1)
+    got = _ext.ext().moe_temperature(s, float(MOE_TEMPERATURE_STEPS), 0.1)
+    assert got.shape == want.shape and abs(float(got) - float(want)) <= 2.0 ** -22
+
+
 @pytest.mark.parametrize("chunks", [1, 2, 7, 8, 9, 15, 16, 17, 33])
 @pytest.mark.parametrize("D", [64, 128])
 def test_state_scan_over_batches_of_chunks(chunks, D):

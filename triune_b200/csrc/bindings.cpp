@@ -348,6 +348,50 @@ std::vector<Tensor> moe_plan_sorted(const Tensor& sorted_keys, const Tensor& ord
   return {pos, keep, row_src, tile_group, offsets, accepted};
 }
 
+// max(1 - step / steps, least) as an fp32 scalar on the device of the step (int64)
+Tensor moe_temperature(const Tensor& step, double steps, double least) {
+  TORCH_CHECK(step.is_cuda() && step.scalar_type() == at::kLong && step.numel() == 1, "moe_temperature: step int64 on the device");
+  c10::cuda::CUDAGuard guard(step.device());
+  Tensor out = torch::empty({}, step.options().dtype(at::kFloat));
+  tb::launch_moe_temperature((const long long*)step.data_ptr<int64_t>(), (float)steps, (float)least, out.data_ptr<float>(), cur_stream());
+  return out;
+}
+
+// [N, E] bf16: 1 for each accepted expert of a token
+Tensor moe_mask(const Tensor& idx, const c10::optional<Tensor>& keep, int64_t E) {
+  TORCH_CHECK(idx.is_cuda() && idx.scalar_type() == at::kLong && idx.dim() == 2 && idx.is_contiguous() && E % 8 == 0, "moe_mask: idx int64 [N, K], E % 8 == 0");
+  const bool has = keep.has_value() && keep->defined();
+  if (has) TORCH_CHECK(keep->is_cuda() && keep->scalar_type() == at::kBool && keep->is_contiguous() && keep->sizes() == idx.sizes(), "moe_mask: keep bool [N, K]");
+  c10::cuda::CUDAGuard guard(idx.device());
+  Tensor mask = torch::empty({idx.size(0), E}, idx.options().dtype(at::kBFloat16));
+  tb::launch_moe_mask((const long long*)idx.data_ptr<int64_t>(), has ? (const unsigned char*)keep->data_ptr<bool>() : nullptr, (int)idx.size(0), (int)E,
+                      (int)idx.size(1), bfm(mask), cur_stream());
+  return mask;
+}
+
+// -> requested, dropped (int64 [E]), pending bias update (fp32 [E]); overflow, load and centroids are updated in place
+std::vector<Tensor> moe_stats(const Tensor& slot_counts, const c10::optional<Tensor>& accepted, const Tensor& sums, Tensor& overflow, Tensor& load,
+                              Tensor& centroids, double target, double rate, double ema) {
+  const int64_t E = slot_counts.size(0), K = slot_counts.size(1), D = centroids.size(1);
+  TORCH_CHECK(slot_counts.is_cuda() && slot_counts.scalar_type() == at::kInt && slot_counts.is_contiguous(), "moe_stats: counts int32 [E, K]");
+  for (const Tensor* t : {&sums, static_cast<const Tensor*>(&centroids)})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->dim() == 2 && t->size(0) == E && t->size(1) == D,
+                "moe_stats: sums and centroids fp32 [E, D]");
+  TORCH_CHECK(load.is_cuda() && load.scalar_type() == at::kFloat && load.is_contiguous() && load.numel() == E, "moe_stats: load fp32 [E]");
+  TORCH_CHECK(overflow.is_cuda() && overflow.scalar_type() == at::kLong && overflow.numel() == 1, "moe_stats: overflow int64");
+  const bool has = accepted.has_value() && accepted->defined();
+  if (has) TORCH_CHECK(accepted->is_cuda() && accepted->scalar_type() == at::kLong && accepted->is_contiguous() && accepted->numel() == E, "moe_stats: accepted int64 [E]");
+  c10::cuda::CUDAGuard guard(slot_counts.device());
+  auto l = slot_counts.options().dtype(at::kLong);
+  Tensor requested = torch::empty({E}, l), dropped = torch::empty({E}, l), pending = torch::empty({E}, sums.options());
+  auto lp = [](const Tensor& t) { return reinterpret_cast<long long*>(t.data_ptr<int64_t>()); };
+  tb::launch_moe_stats({slot_counts.data_ptr<int>(), has ? lp(*accepted) : nullptr, sums.data_ptr<float>(), lp(requested), lp(dropped), lp(overflow),
+                        pending.data_ptr<float>(), load.data_ptr<float>(), centroids.data_ptr<float>(), (int)E, (int)K, (int)D, (float)target,
+                        (float)rate, (float)ema},
+                       cur_stream());
+  return {requested, dropped, pending};
+}
+
 void adamw_flat(Tensor& master, Tensor& m, Tensor& v, const Tensor& grad, const c10::optional<Tensor>& param_bf16,
                 double lr, double beta1, double beta2, double eps, double wd, int64_t step,
                 const c10::optional<Tensor>& grad_scale_ptr, double grad_scale, const c10::optional<Tensor>& hyper) {
@@ -494,6 +538,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_route_topk", &moe_route_topk);
   m.def("moe_route_bwd", &moe_route_bwd);
   m.def("moe_plan_sorted", &moe_plan_sorted);
+  m.def("moe_temperature", &moe_temperature);
+  m.def("moe_mask", &moe_mask);
+  m.def("moe_stats", &moe_stats);
   m.def("adamw_flat", &adamw_flat);
   m.def("sumsq", &sumsq);
   m.def("muon_momentum", &muon_momentum);

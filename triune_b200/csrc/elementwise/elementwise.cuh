@@ -120,6 +120,22 @@ void launch_moe_route_topk(const float* logits, const float* bias, const float* 
                            long long* idx, float* w, void* keys, bool keys32, int* counts, cudaStream_t s);
 void launch_moe_route_bwd(const float* logits, const float* temperature, float temp_value, const long long* idx, const float* w,
                           const float* dw, int N, int E, int K, float* dlogits, cudaStream_t s);
+// Sampling temperature of the router at a training step (device count): max(1 - step / steps, least).
+void launch_moe_temperature(const long long* step, float steps, float least, float* out, cudaStream_t s);
+// One row of E numbers a token: 1 for each accepted expert, 0 elsewhere (bf16, E % 8 == 0). idx [N, K], keep [N, K] or null (all).
+void launch_moe_mask(const long long* idx, const unsigned char* keep, int N, int E, int K, __nv_bfloat16* mask, cudaStream_t s);
+// Statistics of one routing pass, per expert: requests (summed over slots), drops, the pending bias update, running load and
+// centroids. accepted null: all requests.
+struct MoeStats {
+  const int* slot_counts;      // [E, K]
+  const long long* accepted;   // [E] or null
+  const float* sums;           // [E, D]: sums of the accepted tokens' rows
+  long long *requested, *dropped, *overflow;  // [E], [E], [1]: dropped tokens, added
+  float *pending, *load, *centroids;          // [E], [E], [E, D]; the last two updated in place
+  int E, K, D;
+  float target, rate, ema;
+};
+void launch_moe_stats(const MoeStats& p, cudaStream_t s);
 void launch_moe_plan_sorted(const void* sorted_keys, bool keys32, const long long* order, const int* counts, int A, int E, int K, int cap,
                             int R, int* pos, unsigned char* keep, int* row_src, int* tile_group, int* group_offsets,
                             long long* accepted, cudaStream_t s);

@@ -191,6 +191,75 @@ __global__ void __launch_bounds__(256) moe_plan_sorted_kernel(const KeyT* __rest
     for (int e = threadIdx.x; e <= E; e += blockDim.x) group_offsets[e] = exp_pad_start[e];
 }
 
+__global__ void moe_temperature_kernel(const long long* step, float steps, float least, float* out) {
+  *out = fmaxf(1.f - (float)*step / steps, least);
+}
+
+__global__ void __launch_bounds__(256) moe_mask_kernel(const long long* __restrict__ idx, const unsigned char* __restrict__ keep, int N, int E, int K,
+                                                       __nv_bfloat16* __restrict__ mask) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= N) return;
+  unsigned long long set = 0ull;  // up to 64 experts
+  for (int j = 0; j < K; ++j)
+    if (keep == nullptr || keep[(long long)t * K + j]) set |= 1ull << idx[(long long)t * K + j];
+  for (int e = 0; e < E; e += 8) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t lo = (set >> (e + 2 * i)) & 1ull ? 0x3f80u : 0u, hi = (set >> (e + 2 * i + 1)) & 1ull ? 0x3f800000u : 0u;
+      w[i] = lo | hi;
+    }
+    *reinterpret_cast<uint4*>(mask + (long long)t * E + e) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// One CTA per expert. Some thirty element-wise launches on [E] and [E, D] before, 70 us of the device's and 200 of the host's time a pass.
+__global__ void __launch_bounds__(256) moe_stats_kernel(const MoeStats p) {
+  __shared__ float red[8];
+  __shared__ long long total;
+  const int e = blockIdx.x, tid = threadIdx.x;
+  auto requests = [&](int x) {
+    long long n = 0;
+    for (int j = 0; j < p.K; ++j) n += p.slot_counts[x * p.K + j];
+    return n;
+  };
+  auto drops = [&](int x) {
+    const long long r = requests(x), d = p.accepted != nullptr ? r - p.accepted[x] : 0;
+    return d > 0 ? d : 0;
+  };
+  if (e == 0) {
+    if (tid == 0) total = 0;
+    __syncthreads();
+    if (tid < p.E) atomicAdd(reinterpret_cast<unsigned long long*>(&total), (unsigned long long)drops(tid));
+    __syncthreads();
+    if (tid == 0) *p.overflow += total;
+  }
+  const long long requested = requests(e), accepted = p.accepted != nullptr ? p.accepted[e] : requested;
+  if (tid == 0) {
+    p.requested[e] = requested;
+    p.dropped[e] = drops(e);
+    p.pending[e] = -(((float)requested - p.target) / p.target) * p.rate;
+    p.load[e] = p.load[e] * 0.9f + (float)accepted / p.target * 0.1f;
+  }
+  float* c = p.centroids + (long long)e * p.D;
+  float ss = 0.f;
+  for (int i = tid; i < p.D; i += 256) ss += c[i] * c[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) ss += red[i];
+  if (accepted <= 0) return;
+  const bool fresh = sqrtf(ss) < 1e-6f;
+  const float inv = 1.f / (float)accepted;
+  for (int i = tid; i < p.D; i += 256) {
+    const float mean = p.sums[(long long)e * p.D + i] * inv;
+    c[i] = fresh ? mean : c[i] * p.ema + mean * (1.f - p.ema);
+  }
+}
+
 void check(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + " launch failed: " + cudaGetErrorString(e));
@@ -218,6 +287,25 @@ void launch_moe_route_bwd(const float* logits, const float* temperature, float t
   if (N <= 0) return;
   moe_route_bwd_kernel<<<(N + 255) / 256, 256, 0, s>>>(logits, temperature, temp_value, idx, w, dw, N, E, K, dlogits);
   check("moe_route_bwd");
+}
+
+void launch_moe_temperature(const long long* step, float steps, float least, float* out, cudaStream_t s) {
+  moe_temperature_kernel<<<1, 1, 0, s>>>(step, steps, least, out);
+  check("moe_temperature");
+}
+
+void launch_moe_mask(const long long* idx, const unsigned char* keep, int N, int E, int K, __nv_bfloat16* mask, cudaStream_t s) {
+  if (E > MAX_E || E % 8 != 0) throw std::runtime_error("moe_mask: at most 64 experts, in eights");
+  if (N <= 0) return;
+  moe_mask_kernel<<<(N + 255) / 256, 256, 0, s>>>(idx, keep, N, E, K, mask);
+  check("moe_mask");
+}
+
+void launch_moe_stats(const MoeStats& p, cudaStream_t s) {
+  if (p.E > MAX_E) throw std::runtime_error("moe_stats: at most 64 experts");
+  if (p.E <= 0) return;
+  moe_stats_kernel<<<p.E, 256, 0, s>>>(p);
+  check("moe_stats");
 }
 
 void launch_moe_plan_sorted(const void* sorted_keys, bool keys32, const long long* order, const int* counts, int A, int E, int K, int cap,

@@ -163,6 +163,10 @@ class MoE_FFN(nn.Module):
     # --- routing ----------------------------------------------------------------------------
     def _temperature(self):
         if self.training:
+            step = self._global_step
+            if ops._ext.use_kernels(step) and ops._ext.ext_available() and step.dtype == torch.long:
+                ops._tick(1)
+                return ops._ext.ext().moe_temperature(step, float(MOE_TEMPERATURE_STEPS), 0.1)
             return (1.0 - self._global_step.float() / MOE_TEMPERATURE_STEPS).clamp(min=0.1)
         return 1.0
 
@@ -223,10 +227,28 @@ class MoE_FFN(nn.Module):
         return out.to(x.dtype).reshape(B, T, D)
 
     # --- statistics (no gradient, no host sync) ---------------------------------------------
+    def _stats_on_kernels(self, x2, plan) -> bool:
+        """Whether two kernels and the product of centroid sums cover the statistics (the routing kernels' counts, fp32 buffers)."""
+        E, bufs = self.num_experts, (self.expert_load_ratio, self.last_centroids)
+        return (getattr(plan, "slot_counts", None) is not None and x2.is_cuda and x2.dtype == torch.bfloat16 and E % 8 == 0 and E <= 64
+                and x2.shape[1] % 8 == 0 and x2.data_ptr() % 16 == 0 and ops._ext.use_kernels(x2, self._overflow_counter, *bufs)
+                and all(type(b) is torch.Tensor and b.dtype == torch.float32 and b.is_contiguous() for b in bufs))
+
     @torch.no_grad()
     def _update_routing_stats(self, x2, idx, w, keep, plan=None):
         E, N = self.num_experts, x2.shape[0]
         target = max(1.0, float(N * self.top_k / E))
+        if plan is not None and self._stats_on_kernels(x2, plan):
+            sums = ops.gemm(ops._ext.ext().moe_mask(idx, keep, E), x2.contiguous(), a_mn=True, b_mn=True, out_dtype=torch.float32)
+            accepted = plan[4] if keep is not None else None
+            requested, dropped, self._pending_bias_update = ops._ext.ext().moe_stats(
+                plan.slot_counts, accepted, sums, self._overflow_counter, self.expert_load_ratio, self.last_centroids, target,
+                MOE_BIAS_UPDATE_RATE, self.centroid_ema)
+            ops._tick(2)
+            self.last_counts = self.last_requested_counts = requested
+            self.last_accepted_counts, self.last_dropped_counts = requested if accepted is None else accepted, dropped
+            self.last_target = target
+            return
         flat = idx.reshape(-1)
         if plan is not None and getattr(plan, "slot_counts", None) is not None:
             # the routing and plan kernels already counted: no atomics over N * k indices into E bins
