@@ -232,6 +232,26 @@ def test_products_of_few_tiles_against_fp32(M, N, K, a_mn, b_mn, what):
     assert torch.isfinite(got.float()).all()
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (1, 8, 64), (31, 72, 384), (129, 264, 384), (300, 1536, 384), (9001, 1544, 384), (257, 520, 1016), (257, 520, 1024),
+    (1000, 2056, 1536),
+])
+def test_products_with_saved_rows_at_ragged_edges(M, N, K):
+    """Chunks of the second operand read ahead: tiles cut in both directions, several tiles a block, sixteen and eight warps."""
+    from triune_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    a, b, aux, alpha = rnd(M, K), rnd(N, K), rnd(M, N), K ** -0.5
+    want = alpha * a.float() @ b.float().t()
+    x = aux.float()
+    # one rounding to bf16 (2^-9 of the value) over fp32 sums: every element, with the sums' error of sqrt(K) 2^-24 of its size
+    for got, ref in ((ops.gemm(a, b, alpha=alpha, dgelu_aux=aux), want * x),
+                     (ops.gemm(a, b, alpha=alpha, add_aux=aux, beta=-0.75), want - 0.75 * x)):
+        bound = 2.0 ** -8 * ref.abs() + 1e-5 * (1 + x.abs())
+        assert ((got.float() - ref).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("M,N", [(0, 1536), (0, 72), (40, 0), (0, 0)])
 @pytest.mark.parametrize("K", [1536, 8192])
 def test_empty_products_of_long_reductions_do_nothing(M, N, K):

@@ -200,11 +200,13 @@ __global__ void __launch_bounds__(gemm_threads(EW), 1)
     uint8_t* my_stage = smem_epi + (warp - 2) * (8 * EPI_TILE / EW);
     int acc = 0;
     uint32_t acc_phase = 0, buf = 0;
+    AuxChunk<EPI> aux;
     for (int t = blockIdx.x; t < p.total_tiles; t += gridDim.x) {
       Tile tl = decode_tile(p, t);
       if (!tl.valid) continue;
       const bool timed = p.dbg != nullptr && lane == 0 && warp == 2;
       const long long tw0 = timed ? clock64() : 0;
+      aux.load(p, tl, tl.n0 * NOUT, tl.m0, lane_base, lane, col_half * 32);
       bool ok = mbar_wait(&acc_full[acc], acc_phase);
       ok = __all_sync(0xffffffffu, ok);
       if (timed) {
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(gemm_threads(EW), 1)
       }
       tc_fence_after_sync();
       run_epilogue<EPI, EW>(p, tl, &tmC, &tmAux, tmem_base + acc * BN, BN, tl.n0 * NOUT, tl.m0, lane_base, col_half, lane,
-                        my_stage, buf);
+                            my_stage, buf, aux);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -259,21 +261,18 @@ void launch_variant(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtens
   if (e != cudaSuccess) throw std::runtime_error(std::string("tc_gemm launch failed: ") + cudaGetErrorString(e));
 }
 
-int sm_count();
-
 // Epilogue warps. The activation epilogues spend more on arithmetic (two tanh and twenty packed operations per pair of outputs
 // with the derivative) or on reads than a tile's products take, and with two warps per scheduler much of that was latency:
 // sixteen warps there, eight where the epilogue only converts or a tile has few chunks. Before -> after at 65536 x 1536 x 384:
-// GELU 109 -> 91 us, with its derivative 131 -> 119 (3.8 TB/s), times saved rows 150 -> 123; at 8192 x 4096 x 1024 and above the
-// products hide either. Multiplied rows want K below 1024 (8192 x 6144 x 1536: 131 with eight warps, 135 with sixteen) and more than
-// two waves of tiles (1536 columns over 384: 4096 rows 14.0 with eight, 14.6 with sixteen, 12288 rows 29.7 and 26.3); SwiGLU
-// backward gains 2 to 5 % at 2048 and 8192 x 5632 x 2048, its forward loses as much.
+// GELU 109 -> 91 us, with its derivative 131 -> 119 (3.8 TB/s); at 8192 x 4096 x 1024 and above the products hide either.
+// Multiplied rows want K below 1024 (8 warps and 16: 1536 columns over 384, 4096 rows 14.6 and 13.4 us, 65536 rows 129.5 and 108;
+// 8192 x 4096 x 1024: 59.8 and 61.2); SwiGLU backward gains 2 to 5 % at 2048 and 8192 x 5632 x 2048, its forward loses as much.
 template <int BN, bool A_MN, bool B_MN, int EPI>
 void launch_epi(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmAux, const KParams& kp,
                 int grid, cudaStream_t s) {
   constexpr bool more = BN >= 128 && (EPI == EPI_GELU || EPI == EPI_DSWIGLU || EPI == EPI_MULAUX);
   if constexpr (more) {
-    if (EPI != EPI_MULAUX || (kp.K < 1024 && kp.total_tiles > 2 * sm_count())) return launch_variant<BN, A_MN, B_MN, EPI, 16>(tmA, tmB, tmC, tmAux, kp, grid, s);
+    if (EPI != EPI_MULAUX || kp.K < 1024) return launch_variant<BN, A_MN, B_MN, EPI, 16>(tmA, tmB, tmC, tmAux, kp, grid, s);
   }
   if constexpr (!more || EPI == EPI_MULAUX) launch_variant<BN, A_MN, B_MN, EPI, 8>(tmA, tmB, tmC, tmAux, kp, grid, s);
 }

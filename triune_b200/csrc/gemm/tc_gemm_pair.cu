@@ -271,8 +271,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         break;
       }
       tc_fence_after_sync();
+      AuxChunk<EPI> no_aux;
       run_epilogue<EPI>(p, tl, &tmC, &tmAux, tmem_base + acc * 256, NCFG, tl.n0 * NOUT, tl.m0 + (int)rank * BM,
-                        lane_base, col_half, lane, my_stage, buf);
+                        lane_base, col_half, lane, my_stage, buf, no_aux);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {

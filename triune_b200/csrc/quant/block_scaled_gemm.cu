@@ -288,7 +288,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         break;
       }
       tc_fence_after_sync();
-      epilogue_tile<EPI>(p, tl, &tmC, &tmC, tmem_base + acc * BN, BN, n_idx * BN, tl.m0, lane_base, col_half, lane, my_stage, buf);
+      AuxChunk<EPI> no_aux;
+      epilogue_tile<EPI>(p, tl, &tmC, &tmC, tmem_base + acc * BN, BN, n_idx * BN, tl.m0, lane_base, col_half, lane, my_stage, buf, no_aux);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
