@@ -58,6 +58,20 @@ def test_step_gives_the_numbers_of_the_modules(mixer, batch, dim, heads, head_di
     assert int(one.graph.native.status) == 0
 
 
+@pytest.mark.parametrize("batch,dim,heads,hidden,vocab", [(1, 128, 2, 128, 64), (4, 128, 2, 256, 300), (2, 256, 4, 128, 64)])
+def test_ctas_without_blocks_leave_no_copies_behind(batch, dim, heads, hidden, vocab, monkeypatch):
+    # 8 to 64 blocks a phase: which CTAs have one changes from phase to phase, and no norm's weights are like another's
+    m = _model(dim, heads, 64, 6, hidden, vocab, "gated_deltanet")
+    norms = [n for layer in m.layers for n in (layer.input_norm, layer.post_attn_norm)] + [m.norm]
+    with torch.no_grad():
+        for i, n in enumerate(norms):
+            n.weight.copy_(torch.randn(dim, device="cuda") * 2.0 ** (i % 5 - 2))
+    one, got, captured, want = _both(m, batch, 9, 24, monkeypatch)
+    assert isinstance(one.graph, dense_step._Step) and torch.equal(got, want)
+    for a, b in zip(one.states, captured.states):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("ffn,scale,vocab", [("gelu", "none", 512), ("gelu", "fla", 512), ("swiglu", "fla", 517)])
 def test_step_with_biases_scales_and_ragged_vocabularies(ffn, scale, vocab, monkeypatch):
     m = _model(256, 4, 64, 3, 320, vocab, "gla", ffn, scale)

@@ -330,13 +330,14 @@ __global__ void __launch_bounds__((32 << LOG_WARPS) + 32, 1) dense_step_kernel(c
     uint4 next = make_uint4(0u, 0u, 0u, 0u);
     if (tid < PHASE_WORDS && i + 1 < p.phases) next = reinterpret_cast<const uint4*>(p.program + i + 1)[tid];
     const bool normed = ph.norm != nullptr;
-    if (normed) {
+    const int mine_first = own_first(ph.first);
+    const int head = kind == DP_PROJECT && mine_first < ph.strengths ? mine_first : -1;  // whose write strengths this CTA forms
+    const int mine = kind == DP_MIX ? 0 : ph.blocks_each + (mine_first < ph.blocks_more ? 1 : 0);
+    if (normed && (mine > 0 || head >= 0)) {  // only where the copies are waited for: two norms' weights never race for the same words
       const __nv_bfloat16* nw = ph.norm;
       for (int c = tid * 8; c < k; c += CONSUMERS * 8)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(nws + c)), "l"(nw + c) : "memory");
     }
-    const int mine_first = own_first(ph.first);
-    const int head = kind == DP_PROJECT && mine_first < ph.strengths ? mine_first : -1;  // whose write strengths this CTA forms
     uint4 strength_w = make_uint4(0u, 0u, 0u, 0u);
     if (head >= 0 && tid < STRENGTH_THREADS && tid * 8 < k) strength_w = *reinterpret_cast<const uint4*>(ph.extra + (long long)head * k + tid * 8);
     float S[RPT], cs = 1.f, sn = 0.f;
@@ -356,7 +357,6 @@ __global__ void __launch_bounds__((32 << LOG_WARPS) + 32, 1) dense_step_kernel(c
       }
     }
     const uint32_t flag = flag0 + (uint32_t)i;
-    const int mine = kind == DP_MIX ? 0 : ph.blocks_each + (mine_first < ph.blocks_more ? 1 : 0);
     auto publish = [&] {  // the next phase's entry
       if (tid < PHASE_WORDS) reinterpret_cast<uint4*>(&sh.phase[(i + 1) & 1])[tid] = next;
     };
