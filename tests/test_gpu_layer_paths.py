@@ -48,9 +48,27 @@ def test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims):
     (1, 8, 16, 128, 1), (1, 17, 5, 128, 2), (1, 31, 3, 64, 0), (2, 33, 7, 64, 1),          # blocks of sixteen and their remainders
     (4, 12, 16, 64, 1), (4, 11, 16, 128, 1), (4, 12, 16, 128, 0), (8, 24, 16, 64, 1), (8, 23, 16, 128, 1), (8, 24, 16, 128, 2),
     (17, 31, 8, 64, 1), (17, 32, 8, 64, 1), (32, 32, 16, 128, 1), (27, 140, 19, 128, 1), (19, 140, 27, 64, 1),  # ends of the rule, segments
+    (8, 25, 16, 128, 1), (8, 26, 16, 128, 1), (16, 32, 16, 64, 1), (385, 32, 1, 64, 1),
 ])
 def test_rounds_of_sixteen_tokens_against_the_token_recurrence(B, T, H, D, beta_dims):
     test_delta_rule_prompts_against_the_token_recurrence(B, T, H, D, beta_dims)
+
+
+@pytest.mark.parametrize("logits", [0.0, 4.0, 8.0, 10.0, 14.0])
+@pytest.mark.parametrize("T,H,D", [(2048, 6, 64), (2048, 4, 128), (509, 3, 64)])
+def test_delta_rule_prompts_lose_no_bits_of_a_long_memory(T, H, D, logits):
+    """Gates near 1 keep thousands of tokens, so that an error to one side in each of them adds up. Pieces of four tokens take the kernel that
+    goes token by token in fp32; a prompt's state may be off by as much as that one's, or by two roundings (2^-23)."""
+    q, k, v, g, _ = _mixer_inputs(1, T, H, D)
+    g = (g.float() + logits).bfloat16()
+    beta = torch.sigmoid(torch.randn(1, T, H, device="cuda", generator=torch.Generator("cuda").manual_seed(T)))
+    _, s = gla_cuda.gdn_recurrent(q, k, v, g, beta, None, 1.0, True)
+    st = None
+    for t in range(0, T, 4):
+        _, st = gla_cuda.gdn_recurrent(*(x[:, t : t + 4] for x in (q, k, v, g, beta)), st, 1.0, True)
+    gl = F.logsigmoid(g.double()).clamp(min=gla_cuda.GLA_MIN_LOG_DECAY)
+    _, exact = ref.gated_deltanet_recurrent(q.double(), k.double(), v.double(), gl, beta.double(), torch.zeros(1, H, D, D, device="cuda").double(), 1.0)
+    assert _rel(s, exact) < 1.5 * _rel(st, exact) + 2.0 ** -23
 
 
 @pytest.mark.parametrize("E,K,N,D,skew", [(8, 2, 1, 64, 0.0), (8, 1, 257, 72, 4.0), (16, 2, 1000, 384, 0.0), (64, 4, 300, 128, 6.0), (8, 2, 4096, 1536, 3.0)])

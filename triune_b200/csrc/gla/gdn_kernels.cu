@@ -162,29 +162,37 @@ __global__ void __launch_bounds__(D* NPART) gdn_recurrent_kernel(
 // walk runs on B * H * D / 16 CTAs of 16 columns whose four warps share the key rows.
 //
 // The products of the walk are warp-level matrix instructions on tf32 numbers with fp32 sums, each operand as the sum of two:
-// x = hi + lo keeps 22 to 24 bits, hi hi + hi lo + lo hi leaves 2^-23 of a product, and the state stays fp32 (relative error of the
-// state after 8192 tokens 4e-7, as with fp32 multiply-adds). The state is held transposed: the fragment that
+// x = hi + lo keeps 22 to 24 bits, hi hi + hi lo + lo hi leaves 2^-23 of a product. The instruction cuts its sums off towards zero, so
+// nothing that lasts is summed up in it: the state, the value minus what the state holds for it, and the 1 in T are added outside, in fp32, and
+// the later eight tokens of a block, of which a short memory consists, reach the state by fp32 multiply-adds. Relative error of the state
+// against 64 bits after 8192 tokens, 16 heads of 128, gate logits around 0, 2, 4, 8, 10, 14: eight tokens a round in fp32 multiply-adds 9.0e-8,
+// 1.4e-7, 5.8e-7, 1.4e-6, 3.0e-6, 6.4e-6; here 7.4e-8, 1.4e-7, 2.0e-7, 4.1e-7, 1.1e-6, 6.8e-7; all in the instruction 1.4e-7, 1.9e-7, 4.3e-7,
+// 1.1e-5, 1.6e-5, 9.9e-6 (926 instead of 987 us). After 2048 tokens, token by token: 7.0e-8, 1.1e-7, 5.5e-7, 1.3e-6, 8.1e-7, 5.8e-6.
+// The state is held transposed: the fragment that
 // the update leaves it in is the operand that the next round's contraction takes it from, the order of key rows within an
 // instruction being free. Rows of a record are padded so that its fragments are read without bank conflicts.
 //
 // The launch that walks a segment of tokens also forms the next one's records, in CTAs behind its own. A block's outputs wait for the next
-// round's barrier, so that there is one barrier a round. Bound by the issue slots of one warp per scheduler (81 matrix
-// instructions of 12 clocks and 700 others in the 2500 clocks of a round of 128-wide heads; eight warps a CTA repeat more than they hide:
-// 1030 against 930 us). Measured, token by token -> eight tokens a round in fp32 multiply-adds -> here: one sequence of 8192 tokens, 16 heads of
-// 128, 9010 -> 1164 -> 865 us; 6 heads of 64 5007 -> 960 -> 490; four sequences of 16384, 6 heads of 64 2080 -> 1100; 4 x 512, 16 heads of
-// 128 224 -> 169; see gdn_in_blocks for the sizes that take it.
+// round's barrier, so that there is one barrier a round. Bound by the issue slots of one warp per scheduler (69 matrix
+// instructions of 12 clocks and some 800 others a round of 128-wide heads; eight warps a CTA repeat more than they hide: a ninth slower).
+// Whole calls, eight tokens a round in fp32 multiply-adds -> here: one sequence of 8192 tokens, 16 heads of 128, 1229 -> 987 us
+// (9010 token by token); 6 heads of 64 1034 -> 546; four sequences of 16384, 6 heads of 64 2162 -> 1136; 4 x 512, 16 heads of 128 279 -> 231;
+// see gdn_in_blocks for the sizes that take it.
 // ------------------------------------------------------------------------------------------------
 constexpr int GB = 16;  // tokens per block
 template <int D>
-struct GdnRec {  // floats of a record: k P and q P [32][PK] | (beta k) dec [16][PE] | T [16][PT] | A [16][PT] | P_15 [D] | v bf16 [D][24]
+struct GdnRec {  // floats of a record: k P and q P [32][PK] | (beta k) dec [16][PE] | T - 1 [16][PT] | A [16][PT] | P_15 [D] | v bf16 [D][24]
   static constexpr int PK = D + 8, PE = D + 4, PT = 24, PV = 12;
   static constexpr int E = 2 * GB * PK, TRI = E + GB * PE, A = TRI + GB * PT, P = A + GB * PT, COMMON = P + D, FLOATS = COMMON + D * PV;
   static_assert(COMMON % 4 == 0 && PV % 4 == 0, "records are copied in 16-byte words");
 };
 
-// e^gdn_log_decay: a sigmoid where the gates are logits.
+// e^gdn_log_decay: a sigmoid where the gates are logits. Near 1, where errors add up over a long memory, it is formed from its distance to 1,
+// so that only the last subtraction rounds.
 __device__ __forceinline__ float gdn_decay(float x, bool logits) {
-  return logits ? fmaxf(__fdividef(1.f, 1.f + __expf(-x)), 6.7379469990854671e-3f) : __expf(gdn_log_decay(x, false));
+  if (!logits) return __expf(gdn_log_decay(x, false));
+  const float e = __expf(-fabsf(x)), small = __fdividef(e, 1.f + e);
+  return fmaxf(x > 0.f ? 1.f - small : small, 6.7379469990854671e-3f);
 }
 
 // Sum of v[l] over the lanes, in lane l.
@@ -298,14 +306,14 @@ __device__ __forceinline__ void gdn_block_prep(const GdnBlockArgs& a, GdnPrepSha
   for (int i = tid; i < D * 2; i += 128)  // sixteen values of a column: two 16-byte words
     *reinterpret_cast<uint4*>(out + R::COMMON + (i >> 1) * R::PV + (i & 1) * 4) = *reinterpret_cast<const uint4*>(&sh.v[i >> 1][(i & 1) * 4]);
   if (tid < D) {  // k_j P_{j-1}, q_j P_j; tokens past the end write nothing and leave the state as it is
-    float p = 1.f;
+    double p = 1.;  // products of numbers a few units below 1 all round to the same side in fp32
 #pragma unroll
     for (int j = 0; j < GB; ++j) {
-      out[j * R::PK + tid] = __bfloat162float(sh.k[j][tid]) * p;
+      out[j * R::PK + tid] = __bfloat162float(sh.k[j][tid]) * (float)p;
       p *= sh.dec[j][tid];
-      out[(GB + j) * R::PK + tid] = __bfloat162float(sh.q[j][tid]) * p;
+      out[(GB + j) * R::PK + tid] = __bfloat162float(sh.q[j][tid]) * (float)p;
     }
-    out[R::P + tid] = p;
+    out[R::P + tid] = (float)p;
   }
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
@@ -355,14 +363,14 @@ __device__ __forceinline__ void gdn_block_prep(const GdnBlockArgs& a, GdnPrepSha
     }
   }
   __syncthreads();
-  if (tid < GB) {  // column `tid` of (1 + L)^-1
+  if (tid < GB) {  // column `tid` of (1 + L)^-1 - 1
     float t[GB];
 #pragma unroll
     for (int i = 0; i < GB; ++i) {
       t[i] = i == tid ? 1.f : 0.f;
 #pragma unroll
       for (int m = 0; m < i; ++m) t[i] -= sh.L[i][m] * t[m];
-      out[R::TRI + i * R::PT + tid] = t[i];
+      out[R::TRI + i * R::PT + tid] = i == tid ? t[i] - 1.f : t[i];
     }
   }
 }
@@ -388,12 +396,22 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ void operand(const float (&c)[4], Split (&v)[4]) {
   v[0] = split_tf32(c[0]), v[1] = split_tf32(c[2]), v[2] = split_tf32(c[1]), v[3] = split_tf32(c[3]);
 }
-__device__ __forceinline__ void multiply(float (&c)[4], const Split (&a)[4], float b0, float b1) {
-  const Split x = split_tf32(b0), y = split_tf32(b1);
-  mma_tf32(c, a[0].lo, a[1].lo, a[2].lo, a[3].lo, x.hi, y.hi);
-  mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, x.lo, y.lo);
-  mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, x.hi, y.hi);
-}
+// An instruction cuts off what is below the last bit of its largest term, always towards zero. So the small products of a sum are added up by
+// themselves, the large ones in as few instructions as there are, and what has been summed up before is added in fp32.
+struct Sum {
+  float large[4], small[4];
+  __device__ __forceinline__ Sum() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) large[i] = small[i] = 0.f;
+  }
+  __device__ __forceinline__ void multiply(const Split (&a)[4], float b0, float b1) {
+    const Split x = split_tf32(b0), y = split_tf32(b1);
+    mma_tf32(small, a[0].lo, a[1].lo, a[2].lo, a[3].lo, x.hi, y.hi);
+    mma_tf32(small, a[0].hi, a[1].hi, a[2].hi, a[3].hi, x.lo, y.lo);
+    mma_tf32(large, a[0].hi, a[1].hi, a[2].hi, a[3].hi, x.hi, y.hi);
+  }
+  __device__ __forceinline__ float operator[](int i) const { return large[i] + small[i]; }
+};
 
 template <int D>
 struct GdnWalkShared {
@@ -467,7 +485,7 @@ struct GdnWalk {
     f[2] = __uint_as_float(hi << 16), f[3] = __uint_as_float(hi & 0xffff0000u);
   }
 
-  __device__ __forceinline__ void leave(int buf, int part, const float (&f)[4], const float (&s)[4]) const {
+  __device__ __forceinline__ void leave(int buf, int part, const Sum& f, const Sum& s) const {
     sh.red[buf][part][warp][0][lane] = make_float4(f[0], f[1], f[2], f[3]);
     sh.red[buf][part][warp][1][lane] = make_float4(s[0], s[1], s[2], s[3]);
   }
@@ -488,15 +506,46 @@ struct GdnWalk {
            (tok + 1 < left && !(fmaxf(fabsf(o[1]), fabsf(o[3])) < INFINITY && o[1] == o[1] && o[3] == o[3]));
   }
 
+  // u of tokens 8 to 15, of columns g and g + 8
+  __device__ __forceinline__ void gather(const float (&u1)[4], float (&v)[8][2]) const {
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[2 * n + (i & 1)][i >> 1] = __shfl_sync(0xffffffffu, u1[i], (lane & ~3) | n);
+  }
+  // S of eight key rows <- P_15 S + sum_j (beta k_j dec_{j+1..15}) u_j^T. The later eight tokens, of which a short memory consists, in fp32.
+  __device__ __forceinline__ void advance(const float* r, int n, const Split (&u0)[4], const float (&v)[8][2]) {
+    const int d = warp * (D / 4) + 8 * n;
+    const float2 p = *reinterpret_cast<const float2*>(r + R::P + d + 2 * t);
+    const float* e = r + R::E + 2 * t * R::PE + d + g;
+    Sum early;
+    early.multiply(u0, e[0], e[R::PE]);
+    float add[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) add[i] = early[i];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float2 w = *reinterpret_cast<const float2*>(r + R::E + (8 + j) * R::PE + d + 2 * t);
+      add[0] = __fmaf_rn(w.x, v[j][0], add[0]), add[1] = __fmaf_rn(w.y, v[j][0], add[1]);
+      add[2] = __fmaf_rn(w.x, v[j][1], add[2]), add[3] = __fmaf_rn(w.y, v[j][1], add[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) S[n][i] = __fmaf_rn(S[n][i], (i & 1) ? p.y : p.x, add[i]);
+  }
+  // o plus what the tokens of the block itself add to outputs of eight of them: `a0`, `a1` their rows of A
+  __device__ __forceinline__ void add_block(float (&o)[4], int e, const Split (&u0)[4], const Split (&u1)[4], float2 a0, float2 a1) const {
+    Sum sum;
+    sum.multiply(u0, a0.x, a0.y);
+    if (e == 1) sum.multiply(u1, a1.x, a1.y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] += sum[i];
+  }
+
   // A block's round, its record in `r`: outputs of its tokens before `limit`, and the state after all of them. Tokens from
   // `limit` on count as nothing (LIMIT), as they are behind a token that is no number. True where an output is no number.
   template <bool LIMIT>
   __device__ __forceinline__ bool round(const float* r, int blk, int limit) {
-    float acc[4][4];  // [16 columns] x [k P of tokens 0-7, 8-15 | q P of tokens 0-7, 8-15], of this warp's key rows
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
+    Sum acc[4];  // [16 columns] x [k P of tokens 0-7, 8-15 | q P of tokens 0-7, 8-15], of this warp's key rows
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       Split s[4];
@@ -504,7 +553,7 @@ struct GdnWalk {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 b = *reinterpret_cast<const float2*>(r + (8 * j + g) * R::PK + warp * (D / 4) + 8 * n + 2 * t);
-        multiply(acc[j], s, b.x, b.y);
+        acc[j].multiply(s, b.x, b.y);
       }
     }
     const int buf = blk & 1;
@@ -531,41 +580,30 @@ struct GdnWalk {
       const float* tri = r + R::TRI + 2 * t;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        u[e][0] = u[e][1] = u[e][2] = u[e][3] = 0.f;
+        Sum sum;
         const float2 b0 = *reinterpret_cast<const float2*>(tri + (8 * e + g) * R::PT);
-        multiply(u[e], x0, b0.x, b0.y);
+        sum.multiply(x0, b0.x, b0.y);
         if (e == 1) {
           const float2 b1 = *reinterpret_cast<const float2*>(tri + (8 + g) * R::PT + 8);
-          multiply(u[e], x1, b1.x, b1.y);
+          sum.multiply(x1, b1.x, b1.y);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (LIMIT && 8 * e + 2 * t + (i & 1) >= limit) u[e][i] = 0.f;
+        for (int i = 0; i < 4; ++i) u[e][i] = LIMIT && 8 * e + 2 * t + (i & 1) >= limit ? 0.f : x[e][i] + sum[i];
       }
     }
     Split u0[4], u1[4];
     operand(u[0], u0);
     operand(u[1], u1);
+    float after[8][2];
+    gather(u[1], after);
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      const int d = warp * (D / 4) + 8 * n;
-      const float2 p = *reinterpret_cast<const float2*>(r + R::P + d + 2 * t);
-      S[n][0] *= p.x, S[n][1] *= p.y, S[n][2] *= p.x, S[n][3] *= p.y;
-      const float* e = r + R::E + 2 * t * R::PE + d + g;
-      multiply(S[n], u0, e[0], e[R::PE]);
-      multiply(S[n], u1, e[8 * R::PE], e[9 * R::PE]);
-    }
+    for (int n = 0; n < NT; ++n) advance(r, n, u0, after);
     bool odd = false;
     if (warp < 2) {  // outputs of tokens 8 warp + ...
       float o[4];
       total(buf, 1, warp, o);
       const float* tri = r + R::A + (8 * warp + g) * R::PT + 2 * t;
-      const float2 b0 = *reinterpret_cast<const float2*>(tri);
-      multiply(o, u0, b0.x, b0.y);
-      if (warp == 1) {
-        const float2 b1 = *reinterpret_cast<const float2*>(tri + 8);
-        multiply(o, u1, b1.x, b1.y);
-      }
+      add_block(o, warp, u0, u1, *reinterpret_cast<const float2*>(tri), *reinterpret_cast<const float2*>(tri + 8));
       odd = put(o, blk, warp, limit);
     }
     return odd;
@@ -600,8 +638,7 @@ struct GdnWalk {
       if ((warp >> 1) == (blk & 1)) {
         float o[4];
         total(blk & 1, 1, e, o);
-        multiply(o, u0, a0.x, a0.y);
-        if (e == 1) multiply(o, u1, a1.x, a1.y);
+        add_block(o, e, u0, u1, a0, a1);
         odd |= put(o, blk, e, GB);
       }
     };
@@ -611,17 +648,13 @@ struct GdnWalk {
       Split s[NT][4];
 #pragma unroll
       for (int n = 0; n < NT; ++n) operand(S[n], s[n]);
-      float kp[2][4];
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) kp[j][i] = 0.f;
+      Sum kp[2];
 #pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const float2 b = *reinterpret_cast<const float2*>(r + (8 * j + g) * R::PK + warp * (D / 4) + 8 * n + 2 * t);
-          multiply(kp[j], s[n], b.x, b.y);
+          kp[j].multiply(s[n], b.x, b.y);
         }
       leave(buf, 0, kp[0], kp[1]);
       __syncthreads();  // all warps' sums; the record of the block before has been read
@@ -636,11 +669,8 @@ struct GdnWalk {
 #pragma unroll
         for (int i = 0; i < 4; ++i) x[e][i] = f[i] - x[e][i];
       }
-      float u[2][4], qp[2][4];
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) u[e][i] = qp[e][i] = 0.f;
+      float u[2][4];
+      Sum qp[2];
       {
         Split x0[4], x1[4];
         operand(x[0], x0);
@@ -648,31 +678,31 @@ struct GdnWalk {
         const float* tri = r + R::TRI + g * R::PT + 2 * t;
         const float2 b0 = *reinterpret_cast<const float2*>(tri), b1 = *reinterpret_cast<const float2*>(tri + 8 * R::PT),
                      b2 = *reinterpret_cast<const float2*>(tri + 8 * R::PT + 8);
-        multiply(u[0], x0, b0.x, b0.y);
-        multiply(u[1], x0, b1.x, b1.y);
-        multiply(u[1], x1, b2.x, b2.y);
+        Sum sum[2];
+        sum[0].multiply(x0, b0.x, b0.y);
+        sum[1].multiply(x0, b1.x, b1.y);
+        sum[1].multiply(x1, b2.x, b2.y);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) u[e][i] = x[e][i] + sum[e][i];
       }
 #pragma unroll
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const float2 b = *reinterpret_cast<const float2*>(r + (GB + 8 * j + g) * R::PK + warp * (D / 4) + 8 * n + 2 * t);
-          multiply(qp[j], s[n], b.x, b.y);
+          qp[j].multiply(s[n], b.x, b.y);
         }
       leave(buf, 1, qp[0], qp[1]);
       operand(u[0], u0);
       operand(u[1], u1);
       a0 = *reinterpret_cast<const float2*>(r + R::A + (8 * (warp & 1) + g) * R::PT + 2 * t);
       a1 = *reinterpret_cast<const float2*>(r + R::A + (8 * (warp & 1) + g) * R::PT + 2 * t + 8);
+      float after[8][2];
+      gather(u[1], after);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        const int d = warp * (D / 4) + 8 * n;
-        const float2 p = *reinterpret_cast<const float2*>(r + R::P + d + 2 * t);
-        S[n][0] *= p.x, S[n][1] *= p.y, S[n][2] *= p.x, S[n][3] *= p.y;
-        const float* e = r + R::E + 2 * t * R::PE + d + g;
-        multiply(S[n], u0, e[0], e[R::PE]);
-        multiply(S[n], u1, e[8 * R::PE], e[9 * R::PE]);
-      }
+      for (int n = 0; n < NT; ++n) advance(r, n, u0, after);
       if (++at == GDN_STAGES) at = 0, ++lap;
       if (blk + 1 < nb && !late) late = !landed(blk + 1, lap);  // what did not arrive is read as it is, and walked again
     }
@@ -865,15 +895,15 @@ int segment_tokens(int BH, int D) {
 
 // Sixteen tokens a round win where the recurrence is a chain that the chip waits for: the walk's work grows with the heads, the token
 // kernel's time hardly does until its CTAs fill the SMs, and a round costs the same for one token as for sixteen. Token kernel -> blocks,
-// us: 16 heads of 64, 8 tokens 7.1 -> 8.0, 12 tokens 9.5 -> 8.4, 512 tokens 315 -> 40; 128 of 64, 17 tokens 13 -> 15, 24 tokens 17 -> 15; 256
-// of 64, 24 tokens 20 -> 21, 32 tokens 26 -> 21; 512 of 64, 32 tokens 36 -> 35, 130 tokens 137 -> 140, 512 tokens 533 -> 508; 1024 of 64, 130
-// tokens 247 -> 268; 16 of 128, 4 tokens 7.4 -> 9.8, 8 tokens 11.5 -> 10.3; 64 of 128, 8 tokens 11.7 -> 14.4, 12 tokens 16.1 -> 15.0; 128 of
-// 128, 17 tokens 22 -> 28, 24 tokens 28.7 -> 27.5; 512 of 128, 24 tokens 85 -> 93, 32 tokens 111 -> 97, 512 tokens 1676 -> 1353. More than
-// 512 heads would take hundreds of megabytes of records.
+// us: 16 heads of 64, 8 tokens 7.1 -> 8.0, 12 tokens 9.5 -> 8.3, 512 tokens 315 -> 39; 128 of 64, 17 tokens 13 -> 15, 24 tokens 17 -> 15; 256
+// of 64, 24 tokens 20 -> 21, 32 tokens 26 -> 22; 384 of 64, 32 tokens 30 -> 31, 130 tokens 115 -> 116, 512 tokens 449 -> 420; 512 of 64, 32 tokens 36 -> 36, 130 tokens 137 -> 150, 512 tokens 533 -> 534; 16 of 128, 4
+// tokens 7.4 -> 9.8, 8 tokens 11.5 -> 10.7; 64 of 128, 8 tokens 11.7 -> 14.4, 12 tokens 16.1 -> 15.5; 128 of 128, 24 tokens 28.7 -> 29.6, 32
+// tokens 38 -> 30; 512 of 128, 24 tokens 85 -> 93, 32 tokens 111 -> 100, 512 tokens 1676 -> 1433. More than 512 heads would take hundreds of
+// megabytes of records.
 static bool gdn_in_blocks(long long heads, int T, int D) {
   if (D != 64 && D != 128) return false;
-  const int least = D == 128 && heads <= 16 ? 8 : heads <= 64 ? 12 : heads <= 128 ? 24 : 32;
-  return heads <= 512 && T >= least;
+  const int least = D == 128 && heads <= 16 ? 8 : heads <= 64 ? 12 : heads <= 128 ? (D == 128 ? 26 : 24) : 32;
+  return heads <= (D == 128 ? 512 : 384) && T >= least;
 }
 
 long long gdn_block_workspace_floats(int B, int T, int H, int D) {
