@@ -51,7 +51,7 @@ def _both(m, batch, prompt, new, monkeypatch):
 def test_step_gives_the_numbers_of_the_modules(mixer, batch, dim, heads, head_dim, hidden, vocab, monkeypatch):
     m = _model(dim, heads, head_dim, 2, hidden, vocab, mixer)
     one, got, captured, want = _both(m, batch, 9, 12, monkeypatch)
-    assert isinstance(one.graph, dense_step._Step)
+    assert isinstance(one.graph, dense_step.Step)
     assert torch.equal(got, want) and int(one.pos) == int(captured.pos) and torch.equal(one.token, captured.token)
     for a, b in zip(one.states, captured.states):
         assert torch.equal(a, b)
@@ -67,7 +67,7 @@ def test_ctas_without_blocks_leave_no_copies_behind(batch, dim, heads, hidden, v
         for i, n in enumerate(norms):
             n.weight.copy_(torch.randn(dim, device="cuda") * 2.0 ** (i % 5 - 2))
     one, got, captured, want = _both(m, batch, 9, 24, monkeypatch)
-    assert isinstance(one.graph, dense_step._Step) and torch.equal(got, want)
+    assert isinstance(one.graph, dense_step.Step) and torch.equal(got, want)
     for a, b in zip(one.states, captured.states):
         assert torch.equal(a, b)
 
@@ -76,7 +76,7 @@ def test_ctas_without_blocks_leave_no_copies_behind(batch, dim, heads, hidden, v
 def test_step_with_biases_scales_and_ragged_vocabularies(ffn, scale, vocab, monkeypatch):
     m = _model(256, 4, 64, 3, 320, vocab, "gla", ffn, scale)
     one, got, captured, want = _both(m, 2, 21, 10, monkeypatch)
-    assert isinstance(one.graph, dense_step._Step) and torch.equal(got, want)
+    assert isinstance(one.graph, dense_step.Step) and torch.equal(got, want)
     for a, b in zip(one.states, captured.states):
         assert torch.equal(a, b)
 
@@ -115,3 +115,26 @@ def test_other_models_keep_the_captured_step(change):
     finally:
         if handle is not None:
             handle.remove()
+
+
+@pytest.mark.parametrize("how", ["status", "wait"])
+def test_a_step_that_did_not_finish_raises_and_the_next_prompt_starts_over(how):
+    m = _model(128, 2, 64, 2, 256, 512, "gla")
+    ids = torch.randint(0, 512, (1, 9), device="cuda")
+    dec = GraphedGreedyDecoder(m)
+    want = dec.generate(ids, 6)
+    first = dec.graph
+    assert isinstance(first, dense_step.Step)
+    if how == "status":
+        first.status.fill_(4)
+    else:  # nobody forms the first projection, so that the mixer's wait for it runs out after its second
+        entry = first.native.program.view(torch.int32).view(-1, 40)[0]
+        assert entry[16:19].tolist() == [0, 4 * 128, 128] and entry[26:29].tolist() == [32, 0, 32]
+        entry[26:29] = 0
+    with pytest.raises(RuntimeError, match="did not finish"):
+        dec.generate(ids, 6)
+    assert int(first.status) != 0
+    with pytest.raises(RuntimeError, match="prefill"):
+        dec.decode(3)
+    assert torch.equal(dec.generate(ids, 6), want)
+    assert dec.graph is not first and int(dec.graph.status) == 0

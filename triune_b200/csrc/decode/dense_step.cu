@@ -24,7 +24,8 @@
 // copies' matrix steps, sums: 3 to 8 us for 31 phases) and, at the head, by memory (6.6 TB/s).
 //
 // The grid is launched cooperatively (its CTAs wait for one another); every wait has a time limit, after which the step sets the
-// status word and a word that all waits look at, lets its copies land and returns; later steps return at once.
+// status word and a word that all waits look at, lets its copies land and returns; later steps return at once. The host reads
+// the status once a request.
 #include "dense_step.cuh"
 
 #include <cstring>

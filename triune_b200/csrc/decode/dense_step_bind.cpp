@@ -171,6 +171,7 @@ class DenseStepPlan {
 
   bool fits() const { return fits_; }
   Tensor status() const { return words_.slice(0, 2, 3); }
+  Tensor program() const { return program_; }  // bytes of the DensePhase entries
 
   // One token of every sequence, on the current stream.
   void replay() {
@@ -222,5 +223,6 @@ void register_decode(pybind11::module& m) {
            py::arg("out"), py::arg("pos"), py::arg("step"), py::arg("delta"), py::arg("gated"))
       .def_property_readonly("fits", &DenseStepPlan::fits)
       .def_property_readonly("status", &DenseStepPlan::status)
+      .def_property_readonly("program", &DenseStepPlan::program)
       .def("replay", &DenseStepPlan::replay);
 }

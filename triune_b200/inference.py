@@ -417,7 +417,10 @@ class GraphedGreedyDecoder:
 
     @torch.no_grad()
     def decode(self, max_new_tokens: int) -> torch.Tensor:
-        """-> [B, max_new_tokens] token ids (the first one is the token ``prefill`` returned)."""
+        """-> [B, max_new_tokens] token ids (the first one is the token ``prefill`` returned). Raises where a step did not finish; a new prompt
+        has to come before the next tokens then."""
+        if not self.states:
+            raise RuntimeError("no prompt to decode from: call prefill first")
         tables = _cover_positions(self.rotary, self.device, self.host_pos + max_new_tokens, self.max_positions)
         if len(tables) != len(self.tables) or any(a is not b for a, b in zip(tables, self.tables)):
             self.graph = None  # the capture reads the tables that were there before
@@ -457,7 +460,11 @@ class GraphedGreedyDecoder:
             self.step_idx.zero_()
         for _ in range(max_new_tokens):
             self.graph.replay()
-        return self.out[:, :max_new_tokens].clone()
+        tokens = self.out[:, :max_new_tokens].clone()
+        if isinstance(self.graph, dense_step.Step) and self.graph.failed():  # once a request; waits for its tokens
+            self.graph, self.states = None, []  # the next prompt starts over
+            raise RuntimeError("a decoding step did not finish: a wait between its blocks ran out of time, the request's tokens are lost")
+        return tokens
 
     @torch.no_grad()
     def generate(self, input_ids: torch.Tensor, max_new_tokens: int) -> torch.Tensor:

@@ -36,9 +36,13 @@ def _weight(t: Optional[torch.Tensor], like: torch.Tensor) -> bool:
                           and type(t) in (torch.Tensor, nn.Parameter)))
 
 
-class _Step:
+class Step:
     def __init__(self, native):
         self.native, self.status = native, native.status
+
+    def failed(self) -> bool:
+        """Whether a step gave up on a wait. No step after it does anything, and what it left in the states and the output is not to be used."""
+        return int(self.status) != 0
 
     def replay(self) -> None:
         """One token of every sequence, on the current stream."""
@@ -47,7 +51,7 @@ class _Step:
         gla_cuda._note(self.status)
 
 
-def plan(model, states: List[Optional[torch.Tensor]], token, out, pos, step) -> Optional[_Step]:
+def plan(model, states: List[Optional[torch.Tensor]], token, out, pos, step) -> Optional[Step]:
     """The step of ``model`` from and into these buffers (states advanced in place, ``out[:, step] = token``, the next token, position and
     step count plus one), or None where the kernel does not cover it. The plan keeps the tensors that it reads."""
     if type(model) is not UniversalDenseTransformer or not _ext.use_kernels(token) or not _ext.ext_available():
@@ -91,4 +95,4 @@ def plan(model, states: List[Optional[torch.Tensor]], token, out, pos, step) -> 
         return None
     native = _ext.ext().DenseStepPlan(layers, scalars, embed.detach(), model.norm.weight.detach(), model.norm.eps, head.detach(), token, out, pos,
                                       step, delta, gated)
-    return _Step(native) if native.fits else None
+    return Step(native) if native.fits else None
