@@ -108,7 +108,7 @@ def test_prompt_with_and_without_a_state(batch, seq, fmt, gated, delta, monkeypa
         assert after["offset"] == want_after["offset"] == 9 + seq
 
 
-@pytest.mark.parametrize("change", ["hook", "global hook", "backward hook", "forward", "bias", "module", "lora", "float32", "strided", "one token", "tangent"])
+@pytest.mark.parametrize("change", ["hook", "global hook", "backward hook", "forward", "bias", "module", "another module", "lora", "float32", "strided", "one token", "tangent"])
 def test_other_blocks_run_module_by_module(change):
     m, handle = _block(128, 2, 64, False).eval(), None
     x = torch.randn(2, 8, 128, device="cuda").bfloat16()
@@ -124,6 +124,8 @@ def test_other_blocks_run_module_by_module(change):
         m.attn.gla.out_proj.bias = torch.nn.Parameter(torch.zeros(128, device="cuda", dtype=torch.bfloat16))
     elif change == "module":
         m.ffn[0] = torch.nn.Sequential(m.ffn[0])
+    elif change == "another module":
+        m.ffn.append(torch.nn.Identity())
     elif change == "lora":
         m.attn.gla.qkvg_lora = lambda t: t
     elif change == "float32":

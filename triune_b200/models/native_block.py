@@ -110,6 +110,8 @@ def run(norm1, attn, norm2, ffn, x, cache) -> Optional[Any]:
             return None
         up, up_bias, down, down_bias = ffn.gate_up, None, ffn.down.weight, None
     else:
+        if len(ffn._modules) != 3:
+            return None
         first, act, last = ffn._modules.values()
         if not (_plain(first, nn.Linear) and _plain(act, nn.GELU) and _plain(last, nn.Linear)):
             return None
