@@ -52,6 +52,16 @@ def test_training_pass(batch, seq, dim, heads, head_dim, delta, learn_beta, monk
         assert torch.equal(a, b) if n != "x" and not n.startswith("norm1") else (a - b).norm() <= 2 ** -7 * b.norm(), n
 
 
+def test_a_block_s_output_may_be_written_into():
+    m = _block(128, 2, 64, False).train()
+    x = torch.randn(2, 70, 128, device="cuda").bfloat16().requires_grad_(True)
+    y = m(x)[0]
+    (plain,) = torch.autograd.grad((2 * y).float().sum(), x, retain_graph=True)
+    y.mul_(2)
+    (got,) = torch.autograd.grad(y.float().sum(), x)
+    assert torch.equal(got, plain)
+
+
 def test_gradients_added_into_buffers_and_frozen_parameters(monkeypatch):
     m = _block(256, 4, 64, True).train()
     x = torch.randn(2, 130, 256, device="cuda").bfloat16()

@@ -111,9 +111,10 @@ std::vector<Tensor> block_forward(const Tensor& x, const std::vector<Opt>& p, co
   auto n2 = tb_launch::rmsnorm_fwd(a, x2, *p[NORM2], eps2);
   Tensor slope = torch::empty({s.rows, p[UP]->size(0)}, x.options());
   Tensor h = product(n2[0], *p[UP], false, false, 1.0, p[UP_BIAS], tb::GF_GELU, {}, slope);
-  Tensor y = product(h, *p[DOWN], false, false, 1.0, p[DOWN_BIAS]);
-  at::add_out(y, n2[2], y);
-  std::vector<Tensor> r{y.view(x.sizes()), n1[0], n1[1], qkvg, qk, o, n2[2], n2[0], n2[1], slope, h, beta};
+  Tensor y = torch::empty(x.sizes(), x.options()), y2 = y.view({s.rows, s.d});  // no view: a caller may write into it
+  product(h, *p[DOWN], false, false, 1.0, p[DOWN_BIAS], 0, {}, {}, y2);
+  at::add_out(y2, n2[2], y2);
+  std::vector<Tensor> r{y, n1[0], n1[1], qkvg, qk, o, n2[2], n2[0], n2[1], slope, h, beta};
   r.insert(r.end(), mixer.begin(), mixer.end());
   r.push_back(status);
   return r;
