@@ -52,6 +52,32 @@ def test_training_pass(batch, seq, dim, heads, head_dim, delta, learn_beta, monk
         assert torch.equal(a, b) if n != "x" and not n.startswith("norm1") else (a - b).norm() <= 2 ** -7 * b.norm(), n
 
 
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("train", [False, True])
+def test_memory_is_that_of_the_modules(train, delta, monkeypatch):
+    m = _block(512, 8, 64, delta).train(train)
+    x = torch.randn(2, 4096, 512, device="cuda").bfloat16().requires_grad_(train)
+    dy = torch.randn_like(x)
+
+    def peak():
+        def call():
+            if train:
+                return torch.autograd.grad(m(x)[0], (x, *m.parameters()), dy)
+            with torch.no_grad():
+                return m(x, cache=(None, 0))
+
+        call()  # tables and workspaces that stay
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        call()
+        torch.cuda.synchronize()
+        return torch.cuda.max_memory_allocated() - before
+
+    native, modules = peak(), _modules(monkeypatch, peak)
+    assert native <= 1.01 * modules
+
+
 def test_a_block_s_output_may_be_written_into():
     m = _block(128, 2, 64, False).train()
     x = torch.randn(2, 70, 128, device="cuda").bfloat16().requires_grad_(True)

@@ -1,5 +1,5 @@
-"""Whole pre-norm blocks in one native call (``csrc/block/block_bind.cpp``): norm, recurrent mixer, norm with the residual, dense
-feed-forward, residual.
+"""Whole pre-norm blocks (``csrc/block/block_bind.cpp``): norm, recurrent mixer, norm with the residual, dense feed-forward, residual. One
+native call without gradients; with them two in each direction (the norm and the mixer; all that follows).
 
 Issued op by op, the launches of a layer keep the host busy for 240 us (a prompt) to 950 us (forward and backward), which is what small
 batches and chat turns cost; the native call issues the same launches. :func:`run` answers only for blocks of plain modules whose
@@ -40,33 +40,62 @@ def _vec(t, n, dev) -> bool:
                          and t.data_ptr() % 16 == 0)
 
 
-class _BlockFn(torch.autograd.Function):
-    """x and the block's parameters -> the block's output; see ``block_forward`` and ``block_backward``."""
+def _buffers(params, want):
+    """Where gradients of wanted parameters are added to, where they have such a buffer."""
+    return [getattr(p, "main_grad", None) if p is not None and w else None for p, w in zip(params, want)]
+
+
+class _BlockMixerFn(torch.autograd.Function):
+    """x and the parameters up to the mixer -> (output of the mixer, x); see ``mixer_forward`` and ``mixer_backward``. That x goes on from here
+    lets its gradient from all that follows join in the norm's backward pass."""
 
     @staticmethod
-    def forward(ctx, x, norm1, qkvg, beta, out, norm2, up, up_bias, down, down_bias, cos, sin, H, D, eps1, eps2, scale, delta):
-        params = (norm1, qkvg, beta, out, norm2, up, up_bias, down, down_bias)
-        y, *saved, status = _ext.ext().block_forward(x, params, cos, sin, H, D, eps1, eps2, scale, delta)
+    def forward(ctx, x, norm1, qkvg, beta, cos, sin, H, D, eps1, delta):
+        params = (norm1, qkvg, beta)
+        o, *saved, status = _ext.ext().mixer_forward(x, params, cos, sin, H, D, eps1, delta)
         T = x.shape[1]
-        ops._tick(11 if delta else 8 + 3 * (T >= 64) + (T % 64 != 0))
+        ops._tick(6 if delta else 3 + 3 * (T >= 64) + (T % 64 != 0))
         _note(status)
         ctx.save_for_backward(x, *params, cos, sin, *saved)
-        ctx.dims = (H, D, scale, delta)
+        ctx.dims = (H, D, delta)
+        return o, x
+
+    @staticmethod
+    def backward(ctx, dout, ds):
+        x, *rest = ctx.saved_tensors
+        params, cos, sin, saved = rest[:3], rest[3], rest[4], rest[5:]
+        want_x, *want = ctx.needs_input_grad[:4]
+        into = _buffers(params, want)
+        into[2] = None  # the write strengths' weight has its gradient returned, wherever it is kept
+        H, D, delta = ctx.dims
+        *grads, status = _ext.ext().mixer_backward(dout, ds, x, params, into, want_x, want, cos, sin, saved, H, D, delta)
+        T = x.shape[1]
+        ops._tick(17 if delta else 8 + 4 * (T >= 64) + 2 * (T % 64 != 0))
+        _note(status)
+        return (*grads, None, None, None, None, None, None)
+
+
+class _BlockFn(torch.autograd.Function):
+    """The rest of a block: the mixer's output, x and the parameters after the mixer -> the block's output; see ``rest_forward`` and
+    ``rest_backward``."""
+
+    @staticmethod
+    def forward(ctx, o, x, out, norm2, up, up_bias, down, down_bias, eps2, scale):
+        params = (out, norm2, up, up_bias, down, down_bias)
+        y, *saved = _ext.ext().rest_forward(o, x, params, eps2, scale)
+        ops._tick(5)
+        ctx.save_for_backward(o, x, *params, *saved)
+        ctx.scale = scale
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, *rest = ctx.saved_tensors
-        params, cos, sin, saved = rest[:9], rest[9], rest[10], rest[11:]
-        H, D, scale, delta = ctx.dims
-        want = ctx.needs_input_grad[:10]
-        # the write strengths' weight has its gradient returned, wherever it is kept
-        into = [getattr(p, "main_grad", None) if p is not None and w and i != 2 else None for i, (p, w) in enumerate(zip(params, want[1:]))]
-        *grads, status = _ext.ext().block_backward(dy, x, params, into, list(want), cos, sin, saved, H, D, scale, delta)
-        T = x.shape[1]
-        ops._tick(26 if delta else 17 + 4 * (T >= 64) + 2 * (T % 64 != 0))
-        _note(status)
-        return (*grads, None, None, None, None, None, None, None, None)
+        o, x, *rest = ctx.saved_tensors
+        params, saved = rest[:6], rest[6:]
+        want = list(ctx.needs_input_grad[2:8])
+        dout, ds, *grads = _ext.ext().rest_backward(dy, o, x, params, _buffers(params, want), want, saved, ctx.scale)
+        ops._tick(9)
+        return (dout, ds, *grads, None, None)
 
 
 def _note(status) -> None:
@@ -138,13 +167,14 @@ def run(norm1, attn, norm2, ffn, x, cache) -> Optional[Any]:
         if cos.dtype != torch.float32 or not cos.is_contiguous() or not sin.is_contiguous() or cos.shape[1] != D or cos.data_ptr() % 16 or sin.data_ptr() % 16:
             return None
     scale = 1.0 if delta else attn.out_scale
-    params = (w1, qkvg, beta, out, w2, up, up_bias, down, down_bias)
+    mixer, after = (w1, qkvg, beta), (out, w2, up, up_bias, down, down_bias)
     if not grad:
-        y, new_state, status = _ext.ext().block_infer(x, params, cos, sin, offset, state, H, D, norm1.eps, norm2.eps, scale, delta, gated)
+        y, new_state, status = _ext.ext().block_infer(x, mixer, after, cos, sin, offset, state, H, D, norm1.eps, norm2.eps, scale, delta, gated)
         ops._tick(9 if delta else 7 + 3 * (T >= 64) + (T % 64 != 0))
         _note(status)
         return y, format_cache(new_state if cache is not None else None, cache, fmt, offset, T)
     # a mixer without gradients takes other kernels
-    if not (x.requires_grad or w1.requires_grad or qkvg.requires_grad) or not all(p is None or _arena_ok(p) for p in params):
+    if not (x.requires_grad or w1.requires_grad or qkvg.requires_grad) or not all(p is None or _arena_ok(p) for p in (*mixer, *after)):
         return None
-    return _BlockFn.apply(x, *params, cos, sin, H, D, norm1.eps, norm2.eps, scale, delta), None
+    o, x = _BlockMixerFn.apply(x, *mixer, cos, sin, H, D, norm1.eps, delta)
+    return _BlockFn.apply(o, x, *after, norm2.eps, scale), None
