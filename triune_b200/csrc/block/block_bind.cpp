@@ -87,7 +87,7 @@ std::vector<Tensor> block_infer(const Tensor& x, const std::vector<Opt>& p, cons
       state = torch::empty({s.B, H, D, D}, x.options().dtype(at::kFloat));
       if (init) state.copy_(*init);
       else state.zero_();
-      tb_launch::gdn_recurrent(qk, 0, qk, s.HD, qkvg, 2 * s.HD, qkvg, 3 * s.HD, beta, state, o, 0, s.B, s.T, H, D, true, 1.0);
+      status = tb_launch::gdn_recurrent(qk, 0, qk, s.HD, qkvg, 2 * s.HD, qkvg, 3 * s.HD, beta, state, o, 0, s.B, s.T, H, D, true, 1.0);
     } else {
       auto r = tb_launch::gla_fwd(qk, 0, qk, s.HD, qkvg, 2 * s.HD, qkvg, 3 * s.HD, o, 0, init, s.B, s.T, H, true, D);
       state = r[2].view({s.B, H, D, D});

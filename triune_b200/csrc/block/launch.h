@@ -24,9 +24,9 @@ std::vector<Tensor> gla_bwd(const Tensor& q, int64_t qcol, const Tensor& k, int6
                             int64_t gcol, const Tensor& dout, int64_t docol, const Tensor& states, const Tensor& decay, Tensor& dq, int64_t dqcol,
                             Tensor& dk, int64_t dkcol, Tensor& dv, int64_t dvcol, Tensor& dg, int64_t dgcol, int64_t B, int64_t T, int64_t H,
                             bool gate_logits, const Opt& dfin, const Opt& fin, int64_t D, const Opt& before_rest);
-void gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol, const Tensor& g, int64_t gcol,
-                   const Opt& beta, Tensor& state, Tensor& out, int64_t ocol, int64_t B, int64_t T, int64_t H, int64_t D, bool gate_logits,
-                   double scale);
+Tensor gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol, const Tensor& g, int64_t gcol,
+                     const Opt& beta, Tensor& state, Tensor& out, int64_t ocol, int64_t B, int64_t T, int64_t H, int64_t D, bool gate_logits,
+                     double scale);
 std::vector<Tensor> gdn_chunk_fwd(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol, const Tensor& g,
                                   int64_t gcol, const Opt& beta, const Opt& init, Tensor& out, int64_t ocol, int64_t B, int64_t T, int64_t H,
                                   int64_t D, bool gate_logits, double scale, bool keep_scores);

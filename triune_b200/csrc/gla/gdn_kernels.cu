@@ -265,6 +265,7 @@ struct GdnBlockArgs {
   __nv_bfloat16* out;
   int T, H, logits;
   float scale;
+  int* status;
 };
 
 // Record `index` of [B * H, ceil(nt / GB)] for tokens [t0, t0 + nt) of every sequence, by a CTA of four warps. A warp carries the vectors
@@ -618,13 +619,18 @@ struct GdnWalk {
     return odd;
   }
 
-  // The whole segment; true (to all threads) where an output or the state after it is no number. The state in memory is as it was. The rounds
+  // How a walk ended, for all threads: fine; with an output or the state no number, or with a record that came late: to be walked again; with
+  // a record that still had not landed, so that its stage may not be used for anything else.
+  enum End { FINE, AGAIN, LOST };
+
+  // The whole segment. The state in memory is as it was. The rounds
   // are those of round(), in another order: a block's outputs wait for the next round's barrier, so that there is one barrier a
   // round, and what they need from the state is multiplied while the triangle's short chain runs.
-  __device__ __forceinline__ bool walk() {
+  __device__ __forceinline__ End walk() {
     start();
     fetch(0);
     fetch(1);
+    int issued = min(nb, 2);  // records on their way or there, as thread 0 counts them
     load_state();
     bool odd = false, late = !landed(0, 0);
     int at = 0, lap = 0;      // stage of the block, records that it held before
@@ -658,7 +664,7 @@ struct GdnWalk {
         }
       leave(buf, 0, kp[0], kp[1]);
       __syncthreads();  // all warps' sums; the record of the block before has been read
-      fetch(blk + 2);   // in its place
+      if (!late && blk + 2 < nb) fetch(blk + 2), issued = blk + 3;  // in its place
       if (blk > 0) outputs(blk - 1);
       float x[2][4];
 #pragma unroll
@@ -708,7 +714,12 @@ struct GdnWalk {
     }
     __syncthreads();
     if (nb > 0) outputs(nb - 1);
-    return __syncthreads_or(odd || late || state_odd());
+    if (!__syncthreads_or(odd || late || state_odd())) return FINE;
+    // nothing else goes into a stage, and nothing leaves, while a copy into it is in flight
+    bool lost = false;
+    if (tid == 0 && late)
+      for (int b = max(0, issued - GDN_STAGES); b < issued; ++b) lost |= !landed(b, b / GDN_STAGES);
+    return __syncthreads_or(lost) ? LOST : AGAIN;
   }
 
   // The same where something is no number. A later token of a block enters an earlier one's sums times a zero of a triangle, which
@@ -850,18 +861,21 @@ __global__ void __launch_bounds__(128) gdn_block_kernel(const __grid_constant__ 
                                                         float* next_rec, int next_nt) {
   extern __shared__ __align__(16) uint8_t block_smem[];
   if ((int)blockIdx.x >= walks) {
+    if (walks == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.status = ST_OK;  // the first launch, which walks nothing
     gdn_block_prep<D>(a, *reinterpret_cast<GdnPrepShared<D>*>(block_smem), next_rec, t0 + nt, next_nt, (int)blockIdx.x - walks);
     return;
   }
   GdnWalkShared<D>& sh = *reinterpret_cast<GdnWalkShared<D>*>(block_smem);
   GdnWalk<D> w(a, sh, rec, t0, nt);
-  if (w.walk()) gdn_walk_again<D>(a, sh, rec, t0, nt);
-  else w.store_state();
+  const typename GdnWalk<D>::End end = w.walk();
+  if (end == GdnWalk<D>::FINE) w.store_state();
+  else if (end == GdnWalk<D>::AGAIN) gdn_walk_again<D>(a, sh, rec, t0, nt);
+  else if (threadIdx.x == 0) *a.status = ST_TIMEOUT_FULL;
 }
 
 template <int D>
 void run_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode, float* state,
-                const GlaMat& O, int B, int T, int H, bool logits, float scale, float* rec, int seg, cudaStream_t s) {
+                const GlaMat& O, int B, int T, int H, bool logits, float scale, float* rec, int* status, int seg, cudaStream_t s) {
   auto p = [](const GlaMat& m) { return reinterpret_cast<const __nv_bfloat16*>(m.ptr); };
   constexpr int walk_smem = (int)sizeof(GdnWalkShared<D>), prep_smem = (int)sizeof(GdnPrepShared<D>);
   static PerDeviceOnce once;
@@ -870,7 +884,7 @@ void run_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat&
     if (e != cudaSuccess) throw std::runtime_error(std::string("gdn_blocks attribute: ") + cudaGetErrorString(e));
   }
   const GdnBlockArgs a{p(Q), p(K), p(V), p(G), Q.ld, K.ld, V.ld, G.ld, O.ld, Q.col0, K.col0, V.col0, G.col0, O.col0, beta, beta_mode, state,
-                       reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(O.ptr)), T, H, logits ? 1 : 0, scale};
+                       reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(O.ptr)), T, H, logits ? 1 : 0, scale, status};
   auto tokens = [&](int t0) { return T - t0 < seg ? T - t0 : seg; };
   auto records = [&](int nt) { return B * H * ((nt + GB - 1) / GB); };
   float* half[2] = {rec, rec + (long long)records(tokens(0)) * GdnRec<D>::FLOATS};
@@ -914,13 +928,13 @@ long long gdn_block_workspace_floats(int B, int T, int H, int D) {
 
 void launch_gdn_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode,
                        float* state, const GlaMat& O, int B, int T, int H, int D, bool logits, float scale, float* workspace,
-                       cudaStream_t s) {
+                       int* status, cudaStream_t s) {
   if (B <= 0 || T <= 0) return;
   const int seg = segment_tokens(B * H, D);
   if (D == 64)
-    run_blocks<64>(Q, K, V, G, beta, beta_mode, state, O, B, T, H, logits, scale, workspace, seg, s);
+    run_blocks<64>(Q, K, V, G, beta, beta_mode, state, O, B, T, H, logits, scale, workspace, status, seg, s);
   else if (D == 128)
-    run_blocks<128>(Q, K, V, G, beta, beta_mode, state, O, B, T, H, logits, scale, workspace, seg, s);
+    run_blocks<128>(Q, K, V, G, beta, beta_mode, state, O, B, T, H, logits, scale, workspace, status, seg, s);
   else
     throw std::runtime_error("gdn_blocks: head dimension must be 64 or 128");
   cudaError_t e = cudaGetLastError();

@@ -97,11 +97,11 @@ void launch_gdn_recurrent(const GlaMat& Q, const GlaMat& K, const GlaMat& V, con
                           float scale, cudaStream_t s);
 
 // The same, sixteen tokens per round; `workspace`: fp32 [gdn_block_workspace_floats(...)], 16-byte aligned, 0 floats where the token
-// recurrence is the faster one. q, k, v, g rows must start on 8-byte boundaries.
+// recurrence is the faster one. q, k, v, g rows must start on 8-byte boundaries. `status`: device word, 0 or what a wait that ran out left.
 long long gdn_block_workspace_floats(int B, int T, int H, int D);
 void launch_gdn_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat& G, const float* beta, int beta_mode,
                        float* state, const GlaMat& O, int B, int T, int H, int D, bool gate_logits, float scale, float* workspace,
-                       cudaStream_t s);
+                       int* status, cudaStream_t s);
 
 // ---- Gated DeltaNet, chunk-parallel training path (gdn_chunk_kernels.cu) ----
 struct GdnDims {

@@ -190,12 +190,13 @@ std::vector<Tensor> mixer_step(const Tensor& qkvg, const c10::optional<Tensor>& 
   return {out, next};
 }
 
-// Gated DeltaNet recurrence (no gradient): q,k,v,g as [B*T, ld] matrices whose columns col0 + h*D.. hold head h.
+// Gated DeltaNet recurrence (no gradient): q,k,v,g as [B*T, ld] matrices whose columns col0 + h*D.. hold head h. Returns the status of
+// the kernel that takes prompts in blocks (empty where the token kernel ran, which waits for nothing).
 }  // namespace
 namespace tb_launch {
-void gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol,
-                   const Tensor& g, int64_t gcol, const c10::optional<Tensor>& beta, Tensor& state, Tensor& out,
-                   int64_t ocol, int64_t B, int64_t T, int64_t H, int64_t D, bool gate_logits, double scale) {
+Tensor gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol,
+                     const Tensor& g, int64_t gcol, const c10::optional<Tensor>& beta, Tensor& state, Tensor& out,
+                     int64_t ocol, int64_t B, int64_t T, int64_t H, int64_t D, bool gate_logits, double scale) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(state.scalar_type() == at::kFloat && state.is_contiguous() && state.numel() == B * H * D * D,
               "state must be fp32 contiguous [B,H,D,D]");
@@ -209,14 +210,17 @@ void gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol,
     bp = beta->data_ptr<float>();
   }
   const int64_t ws = tb::gdn_block_workspace_floats((int)B, (int)T, (int)H, (int)D);
+  Tensor status = torch::empty({ws > 0 ? 1 : 0}, state.options().dtype(at::kInt));
   if (ws > 0) {
     Tensor work = torch::empty({ws}, state.options());
     tb::launch_gdn_blocks(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), bp, mode, state.data_ptr<float>(), mat(out, ocol),
-                          (int)B, (int)T, (int)H, (int)D, gate_logits, (float)scale, work.data_ptr<float>(), cur_stream());
-    return;
+                          (int)B, (int)T, (int)H, (int)D, gate_logits, (float)scale, work.data_ptr<float>(), status.data_ptr<int>(),
+                          cur_stream());
+    return status;
   }
   tb::launch_gdn_recurrent(mat(q, qcol), mat(k, kcol), mat(v, vcol), mat(g, gcol), bp, mode, state.data_ptr<float>(),
                            mat(out, ocol), (int)B, (int)T, (int)H, (int)D, gate_logits, (float)scale, cur_stream());
+  return status;
 }
 }  // namespace tb_launch
 namespace {

@@ -362,8 +362,10 @@ def gdn_recurrent(q, k, v, g, beta, initial_state, scale, gate_logits):
     qm, km, vm, gm = (_as_matrix(t.to(torch.bfloat16)) for t in (q, k, v, g))
     out = torch.empty(B * T, H * D, device=q.device, dtype=torch.bfloat16)
     bt = None if beta is None else beta.float().contiguous()
-    e.gdn_recurrent(qm, 0, km, 0, vm, 0, gm, 0, bt, st, out, 0, B, T, H, D, gate_logits, float(scale))
+    status = e.gdn_recurrent(qm, 0, km, 0, vm, 0, gm, 0, bt, st, out, 0, B, T, H, D, gate_logits, float(scale))
     _tick(1)
+    if status.numel():
+        _note(status)
     return out.view(B, T, H, D), st
 
 
