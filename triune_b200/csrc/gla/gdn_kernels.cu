@@ -192,7 +192,7 @@ struct GdnRec {  // floats of a record: k P and q P [32][PK] | (beta k) dec [16]
 __device__ __forceinline__ float gdn_decay(float x, bool logits) {
   if (!logits) return __expf(gdn_log_decay(x, false));
   const float e = __expf(-fabsf(x)), small = __fdividef(e, 1.f + e);
-  return fmaxf(x > 0.f ? 1.f - small : small, 6.7379469990854671e-3f);
+  return fmaxf(x > 0.f ? 1.f - small : small, GLA_MIN_DECAY);
 }
 
 // Sum of v[l] over the lanes, in lane l.

@@ -15,6 +15,9 @@
 namespace tb {
 
 constexpr float GLA_MIN_LOG_DECAY = -5.0f;
+// What follows from it: the least decay, and the logit whose log-sigmoid it is, -log(e^5 - 1).
+static_assert(GLA_MIN_LOG_DECAY == -5.0f, "the two numbers below are of -5");
+constexpr float GLA_MIN_DECAY = 6.7379469990854671e-3f, GLA_MIN_LOGIT = -4.9932392505505110f;
 
 // A [B*T rows] x [D cols] bf16 slice of a wider row-major matrix: element (row, c) = ptr[row*ld + col0 + h*D + c].
 struct GlaMat {

@@ -994,8 +994,8 @@ __global__ void __launch_bounds__(256) gla_dg_finalize_kernel(const float* __res
     for (int j = 0; j < 8; ++j) {
       float deriv;
       if (logits) {
-        // d logsigmoid = sigmoid(-x) where logsigmoid(x) is above the clamp: x > -4.99326, between the bf16 numbers -5 and -4.96875
-        deriv = x[j] > -4.9932617f ? __fdividef(1.f, 1.f + __expf(x[j])) : 0.f;
+        // d logsigmoid = sigmoid(-x) where logsigmoid(x) is above the clamp, whose logit lies between the bf16 numbers -5 and -4.96875
+        deriv = x[j] > GLA_MIN_LOGIT ? __fdividef(1.f, 1.f + __expf(x[j])) : 0.f;
       } else {
         deriv = (x[j] <= 0.f && x[j] >= GLA_MIN_LOG_DECAY) ? 1.f : 0.f;
       }
