@@ -1,5 +1,7 @@
 """The one-launch decoding step against the step of the model's modules: the same tokens, states and positions, bit for bit."""
 
+import threading
+
 import pytest
 import torch
 
@@ -138,3 +140,24 @@ def test_a_step_that_did_not_finish_raises_and_the_next_prompt_starts_over(how):
         dec.decode(3)
     assert torch.equal(dec.generate(ids, 6), want)
     assert dec.graph is not first and int(dec.graph.status) == 0
+
+
+def test_two_decoders_on_two_streams_take_turns():
+    models = [_model(256, 4, 64, 3, 320, 512, "gla"), _model(384, 6, 64, 4, 1088, 1000, "gated_deltanet")]
+    prompts = [torch.randint(0, 500, (b, 33), device="cuda") for b in (1, 2)]
+    decoders = [GraphedGreedyDecoder(m, batch_size=p.shape[0]) for m, p in zip(models, prompts)]
+    want = [d.generate(p, 40) for d, p in zip(decoders, prompts)]
+    torch.cuda.synchronize()
+    same = [[], []]
+
+    def serve(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(8):
+                same[i].append(torch.equal(decoders[i].generate(prompts[i], 40), want[i]))
+
+    threads = [threading.Thread(target=serve, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert same == [[True] * 8] * 2

@@ -29,7 +29,9 @@ void check_bf16_cuda(const Tensor& t, const char* name) {
 }
 
 }  // namespace
+
 namespace tb_launch {
+
 std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& res, const Tensor& w, double eps) {
   check_bf16_cuda(x, "x");
   TORCH_CHECK(x.is_contiguous() && w.is_contiguous(), "rmsnorm: contiguous inputs required");
@@ -51,11 +53,9 @@ std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& re
                          rstd.data_ptr<float>(), rows, d, (float)eps, cur_stream());
   return {y, rstd, has_res ? sum_out : Tensor()};
 }
-}  // namespace tb_launch
-namespace {
 
 // Where a gradient's column sums go: into `into` (fp32, added), or a new tensor, bf16 on request and else fp32.
-tb::ColumnSum column_sum(const c10::optional<Tensor>& into, bool bf16, int64_t n, const Tensor& like, Tensor& res) {
+static tb::ColumnSum column_sum(const c10::optional<Tensor>& into, bool bf16, int64_t n, const Tensor& like, Tensor& res) {
   const bool add = into.has_value() && into->defined();
   if (add)
     TORCH_CHECK(into->is_cuda() && into->scalar_type() == at::kFloat && into->is_contiguous() && into->numel() == n, "out must be fp32 [N]");
@@ -65,8 +65,6 @@ tb::ColumnSum column_sum(const c10::optional<Tensor>& into, bool bf16, int64_t n
 }
 
 // Returns (dx, dw): dw as column_sum says.
-}  // namespace
-namespace tb_launch {
 std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& dy, const Tensor& rstd,
                                 const c10::optional<Tensor>& dres, const c10::optional<Tensor>& dw_into, bool dw_bf16) {
   check_bf16_cuda(x, "x");
@@ -84,11 +82,9 @@ std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& 
                          partial.data_ptr<float>(), to, rows, d, cur_stream());
   return {dx, dw};
 }
-}  // namespace tb_launch
-namespace {
 
 // Row pitch of rotary tables: fp32 rows that the kernels read in 16-byte vectors.
-int table_pitch(const Tensor& cs, const Tensor& sn, int64_t T, int64_t D) {
+static int table_pitch(const Tensor& cs, const Tensor& sn, int64_t T, int64_t D) {
   for (const Tensor* t : {&cs, &sn})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 2 && t->stride(1) == 1 && t->stride(0) % 4 == 0 &&
                     t->size(0) >= T && t->size(1) >= D / 2 && t->stride(0) == cs.stride(0) &&
@@ -98,8 +94,6 @@ int table_pitch(const Tensor& cs, const Tensor& sn, int64_t T, int64_t D) {
 }
 
 // in: [tokens, ld] with q at col 0 and k at col k_off; returns [tokens, 2, H, D].
-}  // namespace
-namespace tb_launch {
 Tensor qk_prep_fwd(const Tensor& in, int64_t k_off, const c10::optional<Tensor>& cs, const c10::optional<Tensor>& sn,
                    int64_t T, int64_t H, int64_t D) {
   check_bf16_cuda(in, "in");
@@ -125,11 +119,9 @@ void qk_prep_bwd(const Tensor& in, int64_t k_off, const Tensor& dout, Tensor& d_
                          rope ? cs->data_ptr<float>() : nullptr, rope ? sn->data_ptr<float>() : nullptr, rope ? table_pitch(*cs, *sn, T, D) : 0, in.size(0),
                          (int)T, (int)H, (int)D, cur_stream());
 }
-}  // namespace tb_launch
-namespace {
 
 // Cross entropy that leaves the logits intact: returns (per-row loss, grad_scale * (softmax - onehot) as a new tensor).
-std::vector<Tensor> ce_loss_grad(const Tensor& logits, const Tensor& targets, int64_t ignore_index, double grad_scale) {
+static std::vector<Tensor> ce_loss_grad(const Tensor& logits, const Tensor& targets, int64_t ignore_index, double grad_scale) {
   check_bf16_cuda(logits, "logits");
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1 && logits.stride(0) % 8 == 0, "logits must be [rows, V] with 16-byte rows");
   TORCH_CHECK(targets.scalar_type() == at::kLong && targets.is_contiguous() && targets.numel() == logits.size(0),
@@ -152,14 +144,14 @@ struct RowMat {
   const __nv_bfloat16* p;
   long long ld;
 };
-RowMat rows_of(const Tensor& t, int64_t width, const char* name) {
+static RowMat rows_of(const Tensor& t, int64_t width, const char* name) {
   check_bf16_cuda(t, name);
   TORCH_CHECK(t.dim() == 2 && t.stride(1) == 1 && t.size(1) == width && t.stride(0) % 8 == 0, name,
               ": [rows, width] with contiguous, 16-byte aligned rows expected");
   return RowMat{bf(t), t.stride(0)};
 }
 
-Tensor swiglu_fwd(const Tensor& gate, const Tensor& up) {
+static Tensor swiglu_fwd(const Tensor& gate, const Tensor& up) {
   const int64_t rows = gate.size(0), width = gate.size(1);
   TORCH_CHECK(width % 8 == 0 && up.size(0) == rows, "swiglu: width must be a multiple of 8");
   RowMat g = rows_of(gate, width, "gate"), u = rows_of(up, width, "up");
@@ -169,7 +161,7 @@ Tensor swiglu_fwd(const Tensor& gate, const Tensor& up) {
   return out;
 }
 
-std::vector<Tensor> swiglu_bwd(const Tensor& gate, const Tensor& up, const Tensor& dh) {
+static std::vector<Tensor> swiglu_bwd(const Tensor& gate, const Tensor& up, const Tensor& dh) {
   const int64_t rows = gate.size(0), width = gate.size(1);
   TORCH_CHECK(width % 8 == 0, "swiglu: width must be a multiple of 8");
   RowMat g = rows_of(gate, width, "gate"), u = rows_of(up, width, "up"), d = rows_of(dh, width, "dh");
@@ -184,7 +176,7 @@ std::vector<Tensor> swiglu_bwd(const Tensor& gate, const Tensor& up, const Tenso
 }
 
 // x: [rows = B*T, H*D] bf16 (row pitch free); cos/sin: fp32 [T, D/2] contiguous.
-Tensor rope_apply(const Tensor& x, const Tensor& cs, const Tensor& sn, int64_t T, int64_t H, int64_t D, bool transpose) {
+static Tensor rope_apply(const Tensor& x, const Tensor& cs, const Tensor& sn, int64_t T, int64_t H, int64_t D, bool transpose) {
   RowMat xm = rows_of(x, H * D, "x");
   TORCH_CHECK(D % 16 == 0 && cs.scalar_type() == at::kFloat && sn.scalar_type() == at::kFloat && cs.is_contiguous() &&
                   sn.is_contiguous() && cs.numel() == T * (D / 2) && sn.numel() == T * (D / 2),
@@ -198,7 +190,7 @@ Tensor rope_apply(const Tensor& x, const Tensor& cs, const Tensor& sn, int64_t T
 }
 
 // grad [V, d] fp32 += scatter of dy [tokens, d] bf16 by ids [tokens] int64.
-void embedding_bwd(const Tensor& dy, const Tensor& ids, Tensor& grad) {
+static void embedding_bwd(const Tensor& dy, const Tensor& ids, Tensor& grad) {
   check_bf16_cuda(dy, "dy");
   TORCH_CHECK(dy.dim() == 2 && dy.stride(1) == 1 && dy.stride(0) % 4 == 0 && dy.size(1) % 4 == 0, "dy must be [tokens, d], d % 4 == 0");
   TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && ids.numel() == dy.size(0), "ids must be int64 [tokens]");
@@ -211,7 +203,7 @@ void embedding_bwd(const Tensor& dy, const Tensor& ids, Tensor& grad) {
                            grad.data_ptr<float>(), dy.size(0), (int)dy.size(1), grad.size(0), cur_stream());
 }
 
-Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, int64_t ignore_index, double grad_scale) {
+static Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, int64_t ignore_index, double grad_scale) {
   check_bf16_cuda(logits, "logits");
   TORCH_CHECK(logits.dim() == 2 && logits.stride(1) == 1, "logits must be [rows, V]");
   TORCH_CHECK(targets.scalar_type() == at::kLong && targets.is_contiguous(), "targets must be int64");
@@ -224,8 +216,6 @@ Tensor ce_fwd_bwd(Tensor& logits, const Tensor& targets, int64_t ignore_index, d
 }
 
 // Column sums of a bf16 [M, N] matrix in fp32: returns a new [N] tensor (rounded to bf16 on request), or adds into `out`.
-}  // namespace
-namespace tb_launch {
 Tensor colsum(const Tensor& x, const c10::optional<Tensor>& out, bool bf16) {
   check_bf16_cuda(x, "x");
   TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && x.size(1) % 8 == 0 && x.stride(0) % 8 == 0,
@@ -240,11 +230,9 @@ Tensor colsum(const Tensor& x, const c10::optional<Tensor>& out, bool bf16) {
   tb::launch_colsum(bf(x), x.stride(0), M, N, partial.data_ptr<float>(), parts, to, cur_stream());
   return res;
 }
-}  // namespace tb_launch
-namespace {
 
 // out (int64, one value per row) = index of the largest value of each row of x [rows, V] bf16
-void argmax_rows(const Tensor& x, Tensor& out) {
+static void argmax_rows(const Tensor& x, Tensor& out) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1 && x.size(1) > 0, "argmax_rows: [rows, V] bf16 rows");
   TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kLong && out.is_contiguous() && out.numel() == x.size(0) &&
                   out.get_device() == x.get_device(), "argmax_rows: int64 [rows]");
@@ -253,7 +241,7 @@ void argmax_rows(const Tensor& x, Tensor& out) {
                          cur_stream());
 }
 
-Tensor gather_rows(const Tensor& src, const Tensor& row_src, const c10::optional<Tensor>& row_scale) {
+static Tensor gather_rows(const Tensor& src, const Tensor& row_src, const c10::optional<Tensor>& row_scale) {
   check_bf16_cuda(src, "src");
   TORCH_CHECK(src.dim() == 2 && src.is_contiguous() && src.size(1) % 8 == 0, "src must be [rows, width%8==0]");
   TORCH_CHECK(row_src.scalar_type() == at::kInt, "row_src must be int32");
@@ -265,7 +253,7 @@ Tensor gather_rows(const Tensor& src, const Tensor& row_src, const c10::optional
   return dst;
 }
 
-Tensor combine_rows(const Tensor& src, const Tensor& pos, const c10::optional<Tensor>& w,
+static Tensor combine_rows(const Tensor& src, const Tensor& pos, const c10::optional<Tensor>& w,
                     const c10::optional<Tensor>& add, double add_scale) {
   check_bf16_cuda(src, "src");
   TORCH_CHECK(pos.scalar_type() == at::kInt && pos.dim() == 2 && pos.is_contiguous(), "pos must be int32 [tokens,k]");
@@ -281,13 +269,13 @@ Tensor combine_rows(const Tensor& src, const Tensor& pos, const c10::optional<Te
   return out;
 }
 
-std::vector<int64_t> index_error_word(bool clear) {
+static std::vector<int64_t> index_error_word(bool clear) {
   int w[4];
   tb::index_error_word(w, clear);
   return {w[0], w[1], w[2], w[3]};
 }
 
-Tensor row_dots(const Tensor& a, const Tensor& b, const Tensor& pos) {
+static Tensor row_dots(const Tensor& a, const Tensor& b, const Tensor& pos) {
   check_bf16_cuda(a, "a");
   check_bf16_cuda(b, "b");
   TORCH_CHECK(a.is_contiguous() && b.is_contiguous() && pos.is_contiguous(), "contiguous inputs required");
@@ -298,7 +286,7 @@ Tensor row_dots(const Tensor& a, const Tensor& b, const Tensor& pos) {
   return dots;
 }
 
-std::vector<Tensor> moe_route_topk(const Tensor& logits, const Tensor& bias, const c10::optional<Tensor>& temperature,
+static std::vector<Tensor> moe_route_topk(const Tensor& logits, const Tensor& bias, const c10::optional<Tensor>& temperature,
                                    double temp_value, int64_t K) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.is_contiguous() && logits.scalar_type() == at::kFloat, "logits: contiguous fp32 [N, E]");
   TORCH_CHECK(bias.scalar_type() == at::kFloat && bias.is_contiguous() && bias.numel() == logits.size(1), "bias: fp32 [E]");
@@ -317,7 +305,7 @@ std::vector<Tensor> moe_route_topk(const Tensor& logits, const Tensor& bias, con
   return {idx, w, keys, counts};
 }
 
-Tensor moe_route_bwd(const Tensor& logits, const c10::optional<Tensor>& temperature, double temp_value, const Tensor& idx,
+static Tensor moe_route_bwd(const Tensor& logits, const c10::optional<Tensor>& temperature, double temp_value, const Tensor& idx,
                      const Tensor& w, const Tensor& dw) {
   c10::cuda::CUDAGuard guard(logits.device());
   const int64_t N = logits.size(0), E = logits.size(1), K = idx.size(1);
@@ -329,7 +317,7 @@ Tensor moe_route_bwd(const Tensor& logits, const c10::optional<Tensor>& temperat
   return dl;
 }
 
-std::vector<Tensor> moe_plan_sorted(const Tensor& sorted_keys, const Tensor& order, const Tensor& counts, int64_t N, int64_t K,
+static std::vector<Tensor> moe_plan_sorted(const Tensor& sorted_keys, const Tensor& order, const Tensor& counts, int64_t N, int64_t K,
                                     int64_t cap) {
   const bool keys32 = sorted_keys.scalar_type() == at::kInt;
   TORCH_CHECK((keys32 || sorted_keys.scalar_type() == at::kLong) && order.scalar_type() == at::kLong && counts.scalar_type() == at::kInt,
@@ -349,7 +337,7 @@ std::vector<Tensor> moe_plan_sorted(const Tensor& sorted_keys, const Tensor& ord
 }
 
 // max(1 - step / steps, least) as an fp32 scalar on the device of the step (int64)
-Tensor moe_temperature(const Tensor& step, double steps, double least) {
+static Tensor moe_temperature(const Tensor& step, double steps, double least) {
   TORCH_CHECK(step.is_cuda() && step.scalar_type() == at::kLong && step.numel() == 1, "moe_temperature: step int64 on the device");
   c10::cuda::CUDAGuard guard(step.device());
   Tensor out = torch::empty({}, step.options().dtype(at::kFloat));
@@ -358,7 +346,7 @@ Tensor moe_temperature(const Tensor& step, double steps, double least) {
 }
 
 // [N, E] bf16: 1 for each accepted expert of a token
-Tensor moe_mask(const Tensor& idx, const c10::optional<Tensor>& keep, int64_t E) {
+static Tensor moe_mask(const Tensor& idx, const c10::optional<Tensor>& keep, int64_t E) {
   TORCH_CHECK(idx.is_cuda() && idx.scalar_type() == at::kLong && idx.dim() == 2 && idx.is_contiguous() && E % 8 == 0, "moe_mask: idx int64 [N, K], E % 8 == 0");
   const bool has = keep.has_value() && keep->defined();
   if (has) TORCH_CHECK(keep->is_cuda() && keep->scalar_type() == at::kBool && keep->is_contiguous() && keep->sizes() == idx.sizes(), "moe_mask: keep bool [N, K]");
@@ -370,7 +358,7 @@ Tensor moe_mask(const Tensor& idx, const c10::optional<Tensor>& keep, int64_t E)
 }
 
 // -> requested, dropped (int64 [E]), pending bias update (fp32 [E]); overflow, load and centroids are updated in place
-std::vector<Tensor> moe_stats(const Tensor& slot_counts, const c10::optional<Tensor>& accepted, const Tensor& sums, Tensor& overflow, Tensor& load,
+static std::vector<Tensor> moe_stats(const Tensor& slot_counts, const c10::optional<Tensor>& accepted, const Tensor& sums, Tensor& overflow, Tensor& load,
                               Tensor& centroids, double target, double rate, double ema) {
   const int64_t E = slot_counts.size(0), K = slot_counts.size(1), D = centroids.size(1);
   TORCH_CHECK(slot_counts.is_cuda() && slot_counts.scalar_type() == at::kInt && slot_counts.is_contiguous(), "moe_stats: counts int32 [E, K]");
@@ -392,7 +380,7 @@ std::vector<Tensor> moe_stats(const Tensor& slot_counts, const c10::optional<Ten
   return {requested, dropped, pending};
 }
 
-void adamw_flat(Tensor& master, Tensor& m, Tensor& v, const Tensor& grad, const c10::optional<Tensor>& param_bf16,
+static void adamw_flat(Tensor& master, Tensor& m, Tensor& v, const Tensor& grad, const c10::optional<Tensor>& param_bf16,
                 double lr, double beta1, double beta2, double eps, double wd, int64_t step,
                 const c10::optional<Tensor>& grad_scale_ptr, double grad_scale, const c10::optional<Tensor>& hyper) {
   TORCH_CHECK(master.scalar_type() == at::kFloat && master.is_contiguous(), "master must be fp32 contiguous");
@@ -411,13 +399,13 @@ void adamw_flat(Tensor& master, Tensor& m, Tensor& v, const Tensor& grad, const 
                         hyper.has_value() && hyper->defined() ? hyper->data_ptr<float>() : nullptr, cur_stream());
 }
 
-void sumsq(const Tensor& x, Tensor& out) {
+static void sumsq(const Tensor& x, Tensor& out) {
   TORCH_CHECK(x.is_contiguous() && out.scalar_type() == at::kFloat, "sumsq: contiguous x, fp32 out");
   c10::cuda::CUDAGuard guard(x.device());
   tb::launch_sumsq(x.data_ptr(), x.scalar_type() == at::kFloat, x.numel(), out.data_ptr<float>(), cur_stream());
 }
 
-void muon_momentum(Tensor& mom, const Tensor& grad, Tensor& u_out, double beta, bool nesterov,
+static void muon_momentum(Tensor& mom, const Tensor& grad, Tensor& u_out, double beta, bool nesterov,
                    const c10::optional<Tensor>& grad_scale_ptr) {
   c10::cuda::CUDAGuard guard(mom.device());
   const bool hs = grad_scale_ptr.has_value() && grad_scale_ptr->defined();
@@ -426,7 +414,7 @@ void muon_momentum(Tensor& mom, const Tensor& grad, Tensor& u_out, double beta, 
                            cur_stream());
 }
 
-void muon_apply(Tensor& master, const Tensor& o, const c10::optional<Tensor>& param_bf16, double lr, double wd,
+static void muon_apply(Tensor& master, const Tensor& o, const c10::optional<Tensor>& param_bf16, double lr, double wd,
                 double scale, const c10::optional<Tensor>& hyper) {
   c10::cuda::CUDAGuard guard(master.device());
   const bool hp = param_bf16.has_value() && param_bf16->defined();
@@ -437,7 +425,7 @@ void muon_apply(Tensor& master, const Tensor& o, const c10::optional<Tensor>& pa
 }
 
 // X [batch, m, n] bf16 contiguous (m <= n) -> X / safe spectral bound, bf16 (see launch_ns_prepare)
-Tensor ns_prepare(const Tensor& x, double eps) {
+static Tensor ns_prepare(const Tensor& x, double eps) {
   check_bf16_cuda(x, "x");
   TORCH_CHECK(x.dim() == 3 && x.is_contiguous() && x.size(2) % 8 == 0 && x.size(1) <= x.size(2),
               "ns_prepare: contiguous [batch, m, n] with m <= n and n % 8 == 0");
@@ -450,12 +438,12 @@ Tensor ns_prepare(const Tensor& x, double eps) {
   return y;
 }
 
-void axpby_bf16(Tensor& x, const Tensor& y, double a, double b) {
+static void axpby_bf16(Tensor& x, const Tensor& y, double a, double b) {
   c10::cuda::CUDAGuard guard(x.device());
   tb::launch_axpby_bf16(bfm(x), bf(y), (float)a, (float)b, x.numel(), cur_stream());
 }
 
-Tensor triangular_adamw(const Tensor& S, Tensor& m, Tensor& v, double beta1, double beta2, double eps, int64_t step,
+static Tensor triangular_adamw(const Tensor& S, Tensor& m, Tensor& v, double beta1, double beta2, double eps, int64_t step,
                         bool triu, const c10::optional<Tensor>& hyper) {
   TORCH_CHECK(S.scalar_type() == at::kFloat && S.is_contiguous() && S.dim() == 3 && S.size(1) == S.size(2),
               "S must be fp32 [n, r, r]");
@@ -468,13 +456,13 @@ Tensor triangular_adamw(const Tensor& S, Tensor& m, Tensor& v, double beta1, dou
   return delta;
 }
 
-void steer_update(Tensor& P, const Tensor& G, double momentum, double steer) {
+static void steer_update(Tensor& P, const Tensor& G, double momentum, double steer) {
   c10::cuda::CUDAGuard guard(P.device());
   tb::launch_steer_update(P.data_ptr<float>(), G.data_ptr<float>(), P.numel(), (float)momentum, (float)steer,
                           cur_stream());
 }
 
-std::vector<Tensor> route_tiers(const Tensor& logits, double threshold) {
+static std::vector<Tensor> route_tiers(const Tensor& logits, double threshold) {
   TORCH_CHECK(logits.scalar_type() == at::kFloat && logits.is_contiguous() && logits.size(-1) == 3, "logits [rows,3]");
   c10::cuda::CUDAGuard guard(logits.device());
   Tensor tiers = torch::empty({logits.size(0)}, logits.options().dtype(at::kInt));
@@ -484,7 +472,7 @@ std::vector<Tensor> route_tiers(const Tensor& logits, double threshold) {
   return {tiers, flag};
 }
 
-Tensor neuron_heatmap(const Tensor& act, int64_t num_bins) {
+static Tensor neuron_heatmap(const Tensor& act, int64_t num_bins) {
   TORCH_CHECK(act.scalar_type() == at::kFloat && act.is_contiguous(), "act must be fp32 contiguous");
   c10::cuda::CUDAGuard guard(act.device());
   Tensor scratch = torch::empty({num_bins}, act.options());
@@ -494,7 +482,7 @@ Tensor neuron_heatmap(const Tensor& act, int64_t num_bins) {
   return rgba;
 }
 
-Tensor tier_render(const Tensor& act, const Tensor& tiers) {
+static Tensor tier_render(const Tensor& act, const Tensor& tiers) {
   TORCH_CHECK(act.scalar_type() == at::kFloat && act.is_contiguous() && act.dim() == 2, "act must be fp32 [rows,w]");
   c10::cuda::CUDAGuard guard(act.device());
   Tensor rgba = torch::empty({act.size(0), act.size(1)}, act.options().dtype(at::kInt));
@@ -503,7 +491,7 @@ Tensor tier_render(const Tensor& act, const Tensor& tiers) {
   return rgba;
 }
 
-}  // namespace
+}  // namespace tb_launch
 
 void register_gemm(pybind11::module& m);
 void register_decode(pybind11::module& m);

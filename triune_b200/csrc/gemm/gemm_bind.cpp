@@ -24,10 +24,12 @@ void check_bf16_cuda(const Tensor& t, const char* name) {
   TORCH_CHECK((reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0, name, " must start on a 16-byte boundary");
 }
 
+}  // namespace
+
+namespace tb_launch {
+
 // C[b] = alpha * op(A[b]) * op(B[b])^T with the fused epilogue. a: [batch?, M, K] (or [batch?, K, M] when
 // a_mn_major), b: [batch?, N, K] (or [batch?, K, N] when b_mn_major). Inner dims must be contiguous.
-}  // namespace
-namespace tb_launch {
 void tc_gemm(const Tensor& a, const Tensor& b, Tensor& c, bool a_mn_major, bool b_mn_major, int64_t mode, int64_t flags,
              double alpha, const c10::optional<Tensor>& bias, const c10::optional<Tensor>& aux_in,
              const c10::optional<Tensor>& aux_out, const c10::optional<Tensor>& row_scale,
@@ -124,14 +126,10 @@ void tc_gemm(const Tensor& a, const Tensor& b, Tensor& c, bool a_mn_major, bool 
   }
   tb::launch_tc_gemm(g, cur_stream());
 }
-}  // namespace tb_launch
-namespace {
 
 // SwiGLU over the fused gate/up weight inside the GEMM: h [M, H] = silu(x Wg^T) * (x Wu^T) with w13 = [Wg ; Wu]
 // ([2H, K]); gu (optional, [M, 2H]) receives both pre-activations for the backward pass. act: 0 silu, 1 relu, 2 clamped
 // (see GemmArgs::glu_act); bias: fp32 [2H] or none (forward only, as the last two activations are).
-}  // namespace
-namespace tb_launch {
 void tc_gemm_swiglu(const Tensor& x, const Tensor& w13, Tensor& h, const c10::optional<Tensor>& gu, int64_t act,
                     const c10::optional<Tensor>& bias, double limit, double alpha) {
   check_bf16_cuda(x, "x");
@@ -164,13 +162,11 @@ void tc_gemm_swiglu(const Tensor& x, const Tensor& w13, Tensor& h, const c10::op
   }
   tb::launch_tc_gemm(g, cur_stream());
 }
-}  // namespace tb_launch
-namespace {
 
 // Backward of the SwiGLU epilogue inside the GEMM that forms d(hidden): dgu [M, 2H] = (d gate | d up) from
 // dh = dy op(w) ([M, H], never written) and the saved pre-activations gu [M, 2H]. w is [H, K] (K-major) or, with
 // w_mn_major, stored [K, H] (the FFN's down projection as it is stored).
-void tc_gemm_dswiglu(const Tensor& dy, const Tensor& w, bool w_mn_major, const Tensor& gu, Tensor& dgu) {
+static void tc_gemm_dswiglu(const Tensor& dy, const Tensor& w, bool w_mn_major, const Tensor& gu, Tensor& dgu) {
   check_bf16_cuda(dy, "dy");
   check_bf16_cuda(w, "w");
   check_bf16_cuda(gu, "gu");
@@ -192,7 +188,7 @@ void tc_gemm_dswiglu(const Tensor& dy, const Tensor& w, bool w_mn_major, const T
   tb::launch_tc_gemm(g, cur_stream());
 }
 
-}  // namespace
+}  // namespace tb_launch
 
 void register_gemm(pybind11::module& m) {
   using namespace tb_launch;

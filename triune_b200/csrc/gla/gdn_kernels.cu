@@ -211,13 +211,13 @@ __device__ __forceinline__ float reduce_scatter32(float (&v)[32], int lane) {
 }
 
 template <int N>
-__device__ __forceinline__ void load_bf16_row(const __nv_bfloat16* p, bool ok, uint32_t (&w)[N / 2]) {
+__device__ __forceinline__ void load_bf16_row(const __nv_bfloat16* p, uint32_t (&w)[N / 2]) {
   if constexpr (N == 4) {
-    const uint2 x = ok ? *reinterpret_cast<const uint2*>(p) : make_uint2(0u, 0u);
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
     w[0] = x.x;
     w[1] = x.y;
   } else {
-    w[0] = ok ? *reinterpret_cast<const uint32_t*>(p) : 0u;
+    w[0] = *reinterpret_cast<const uint32_t*>(p);
   }
 }
 template <int N>
@@ -334,8 +334,8 @@ __device__ __forceinline__ void gdn_block_prep(const GdnBlockArgs& a, GdnPrepSha
       if (j >= i) {  // the same for all lanes
         uint32_t kw[N / 2], qw[N / 2];
         float kf[N], qf[N], dec[N];
-        load_bf16_row<N>(&sh.k[j][lane * N], true, kw);
-        load_bf16_row<N>(&sh.q[j][lane * N], true, qw);
+        load_bf16_row<N>(&sh.k[j][lane * N], kw);
+        load_bf16_row<N>(&sh.q[j][lane * N], qw);
         unpack_bf16<N>(kw, kf);
         unpack_bf16<N>(qw, qf);
         load_rec<N>(&sh.dec[j][lane * N], dec);
@@ -479,7 +479,7 @@ struct GdnWalk {
   }
   // False where it never arrived. `nth`: how many records this stage held before this one.
   __device__ __forceinline__ bool landed(int blk, int nth) { return mbar_wait(&sh.full[blk % GDN_STAGES], nth & 1); }
-  // x = v - s for tokens 8 e + 2 t, 8 e + 2 t + 1 of columns g, then of g + 8.
+  // Values of tokens 8 e + 2 t, 8 e + 2 t + 1 of columns g, then of g + 8.
   __device__ __forceinline__ void values(const float* r, int e, float (&f)[4]) const {
     const uint32_t lo = __float_as_uint(r[R::COMMON + g * R::PV + 4 * e + t]), hi = __float_as_uint(r[R::COMMON + (g + 8) * R::PV + 4 * e + t]);
     f[0] = __uint_as_float(lo << 16), f[1] = __uint_as_float(lo & 0xffff0000u);
@@ -897,9 +897,10 @@ void run_blocks(const GlaMat& Q, const GlaMat& K, const GlaMat& V, const GlaMat&
 
 constexpr int rec_floats(int D) { return D == 64 ? GdnRec<64>::FLOATS : GdnRec<128>::FLOATS; }
 
-// Tokens per segment: whole blocks whose records fill at most 40 MB (with the next segment's they are read back from the 126 MB
-// L2), at least 128 tokens so that the launch of a segment stays small beside its walk (256 heads of 128, 512 tokens:
-// 702 us, and 806 with 64).
+// Tokens per segment: whole blocks whose records (36 KB for heads of 128, 20 KB for 64) fill at most 40 MB, so that with the next segment's
+// they are read back from the 126 MB L2, but at least 128 tokens, so that the launch of a segment stays small beside its walk (256 heads of
+// 128, 512 tokens: 702 us, and 806 with 64). Above 147 heads of 128 or 262 of 64 the second rule holds and records come from
+// memory in part: 512 heads of 128 have 146 MB a segment, 291 MB with the next one's.
 int segment_tokens(int BH, int D) {
   const long long blocks = (40ll << 20) / ((long long)BH * rec_floats(D) * 4);
   return (int)(blocks < 8 ? 8 : blocks) * GB;
@@ -912,8 +913,8 @@ int segment_tokens(int BH, int D) {
 // us: 16 heads of 64, 8 tokens 7.1 -> 8.0, 12 tokens 9.5 -> 8.3, 512 tokens 315 -> 39; 128 of 64, 17 tokens 13 -> 15, 24 tokens 17 -> 15; 256
 // of 64, 24 tokens 20 -> 21, 32 tokens 26 -> 22; 384 of 64, 32 tokens 30 -> 31, 130 tokens 115 -> 116, 512 tokens 449 -> 420; 512 of 64, 32 tokens 36 -> 36, 130 tokens 137 -> 150, 512 tokens 533 -> 534; 16 of 128, 4
 // tokens 7.4 -> 9.8, 8 tokens 11.5 -> 10.7; 64 of 128, 8 tokens 11.7 -> 14.4, 12 tokens 16.1 -> 15.5; 128 of 128, 24 tokens 28.7 -> 29.6, 32
-// tokens 38 -> 30; 512 of 128, 24 tokens 85 -> 93, 32 tokens 111 -> 100, 512 tokens 1676 -> 1433. More than 512 heads would take hundreds of
-// megabytes of records.
+// tokens 38 -> 30; 512 of 128, 24 tokens 85 -> 93, 32 tokens 111 -> 100, 512 tokens 1676 -> 1433. More than 512 heads would take more
+// than 291 MB of records.
 static bool gdn_in_blocks(long long heads, int T, int D) {
   if (D != 64 && D != 128) return false;
   const int least = D == 128 && heads <= 16 ? 8 : heads <= 64 ? 12 : heads <= 128 ? (D == 128 ? 26 : 24) : 32;

@@ -28,12 +28,14 @@ Tensor state_of(const Tensor& t, const Tensor& q, int64_t numel, const char* wha
   return t.to(at::kFloat).contiguous();
 }
 
+}  // namespace
+
+namespace tb_launch {
+
 // Forward over [B*T] rows: whole chunks of 64 tokens on the chunk kernels, the T % 64 tokens after them one by one in fp32
 // (all of them where T < 64, and then without the chunk kernels' clamp of the log decay, which that case never had).
 // Returns (states bf16 [BH*NT,D,D], decay fp32 [BH*NT,D], final_state fp32 [BH,D,D], status) and, where there are both
 // chunks and further tokens, the state between them (fp32 [BH,D,D]); writes out.
-}  // namespace
-namespace tb_launch {
 std::vector<Tensor> gla_fwd(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol,
                             const Tensor& g, int64_t gcol, Tensor& out, int64_t ocol, const c10::optional<Tensor>& init,
                             int64_t B, int64_t T, int64_t H, bool gate_logits, int64_t D) {
@@ -73,15 +75,11 @@ std::vector<Tensor> gla_fwd(const Tensor& q, int64_t qcol, const Tensor& k, int6
   if (NT > 0 && rest > 0) r.push_back(mid);
   return r;
 }
-}  // namespace tb_launch
-namespace {
 
 // Backward: writes dq, dk, dv, dg into the given matrices. With `dfin` (gradient of the final state, fp32
 // [BH,D,D]) and `fin` (the final state itself) the reverse scan starts from dfin instead of zero and the gate
 // gradient receives rowsum(dfin * fin). `before_rest`: the state before the T % 64 last tokens (the initial state where
 // T < 64; none: zero). Returns (status, gradient of the initial state [BH,D,D] fp32).
-}  // namespace
-namespace tb_launch {
 std::vector<Tensor> gla_bwd(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol, const Tensor& g,
                int64_t gcol, const Tensor& dout, int64_t docol, const Tensor& states, const Tensor& decay, Tensor& dq,
                int64_t dqcol, Tensor& dk, int64_t dkcol, Tensor& dv, int64_t dvcol, Tensor& dg, int64_t dgcol, int64_t B,
@@ -131,10 +129,8 @@ std::vector<Tensor> gla_bwd(const Tensor& q, int64_t qcol, const Tensor& k, int6
   tb::launch_gla_dg_finalize(dgl.data_ptr<float>(), tot.data_ptr<float>(), mat(g, gcol), mat(dg, dgcol), d, s, fp(end_term));
   return {status, dinit};
 }
-}  // namespace tb_launch
-namespace {
 
-void gla_decode(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol, const Tensor& g,
+static void gla_decode(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol, const Tensor& g,
                 int64_t gcol, Tensor& state, Tensor& out, int64_t ocol, int64_t B, int64_t H, bool gate_logits) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(state.scalar_type() == at::kFloat && state.is_contiguous(), "state must be fp32 contiguous [B,H,64,64]");
@@ -143,7 +139,7 @@ void gla_decode(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, co
 }
 
 // One decoding step: qkvg [B, 4 H D] -> (out [B, H D], state after the step). `inplace`: the state is updated where it is.
-std::vector<Tensor> mixer_step(const Tensor& qkvg, const c10::optional<Tensor>& cos, const c10::optional<Tensor>& sin,
+static std::vector<Tensor> mixer_step(const Tensor& qkvg, const c10::optional<Tensor>& cos, const c10::optional<Tensor>& sin,
                                const c10::optional<Tensor>& pos, int64_t pos_host, const Tensor& state, bool inplace, bool delta,
                                const c10::optional<Tensor>& x, const c10::optional<Tensor>& beta_w) {
   c10::cuda::CUDAGuard guard(qkvg.device());
@@ -192,8 +188,6 @@ std::vector<Tensor> mixer_step(const Tensor& qkvg, const c10::optional<Tensor>& 
 
 // Gated DeltaNet recurrence (no gradient): q,k,v,g as [B*T, ld] matrices whose columns col0 + h*D.. hold head h. Returns the status of
 // the kernel that takes prompts in blocks (empty where the token kernel ran, which waits for nothing).
-}  // namespace
-namespace tb_launch {
 Tensor gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v, int64_t vcol,
                      const Tensor& g, int64_t gcol, const c10::optional<Tensor>& beta, Tensor& state, Tensor& out,
                      int64_t ocol, int64_t B, int64_t T, int64_t H, int64_t D, bool gate_logits, double scale) {
@@ -222,16 +216,12 @@ Tensor gdn_recurrent(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kco
                            mat(out, ocol), (int)B, (int)T, (int)H, (int)D, gate_logits, (float)scale, cur_stream());
   return status;
 }
-}  // namespace tb_launch
-namespace {
-inline const __nv_bfloat16* bfc(const Tensor& t) { return reinterpret_cast<const __nv_bfloat16*>(t.data_ptr()); }
-inline __nv_bfloat16* bfp(Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); }
+static const __nv_bfloat16* bfc(const Tensor& t) { return reinterpret_cast<const __nv_bfloat16*>(t.data_ptr()); }
+static __nv_bfloat16* bfp(Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); }
 
 // Chunk-parallel Gated DeltaNet forward. q, k, v, g: [B*T, ld] bf16 matrices with head h at columns col + h*D;
 // beta fp32 [B*T, H] or None; init fp32 [B*H, D, D] or None. Writes `out`; returns
 // [U0, W, Tm, Kend, decay, Lraw (empty when not kept), U, states, fin, status].
-}  // namespace
-namespace tb_launch {
 std::vector<Tensor> gdn_chunk_fwd(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v,
                                   int64_t vcol, const Tensor& g, int64_t gcol, const c10::optional<Tensor>& beta,
                                   const c10::optional<Tensor>& init, Tensor& out, int64_t ocol, int64_t B, int64_t T,
@@ -265,13 +255,9 @@ std::vector<Tensor> gdn_chunk_fwd(const Tensor& q, int64_t qcol, const Tensor& k
                            (float)scale, status.data_ptr<int>(), cur_stream());
   return {U0, W, Tm, Kend, decay, Lraw, U, states, fin, status};
 }
-}  // namespace tb_launch
-namespace {
 
 // Backward. `saved` is the list returned by gdn_chunk_fwd. Writes dq, dk, dv, dg into the given matrices; returns
 // [dbeta (fp32 [B*T, H], empty without beta), dS0 (fp32 [B*H, D, D]), status, then the per-chunk intermediates].
-}  // namespace
-namespace tb_launch {
 std::vector<Tensor> gdn_chunk_bwd(const Tensor& q, int64_t qcol, const Tensor& k, int64_t kcol, const Tensor& v,
                                   int64_t vcol, const Tensor& g, int64_t gcol, const Tensor& dout, int64_t docol,
                                   const c10::optional<Tensor>& beta, const c10::optional<Tensor>& dfin,
@@ -322,10 +308,8 @@ std::vector<Tensor> gdn_chunk_bwd(const Tensor& q, int64_t qcol, const Tensor& k
   // the per-chunk intermediates follow for inspection (stage-by-stage comparison against the PyTorch oracle)
   return {dbeta, dS0, status, G1, H1, dU, dSend, dq1, dkw1, dkr1, dW, dLraw, dgl, tot};
 }
-}  // namespace tb_launch
-namespace {
 
-void strength_operands(const Tensor& x, const Tensor& w) {
+static void strength_operands(const Tensor& x, const Tensor& w) {
   (void)mat(x, 0);
   (void)mat(w, 0);
   TORCH_CHECK(w.is_contiguous() && w.size(1) == x.size(1) && w.size(0) <= tb::STRENGTH_MAX_HEADS && x.get_device() == w.get_device(),
@@ -333,8 +317,6 @@ void strength_operands(const Tensor& x, const Tensor& w) {
 }
 
 // beta [rows, H] fp32 = sigmoid(x w^T)
-}  // namespace
-namespace tb_launch {
 Tensor strength_fwd(const Tensor& x, const Tensor& w) {
   strength_operands(x, w);
   c10::cuda::CUDAGuard guard(x.device());
@@ -342,12 +324,8 @@ Tensor strength_fwd(const Tensor& x, const Tensor& w) {
   tb::launch_strength_fwd(bfc(x), x.stride(0), bfc(w), beta.data_ptr<float>(), (int)x.size(0), (int)x.size(1), (int)w.size(0), cur_stream());
   return beta;
 }
-}  // namespace tb_launch
-namespace {
 
 // (dx bf16 [rows, dim], dw bf16 [H, dim]) from the gradient of beta (fp32 [rows, H])
-}  // namespace
-namespace tb_launch {
 std::vector<Tensor> strength_bwd(const Tensor& dbeta, const Tensor& beta, const Tensor& x, const Tensor& w) {
   strength_operands(x, w);
   const int64_t rows = x.size(0), dim = x.size(1), H = w.size(0);
@@ -363,9 +341,8 @@ std::vector<Tensor> strength_bwd(const Tensor& dbeta, const Tensor& beta, const 
   tb::launch_column_parts(partial.data_ptr<float>(), parts, (int)(H * dim), {nullptr, bfp(dw), false}, s);
   return {dx, dw};
 }
+
 }  // namespace tb_launch
-namespace {
-}  // namespace
 
 void register_gla(pybind11::module& m) {
   namespace py = pybind11;
