@@ -55,6 +55,25 @@ def test_training_pass(batch, seq, dim, heads, head_dim, delta, learn_beta, monk
 
 
 @pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("frozen", ["", "x", "ffn", "norm1"])
+def test_two_functions_give_the_numbers_of_one(delta, frozen, monkeypatch):
+    m = _block(256, 4, 64, delta).train()
+    x = torch.randn(2, 100, 256, device="cuda").bfloat16().requires_grad_(frozen != "x")
+    dy = torch.randn_like(x)
+    for n, p in m.named_parameters():
+        p.requires_grad_(not frozen or not n.startswith(frozen))
+    wanted = [t for t in (x, *m.parameters()) if t.requires_grad]
+    y = m(x)[0]
+    assert type(y.grad_fn).__name__ == "_BlockFnBackward"
+    grads = torch.autograd.grad(y, wanted, dy)
+    monkeypatch.setattr(native_block, "ONE_FUNCTION", 0)
+    z = m(x)[0]
+    assert type(z.grad_fn).__name__ == "_BlockRestFnBackward" and torch.equal(y, z)
+    for a, b in zip(torch.autograd.grad(z, wanted, dy), grads):
+        assert torch.equal(a, b) if not delta else (a - b).norm() <= 2 ** -7 * b.norm()  # strengths' gradients are summed up in any order
+
+
+@pytest.mark.parametrize("delta", [False, True])
 @pytest.mark.parametrize("train", [False, True])
 def test_memory_is_that_of_the_modules(train, delta, monkeypatch):
     m = _block(512, 8, 64, delta).train(train)

@@ -40,22 +40,74 @@ def _vec(t, n, dev) -> bool:
                          and t.data_ptr() % 16 == 0)
 
 
+# Elements of x up to which a block is one autograd function, not two. Such blocks wait for the host, to which the second function is 40 us (forward
+# and backward over 2 x 300 x 384: 587 us with two, 552 with one; 7 x 256 x 768: 527 and 482). What the feed-forward saved stays until the
+# mixer's gradients are there then, ten times x where it is four times as wide: 42 MB here. Above, that is memory the modules do not take.
+ONE_FUNCTION = 1 << 21
+
+
 def _buffers(params, want):
     """Where gradients of wanted parameters are added to, where they have such a buffer."""
     return [getattr(p, "main_grad", None) if p is not None and w else None for p, w in zip(params, want)]
 
 
+def _mixer_forward(x, params, cos, sin, dims, eps1):
+    o, *saved, status = _ext.ext().mixer_forward(x, params, cos, sin, dims[0], dims[1], eps1, dims[2])
+    T = x.shape[1]
+    ops._tick(6 if dims[2] else 3 + 3 * (T >= 64) + (T % 64 != 0))
+    _note(status)
+    return o, saved
+
+
+def _mixer_backward(dout, ds, x, params, want_x, want, cos, sin, saved, dims):
+    into = _buffers(params, want)
+    into[2] = None  # the write strengths' weight has its gradient returned, wherever it is kept
+    *grads, status = _ext.ext().mixer_backward(dout, ds, x, params, into, want_x, want, cos, sin, saved, *dims)
+    T = x.shape[1]
+    ops._tick(17 if dims[2] else 8 + 4 * (T >= 64) + 2 * (T % 64 != 0))
+    _note(status)
+    return grads
+
+
+def _rest_forward(o, x, params, eps2, scale):
+    ops._tick(5)
+    return _ext.ext().rest_forward(o, x, params, eps2, scale)
+
+
+def _rest_backward(dy, o, x, params, want, saved, scale):
+    ops._tick(9)
+    return _ext.ext().rest_backward(dy, o, x, params, _buffers(params, want), want, saved, scale)
+
+
+class _BlockFn(torch.autograd.Function):
+    """x, the parameters up to the mixer and those after it -> the block's output."""
+
+    @staticmethod
+    def forward(ctx, x, norm1, qkvg, beta, out, norm2, up, up_bias, down, down_bias, cos, sin, H, D, eps1, eps2, scale, delta):
+        mixer, after = (norm1, qkvg, beta), (out, norm2, up, up_bias, down, down_bias)
+        o, first = _mixer_forward(x, mixer, cos, sin, (H, D, delta), eps1)
+        y, *second = _rest_forward(o, x, after, eps2, scale)
+        ctx.save_for_backward(x, *mixer, *after, cos, sin, o, *second, *first)
+        ctx.dims, ctx.scale = (H, D, delta), scale
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, *rest = ctx.saved_tensors
+        mixer, after, (cos, sin, o), second, first = rest[:3], rest[3:9], rest[9:12], rest[12:17], rest[17:]
+        want_x, *want = ctx.needs_input_grad[:10]
+        dout, ds, *grads = _rest_backward(dy, o, x, after, want[3:], second, ctx.scale)
+        return (*_mixer_backward(dout, ds, x, mixer, want_x, want[:3], cos, sin, first, ctx.dims), *grads, None, None, None, None, None, None, None, None)
+
+
 class _BlockMixerFn(torch.autograd.Function):
-    """x and the parameters up to the mixer -> (output of the mixer, x); see ``mixer_forward`` and ``mixer_backward``. That x goes on from here
-    lets its gradient from all that follows join in the norm's backward pass."""
+    """x and the parameters up to the mixer -> (output of the mixer, x). That x goes on from here lets its gradient from all that follows join in
+    the norm's backward pass."""
 
     @staticmethod
     def forward(ctx, x, norm1, qkvg, beta, cos, sin, H, D, eps1, delta):
         params = (norm1, qkvg, beta)
-        o, *saved, status = _ext.ext().mixer_forward(x, params, cos, sin, H, D, eps1, delta)
-        T = x.shape[1]
-        ops._tick(6 if delta else 3 + 3 * (T >= 64) + (T % 64 != 0))
-        _note(status)
+        o, saved = _mixer_forward(x, params, cos, sin, (H, D, delta), eps1)
         ctx.save_for_backward(x, *params, cos, sin, *saved)
         ctx.dims = (H, D, delta)
         return o, x
@@ -63,27 +115,17 @@ class _BlockMixerFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout, ds):
         x, *rest = ctx.saved_tensors
-        params, cos, sin, saved = rest[:3], rest[3], rest[4], rest[5:]
         want_x, *want = ctx.needs_input_grad[:4]
-        into = _buffers(params, want)
-        into[2] = None  # the write strengths' weight has its gradient returned, wherever it is kept
-        H, D, delta = ctx.dims
-        *grads, status = _ext.ext().mixer_backward(dout, ds, x, params, into, want_x, want, cos, sin, saved, H, D, delta)
-        T = x.shape[1]
-        ops._tick(17 if delta else 8 + 4 * (T >= 64) + 2 * (T % 64 != 0))
-        _note(status)
-        return (*grads, None, None, None, None, None, None)
+        return (*_mixer_backward(dout, ds, x, rest[:3], want_x, want, rest[3], rest[4], rest[5:], ctx.dims), None, None, None, None, None, None)
 
 
-class _BlockFn(torch.autograd.Function):
-    """The rest of a block: the mixer's output, x and the parameters after the mixer -> the block's output; see ``rest_forward`` and
-    ``rest_backward``."""
+class _BlockRestFn(torch.autograd.Function):
+    """The mixer's output, x and the parameters after the mixer -> the block's output."""
 
     @staticmethod
     def forward(ctx, o, x, out, norm2, up, up_bias, down, down_bias, eps2, scale):
         params = (out, norm2, up, up_bias, down, down_bias)
-        y, *saved = _ext.ext().rest_forward(o, x, params, eps2, scale)
-        ops._tick(5)
+        y, *saved = _rest_forward(o, x, params, eps2, scale)
         ctx.save_for_backward(o, x, *params, *saved)
         ctx.scale = scale
         return y
@@ -91,11 +133,7 @@ class _BlockFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         o, x, *rest = ctx.saved_tensors
-        params, saved = rest[:6], rest[6:]
-        want = list(ctx.needs_input_grad[2:8])
-        dout, ds, *grads = _ext.ext().rest_backward(dy, o, x, params, _buffers(params, want), want, saved, ctx.scale)
-        ops._tick(9)
-        return (dout, ds, *grads, None, None)
+        return (*_rest_backward(dy, o, x, rest[:6], list(ctx.needs_input_grad[2:8]), rest[6:], ctx.scale), None, None)
 
 
 def _note(status) -> None:
@@ -176,5 +214,7 @@ def run(norm1, attn, norm2, ffn, x, cache) -> Optional[Any]:
     # a mixer without gradients takes other kernels
     if not (x.requires_grad or w1.requires_grad or qkvg.requires_grad) or not all(p is None or _arena_ok(p) for p in (*mixer, *after)):
         return None
+    if x.numel() <= ONE_FUNCTION:
+        return _BlockFn.apply(x, *mixer, *after, cos, sin, H, D, norm1.eps, norm2.eps, scale, delta), None
     o, x = _BlockMixerFn.apply(x, *mixer, cos, sin, H, D, norm1.eps, delta)
-    return _BlockFn.apply(o, x, *after, norm2.eps, scale), None
+    return _BlockRestFn.apply(o, x, *after, norm2.eps, scale), None
