@@ -1,6 +1,6 @@
 // A whole pre-norm block (norm, recurrent mixer, norm with the residual, feed-forward, residual) on the launchers of its parts: one call from
-// Python without gradients, two in each direction with them (the norm and the mixer; all that follows), so that what the feed-forward saved is
-// given back before the mixer's gradients are formed.
+// Python without gradients; one in each direction with them where the host is waited for, and else two (the norm and the mixer; all that
+// follows), so that what the feed-forward saved is given back before the mixer's gradients are formed.
 //
 // A layer's pass is 12 (forward) to 44 launches (both directions) whose device time is 70 to 230 us for small batches and chat turns;
 // issued from Python, one autograd function or op after the other, the host needs 240 to 950 us for them. From here it needs about a third.
@@ -246,10 +246,40 @@ std::vector<Tensor> mixer_backward(const Tensor& dout, const Tensor& ds, const T
   return g.out;
 }
 
+// Both halves in one call, for blocks that wait for the host.
+
+// -> [y, output of the mixer, five tensors of rest_forward, those of mixer_forward ..., status].
+std::vector<Tensor> block_forward(const Tensor& x, const std::vector<Opt>& p, const std::vector<Opt>& f, const Opt& cos, const Opt& sin, int64_t H,
+                                  int64_t D, double eps1, double eps2, double out_scale, bool delta) {
+  auto m = mixer_forward(x, p, cos, sin, H, D, eps1, delta);
+  auto r = rest_forward(m[0], x, f, eps2, out_scale);
+  std::vector<Tensor> out{r[0], m[0]};
+  out.insert(out.end(), r.begin() + 1, r.end());
+  out.insert(out.end(), m.begin() + 1, m.end());
+  return out;
+}
+
+// `saved`: what block_forward returned between y and the status; `into` and `want` of the nine parameters. Returns the gradients of x and the
+// parameters, and the status.
+std::vector<Tensor> block_backward(const Tensor& dy, const Tensor& x, const std::vector<Opt>& p, const std::vector<Opt>& f, const std::vector<Opt>& into,
+                                   bool want_x, const std::vector<bool>& want, const Opt& cos, const Opt& sin, const std::vector<Opt>& saved, int64_t H,
+                                   int64_t D, double out_scale, bool delta) {
+  TORCH_CHECK(into.size() == MIXER_PARAMS + REST_PARAMS && want.size() == into.size() && saved.size() > 6, "block_backward: lists");
+  std::vector<Tensor> second;
+  for (int i = 1; i < 6; ++i) second.push_back(*saved[i]);
+  auto r = rest_backward(dy, *saved[0], x, f, {into.begin() + MIXER_PARAMS, into.end()}, {want.begin() + MIXER_PARAMS, want.end()}, second, out_scale);
+  auto m = mixer_backward(r[0], r[1], x, p, {into.begin(), into.begin() + MIXER_PARAMS}, want_x, {want.begin(), want.begin() + MIXER_PARAMS}, cos, sin,
+                          {saved.begin() + 6, saved.end()}, H, D, delta);
+  m.insert(m.end() - 1, r.begin() + 2, r.end());
+  return m;
+}
+
 }  // namespace
 
 void register_block(pybind11::module& m) {
   m.def("block_infer", &block_infer);
+  m.def("block_forward", &block_forward);
+  m.def("block_backward", &block_backward);
   m.def("mixer_forward", &mixer_forward);
   m.def("rest_forward", &rest_forward);
   m.def("rest_backward", &rest_backward);

@@ -1,5 +1,5 @@
 """Whole pre-norm blocks (``csrc/block/block_bind.cpp``): norm, recurrent mixer, norm with the residual, dense feed-forward, residual. One
-native call without gradients; with them two in each direction (the norm and the mixer; all that follows).
+native call without gradients; with them one in each direction, or two (the norm and the mixer; all that follows) for large blocks.
 
 Issued op by op, the launches of a layer keep the host busy for 240 us (a prompt) to 950 us (forward and backward), which is what small
 batches and chat turns cost; the native call issues the same launches. :func:`run` answers only for blocks of plain modules whose
@@ -41,73 +41,60 @@ def _vec(t, n, dev) -> bool:
 
 
 # Elements of x up to which a block is one autograd function, not two. Such blocks wait for the host, to which the second function is 40 us (forward
-# and backward over 2 x 300 x 384: 587 us with two, 552 with one; 7 x 256 x 768: 527 and 482). What the feed-forward saved stays until the
-# mixer's gradients are there then, ten times x where it is four times as wide: 42 MB here. Above, that is memory the modules do not take.
+# and backward over 2 x 300 x 384: 44 of 587 us; 7 x 256 x 768: 39 of 527). What the feed-forward saved stays until the mixer's gradients
+# are there then, ten times x where it is four times as wide: 42 MB here. Above, that is memory the modules do not take.
 ONE_FUNCTION = 1 << 21
 
 
-def _buffers(params, want):
-    """Where gradients of wanted parameters are added to, where they have such a buffer."""
-    return [getattr(p, "main_grad", None) if p is not None and w else None for p, w in zip(params, want)]
+def _buffers(params, want, returned=-1):
+    """Where gradients of wanted parameters are added to, where they have such a buffer. The write strengths' weight (``returned``) has its
+    gradient returned, wherever it is kept."""
+    return [getattr(p, "main_grad", None) if p is not None and w and i != returned else None for i, (p, w) in enumerate(zip(params, want))]
 
 
-def _mixer_forward(x, params, cos, sin, dims, eps1):
-    o, *saved, status = _ext.ext().mixer_forward(x, params, cos, sin, dims[0], dims[1], eps1, dims[2])
-    T = x.shape[1]
-    ops._tick(6 if dims[2] else 3 + 3 * (T >= 64) + (T % 64 != 0))
-    _note(status)
-    return o, saved
+def _forward_launches(T, delta):
+    """Launches of the first half, forward."""
+    return 6 if delta else 3 + 3 * (T >= 64) + (T % 64 != 0)
 
 
-def _mixer_backward(dout, ds, x, params, want_x, want, cos, sin, saved, dims):
-    into = _buffers(params, want)
-    into[2] = None  # the write strengths' weight has its gradient returned, wherever it is kept
-    *grads, status = _ext.ext().mixer_backward(dout, ds, x, params, into, want_x, want, cos, sin, saved, *dims)
-    T = x.shape[1]
-    ops._tick(17 if dims[2] else 8 + 4 * (T >= 64) + 2 * (T % 64 != 0))
-    _note(status)
-    return grads
-
-
-def _rest_forward(o, x, params, eps2, scale):
-    ops._tick(5)
-    return _ext.ext().rest_forward(o, x, params, eps2, scale)
-
-
-def _rest_backward(dy, o, x, params, want, saved, scale):
-    ops._tick(9)
-    return _ext.ext().rest_backward(dy, o, x, params, _buffers(params, want), want, saved, scale)
+def _backward_launches(T, delta):
+    return 17 if delta else 8 + 4 * (T >= 64) + 2 * (T % 64 != 0)
 
 
 class _BlockFn(torch.autograd.Function):
-    """x, the parameters up to the mixer and those after it -> the block's output."""
+    """x, the parameters up to the mixer and those after it -> the block's output; see ``block_forward`` and ``block_backward``."""
 
     @staticmethod
     def forward(ctx, x, norm1, qkvg, beta, out, norm2, up, up_bias, down, down_bias, cos, sin, H, D, eps1, eps2, scale, delta):
         mixer, after = (norm1, qkvg, beta), (out, norm2, up, up_bias, down, down_bias)
-        o, first = _mixer_forward(x, mixer, cos, sin, (H, D, delta), eps1)
-        y, *second = _rest_forward(o, x, after, eps2, scale)
-        ctx.save_for_backward(x, *mixer, *after, cos, sin, o, *second, *first)
-        ctx.dims, ctx.scale = (H, D, delta), scale
+        y, *saved, status = _ext.ext().block_forward(x, mixer, after, cos, sin, H, D, eps1, eps2, scale, delta)
+        ops._tick(_forward_launches(x.shape[1], delta) + 5)
+        _note(status)
+        ctx.save_for_backward(x, *mixer, *after, cos, sin, *saved)
+        ctx.dims = (H, D, scale, delta)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, *rest = ctx.saved_tensors
-        mixer, after, (cos, sin, o), second, first = rest[:3], rest[3:9], rest[9:12], rest[12:17], rest[17:]
+        params, cos, sin, saved = rest[:9], rest[9], rest[10], rest[11:]
         want_x, *want = ctx.needs_input_grad[:10]
-        dout, ds, *grads = _rest_backward(dy, o, x, after, want[3:], second, ctx.scale)
-        return (*_mixer_backward(dout, ds, x, mixer, want_x, want[:3], cos, sin, first, ctx.dims), *grads, None, None, None, None, None, None, None, None)
+        *grads, status = _ext.ext().block_backward(dy, x, params[:3], params[3:], _buffers(params, want, 2), want_x, want, cos, sin, saved, *ctx.dims)
+        ops._tick(_backward_launches(x.shape[1], ctx.dims[3]) + 9)
+        _note(status)
+        return (*grads, None, None, None, None, None, None, None, None)
 
 
 class _BlockMixerFn(torch.autograd.Function):
-    """x and the parameters up to the mixer -> (output of the mixer, x). That x goes on from here lets its gradient from all that follows join in
-    the norm's backward pass."""
+    """x and the parameters up to the mixer -> (output of the mixer, x); see ``mixer_forward`` and ``mixer_backward``. That x goes on from here
+    lets its gradient from all that follows join in the norm's backward pass."""
 
     @staticmethod
     def forward(ctx, x, norm1, qkvg, beta, cos, sin, H, D, eps1, delta):
         params = (norm1, qkvg, beta)
-        o, saved = _mixer_forward(x, params, cos, sin, (H, D, delta), eps1)
+        o, *saved, status = _ext.ext().mixer_forward(x, params, cos, sin, H, D, eps1, delta)
+        ops._tick(_forward_launches(x.shape[1], delta))
+        _note(status)
         ctx.save_for_backward(x, *params, cos, sin, *saved)
         ctx.dims = (H, D, delta)
         return o, x
@@ -115,17 +102,22 @@ class _BlockMixerFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout, ds):
         x, *rest = ctx.saved_tensors
+        params, cos, sin, saved = rest[:3], rest[3], rest[4], rest[5:]
         want_x, *want = ctx.needs_input_grad[:4]
-        return (*_mixer_backward(dout, ds, x, rest[:3], want_x, want, rest[3], rest[4], rest[5:], ctx.dims), None, None, None, None, None, None)
+        *grads, status = _ext.ext().mixer_backward(dout, ds, x, params, _buffers(params, want, 2), want_x, want, cos, sin, saved, *ctx.dims)
+        ops._tick(_backward_launches(x.shape[1], ctx.dims[2]))
+        _note(status)
+        return (*grads, None, None, None, None, None, None)
 
 
 class _BlockRestFn(torch.autograd.Function):
-    """The mixer's output, x and the parameters after the mixer -> the block's output."""
+    """The mixer's output, x and the parameters after the mixer -> the block's output; see ``rest_forward`` and ``rest_backward``."""
 
     @staticmethod
     def forward(ctx, o, x, out, norm2, up, up_bias, down, down_bias, eps2, scale):
         params = (out, norm2, up, up_bias, down, down_bias)
-        y, *saved = _rest_forward(o, x, params, eps2, scale)
+        y, *saved = _ext.ext().rest_forward(o, x, params, eps2, scale)
+        ops._tick(5)
         ctx.save_for_backward(o, x, *params, *saved)
         ctx.scale = scale
         return y
@@ -133,7 +125,11 @@ class _BlockRestFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         o, x, *rest = ctx.saved_tensors
-        return (*_rest_backward(dy, o, x, rest[:6], list(ctx.needs_input_grad[2:8]), rest[6:], ctx.scale), None, None)
+        params, saved = rest[:6], rest[6:]
+        want = list(ctx.needs_input_grad[2:8])
+        grads = _ext.ext().rest_backward(dy, o, x, params, _buffers(params, want), want, saved, ctx.scale)
+        ops._tick(9)
+        return (*grads, None, None)
 
 
 def _note(status) -> None:
