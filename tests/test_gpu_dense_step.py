@@ -142,6 +142,19 @@ def test_a_step_that_did_not_finish_raises_and_the_next_prompt_starts_over(how):
     assert dec.graph is not first and int(dec.graph.status) == 0
 
 
+def test_steps_may_be_captured():
+    m = _model(128, 2, 64, 2, 256, 512, "gla")
+    ids = torch.randint(0, 512, (1, 9), device="cuda")
+    dec = GraphedGreedyDecoder(m)
+    want = dec.generate(ids, 6)[:, 9:]
+    dec.prefill(ids)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = dec.decode(6)
+    graph.replay()
+    assert torch.equal(got, want)
+
+
 def test_two_decoders_on_two_streams_take_turns():
     models = [_model(256, 4, 64, 3, 320, 512, "gla"), _model(384, 6, 64, 4, 1088, 1000, "gated_deltanet")]
     prompts = [torch.randint(0, 500, (b, 33), device="cuda") for b in (1, 2)]

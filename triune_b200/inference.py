@@ -461,8 +461,8 @@ class GraphedGreedyDecoder:
         for _ in range(max_new_tokens):
             self.graph.replay()
         tokens = self.out[:, :max_new_tokens].clone()
-        if isinstance(self.graph, dense_step.Step) and self.graph.failed():  # once a request; waits for its tokens
-            self.graph, self.states = None, []  # the next prompt starts over
+        if isinstance(self.graph, dense_step.Step) and not torch.cuda.is_current_stream_capturing() and self.graph.failed():
+            self.graph, self.states = None, []  # looked at once a request, which waits for its tokens; the next prompt starts over
             raise RuntimeError("a decoding step did not finish: a wait between its blocks ran out of time, the request's tokens are lost")
         return tokens
 
