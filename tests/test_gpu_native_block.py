@@ -203,3 +203,13 @@ def test_other_blocks_run_module_by_module(change):
     finally:
         if handle is not None:
             handle.remove()
+
+
+@pytest.mark.parametrize("module,name", [(torch.jit, "is_tracing"), (torch.compiler, "is_compiling")])
+def test_traced_and_compiled_calls_run_module_by_module(module, name, monkeypatch):
+    m = _block(128, 2, 64, False).eval()
+    x = torch.randn(2, 8, 128, device="cuda").bfloat16()
+    with torch.no_grad():
+        assert native_block.run(m.norm1, m.attn, m.norm2, m.ffn, x, None) is not None
+        monkeypatch.setattr(module, name, lambda: True)
+        assert native_block.run(m.norm1, m.attn, m.norm2, m.ffn, x, None) is None
