@@ -168,9 +168,8 @@ __global__ void __launch_bounds__(D* NPART) gdn_recurrent_kernel(
 // against 64 bits after 8192 tokens, 16 heads of 128, gate logits around 0, 2, 4, 8, 10, 14: eight tokens a round in fp32 multiply-adds 9.0e-8,
 // 1.4e-7, 5.8e-7, 1.4e-6, 3.0e-6, 6.4e-6; here 7.4e-8, 1.4e-7, 2.0e-7, 4.1e-7, 1.1e-6, 6.8e-7; all in the instruction 1.4e-7, 1.9e-7, 4.3e-7,
 // 1.1e-5, 1.6e-5, 9.9e-6 (926 instead of 987 us). After 2048 tokens, token by token: 7.0e-8, 1.1e-7, 5.5e-7, 1.3e-6, 8.1e-7, 5.8e-6.
-// The state is held transposed: the fragment that
-// the update leaves it in is the operand that the next round's contraction takes it from, the order of key rows within an
-// instruction being free. Rows of a record are padded so that its fragments are read without bank conflicts.
+// The state is held transposed: the fragment that the update leaves it in is the operand that the next round's contraction takes it from,
+// the order of key rows within an instruction being free. Rows of a record are padded so that its fragments are read without bank conflicts.
 //
 // The launch that walks a segment of tokens also forms the next one's records, in CTAs behind its own. A block's outputs wait for the next
 // round's barrier, so that there is one barrier a round. Bound by the issue slots of one warp per scheduler (69 matrix
@@ -909,12 +908,13 @@ int segment_tokens(int BH, int D) {
 }  // namespace
 
 // Sixteen tokens a round win where the recurrence is a chain that the chip waits for: the walk's work grows with the heads, the token
-// kernel's time hardly does until its CTAs fill the SMs, and a round costs the same for one token as for sixteen. Token kernel -> blocks,
-// us: 16 heads of 64, 8 tokens 7.1 -> 8.0, 12 tokens 9.5 -> 8.3, 512 tokens 315 -> 39; 128 of 64, 17 tokens 13 -> 15, 24 tokens 17 -> 15; 256
-// of 64, 24 tokens 20 -> 21, 32 tokens 26 -> 22; 384 of 64, 32 tokens 30 -> 31, 130 tokens 115 -> 116, 512 tokens 449 -> 420; 512 of 64, 32 tokens 36 -> 36, 130 tokens 137 -> 150, 512 tokens 533 -> 534; 16 of 128, 4
-// tokens 7.4 -> 9.8, 8 tokens 11.5 -> 10.7; 64 of 128, 8 tokens 11.7 -> 14.4, 12 tokens 16.1 -> 15.5; 128 of 128, 24 tokens 28.7 -> 29.6, 32
-// tokens 38 -> 30; 512 of 128, 24 tokens 85 -> 93, 32 tokens 111 -> 100, 512 tokens 1676 -> 1433. More than 512 heads would take more
-// than 291 MB of records.
+// kernel's time hardly does until its CTAs fill the SMs, and a round costs the same for one token as for sixteen. Token kernel -> blocks, us:
+// heads of 64: 16 heads, 8 tokens 7.1 -> 8.0, 12 tokens 9.5 -> 8.3, 512 tokens 315 -> 39; 128 heads, 17 tokens 13 -> 15, 24 tokens 17 -> 15; 256
+// heads, 24 tokens 20 -> 21, 32 tokens 26 -> 22; 384 heads, 32 tokens 30 -> 31, 130 tokens 115 -> 116, 512 tokens 449 -> 420; 512 heads, 32
+// tokens 36 -> 36, 130 tokens 137 -> 150, 512 tokens 533 -> 534.
+// Heads of 128: 16 heads, 4 tokens 7.4 -> 9.8, 8 tokens 11.5 -> 10.7; 64 heads, 8 tokens 11.7 -> 14.4, 12 tokens 16.1 -> 15.5; 128 heads, 24
+// tokens 28.7 -> 29.6, 32 tokens 38 -> 30; 512 heads, 24 tokens 85 -> 93, 32 tokens 111 -> 100, 512 tokens 1676 -> 1433. More than 512 heads
+// would take more than 291 MB of records.
 static bool gdn_in_blocks(long long heads, int T, int D) {
   if (D != 64 && D != 128) return false;
   const int least = D == 128 && heads <= 16 ? 8 : heads <= 64 ? 12 : heads <= 128 ? (D == 128 ? 26 : 24) : 32;
